@@ -1,4 +1,4 @@
-// Split GEMM on CTA pairs (sm_100a): the same computation as tq_gemm_tail.cu -- dense INT4 x INT4 part on tcgen05
+// Split GEMM on CTA pairs (sm_100a): the computation of tq_split_gemm.cu -- dense INT4 x INT4 part on tcgen05
 // kind::i8, tail as a bf16 tcgen05 product over the zero-filled tail tile, one fused epilogue -- but two CTAs of a
 // cluster share one 256 x 256 output tile: tcgen05.mma.cta_group::2 with M = 256.
 //
@@ -16,7 +16,7 @@
 //   * "accumulator empty" collects the epilogue threads of both CTAs in the leader;
 //   * tensor memory is allocated / freed by warp 1 of both CTAs with the cta_group::2 forms; the kernel starts
 //     and ends with a cluster-wide barrier so that no CTA touches a peer that has not started or has left.
-// Every mbarrier wait is bounded as in the one-CTA kernel.
+// Every mbarrier wait is bounded (see mbar_wait).
 #include "tq_common.cuh"
 #include "tq_ptx.cuh"
 
@@ -52,7 +52,7 @@ constexpr int P_BN = 256;         // output channels per pair tile
 constexpr int P_BH = P_BN / 2;    // B rows (output channels) loaded by each CTA
 
 struct PS {
-  static constexpr int SU = 6;                            // operand slots
+  static constexpr int SU = 6;                            // operand slots (a multiple of the three uses of a K slice)
   static constexpr int SP = 4;                            // packed-weight staging buffers
   static constexpr int SLOT = (P_BM + P_BH) * 128;        // A region (16 KB) then this CTA's half of B (16 KB)
   static constexpr int B_OFF = P_BM * 128;
@@ -275,96 +275,119 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a8, const __grid_const
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer: packed INT4 weights
-    if (lane == 0) {
-      for (int g = 0; g < G; ++g) {
-        const int sp = g % S::SP;
-        const uint32_t php = (uint32_t)((g / S::SP) & 1);
-        TQ_TRACE(6, g * uses, 0);
-        if (!TQ_WAIT(0, mbar_wait(empty_p(sp), php ^ 1u, abort_flag, 0x1000u))) break;
-        TQ_TRACE(6, g * uses, 1);
-        const int i = g / kbt, kb = g - i * kbt;
-        mbar_arrive_expect_tx(full_p(sp), S::STAGE);
-        tma_load_2d(base + S::STAGE_OFF + sp * S::STAGE, &tmap_b4, kb * (P_BK / 2), tile_nt(i) * BN + (int)rank * P_BH,
-                    full_p(sp));
+    if (elect_one()) {
+      int sp = 0;
+      uint32_t ph = 1;   // parity of the release that a load waits for
+      bool ok = true;
+      for (int i = 0; ok && i < my_tiles; ++i) {
+        const int nrow = tile_nt(i) * BN + (int)rank * P_BH;
+        for (int kb = 0; kb < kbt; ++kb) {
+          if (!(ok = TQ_WAIT(0, mbar_wait(empty_p(sp), ph, abort_flag, 0x1000u)))) break;
+          mbar_arrive_expect_tx(full_p(sp), S::STAGE);
+          tma_load_2d(base + S::STAGE_OFF + sp * S::STAGE, &tmap_b4, kb * (P_BK / 2), nrow, full_p(sp));
+          if (++sp == S::SP) {
+            sp = 0;
+            ph ^= 1u;
+          }
+        }
       }
     }
   } else if (warp == 6 + P_BUILD_WARPS) {
     // ------------------------------------------------------------------ TMA producer: INT8 activations
-    if (lane == 0) {
-      for (int g = 0; g < G; ++g) {
-        const int q = g * uses, s = slot_of(q);
-        TQ_TRACE(1, q, 0);
-        if (!TQ_WAIT(1, mbar_wait(empty_u(s), par_of(q) ^ 1u, abort_flag, 0x2000u))) break;
-        TQ_TRACE(1, q, 1);
-        const int i = g / kbt, kb = g - i * kbt;
-        if (rank == 0) mbar_arrive_expect_tx(full_u(s), 2 * P_BM * 128);  // the A tiles of both CTAs
-        tma_load_2d_pair(base + s * S::SLOT, &tmap_a8, kb * P_BK, (2 * tile_mt(i) + (int)rank) * P_BM, lead(full_u(s)));
-        TQ_TRACE(1, q, 2);
+    if (elect_one()) {
+      int s = 0;
+      uint32_t ph = 1;
+      bool ok = true;
+      for (int i = 0; ok && i < my_tiles; ++i) {
+        const int mrow = (2 * tile_mt(i) + (int)rank) * P_BM;
+        for (int kb = 0; kb < kbt; ++kb) {
+          if (!(ok = TQ_WAIT(1, mbar_wait(empty_u(s), ph, abort_flag, 0x2000u)))) break;
+          if (rank == 0) mbar_arrive_expect_tx(full_u(s), 2 * P_BM * 128);  // the A tiles of both CTAs
+          tma_load_2d_pair(base + s * S::SLOT, &tmap_a8, kb * P_BK, mrow, lead(full_u(s)));
+          s += uses;
+          if (s >= S::SU) {
+            s -= S::SU;
+            ph ^= 1u;
+          }
+        }
       }
     }
   } else if (warp == 6 + P_BUILD_WARPS + 1) {
     // ------------------------------------------------------------------ TMA producer: bf16 weight rows
-    if (lane == 0 && has_tail) {
+    if (has_tail && elect_one()) {
+      int s = 1;
+      uint32_t ph = 1;
       bool ok = true;
-      for (int g = 0; g < G && ok; ++g) {
-        const int i = g / kbt, kb = g - i * kbt;
+      for (int i = 0; ok && i < my_tiles; ++i) {
         const int nrow = tile_nt(i) * BN + (int)rank * P_BH;
-        for (int h = 0; h < 2; ++h) {
-          const int q = 3 * g + 1 + h, s = slot_of(q);
-          TQ_TRACE(2, q, 0);
-          if (!(ok = TQ_WAIT(2, mbar_wait(empty_u(s), par_of(q) ^ 1u, abort_flag, 0x4000u)))) break;
-          TQ_TRACE(2, q, 1);
-          if (rank == 0) mbar_arrive_expect_tx(full_u(s), BN * 128);  // both halves of the bf16 B tile
-          tma_load_2d_pair(base + s * S::SLOT + S::B_OFF, &tmap_w, kb * P_BK + h * 64, nrow, lead(full_u(s)));
-          TQ_TRACE(2, q, 2);
+        for (int kb = 0; kb < kbt && ok; ++kb) {
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {   // (six slots, three uses per slice: both halves lie in front of the wrap)
+            if (!(ok = TQ_WAIT(2, mbar_wait(empty_u(s + h), ph, abort_flag, 0x4000u)))) break;
+            if (rank == 0) mbar_arrive_expect_tx(full_u(s + h), BN * 128);  // both halves of the bf16 B tile
+            tma_load_2d_pair(base + (s + h) * S::SLOT + S::B_OFF, &tmap_w, kb * P_BK + h * 64, nrow, lead(full_u(s + h)));
+          }
+          s += 3;
+          if (s >= S::SU) {
+            s -= S::SU;
+            ph ^= 1u;
+          }
         }
       }
     }
   } else if (warp == 1) {
-    // ------------------------------------------------------------------ MMA issuer (leader CTA only)
-    if (lane == 0 && rank == 0) {
+    // ------------------------------------------------------------------ MMA issuer (leader CTA only).  One elected
+    // thread, in the form the compiler recognises as such (operands stay in uniform registers), and nothing but waits,
+    // MMAs and commits in the loop: with `lane == 0` and per-slot address arithmetic the issue of an MMA took longer
+    // than its execution.
+    if (rank == 0 && elect_one()) {
       constexpr uint32_t idesc_i8 = make_idesc_i8<BN, 256>();
       constexpr uint32_t idesc_bf = make_idesc_bf16<BN, 256>();
-      int q = 0;
+      const uint64_t desc0 = make_smem_desc(base);   // address field in units of 16 bytes
+      uint64_t d = desc0;
+      uint32_t fb = full_u(0), ph = 0;
+      constexpr uint32_t TO_EMPTY = 8u * S::SU;
+      constexpr uint64_t B = S::B_OFF >> 4;
+      auto next = [&]() {
+        fb += 8u;
+        d += S::SLOT >> 4;
+        if (fb == full_u(S::SU)) {
+          fb = full_u(0);
+          d = desc0;
+          ph ^= 1u;
+        }
+      };
       bool ok = true;
       for (int i = 0; ok && i < my_tiles; ++i) {
         const int ab = acc_buf(i);
         const uint32_t acc_tmem = tmem_base + (uint32_t)(ab * BN);
         if (!(ok = TQ_WAIT(3, mbar_wait(acc_empty(ab), (uint32_t)(acc_use(i) & 1) ^ 1u, abort_flag, 0x8000u)))) break;
         tc_fence_after();
-        for (int kb = 0; kb < kbt && ok; ++kb) {
-          {
-            const int s = slot_of(q);
-            TQ_TRACE(0, q, 0);
-            if (!(ok = TQ_WAIT(4, mbar_wait(full_u(s), par_of(q), abort_flag, 0x10000u)))) break;
-            TQ_TRACE(0, q, 1);
-            tc_fence_after();
-            const uint32_t a_addr = base + s * S::SLOT, b_addr = a_addr + S::B_OFF;
-#pragma unroll
-            for (int k = 0; k < 4; ++k)
-              umma_i8_pair(acc_tmem, make_smem_desc(a_addr + k * 32), make_smem_desc(b_addr + k * 32), idesc_i8,
-                      (kb > 0 || k > 0) ? 1u : 0u);
-            umma_commit_pair(empty_u(s));
-            TQ_TRACE(0, q, 2);
-            ++q;
-          }
+        uint32_t acc = 0;
+        for (int kb = 0; kb < kbt; ++kb) {
+          if (!(ok = TQ_WAIT(4, mbar_wait(fb, ph, abort_flag, 0x10000u)))) break;
+          tc_fence_after();
+          umma_i8_pair(acc_tmem, d, d + B, idesc_i8, acc);
+          umma_i8_pair(acc_tmem, d + 2, d + B + 2, idesc_i8, 1u);   // 32 bytes of K further: + 2
+          umma_i8_pair(acc_tmem, d + 4, d + B + 4, idesc_i8, 1u);
+          umma_i8_pair(acc_tmem, d + 6, d + B + 6, idesc_i8, 1u);
+          umma_commit_pair(fb + TO_EMPTY);
+          next();
           if (has_tail) {
-            for (int h = 0; h < 2; ++h) {
-              const int s = slot_of(q);
-              TQ_TRACE(0, q, 0);
-              if (!(ok = TQ_WAIT(5, mbar_wait(full_u(s), par_of(q), abort_flag, 0x20000u)))) break;
-              TQ_TRACE(0, q, 1);
-              tc_fence_after();
-              const uint32_t a_addr = base + s * S::SLOT, b_addr = a_addr + S::B_OFF;
 #pragma unroll
-              for (int k = 0; k < 4; ++k)
-                umma_bf16_pair(tmem_base + BN, make_smem_desc(a_addr + k * 32), make_smem_desc(b_addr + k * 32), idesc_bf,
-                          (kb > 0 || h > 0 || k > 0) ? 1u : 0u);
-              umma_commit_pair(empty_u(s));
-              TQ_TRACE(0, q, 2);
-              ++q;
+            for (int h = 0; h < 2; ++h) {
+              if (!(ok = TQ_WAIT(5, mbar_wait(fb, ph, abort_flag, 0x20000u)))) break;
+              tc_fence_after();
+              umma_bf16_pair(tmem_base + BN, d, d + B, idesc_bf, h > 0 ? 1u : acc);
+              umma_bf16_pair(tmem_base + BN, d + 2, d + B + 2, idesc_bf, 1u);
+              umma_bf16_pair(tmem_base + BN, d + 4, d + B + 4, idesc_bf, 1u);
+              umma_bf16_pair(tmem_base + BN, d + 6, d + B + 6, idesc_bf, 1u);
+              umma_commit_pair(fb + TO_EMPTY);
+              next();
             }
+            if (!ok) break;
           }
+          acc = 1u;
         }
         if (!ok) break;
         umma_commit_pair(acc_full(ab));

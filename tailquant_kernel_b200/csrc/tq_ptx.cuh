@@ -68,6 +68,20 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map
       : "memory");
 }
 
+__device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map, int x, int y, int z, uint32_t bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
+      ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(z), "r"(bar)
+      : "memory");
+}
+
+// One lane of a converged warp, in the form the compiler recognises as a single active thread.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t ok;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(ok));
+  return ok != 0u;
+}
+
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
@@ -224,6 +238,26 @@ inline bool make_tensor_map_2d(CUtensorMap* map, CUtensorMapDataType dt, int esi
   CUresult r = fn(map, dt, 2, const_cast<void*>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                   swizzle128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
                   CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS)
+    set_last_error_text("cuTensorMapEncodeTiled rejected a tensor map (base address, pitch or box of an operand)");
+  return r == CUDA_SUCCESS;
+}
+
+// Row-major bf16 [outer, K] seen as K / 64 column blocks of [outer, 64]: a box is `blocks` consecutive blocks of `rows`
+// rows, each block written as a 128-byte-swizzled operand tile (blocks one after the other); K % 64 == 0.
+inline bool make_tensor_map_kblocks(CUtensorMap* map, const void* ptr, uint64_t K, uint64_t outer, int rows, int blocks) {
+  EncodeTiledFn fn = encode_fn();
+  if (!fn) {
+    set_last_error_text("cuTensorMapEncodeTiled is not available from this driver");
+    return false;
+  }
+  cuuint64_t dims[3] = {64, (cuuint64_t)outer, (cuuint64_t)(K / 64)};
+  cuuint64_t strides[2] = {(cuuint64_t)(K * 2), 128};
+  cuuint32_t box[3] = {64, (cuuint32_t)rows, (cuuint32_t)blocks};
+  cuuint32_t estr[3] = {1, 1, 1};
+  CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(ptr), dims, strides, box, estr,
+                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS)
     set_last_error_text("cuTensorMapEncodeTiled rejected a tensor map (base address, pitch or box of an operand)");
   return r == CUDA_SUCCESS;
