@@ -18,6 +18,7 @@ bounded sample).  `--impl reference` times only that CPU oracle.
 from __future__ import annotations
 
 import argparse
+import dataclasses
 import json
 import os
 import sys
@@ -498,7 +499,7 @@ def run_ours(args) -> None:
     h2d = sum(int(h.numel() * h.element_size()) for h in host_x)
     d2h = sum(int(h.numel() * h.element_size()) for h in host_y)
     # The dominant kernel: with the tensor-core tail all four projections of the layer run on CTA pairs
-    # (pair_gemm_kernel: each has more than 74 one-CTA tiles); the roofline entry sums its four launches of a step.
+    # (pair_gemm_kernel); the roofline entry sums its four launches of a step.
     if mma:
         dom = [n for (n, K, N) in LAYER]
         kname = ("pair_gemm_kernel (tcgen05 cta_group::2: kind::i8 dense + kind::f16 tail, fused dequant); launches: "
@@ -699,33 +700,30 @@ def run_extra(args) -> None:
             b_copies = [lin.w.b_col] + [lin.w.b_col.clone() for _ in range(n_copies - 1)]
             for M in (1, 8, 32, 64):
                 x, _ = data(M, K, N, 11 + M)
-                ws = lin.prologue(x)
-                from tailquant_kernel_b200 import ops as _ops
                 t_all = graph_ms_of(lambda: lin.forward(x))
-                # the weight stream is timed with the packed weights rotating through > 300 MB of copies inside
-                # one graph, so that every launch reads them from HBM and not from the 126 MB L2
-                tc = lin._decode_uses_tc(M)  # the layer's dispatch of the dense part
-                part = torch.empty((_ops.gemv_plan(M, N, K), M, N), dtype=torch.int32, device=dev)
+                # the linear behind the prologue is timed with the packed weights rotating through > 300 MB of copies
+                # inside one graph, so that every launch reads them from HBM and not from the 126 MB L2
+                lins = []
+                for b in b_copies:
+                    w = dataclasses.replace(lin.w, b_col=b)
+                    lins.append(SplitLinear.from_prepared(w, ratio=RATIO, tail_engine="gather"))
+                    lins[-1].prologue(x)
 
                 def all_copies():
-                    for b in b_copies:
-                        if tc:
-                            _ops.matmul_splitk(ws.pro.a_pack, b, part[0], lin._pick_split_k(M))
-                        else:
-                            _ops.gemv_partials(ws.pro.a_pack, b, part)
-                t_gemm = graph_ms_of(all_copies) / len(b_copies)
+                    for l in lins:
+                        l.compute(l.workspace(M), M)
+                t_lin = graph_ms_of(all_copies) / len(lins)
                 t_pro = graph_ms_of(lambda: lin.prologue(x))
-                t_tail = graph_ms_of(lambda: _ops.tail_gather_small(ws.pro.tail_idx, ws.pro.tail_val, lin.w.w_t, ws.tail, lin.R))
                 wbytes = K * N / 2
                 print(json.dumps({"workload": "decode", "linear": name, "M": M, "K": K, "N": N, "R": lin.R,
-                                  "linear_ms": t_all, "splitk_gemm_ms": t_gemm,
-                                  "dense_kernel": "tcgen05 split-K GEMM (int32 atomics)" if tc else "weight-streaming GEMV (mma.sync s8), partial sums per K range",
-                                  "prologue_ms": t_pro, "tail_gather_ms": t_tail,
-                                  "timing": "CUDA graph replay; splitk_gemm_ms = mean launch of the partial-sum GEMV over %d weight copies "
-                                            "(HBM-resident), the other figures with L2-warm operands" % len(b_copies),
-                                  "int4_weight_gbs": wbytes / (t_gemm * 1e-3) / 1e9,
-                                  "frac_of_hbm_peak": wbytes / (t_gemm * 1e-3) / 1e9 / peaks["hbm_gbs"],
+                                  "linear_ms": t_all, "compute_ms": t_lin, "prologue_ms": t_pro,
+                                  "timing": "CUDA graph replay; compute_ms = mean launch of the decode linear behind the prologue "
+                                            "over %d weight copies (packed weights from HBM), the other figures with L2-warm "
+                                            "operands" % len(lins),
+                                  "int4_weight_gbs": wbytes / (t_lin * 1e-3) / 1e9,
+                                  "frac_of_hbm_peak": wbytes / (t_lin * 1e-3) / 1e9 / peaks["hbm_gbs"],
                                   "tail_row_bytes": 2.0 * M * lin.R * N}), flush=True)
+                del lins
             del b_copies
     elif args.workload == "latency_table":
         # the seven per-projection shapes of a Qwen3-8B layer (the policy's units), ratios of the policy grid

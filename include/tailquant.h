@@ -170,9 +170,10 @@ int tq_split_gemm_fused(const uint8_t* a_pack, const float* body_scale, const ui
  * prototypes (tools/quarot_split_fused_epilogue_ext_v1.py:283-432).
  *   a_q8      [M,K] i8 from tq_split_prologue       w_rot  [N,K] bf16 from tq_prepare_weight (R > 0)
  *   tail_ptr, tail_rec, tail_cnt  from tq_split_prologue (R > 0)
- *   tail_dense  optional [M,K] bf16 from tq_split_prologue: with it, the 32-row blocks of a half slice in which a
- *               row has more than TQ_TAIL_REC_CAP entries are loaded from it by TMA (CTA-pair kernel); without
- *               it those rows are completed from tail_idx16 / tail_val.  Same results either way.
+ *   tail_dense  optional [M,K] bf16 from tq_split_prologue: the operand of the kernel for few and medium row counts (which
+ *               then needs none of the tail lists); the CTA-pair kernel loads the 32-row blocks of a half slice in which
+ *               a row has more than TQ_TAIL_REC_CAP entries from it by TMA and completes those rows from tail_idx16 /
+ *               tail_val without it.
  *   dbg_acc   optional [M,N] i32: accumulators      dbg_tail  optional [M,N] f32: tail sums */
 int tq_split_gemm_mma(const int8_t* a_q8, const float* body_scale, const uint8_t* b_col,
                       const float* w_scale, const void* w_rot, const uint16_t* tail_idx16,
@@ -193,10 +194,10 @@ int tq_split_gemm_mma_swiglu(const int8_t* a_q8, const float* body_scale, const 
                              const uint32_t* tail_rec, const uint16_t* tail_cnt, const void* tail_dense, int R,
                              const float* bias, void* out_bf16, int M, int N, int K, void* stream);
 
-/* tq_split_gemm_mma has two kernels: one CTA per 128 x 256 tile, and CTA pairs on 256 x 256 tiles
- * (tcgen05 cta_group::2; each CTA loads half of the weight tiles).  mode -1 (default) chooses by shape (pairs
- * without a tail or when there are more than 74 one-CTA tiles), 0 / 1 force one of them.  A tuning knob without
- * a reference counterpart. */
+/* tq_split_gemm_mma has two kernels: tiles of 128 channels x up to 176 rows whose K range a cluster of CTAs shares (for
+ * few and medium row counts; with a tail it needs tail_dense), and CTA pairs on 256 x 256 tiles (tcgen05 cta_group::2).
+ * mode -1 (default) chooses by shape, 0 takes the first wherever it can run, 1 the second always.  A tuning knob
+ * without a reference counterpart. */
 int tq_set_gemm_pair_mode(int mode);
 
 /* The prologue has two kernels with identical outputs: one specialised for K = 4096, 12288 and 14336 (a thread per
@@ -271,6 +272,49 @@ int tq_sparse_top_write(void* out, int out_dtype, const int8_t* top_q, const voi
                         const uint8_t* b_row, const float* top_scale, const float* w_scale,
                         int M, int N, int K, int R, void* stream);
 int tq_idx_i32_to_u16(const int32_t* idx, uint16_t* out, long long n, void* stream);
+
+/* ---------------------------------------------------------------------------------------
+ * Forward of one linear in one call (the role of `RealPolicyLinear.forward`, restated in
+ * tools/profile_multimodel_split_components_v34.py:93-272): everything that stays the same from call to call -- weights,
+ * workspace, options -- is described once by a tq_linear_call; x [M,K] bf16 and out ([M,N] bf16, [M,N/2] with act = 1)
+ * come with each call.  tq_linear_forward enqueues the prologue and the linear; tq_linear_prologue and tq_linear_compute
+ * are its two halves (linears that share one input run tq_linear_compute on one set of prologue outputs).
+ *   engine TQ_LINEAR_DECODE  M <= 64: one kernel behind the prologue, sums as tq_int4_gemv_splitk +
+ *                            tq_tail_gather_small + tq_dequant_finish (needs a_pack, w_t, tail_idx16 / tail_val)
+ *          TQ_LINEAR_FUSED   as tq_split_gemm_mma (needs a_q8, w_rot and the tail arrays)
+ *          TQ_LINEAR_GATHER  as tq_tail_gather + tq_split_gemm_fused (needs a_pack, w_t and `tail`)
+ * Fields the engine or R = 0 does not need may be NULL / 0. */
+#define TQ_LINEAR_DECODE 0
+#define TQ_LINEAR_FUSED 1
+#define TQ_LINEAR_GATHER 2
+typedef struct tq_linear_call {
+  int M, N, K, R;
+  int had_kind, descending_rank, engine, act; /* act = 1: SwiGLU over interleaved channel pairs */
+  int tail_ld, ptr_ld;
+  float eps, rms_eps;
+  /* weights */
+  const uint8_t* b_col;
+  const float* w_scale;
+  const void* w_rot;
+  const void* w_t;
+  const float* bias;
+  const void* rms_weight; /* NULL: x is used as it is */
+  /* workspace: the outputs of tq_split_prologue, and [M,N] f32 tail sums (gather engine; decode engine beyond 8 rows) */
+  uint8_t* a_pack;
+  int8_t* a_q8;
+  float* body_scale;
+  float* top_scale;
+  uint16_t* tail_idx16;
+  void* tail_val;
+  uint16_t* tail_ptr;
+  uint32_t* tail_rec;
+  uint16_t* tail_cnt;
+  void* tail_dense;
+  float* tail;
+} tq_linear_call;
+int tq_linear_forward(const tq_linear_call* call, const void* x, void* out, void* stream);
+int tq_linear_prologue(const tq_linear_call* call, const void* x, void* stream);
+int tq_linear_compute(const tq_linear_call* call, void* out, void* stream);
 
 /* Split-K linear for callers that cannot allocate device memory: the same computation as
  * tq_int4_matmul(split_k) followed by tq_dequant_finish,

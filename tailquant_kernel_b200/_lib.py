@@ -14,7 +14,19 @@ LIB_PATH = os.environ.get("TAILQUANT_LIB") or os.path.join(HERE, "libtailquant.s
 TQ_HAD_NONE, TQ_HAD_WHT, TQ_HAD_KRON12, TQ_HAD_BLOCK128 = 0, 1, 2, 3
 TQ_BF16, TQ_FP16 = 0, 1
 
+TQ_LINEAR_DECODE, TQ_LINEAR_FUSED, TQ_LINEAR_GATHER = 0, 1, 2
+
 _P, _I, _F, _LL = C.c_void_p, C.c_int, C.c_float, C.c_longlong
+
+
+class LinearCall(C.Structure):
+    """tq_linear_call of include/tailquant.h."""
+    _fields_ = ([(n, _I) for n in ("M", "N", "K", "R", "had_kind", "descending_rank", "engine", "act", "tail_ld", "ptr_ld")]
+                + [(n, _F) for n in ("eps", "rms_eps")]
+                + [(n, _P) for n in ("b_col", "w_scale", "w_rot", "w_t", "bias", "rms_weight", "a_pack", "a_q8", "body_scale",
+                                     "top_scale", "tail_idx16", "tail_val", "tail_ptr", "tail_rec", "tail_cnt", "tail_dense",
+                                     "tail")])
+
 
 # name -> argument types; must list every function declared in include/tailquant.h
 SIGNATURES = {
@@ -45,6 +57,9 @@ SIGNATURES = {
     "tq_tail_gather_small": [_P, _P, _P, _P, _I, _I, _I, _I, _I, _P],
     "tq_set_gemm_pair_mode": [_I],
     "tq_set_prologue_mode": [_I],
+    "tq_linear_forward": [_P, _P, _P, _P],
+    "tq_linear_prologue": [_P, _P, _P],
+    "tq_linear_compute": [_P, _P, _P],
     "tq_gemm_status": [_P],
 }
 _CHAR_P_RETURNS = {"tq_error_string", "tq_last_cuda_error"}

@@ -1,0 +1,526 @@
+// Split GEMM for few and medium row counts (sm_100a): the computation of tq_gemm_pair.cu on tiles of 128 output channels
+// x T token rows (T a multiple of 16, at most 176), the K range of a tile shared by a CLUSTER of S CTAs.
+//
+// What bounds it: up to a few hundred rows every weight byte (N K / 2 packed INT4 + 2 N K bf16) is used for so few rows
+// that the weight stream is the floor, and 256 x 256 or 128 x 256 tiles leave most of the chip without work (32 tiles
+// for N = 4096 at 300 rows).  Hence
+//   * the WEIGHTS are the 128-row operand of tcgen05.mma and the tokens the N operand, so a tile does no work for rows
+//     that only pad M to 128, and the slots of the ring spend their bytes on weights;
+//   * S CTAs take S ranges of K; their int32 / fp32 accumulators meet over distributed shared memory (one pass, no
+//     global scratch, no atomics; the integer part stays exact) and CTA r finishes rows [r T / S, (r+1) T / S);
+//   * the tail operand is loaded by TMA from the zero-filled tail matrix of the prologue like every other operand: no
+//     builder warps, and the cost does not depend on how the tail entries are distributed;
+//   * the kernel is a programmatic dependent of the prologue: its weight loads fill the ring while the prologue runs.
+//
+// Operand slots are [128 rows x 128 B weights | T rows x 128 B tokens], in two rings: INT8 slots (a 128-wide K slice; the
+// weights arrive as INT4 by TMA in a staging buffer and are widened x16 by four warps) and bf16 slots (HB 64-wide halves
+// of a slice, one tiled load per operand for all of them).
+// Warp roles: 0 = producer of packed weights, 1 = MMA issuer (+ tensor memory), 2 = producer of the bf16 weight rows,
+// 3 = producer of the token operands, 4..7 = wideners, then accumulator export; all warps share the final reduction.
+// (One thread that waits for a slot, announces its bytes and issues its loads takes about 400 cycles per load: with one
+// producer for everything a K slice took 2700 cycles however few rows there were.)
+// Every mbarrier wait is bounded (see mbar_wait).
+#include "tq_common.cuh"
+#include "tq_ptx.cuh"
+
+namespace tq {
+namespace {
+
+constexpr int ST_THREADS = 256;
+constexpr int ST_SP = 3;              // packed-weight staging buffers
+constexpr int ST_STAGE = 128 * 64;    // [128 channels][128 k] INT4
+constexpr int ST_MAX_SLOTS = 8;       // slots of either ring
+constexpr int ST_MAX_T = 176;         // rows per tile (the exchange buffer of a tile must fit in the rings)
+constexpr int ST_SMEM = 222 * 1024;
+
+struct StreamParams {
+  int M, N, K, T, has_tail, act, tiles_n;
+  int si, sb;   // INT8 slots, bf16 slots
+  const float* sx;
+  const float* sw;
+  const float* bias;
+  uint16_t* out;
+  int32_t* dbg_acc;
+  float* dbg_tail;
+};
+
+__device__ __forceinline__ void st_cluster_v4(uint32_t addr, const uint32_t* v) {
+  asm volatile("st.shared::cluster.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]) : "memory");
+}
+__device__ __forceinline__ void st_shared_v4(uint32_t addr, const uint32_t* v) {
+  asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]) : "memory");
+}
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr));
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+
+template <int HB>   // 64-wide halves per bf16 slot
+__global__ void __launch_bounds__(ST_THREADS, 1)
+stream_gemm_kernel(const __grid_constant__ CUtensorMap tmap_b4, const __grid_constant__ CUtensorMap tmap_w,
+                   const __grid_constant__ CUtensorMap tmap_a8, const __grid_constant__ CUtensorMap tmap_tail,
+                   const StreamParams p) {
+  extern __shared__ unsigned char smem_dyn[];
+  const uint32_t raw = smem_u32(smem_dyn);
+  const uint32_t base = (raw + 1023u) & ~1023u;
+  unsigned char* sm = smem_dyn + (base - raw);
+
+  const int T = p.T, SI = p.si, SB = p.sb;
+  const uint32_t slot_bytes = (uint32_t)(128 + T) * 128u;
+  const uint32_t bf_off = (uint32_t)SI * slot_bytes;
+  const uint32_t bf_bytes = (uint32_t)HB * slot_bytes;   // [HB][128 rows] weights, then [HB][T rows] tail
+  const uint32_t stage_off = bf_off + (uint32_t)SB * bf_bytes;
+  const uint32_t bar_off = stage_off + ST_SP * ST_STAGE;
+  const uint32_t bars = base + bar_off;
+  auto full_p = [&](int s) { return bars + 8u * s; };
+  auto empty_p = [&](int s) { return bars + 8u * (ST_SP + s); };
+  auto full_i = [&](int s) { return bars + 8u * (2 * ST_SP + s); };
+  auto empty_i = [&](int s) { return bars + 8u * (2 * ST_SP + ST_MAX_SLOTS + s); };
+  auto full_b = [&](int s) { return bars + 8u * (2 * ST_SP + 2 * ST_MAX_SLOTS + s); };
+  auto empty_b = [&](int s) { return bars + 8u * (2 * ST_SP + 3 * ST_MAX_SLOTS + s); };
+  const uint32_t acc_full = bars + 8u * (2 * ST_SP + 4 * ST_MAX_SLOTS);
+  volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(sm + bar_off + 8 * (2 * ST_SP + 4 * ST_MAX_SLOTS + 1));
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  float* s_sx = reinterpret_cast<float*>(sm + bar_off + 8 * (2 * ST_SP + 4 * ST_MAX_SLOTS + 1) + 16);   // [T]
+
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int S = (int)gridDim.x, rank = (int)blockIdx.x;   // the cluster spans blockIdx.x
+  const int nt = (int)blockIdx.y % p.tiles_n, mt = (int)blockIdx.y / p.tiles_n;
+  const int kb_total = p.K / 128;
+  const int kb0 = rank * kb_total / S, kb1 = (rank + 1) * kb_total / S;
+  const bool has_tail = p.has_tail != 0;
+  const uint32_t tmem_cols = 2 * T <= 32 ? 32u : 2 * T <= 64 ? 64u : 2 * T <= 128 ? 128u : 2 * T <= 256 ? 256u : 512u;
+
+  if (tid == 0) {
+    asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tmap_b4)) : "memory");
+    asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tmap_w)) : "memory");
+    asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tmap_a8)) : "memory");
+    asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tmap_tail)) : "memory");
+    for (int s = 0; s < ST_SP; ++s) {
+      mbar_init(full_p(s), 1);
+      mbar_init(empty_p(s), 4);
+    }
+    for (int s = 0; s < SI; ++s) {
+      mbar_init(full_i(s), 4 + 1);   // the widener warps + the token producer
+      mbar_init(empty_i(s), 1);
+    }
+    for (int s = 0; s < SB; ++s) {
+      mbar_init(full_b(s), 2);       // the two producers
+      mbar_init(empty_b(s), 1);
+    }
+    mbar_init(acc_full, 1);
+    *abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32((const void*)tmem_slot)), "r"(tmem_cols) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+
+  if (warp == 0) {
+    // ------------------------------------------------------------------ packed weights -> staging
+    if (lane == 0) {
+      int sp = 0;
+      uint32_t ph = 0;
+      for (int kb = kb0; kb < kb1; ++kb) {
+        if (!mbar_wait(empty_p(sp), ph ^ 1u, abort_flag, 0x1000u)) break;
+        mbar_arrive_expect_tx(full_p(sp), ST_STAGE);
+        tma_load_2d(base + stage_off + sp * ST_STAGE, &tmap_b4, kb * 64, nt * 128, full_p(sp));
+        if (++sp == ST_SP) {
+          sp = 0;
+          ph ^= 1u;
+        }
+      }
+    }
+  } else if (warp == 2) {
+    // ------------------------------------------------------------------ bf16 weight rows
+    if (lane == 0 && has_tail) {
+      int s = 0;
+      uint32_t ph = 1;   // parity of the release that a use waits for
+      for (int k = kb0 * 2; k < kb1 * 2; k += HB) {
+        if (!mbar_wait(empty_b(s), ph, abort_flag, 0x2000u)) break;
+        mbar_arrive_expect_tx(full_b(s), (uint32_t)HB * 16384u);
+        tma_load_3d(base + bf_off + s * bf_bytes, &tmap_w, 0, nt * 128, k, full_b(s));
+        if (++s == SB) {
+          s = 0;
+          ph ^= 1u;
+        }
+      }
+    }
+  } else if (warp == 3) {
+    // ------------------------------------------------------------------ token codes and tail rows
+    if (lane == 0) {
+      const uint32_t tok = (uint32_t)T * 128u;
+      const int m0 = mt * T;
+      int si = 0, sb = 0;
+      uint32_t phi = 1, phb = 1;
+      bool ok = true;
+      pdl_wait();   // the prologue's outputs; everything else is on its way already
+      for (int k = kb0 * 128; k < kb1 * 128 && ok; k += 128) {
+        if (!(ok = mbar_wait(empty_i(si), phi, abort_flag, 0x40000u))) break;
+        mbar_arrive_expect_tx(full_i(si), tok);
+        tma_load_2d(base + si * slot_bytes + 16384u, &tmap_a8, k, m0, full_i(si));
+        if (++si == SI) {
+          si = 0;
+          phi ^= 1u;
+        }
+        if (has_tail) {
+          for (int h = 0; h < 2; h += HB) {
+            if (!(ok = mbar_wait(empty_b(sb), phb, abort_flag, 0x80000u))) break;
+            mbar_arrive_expect_tx(full_b(sb), (uint32_t)HB * tok);
+            tma_load_3d(base + bf_off + sb * bf_bytes + (uint32_t)HB * 16384u, &tmap_tail, 0, m0, k / 64 + h, full_b(sb));
+            if (++sb == SB) {
+              sb = 0;
+              phb ^= 1u;
+            }
+          }
+        }
+      }
+    }
+  } else if (warp == 1) {
+    // ------------------------------------------------------------------ MMA issuer (the role that bounds tiles of few
+    // rows: about 45 cycles per MMA up to T = 64, so its loop holds nothing but waits, MMAs and commits)
+    if (elect_one()) {
+      const uint32_t idesc_i8 = make_idesc_i8<0>() | ((uint32_t)(T >> 3) << 17);
+      const uint32_t idesc_bf = make_idesc_bf16<0>() | ((uint32_t)(T >> 3) << 17);
+      const uint64_t desc0 = make_smem_desc(base);            // address field: 16-byte units
+      const uint64_t tok_rows = (uint64_t)(T * 128) >> 4;
+      uint32_t phi = 0, phb = 0, acc = 0;
+      uint32_t fi = full_i(0), fb = full_b(0);
+      uint64_t di = desc0, db = desc0 + (bf_off >> 4);
+      const uint32_t fi_end = full_i(SI), fb_end = full_b(SB);
+      constexpr uint32_t TO_EMPTY = 8u * ST_MAX_SLOTS;
+      bool ok = true;
+      for (int kb = kb0; kb < kb1; ++kb) {
+        if (!(ok = mbar_wait(fi, phi, abort_flag, 0x4000u))) break;
+        tc_fence_after();
+        umma_i8(tmem_base, di, di + 1024, idesc_i8, acc);
+        umma_i8(tmem_base, di + 2, di + 1026, idesc_i8, 1u);   // 32 bytes of K further: + 2
+        umma_i8(tmem_base, di + 4, di + 1028, idesc_i8, 1u);
+        umma_i8(tmem_base, di + 6, di + 1030, idesc_i8, 1u);
+        umma_commit(fi + TO_EMPTY);
+        fi += 8u;
+        di += slot_bytes >> 4;
+        if (fi == fi_end) {
+          fi = full_i(0);
+          di = desc0;
+          phi ^= 1u;
+        }
+        if (has_tail) {
+          uint32_t accf = acc;
+#pragma unroll
+          for (int h = 0; h < 2; h += HB) {
+            if (!(ok = mbar_wait(fb, phb, abort_flag, 0x100000u))) break;
+            tc_fence_after();
+#pragma unroll
+            for (int e = 0; e < HB; ++e) {
+              const uint64_t ad = db + e * 1024, bd = db + HB * 1024 + e * tok_rows;
+              umma_bf16(tmem_base + (uint32_t)T, ad, bd, idesc_bf, accf);
+              accf = 1u;
+              umma_bf16(tmem_base + (uint32_t)T, ad + 2, bd + 2, idesc_bf, 1u);
+              umma_bf16(tmem_base + (uint32_t)T, ad + 4, bd + 4, idesc_bf, 1u);
+              umma_bf16(tmem_base + (uint32_t)T, ad + 6, bd + 6, idesc_bf, 1u);
+            }
+            umma_commit(fb + TO_EMPTY);
+            fb += 8u;
+            db += bf_bytes >> 4;
+            if (fb == fb_end) {
+              fb = full_b(0);
+              db = desc0 + (bf_off >> 4);
+              phb ^= 1u;
+            }
+          }
+          if (!ok) break;
+        }
+        acc = 1u;
+      }
+      if (ok) umma_commit(acc_full);
+    }
+  } else if (warp >= 4) {
+    // ------------------------------------------------------------------ wideners
+    const int wtid = tid - 128;
+    int sp = 0, s = 0;
+    uint32_t php = 0, phu = 1;
+    for (int kb = kb0; kb < kb1; ++kb) {
+      if (!mbar_wait(full_p(sp), php, abort_flag, 0x8000u)) break;
+      if (!mbar_wait(empty_i(s), phu, abort_flag, 0x10000u)) break;
+      const unsigned char* src = sm + stage_off + sp * ST_STAGE;
+      unsigned char* dst = sm + s * slot_bytes;
+#pragma unroll
+      for (int task = wtid; task < 512; task += 128) {
+        const int row = task >> 2, pc = task & 3;
+        const uint4 w = *reinterpret_cast<const uint4*>(src + row * 64 + pc * 16);
+        unsigned char* drow = dst + (row >> 3) * 1024 + (row & 7) * 128;
+        uint4 lo, hi;
+        lo.x = (w.x << 4) & 0xf0f0f0f0u;
+        lo.y = w.x & 0xf0f0f0f0u;
+        lo.z = (w.y << 4) & 0xf0f0f0f0u;
+        lo.w = w.y & 0xf0f0f0f0u;
+        hi.x = (w.z << 4) & 0xf0f0f0f0u;
+        hi.y = w.z & 0xf0f0f0f0u;
+        hi.z = (w.w << 4) & 0xf0f0f0f0u;
+        hi.w = w.w & 0xf0f0f0f0u;
+        *reinterpret_cast<uint4*>(drow + (((2 * pc) ^ (row & 7)) << 4)) = lo;
+        *reinterpret_cast<uint4*>(drow + (((2 * pc + 1) ^ (row & 7)) << 4)) = hi;
+      }
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) {
+        mbar_arrive(full_i(s));
+        mbar_arrive(empty_p(sp));
+      }
+      if (++sp == ST_SP) {
+        sp = 0;
+        php ^= 1u;
+      }
+      if (++s == SI) {
+        s = 0;
+        phu ^= 1u;
+      }
+    }
+    mbar_wait(acc_full, 0, abort_flag, 0x20000u);
+    tc_fence_after();
+  }
+  __syncwarp();
+  pdl_wait();      // (scales below; every thread, so that the kernel does not complete before its predecessor)
+  pdl_trigger();
+  // scales of the rows and of this thread's two channels (its column in the final loop), while the last MMAs run
+  const int oc = (tid & 63) * 2, on = nt * 128 + oc;
+  float2 sw = make_float2(0.0f, 0.0f), bias = make_float2(0.0f, 0.0f);
+  if (on < p.N) {
+    sw = *reinterpret_cast<const float2*>(p.sw + on);
+    if (p.bias) bias = *reinterpret_cast<const float2*>(p.bias + on);
+  }
+  if (warp < 4)
+    for (int t = tid; t < T; t += 128) s_sx[t] = mt * T + t < p.M ? p.sx[mt * T + t] : 0.0f;
+  cluster_sync_all();   // every CTA's MMAs are done: the rings are free
+
+  // ---- accumulators -> shared memory of the CTA that finishes the row: [source][row / 4][channel][4 rows], int32 then
+  // fp32 (128-bit stores of four rows of a channel: with one word per store the export took 1 us per 16 rows)
+  const int TS = ((T + S - 1) / S + 3) & ~3;     // rows per CTA
+  const uint32_t half = (uint32_t)(S * TS * 128) * 4u;
+  if (warp >= 4) {
+    const int ch = (warp & 3) * 32 + lane;
+    const uint32_t lane_addr = tmem_base + ((uint32_t)((warp & 3) * 32) << 16);
+    const int rows = min(T, p.M - mt * T);   // (rows beyond M are not exported)
+    const uint32_t mine = base + (uint32_t)(rank * TS * 128 + ch * 4) * 4u;
+    int owner = 0, left = TS;                // CTA that finishes the current rows, rows left in its share
+    uint32_t off = 0, peer = map_to_cta(mine, 0u);
+    for (int t0 = 0; t0 < rows; t0 += 16) {
+      uint32_t ri[16], rf[16];
+      tmem_ld16(lane_addr + (uint32_t)t0, ri);
+      if (has_tail) tmem_ld16(lane_addr + (uint32_t)(T + t0), rf);
+#pragma unroll
+      for (int i = 0; i < 16; i += 4) {
+        if (owner == rank) {
+          st_shared_v4(mine + off, ri + i);
+          if (has_tail) st_shared_v4(mine + off + half, rf + i);
+        } else {
+          st_cluster_v4(peer + off, ri + i);
+          if (has_tail) st_cluster_v4(peer + off + half, rf + i);
+        }
+        off += 2048u;
+        if ((left -= 4) == 0) {
+          left = TS;
+          off = 0;
+          owner = min(owner + 1, S - 1);   // (past the last share only rows beyond T)
+          peer = map_to_cta(mine, (uint32_t)owner);
+        }
+      }
+    }
+    tc_fence_before();
+  }
+  cluster_sync_all();
+  if (warp == 1) {
+    tc_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(tmem_cols) : "memory");
+  }
+
+  // ---- rows [rank TS, (rank + 1) TS) of the tile: a thread takes two channels of four rows
+  for (int i = tid; i < (TS / 4) * 64; i += ST_THREADS) {
+    const int t = rank * TS + (i >> 6) * 4, row0 = mt * T + t;
+    if (t >= T || row0 >= p.M || on >= p.N) continue;
+    int a[2][4] = {};
+    float f[2][4] = {};
+    const unsigned char* src = sm + (size_t)((i >> 6) * 512 + oc * 4) * 4;
+    for (int q = 0; q < S; ++q) {
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const int4 v = *reinterpret_cast<const int4*>(src + (size_t)q * TS * 512 + e * 16);
+        a[e][0] += v.x;
+        a[e][1] += v.y;
+        a[e][2] += v.z;
+        a[e][3] += v.w;
+        if (has_tail) {
+          const float4 w = *reinterpret_cast<const float4*>(src + half + (size_t)q * TS * 512 + e * 16);
+          f[e][0] = __fadd_rn(f[e][0], w.x);
+          f[e][1] = __fadd_rn(f[e][1], w.y);
+          f[e][2] = __fadd_rn(f[e][2], w.z);
+          f[e][3] = __fadd_rn(f[e][3], w.w);
+        }
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      const int row = row0 + r;
+      if (row >= p.M) break;
+      const float sx = s_sx[t + r];
+      const int a0 = a[0][r] >> 4, a1 = a[1][r] >> 4;   // (the weights carried a factor 16)
+      float d0 = __fmul_rn(__fmul_rn((float)a0, sx), sw.x), d1 = __fmul_rn(__fmul_rn((float)a1, sx), sw.y);
+      if (has_tail) {
+        d0 = __fadd_rn(d0, f[0][r]);
+        d1 = __fadd_rn(d1, f[1][r]);
+      }
+      if (p.bias) {
+        d0 = __fadd_rn(d0, bias.x);
+        d1 = __fadd_rn(d1, bias.y);
+      }
+      const size_t o = (size_t)row * p.N + on;
+      if (p.act)
+        p.out[o / 2] = (uint16_t)swiglu_bf16_bits(d0, d1);
+      else
+        *reinterpret_cast<uint32_t*>(p.out + o) = f32_to_bf16_bits(d0) | (f32_to_bf16_bits(d1) << 16);
+      if (p.dbg_acc) *reinterpret_cast<int2*>(p.dbg_acc + o) = make_int2(a0, a1);
+      if (p.dbg_tail) *reinterpret_cast<float2*>(p.dbg_tail + o) = make_float2(f[0][r], f[1][r]);
+    }
+  }
+}
+
+}  // namespace
+
+// Clusters of S CTAs that can be resident at once: the SMs of a GPC that a cluster size does not divide stay empty (of
+// 148 SMs, 48 clusters of three need two rounds).
+static int stream_active_clusters(int S) {
+  static int known[64][9] = {};
+  int dev = 0;
+  const int sms = current_device_sms(&dev);
+  if (S <= 1) return sms;
+  if (dev < 64 && known[dev][S]) return known[dev][S];
+  int n = 0;
+  if (cudaFuncSetAttribute(stream_gemm_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, ST_SMEM) == cudaSuccess) {
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = (unsigned)S;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    cfg.gridDim = dim3((unsigned)S, 1024);
+    cfg.blockDim = dim3(ST_THREADS);
+    cfg.dynamicSmemBytes = ST_SMEM;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    if (cudaOccupancyMaxActiveClusters(&n, stream_gemm_kernel<2>, &cfg) != cudaSuccess) n = 0;
+  }
+  cudaGetLastError();
+  if (n < 1) n = sms / S > 1 ? sms / S - 1 : 1;
+  if (dev < 64) known[dev][S] = n;
+  return n;
+}
+
+// Work split of a call and its estimated time.  The constants are a fit to timings at 8..512 rows of N = 1024..24576,
+// K = 1024..14336 (weights from HBM): a K slice of a tile of T rows takes 0.44 + 0.0024 T us with a tail and 0.36 without
+// (MMA issue and operand loads of one SM), a tile costs 2.4 + 0.045 T us around its main loop (launch, ring fill,
+// accumulator exchange, output), and the weights cannot arrive faster than 5.2 TB/s.
+struct StreamPlan {
+  int T, tiles_m, tiles_n, S;
+  float us;
+};
+static StreamPlan plan_stream(int M, int N, int K, bool tail) {
+  StreamPlan best = {};
+  best.us = 1e30f;
+  const int tiles_n = (N + 127) / 128, kb = K / 128;
+  const float hbm = (float)N * (float)K * (tail ? 2.5f : 0.5f) / 5.2e6f;
+  const int tm0 = (M + ST_MAX_T - 1) / ST_MAX_T;
+  for (int tm = tm0; tm <= tm0 + 2; ++tm) {
+    const int T = ((M + tm - 1) / tm + 15) / 16 * 16;
+    const float slice = tail ? 0.44f + 0.0024f * T : 0.36f + 0.0003f * T, around = 2.4f + 0.045f * T;
+    for (int S = 1; S <= 8 && S <= kb; ++S) {
+      const int tiles = tm * tiles_n, fit = stream_active_clusters(S), waves = (tiles + fit - 1) / fit;
+      const float one = (float)((kb + S - 1) / S) * slice + around + (S > 1 ? 0.8f : 0.0f);
+      float us = waves * one;
+      if (us < hbm + waves * around) us = hbm + waves * around;
+      if (waves > 1) us *= 1.2f;
+      if (us < best.us) {
+        best.T = T;
+        best.tiles_m = tm;
+        best.tiles_n = tiles_n;
+        best.S = S;
+        best.us = us;
+      }
+    }
+  }
+  return best;
+}
+
+int run_stream_gemm(const int8_t* a_q8, const float* body_scale, const uint8_t* b_col, const float* w_scale,
+                    const void* w_rot, const void* tail_dense, int R, const float* bias, void* out_bf16,
+                    int32_t* dbg_acc, float* dbg_tail, int M, int N, int K, int act, cudaStream_t st) {
+  const StreamPlan pl = plan_stream(M, N, K, R > 0);
+  StreamParams p = {};
+  p.M = M;
+  p.N = N;
+  p.K = K;
+  p.T = pl.T;
+  p.has_tail = R > 0 ? 1 : 0;
+  p.act = act;
+  p.tiles_n = pl.tiles_n;
+  p.sx = body_scale;
+  p.sw = w_scale;
+  p.bias = bias;
+  p.out = reinterpret_cast<uint16_t*>(out_bf16);
+  p.dbg_acc = dbg_acc;
+  p.dbg_tail = dbg_tail;
+  // Slots that fit beside the staging buffers: two bf16 slots of a whole slice and two INT8 slots up to 128 rows (half the
+  // load instructions and waits), three of half a slice beyond; what is left goes to bf16, then INT8 slots.
+  const int slot = (128 + pl.T) * 128;
+  const int fixed = ST_SP * ST_STAGE + 8 * (2 * ST_SP + 4 * ST_MAX_SLOTS + 1) + 16 + 4 * ST_MAX_T + 1024;
+  const int units = (ST_SMEM - fixed) / slot;   // 5 at T = 176, 10 at T = 16
+  int hb = 1;
+  if (R > 0) {
+    hb = units >= 6 ? 2 : 1;
+    p.si = units >= 9 ? 3 : 2;
+    p.sb = (units - p.si) / hb;
+    if (p.sb > ST_MAX_SLOTS) p.sb = ST_MAX_SLOTS;
+  } else {
+    p.si = units < ST_MAX_SLOTS ? units : ST_MAX_SLOTS;
+    p.sb = 0;
+  }
+  auto kern = hb == 2 ? stream_gemm_kernel<2> : stream_gemm_kernel<1>;
+  static bool configured[64][2] = {};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (!(dev < 64 && configured[dev][hb - 1])) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, ST_SMEM);
+    if (e != cudaSuccess) {
+      set_last_cuda_error(e);
+      return TQ_ERR_CUDA;
+    }
+    if (dev < 64) configured[dev][hb - 1] = true;
+  }
+  CUtensorMap mb, mw, ma, mt;
+  if (!make_tensor_map_2d(&mb, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, b_col, (uint64_t)(K / 2), (uint64_t)N, (uint64_t)(K / 2),
+                          64, 128) ||
+      !make_tensor_map_2d(&ma, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, a_q8, (uint64_t)K, (uint64_t)M, (uint64_t)K, 128, pl.T,
+                          true))
+    return TQ_ERR_CUDA;
+  if (R > 0) {
+    if (!make_tensor_map_kblocks(&mw, w_rot, (uint64_t)K, (uint64_t)N, 128, hb) ||
+        !make_tensor_map_kblocks(&mt, tail_dense, (uint64_t)K, (uint64_t)M, pl.T, hb))
+      return TQ_ERR_CUDA;
+  } else {
+    mw = mb;   // never read
+    mt = ma;
+  }
+  return launch_pdl(kern, dim3(pl.S, pl.tiles_n * pl.tiles_m), dim3(ST_THREADS), (size_t)ST_SMEM, st, pl.S,
+                    mb, mw, ma, mt, p);
+}
+
+}  // namespace tq

@@ -1,0 +1,99 @@
+// The forward of one linear as ONE host call: prologue and fused linear enqueued back to back.  The Python layer used
+// to issue every kernel, event and scratch buffer of a forward itself (about 70 us of host time per small call, five
+// times the GPU's); it now fills a tq_linear_call once per (layer, row count) and passes it with the two pointers that
+// change.
+#include "tq_common.cuh"
+
+namespace tq {
+namespace {
+
+// The part of a workspace that a forward of this call fills and reads; a prologue on its own fills all of it, since
+// another linear, of another width and hence perhaps on another kernel, may run on it.  The sorted tail lists and the
+// records cost a small call about 3 us, the zero-filled matrix a large one 2 bytes per element.
+//
+// Whether the fused engine of this call runs the stream kernel (which reads the tail from the zero-filled matrix).
+bool linear_streams(const tq_linear_call& c) {
+  return c.engine == TQ_LINEAR_FUSED && c.M > 0 && (c.R == 0 || c.tail_dense) && stream_is_faster(c.M, c.N, c.K, c.R);
+}
+
+tq_linear_call linear_own_part(tq_linear_call c) {
+  const bool fused = c.engine == TQ_LINEAR_FUSED, streams = linear_streams(c);
+  if (fused)
+    c.a_pack = nullptr;
+  else
+    c.a_q8 = nullptr;
+  if (streams) {
+    c.tail_idx16 = nullptr;
+    c.tail_val = nullptr;
+  }
+  if (!fused || streams) {
+    c.tail_ptr = nullptr;
+    c.tail_rec = nullptr;
+    c.tail_cnt = nullptr;
+  }
+  if (!streams && !(fused && c.had_kind == TQ_HAD_BLOCK128)) c.tail_dense = nullptr;
+  return c;
+}
+
+int linear_prologue(const tq_linear_call& c, const void* x, void* stream) {
+  return run_prologue(x, c.M, c.K, c.had_kind, c.R, c.descending_rank, c.eps, 0, c.a_pack, c.a_q8, c.body_scale,
+                      c.top_scale, c.tail_idx16, c.tail_val, c.tail_ld, c.tail_ptr, c.ptr_ld, c.tail_rec, c.tail_cnt,
+                      nullptr, nullptr, nullptr, c.rms_weight, c.rms_eps, (cudaStream_t)stream, TQ_BF16, c.tail_dense);
+}
+
+int linear_compute(const tq_linear_call& c, void* out, void* stream) {
+  if (c.engine == TQ_LINEAR_DECODE) {
+    if (!c.a_pack || !c.body_scale || !c.b_col || !c.w_scale || !out || c.M < 0 || c.M > 64 || c.R < 0 || c.R >= c.K)
+      return TQ_ERR_BAD_ARG;
+    if (c.R > 0 && (!c.w_t || !c.tail_idx16 || !c.tail_val || c.tail_ld < c.R)) return TQ_ERR_BAD_ARG;
+    if (!aligned16(c.a_pack) || !aligned16(c.b_col) || (c.R > 0 && !aligned16(c.w_t))) return TQ_ERR_MISALIGNED;
+    if (c.M == 0) return TQ_OK;
+    DecodeLinearParams p = {};
+    p.a_pack = c.a_pack;
+    p.sx = c.body_scale;
+    p.idx = c.tail_idx16;
+    p.val = reinterpret_cast<const uint16_t*>(c.tail_val);
+    p.b_col = c.b_col;
+    p.w_t = reinterpret_cast<const uint16_t*>(c.w_t);
+    p.sw = c.w_scale;
+    p.bias = c.bias;
+    p.out = reinterpret_cast<uint16_t*>(out);
+    p.M = c.M;
+    p.N = c.N;
+    p.K = c.K;
+    p.R = c.R;
+    p.ld = c.tail_ld;
+    p.act = c.act;
+    return run_decode_linear(p, c.tail, (cudaStream_t)stream);
+  }
+  if (c.engine == TQ_LINEAR_GATHER) {
+    if (c.R > 0) {
+      const int rc = tq_tail_gather(c.tail_idx16, c.tail_val, c.w_t, c.tail, c.M, c.N, c.K, c.R, c.tail_ld, stream);
+      if (rc != TQ_OK) return rc;
+    }
+    return tq_split_gemm_fused(c.a_pack, c.body_scale, c.b_col, c.w_scale, c.R > 0 ? c.tail : nullptr, c.bias, out, c.M,
+                               c.N, c.K, stream);
+  }
+  if (c.engine != TQ_LINEAR_FUSED) return TQ_ERR_BAD_ARG;
+  return run_split_gemm_mma(c.a_q8, c.body_scale, c.b_col, c.w_scale, c.w_rot, c.tail_idx16, c.tail_val, c.tail_ld,
+                            c.tail_ptr, c.ptr_ld, c.tail_rec, c.tail_cnt, c.tail_dense, c.R, c.bias, out, nullptr, nullptr,
+                            c.M, c.N, c.K, c.act, stream);
+}
+
+}  // namespace
+}  // namespace tq
+
+extern "C" int tq_linear_forward(const tq_linear_call* call, const void* x, void* out, void* stream) {
+  if (!call) return TQ_ERR_BAD_ARG;
+  const tq_linear_call own = tq::linear_own_part(*call);
+  const int rc = tq::linear_prologue(own, x, stream);
+  return rc != TQ_OK ? rc : tq::linear_compute(own, out, stream);
+}
+
+extern "C" int tq_linear_prologue(const tq_linear_call* call, const void* x, void* stream) {
+  return call ? tq::linear_prologue(*call, x, stream) : TQ_ERR_BAD_ARG;
+}
+
+extern "C" int tq_linear_compute(const tq_linear_call* call, void* out, void* stream) {
+  return call ? tq::linear_compute(*call, out, stream) : TQ_ERR_BAD_ARG;
+}

@@ -231,6 +231,8 @@ __global__ void __launch_bounds__(NT, min_ctas(K)) prologue_kernel(const Prologu
   const int fbase = BLOCK ? ((tid & 15) + 128 * (tid >> 4)) : tid;  // index = fbase + eoff(e)
   auto eoff = [](int e) -> int { return BLOCK ? (2048 * (e >> 3) + 16 * (e & 7)) : 256 * e; };
 
+  pdl_wait();  // the rows may come from the kernel in front
+  pdl_trigger();
   for (int m = blockIdx.x; m < p.M; m += gridDim.x) {
     const __nv_bfloat16* xrow = p.x + (size_t)m * K;
     // ---- optional RMSNorm in front of the rotation: inv = 1 / sqrt(mean(x^2) + eps) with the squares summed per
@@ -582,15 +584,12 @@ int launch(const PrologueParams& p, cudaStream_t st) {
     if (dev < 64) configured[dev] = true;
   }
   if (smem > 160 * 1024) return TQ_ERR_UNSUPPORTED;
-  int sms = 148;
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  int per_sm = 1;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, NT, smem);
+  int per_sm = 1;  // (the occupancy query costs host time and only matters when there are more rows than SMs)
+  if (p.M > current_device_sms()) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, NT, smem);
   if (per_sm < 1) per_sm = 1;
-  int grid = sms * per_sm;
+  int grid = current_device_sms() * per_sm;
   if (grid > p.M) grid = p.M;
-  kern<<<grid, NT, smem, st>>>(p);
-  return check_launch();
+  return launch_pdl(kern, dim3(grid), dim3(NT), smem, st, 1, p);
 }
 
 #define TQ_CASE(KIND, KK) \

@@ -299,6 +299,8 @@ prologue_fast_kernel(const __grid_constant__ CUtensorMap tmap_x, const PrologueP
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   __syncthreads();
+  pdl_wait();  // the rows may come from the kernel in front
+  pdl_trigger();
 
   uint32_t phase = 0;
   for (int m = blockIdx.x; m < p.M; m += gridDim.x, phase ^= 1u) {
@@ -862,8 +864,8 @@ int launch_fast(const PrologueParams& p, cudaStream_t st) {
       set_last_cuda_error(e);
       return TQ_ERR_CUDA;
     }
-    int sms = 148, per_sm = 1;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    int per_sm = 1;
+    const int sms = current_device_sms();
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, S::NT, S::DYN);
     if (per_sm < 1) per_sm = 1;
     if (dev < 64) {
@@ -877,8 +879,7 @@ int launch_fast(const PrologueParams& p, cudaStream_t st) {
     return TQ_ERR_CUDA;
   int grid = dev < 64 ? grid_per_dev[dev] : 148;
   if (grid > p.M) grid = p.M;
-  kern<<<grid, S::NT, S::DYN, st>>>(mx, p);
-  return check_launch();
+  return launch_pdl(kern, dim3(grid), dim3(S::NT), (size_t)S::DYN, st, 1, mx, p);
 }
 
 }  // namespace

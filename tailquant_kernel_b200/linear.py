@@ -4,31 +4,22 @@ reference's drop-in adapter discovers.
 Forward of one linear (mirrors the step list of `RealPolicyLinear.forward` as restated in
 tools/profile_multimodel_split_components_v34.py:93-272):
     prologue (rotation + select + pack)  ->  tail gather (R > 0)  ->  GEMM with fused dequant,
-    tail add and bias.  Rows M <= `small_m` take the split-K GEMM and a finisher instead.
-Everything runs on the current CUDA stream out of per-(M) workspaces that are allocated once, so
+    tail add and bias.  Rows M <= `small_m` take the decode kernel instead.
+The kernels of a forward are enqueued by one native call (`tq_linear_forward`) on a description that is filled in once
+per row count.  Everything runs on the current CUDA stream out of per-(M) workspaces that are allocated once, so
 a forward is capturable in a CUDA graph after its first call, as the reference's benches require
 (tools/bench_hadamard_three_schemes_quarot_dense_sharedqkv_inplace_fusedtopr_v43.py:105-123).
 """
 from __future__ import annotations
 
+import ctypes
 import weakref
 from collections import OrderedDict
 from typing import Dict, Optional, Tuple
 
 import torch
 
-from . import ops
-
-
-_SIDE: Dict[int, "torch.cuda.Stream"] = {}
-
-
-def _side_stream(device) -> "torch.cuda.Stream":
-    idx = device.index if device.index is not None else torch.cuda.current_device()
-    st = _SIDE.get(idx)
-    if st is None:
-        st = _SIDE[idx] = torch.cuda.Stream(device=idx)
-    return st
+from . import _lib, ops
 
 
 def interleave_gate_up(w_gate: torch.Tensor, w_up: torch.Tensor) -> torch.Tensor:
@@ -44,31 +35,35 @@ class _Workspace:
     another layer's prologue) and the layer's own output and scratch."""
 
     def __init__(self, M: int, K: int, N: int, R: int, device, mma: bool, small: bool, n_out: Optional[int] = None,
-                 with_pro: bool = True, dense: bool = False):
+                 with_pro: bool = True, dense: bool = False, both: bool = False):
+        """`mma` / `small`: the fused kernels / the decode kernel run on this; `both`: room for the prologue outputs of
+        either, since layers that share one prologue may differ in which one they take (few rows)."""
         ld = (R + 7) // 8 * 8
-        q8 = mma and not small  # the fused GEMM takes INT8 codes; the decode GEMV is faster on the packed form
-        self.M, self.K, self.R, self.q8 = M, K, R, q8
+        q8 = mma or both
+        empty = lambda shape, dtype: torch.empty(shape, dtype=dtype, device=device)  # noqa: E731
+        half_slices = (2 * ((M + 255) // 256), K // 64, 128)
+        self.M, self.K, self.R = M, K, R
         self.pro = None if not with_pro else ops.PrologueOut(
-            a_pack=None if q8 else torch.empty((M, K // 2), dtype=torch.uint8, device=device),
-            a_q8=torch.empty((M, K), dtype=torch.int8, device=device) if q8 else None,
-            tail_ptr=torch.empty((M, K // 128 + 1), dtype=torch.int16, device=device) if (mma and R) else None,
-            tail_rec=torch.empty((2 * ((M + 255) // 256), K // 64, 128, ops.TAIL_REC_CAP), dtype=torch.int32, device=device)
-            if (mma and R) else None,
-            tail_cnt=torch.zeros((2 * ((M + 255) // 256), K // 64, 128), dtype=torch.int16, device=device)
-            if (mma and R) else None,
-            body_scale=torch.empty(M, dtype=torch.float32, device=device),
-            top_scale=torch.empty(M, dtype=torch.float32, device=device),
+            a_pack=None if mma and not both else empty((M, K // 2), torch.uint8),
+            a_q8=empty((M, K), torch.int8) if q8 else None,
+            # what the pair kernel reads (few rows never take it)
+            tail_ptr=empty((M, K // 128 + 1), torch.int16) if (mma and not both and R) else None,
+            tail_rec=empty((*half_slices, ops.TAIL_REC_CAP), torch.int32) if (mma and not both and R) else None,
+            tail_cnt=torch.zeros(half_slices, dtype=torch.int16, device=device) if (mma and not both and R) else None,
+            body_scale=empty(M, torch.float32),
+            top_scale=empty(M, torch.float32),
             tail_idx=torch.zeros((M, ld), dtype=torch.int16, device=device) if R else None,
             tail_val=torch.zeros((M, ld), dtype=torch.bfloat16, device=device) if R else None,
-            # block-diagonal rotations leave the tail concentrated in a few 128-blocks: the fused GEMM then loads
-            # whole operand rows of the zero-filled tail matrix instead of walking long runs entry by entry
-            tail_dense=torch.empty((M, K), dtype=torch.bfloat16, device=device) if (dense and q8 and R) else None,
+            # the operand of the kernel for few and medium row counts; and block-diagonal rotations leave the tail
+            # concentrated in a few 128-blocks: the pair kernel then loads whole operand rows of this matrix instead
+            # of walking long runs entry by entry
+            tail_dense=empty((M, K), torch.bfloat16) if (dense and q8 and R) else None,
             R=R)
-        self.tail = torch.empty((M, N), dtype=torch.float32, device=device) if (R and not mma) else None
-        self.acc = None  # int32 [splits, M, N], decode path only
+        self.tail = torch.empty((M, N), dtype=torch.float32, device=device) if (R and not mma and (M > 8 or not small)) else None
         self.out = torch.empty((M, N if n_out is None else n_out), dtype=torch.bfloat16, device=device)
-        if small and R:
-            self.ev_fork, self.ev_join = torch.cuda.Event(), torch.cuda.Event()
+        self.engine = _lib.TQ_LINEAR_FUSED if mma else _lib.TQ_LINEAR_DECODE if small else _lib.TQ_LINEAR_GATHER
+        self.call = None   # the native description of a forward out of these buffers, and the prologue outputs it names
+        self.call_pro = None
 
 
 class SplitLinear:
@@ -172,46 +167,46 @@ class SplitLinear:
                                  rms_eps=float(h.get("rms_eps") or 1e-6))
 
     def _use_mma(self, M: int) -> bool:
-        # the fused prefill kernels also serve 48..64 rows of the wide projections: there the row-gather tail of the
-        # small-M path reads M R weight rows of 2 N bytes and takes longer than a whole 128-row tile (gate_up at 64
-        # rows: 137 us against 107 us)
-        return self.tail_engine == "mma" and (M > self.small_m or (M >= 48 and self.N >= 12288))
-
-    def _decode_uses_tc(self, M: int) -> bool:
-        # dense part of the small-M path: the weight-streaming GEMV, except beyond 48 rows on the widest projections,
-        # where the tcgen05 split-K GEMM (int32 atomics into one slab) is ahead (34 against 38 us on gate_up at 64)
-        return M > 48 and self.N >= 16384
+        # The decode kernel reads only the M R tail rows it needs, the fused kernels stream all of the bf16 weights: from a
+        # few rows on the second is faster (N = K = 4096, ratio 0.05: 8.8 us against 11.3 at 4 rows, 15.5 against 11.2
+        # at 8; N = 24576: 31 / 52 and 59 / 51; ratio 0.01: 9.2 / 11.2 at 8 rows).  Without a tail the GEMV holds out to 32
+        # rows (N = 24576: 27 us against 35), and narrow projections stay on it up to `small_m`.
+        if self.tail_engine != "mma":
+            return False
+        if M > self.small_m:
+            return True
+        if self.N <= 1024:
+            return False
+        if not self.R:
+            return M > 32
+        return M > 8 or (M > 2 and M * self.R > 0.22 * self.K)
 
     @property
     def N_out(self) -> int:
         return self.N // 2 if self.epilogue == "swiglu" else self.N
 
+    def _new_workspace(self, M: int, with_pro: bool) -> _Workspace:
+        mma = self._use_mma(M)
+        return _Workspace(M, self.K, self.N, self.R, self.w.b_col.device, mma, not mma and M <= self.small_m, self.N_out,
+                          with_pro=with_pro, dense=self.w.had_kind == ops.TQ_HAD_BLOCK128 or M <= 1024,
+                          both=self.tail_engine == "mma" and M <= min(self.small_m, 64))
+
     def workspace(self, M: int) -> _Workspace:
         ws = self._ws.get(M)
         if ws is None:
-            ws = self._ws[M] = _Workspace(M, self.K, self.N, self.R, self.w.b_col.device, self._use_mma(M),
-                                          not self._use_mma(M) and M <= self.small_m, self.N_out,
-                                          dense=self.w.had_kind == ops.TQ_HAD_BLOCK128)
+            ws = self._ws[M] = self._new_workspace(M, True)
         return ws
 
     def _own_buffers(self, ws: _Workspace, M: int) -> _Workspace:
         """Output and scratch of THIS layer for a prologue workspace that may belong to another layer."""
         if self._ws.get(M) is ws:
             return ws
-        if (ws.K, ws.R, ws.M) != (self.K, self.R, M) or ws.q8 != self._use_mma(M):
+        if (ws.K, ws.R, ws.M) != (self.K, self.R, M) or (ws.pro.a_q8 if self._use_mma(M) else ws.pro.a_pack) is None:
             raise RuntimeError("a shared prologue needs the same K, R, row count and operand format in both layers")
         own = self._ws_shared.get(M)
         if own is None:
-            own = self._ws_shared[M] = _Workspace(M, self.K, self.N, self.R, self.w.b_col.device, self._use_mma(M),
-                                                  not self._use_mma(M) and M <= self.small_m, self.N_out,
-                                                  with_pro=False)
+            own = self._ws_shared[M] = self._new_workspace(M, False)
         return own
-
-    def _pick_split_k(self, M: int) -> int:
-        if self.split_k > 0:
-            return self.split_k
-        tiles = ((M + 127) // 128) * ((self.N + 127) // 128)
-        return max(1, min(self.K // 128, (148 + tiles - 1) // tiles))
 
     def prepare_decode(self) -> None:
         """Builds the [K, N] transpose of the rotated weights that the small-M tail reads, ahead of the first small-M
@@ -219,71 +214,69 @@ class SplitLinear:
         if self.R and self.w.w_t is None:
             self.w.w_t = self.w.w_rot.t().contiguous()
 
+    def _call(self, own: _Workspace, pro: "ops.PrologueOut") -> "_lib.LinearCall":
+        """Description of this layer's forward: prologue outputs `pro` (own or another layer's), output side `own`."""
+        if own.call is not None and own.call_pro is pro:
+            return own.call
+        if own.engine == _lib.TQ_LINEAR_DECODE:
+            self.prepare_decode()
+        w, p = self.w, ops._ptr
+        own.call_pro = pro
+        own.call = _lib.LinearCall(
+            M=own.M, N=self.N, K=self.K, R=self.R, had_kind=w.had_kind, descending_rank=self.descending_rank,
+            engine=own.engine, act=1 if self.epilogue == "swiglu" else 0,
+            tail_ld=pro.tail_idx.shape[1] if pro.tail_idx is not None else 0,
+            ptr_ld=pro.tail_ptr.shape[1] if pro.tail_ptr is not None else 0, eps=ops.EPS, rms_eps=self.rms_eps,
+            b_col=p(w.b_col), w_scale=p(w.w_scale), w_rot=p(w.w_rot), w_t=p(w.w_t), bias=p(w.bias),
+            rms_weight=p(self.rms_weight), a_pack=p(pro.a_pack), a_q8=p(pro.a_q8), body_scale=p(pro.body_scale),
+            top_scale=p(pro.top_scale), tail_idx16=p(pro.tail_idx), tail_val=p(pro.tail_val), tail_ptr=p(pro.tail_ptr),
+            tail_rec=p(pro.tail_rec), tail_cnt=p(pro.tail_cnt), tail_dense=p(pro.tail_dense), tail=p(own.tail))
+        return own.call
+
+    def _what(self, M: int) -> str:
+        return f"SplitLinear(M={M}, N={self.N}, K={self.K}, R={self.R}, had_kind={self.w.had_kind})"
+
     def prologue(self, x2d: torch.Tensor) -> _Workspace:
+        ops._check_cuda(x2d, "x", torch.bfloat16)
+        ops._check(x2d.dim() == 2 and x2d.shape[1] == self.K, "x must be [M, K]")
         ws = self.workspace(x2d.shape[0])
-        ops.split_prologue(x2d, self.w.had_kind, self.R, self.descending_rank, out=ws.pro,
-                           rms_weight=self.rms_weight, rms_eps=self.rms_eps)
+        rc = _lib.load().tq_linear_prologue(ctypes.byref(self._call(ws, ws.pro)), x2d.data_ptr(), ops._stream())
+        if rc:
+            _lib.check(rc, self._what(ws.M))
         return ws
 
-    def compute(self, ws: _Workspace, M: int) -> torch.Tensor:
+    def compute(self, ws: _Workspace, M: int, out: Optional[torch.Tensor] = None) -> torch.Tensor:
         """GEMM + tail for a workspace whose prologue outputs are filled.  `ws` may be ANOTHER layer's workspace
         (shared-prologue use: several linears with the same K, R, rank and rotation run `compute` on one prologue,
         the way the reference shares one prepare between q/k/v and gate/up:
         tools/bench_prefill_bf16_romeoquarotdense_split_total_v61_sharedprepare.py:124-134); the output then goes to
-        this layer's own buffer of its own width."""
-        w, pro = self.w, ws.pro
+        this layer's own buffer of its own width, or to `out`."""
         own = self._own_buffers(ws, M)
-        if self._use_mma(M):
-            return ops.split_gemm_mma(pro.a_q8, pro.body_scale, w.b_col, w.w_scale, own.out, w_rot=w.w_rot, pro=pro,
-                                      R=self.R, bias=w.bias, act=self.epilogue)
-        if M <= self.small_m:  # decode: weight-streaming GEMV + row gather, both HBM-bound
-            tc = self._decode_uses_tc(M)
-            if own.acc is None:  # partial sums per K range: one GEMV launch (no zeroing, no atomics) + the finisher
-                splits = 1 if tc else ops.gemv_plan(M, self.N, self.K)
-                own.acc = torch.empty((splits, M, self.N), dtype=torch.int32, device=own.out.device)
-            self.prepare_decode()
-
-            def dense():
-                if tc:
-                    ops.matmul_splitk(pro.a_pack, w.b_col, own.acc[0], self._pick_split_k(M))
-                else:
-                    ops.gemv_partials(pro.a_pack, w.b_col, own.acc)
-            if self.R:
-                if own.tail is None:
-                    own.tail = torch.empty((M, self.N), dtype=torch.float32, device=own.out.device)
-                # the tail sums and the GEMV only depend on the prologue and neither fills the GPU at these sizes:
-                # the tail runs on a side stream next to the GEMV (a parallel branch when captured in a CUDA graph)
-                cur = torch.cuda.current_stream()
-                side = _side_stream(own.out.device)
-                own.ev_fork.record(cur)
-                side.wait_event(own.ev_fork)
-                with torch.cuda.stream(side):
-                    ops.tail_gather_small(pro.tail_idx, pro.tail_val, w.w_t, own.tail, self.R)
-                    own.ev_join.record(side)
-                dense()
-                cur.wait_event(own.ev_join)
-            else:
-                dense()
-            ops.dequant_finish_partials(own.acc, pro.body_scale, w.w_scale, own.out, tail=own.tail, bias=w.bias,
-                                        act=self.epilogue)
-            return own.out
-        if self.R:
-            ops.tail_gather(pro.tail_idx, pro.tail_val, w.w_t, own.tail, self.R)
-        ops.split_gemm_fused(pro.a_pack, pro.body_scale, w.b_col, w.w_scale, own.out, tail=own.tail, bias=w.bias)
-        return own.out
+        if out is None:
+            out = own.out
+        rc = _lib.load().tq_linear_compute(ctypes.byref(self._call(own, ws.pro)), out.data_ptr(), ops._stream())
+        if rc:
+            _lib.check(rc, self._what(M))
+        return out
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
-        lead = x.shape[:-1]
-        x2d = x.reshape(-1, self.K)
-        if x2d.dtype != torch.bfloat16:
-            x2d = x2d.to(torch.bfloat16)
-        x2d = x2d.contiguous()
-        M = x2d.shape[0]
-        ws = self.prologue(x2d)
-        y = self.compute(ws, M)
-        if not self.reuse_output:
-            y = y.clone()
-        return y.view(*lead, self.N_out)
+        shape = x.shape
+        if x.dtype is not torch.bfloat16:
+            x = x.to(torch.bfloat16)
+        if shape[-1] != self.K or not x.is_contiguous():
+            x = x.reshape(-1, self.K).contiguous()
+        if not x.is_cuda:
+            raise RuntimeError("x must be a CUDA tensor")
+        M = x.numel() // self.K
+        ws = self._ws.get(M)
+        if ws is None:
+            ws = self.workspace(M)
+        call = ws.call if ws.call is not None else self._call(ws, ws.pro)
+        y = ws.out if self.reuse_output else torch.empty_like(ws.out)
+        rc = _lib.load().tq_linear_forward(ctypes.byref(call), x.data_ptr(), y.data_ptr(), ops._stream())
+        if rc:
+            _lib.check(rc, self._what(M))
+        return y.view(*shape[:-1], self.N_out)
 
     __call__ = forward
 
@@ -351,7 +344,7 @@ def split_linear_forward(x: torch.Tensor, weight: torch.Tensor, bias: Optional[t
     x2d = x2d.contiguous()
     M = x2d.shape[0]
     skey = (x.device.index, x2d.data_ptr(), x._version, M, lin.K, lin.R, lin.descending_rank, lin.w.had_kind,
-            lin._use_mma(M), torch.cuda.current_stream().cuda_stream)
+            ops._stream())
     hit = _SHARED.get(skey) if x2d.data_ptr() == x.data_ptr() else None
     if hit is not None and hit[0]() is x:
         ws = hit[1]
@@ -360,6 +353,6 @@ def split_linear_forward(x: torch.Tensor, weight: torch.Tensor, bias: Optional[t
         if x2d.data_ptr() == x.data_ptr():  # only inputs that were used as they are can be recognised again
             _SHARED.clear()                  # one entry: the prologue outputs live in a workspace that the next
             _SHARED[skey] = (weakref.ref(x), ws)  # prologue of that layer overwrites
-    y = lin.compute(ws, M).clone()
+    y = lin.compute(ws, M, torch.empty((M, lin.N_out), dtype=torch.bfloat16, device=x2d.device))
     y = y.view(*x.shape[:-1], lin.N_out)
     return y if y.dtype == x.dtype else y.to(x.dtype)

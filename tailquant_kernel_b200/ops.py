@@ -32,8 +32,13 @@ TAIL_REC_CAP = 12  # TQ_TAIL_REC_CAP of include/tailquant.h
 
 
 # --------------------------------------------------------------------------- helpers
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)  # (absent in a CPU-only build)
+
+
 def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    if _raw_stream is None:
+        return torch.cuda.current_stream().cuda_stream
+    return _raw_stream(torch.cuda.current_device())
 
 
 def _ptr(t: Optional[torch.Tensor]) -> Optional[int]:
@@ -334,7 +339,8 @@ def split_gemm_mma(a_q8, body_scale, B_pack, w_scale, out, w_rot=None, pro: Opti
 
 
 def set_gemm_pair_mode(mode: int) -> None:
-    """-1: split_gemm_mma picks its kernel by problem size; 0: one CTA per tile; 1: CTA pairs (256 x 256 tiles)."""
+    """-1: split_gemm_mma picks its kernel by problem size; 0: 128-channel tiles with the K range shared by a cluster,
+    wherever that kernel can run (with a tail it needs `tail_dense`); 1: CTA pairs (256 x 256 tiles)."""
     _lib.check(_lib.load().tq_set_gemm_pair_mode(int(mode)), "set_gemm_pair_mode")
 
 

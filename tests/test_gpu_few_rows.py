@@ -1,0 +1,84 @@
+"""The kernels for few and medium row counts at the sizes where they can go wrong: edges of row and channel tiles, K ranges
+that do not divide, entries beyond a buffer, layers that share a prologue but not a kernel.  Against the CPU oracle."""
+import numpy as np
+import pytest
+import torch
+
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+ops = None
+
+
+@pytest.fixture(scope="module", autouse=True)
+def _load():
+    global ops
+    from tailquant_kernel_b200 import ops as _ops
+    ops = _ops
+    import test_gpu_parity
+    test_gpu_parity.ops = _ops
+    yield
+    assert ops.gemm_status() == 0, "a bounded device-side wait ran out"
+
+
+def dev(bits):
+    return torch.from_numpy(bits.view(np.int16).copy()).cuda().view(torch.bfloat16)
+
+
+def host(t):
+    return t.detach().contiguous().view(torch.int16).cpu().numpy().view(np.uint16)
+
+
+@pytest.mark.parametrize("M,N,K,R", [(16, 128, 256, 13), (17, 136, 512, 26), (64, 1032, 4096, 205), (65, 264, 1024, 0),
+                                     (112, 4096, 512, 60), (176, 256, 4096, 205), (177, 264, 2048, 1), (300, 520, 14336, 717),
+                                     (61, 4096, 12288, 615), (353, 128, 1152, 40), (1, 8, 128, 5)])
+def test_shared_k_range_gemm(M, N, K, R):
+    """128-channel tiles with the K range of a tile shared by a cluster: accumulators exact, tail sums and outputs inside
+    the bounds, at row counts around the 16-row steps and the 176-row tile."""
+    from test_gpu_parity import _run_split_gemm_mma
+    _run_split_gemm_mma(M, N, K, R, bias=True, cluster=False, pair=0, dense=True)
+
+
+@pytest.mark.parametrize("M", [1, 2, 4, 5, 8, 9, 16, 17, 33, 64])
+@pytest.mark.parametrize("N,K,kind,ratio", [(1000, 512, O.HAD_WHT, 0.05), (136, 12288, O.HAD_KRON12, 0.05),
+                                            (72, 4096, O.HAD_WHT, 0.4), (264, 2048, O.HAD_BLOCK128, 0.0)])
+def test_decode_linear_exact(M, N, K, kind, ratio):
+    """The one-launch decode linear: bf16 bits of the eight-chain order, ragged channel tiles, few and many tail entries."""
+    from tailquant_kernel_b200 import SplitLinear
+    xb = O.make_activations(M, K, seed=M, n_outlier=max(1, K // 256))
+    wb = O.make_weights(N, K, seed=N)
+    b = np.random.default_rng(3).standard_normal(N, dtype=np.float32)
+    R = O.ceil_ratio_count(K, ratio)
+    ref = O.split_linear_t16(xb, O.prepare_weight(wb, kind), kind, R, bias=b, tail_chains=8)[0]
+    lin = SplitLinear(dev(wb), torch.from_numpy(b).cuda(), ratio=ratio, had_kind=kind)
+    for _ in range(2):
+        assert np.array_equal(host(lin(dev(xb))), ref)
+
+
+@pytest.mark.parametrize("M,N", [(1, 2056), (2, 6152), (3, 2056), (8, 2056), (40, 2056)])
+def test_few_rows_on_wider_layers(M, N):
+    """Widths on which the dispatch between the decode and the fused kernels depends on rows x tail entries."""
+    from tailquant_kernel_b200 import SplitLinear
+    K, ratio = 1024, 0.05
+    xb, wb = O.make_activations(M, K, seed=1, n_outlier=4), O.make_weights(N, K, seed=2)
+    R = O.ceil_ratio_count(K, ratio)
+    yb, y32, _, _ = O.split_linear_t16(xb, O.prepare_weight(wb, O.HAD_WHT), O.HAD_WHT, R, tail_chains=8)
+    got = host(SplitLinear(dev(wb), ratio=ratio)(dev(xb)))
+    diff = got != yb
+    assert diff.mean() < 0.01 and np.abs(O.bf16_bits_to_f32(got[diff]) - y32[diff]).max(initial=0.0) <= 0.04
+
+
+@pytest.mark.parametrize("M,ratio", [(8, 0.05), (40, 0.01), (430, 0.10), (700, 0.05)])
+def test_layers_on_different_kernels_share_a_prologue(M, ratio):
+    """A wide and a narrow layer on one prologue (they may run on different kernels, which read different parts of its
+    outputs) give the bits of their own forwards."""
+    from tailquant_kernel_b200 import SplitLinear
+    K = 1024
+    x = dev(O.make_activations(M, K, seed=5, n_outlier=4))
+    wide, narrow = (SplitLinear(dev(O.make_weights(n, K, seed=n)), ratio=ratio) for n in (8192, 136))
+    want = [wide(x).clone(), narrow(x).clone()]
+    for first, second, a, b in ((wide, narrow, 0, 1), (narrow, wide, 1, 0)):
+        ws = first.prologue(x)
+        ya, yb = first.compute(ws, M), second.compute(ws, M)
+        assert torch.equal(ya, want[a]) and torch.equal(yb, want[b])
