@@ -967,7 +967,7 @@ def main() -> None:
     ap.add_argument("--probe", default="gemm", choices=["prologue", "gemm"], help="probe: which kernel of the linear to launch")
     ap.add_argument("--ratio", type=float, default=RATIO, help="probe: tail ratio (0 = pure W4A4)")
     ap.add_argument("--prologue-mode", type=int, default=-1, choices=[-1, 0],
-                    help="probe: 0 = the general prologue kernel also where the specialised one is built")
+                    help="probe: 0 = the prologue kernel with 16 elements per thread also for many rows")
     ap.add_argument("--layers", type=int, default=36, help="prefill36: decoder layers")
     ap.add_argument("--seq-len", type=int, default=4096, help="prefill36: tokens")
     ap.add_argument("--with-bf16", action="store_true", help="prefill36: also time the same stack on bf16 cuBLAS linears")

@@ -200,10 +200,9 @@ int tq_split_gemm_mma_swiglu(const int8_t* a_q8, const float* body_scale, const 
  * without a reference counterpart. */
 int tq_set_gemm_pair_mode(int mode);
 
-/* The prologue has two kernels with identical outputs: one specialised for K = 4096, 12288 and 14336 (a thread per
- * 64 contiguous elements, the row staged by one TMA load) and a general one for every other built width.  mode -1
- * (default) uses the specialised kernel where it applies, 0 forces the general one.  A comparison switch without a
- * reference counterpart. */
+/* The prologue has two kernels with identical outputs: 16 elements per thread (every built width), and 64 elements per
+ * thread with the row staged by one TMA load (K = 4096, 12288, 14336).  mode -1 (default) takes the second for many rows of
+ * its widths, 0 always the first.  A comparison switch without a reference counterpart. */
 int tq_set_prologue_mode(int mode);
 
 /* Finisher of the split-K path: out = bf16((float(C)*body_scale[m])*w_scale[n] + tail + bias). */

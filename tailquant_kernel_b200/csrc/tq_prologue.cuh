@@ -1,4 +1,4 @@
-// Types and small helpers shared by the two prologue kernels (tq_prologue.cu, tq_prologue_fast.cu).
+// Types and small helpers shared by the two prologue kernels (tq_prologue_wide.cu, tq_prologue_fast.cu).
 #pragma once
 
 #include "tq_common.cuh"
@@ -38,8 +38,9 @@ __device__ __forceinline__ float make_scale(float t, float eps, int mode) {
 
 }  // namespace
 
-// Kernel of tq_prologue_fast.cu for the (rotation, K, dtype) combinations it is built for; TQ_ERR_UNSUPPORTED
-// otherwise (the caller then runs the general kernel).
+// Kernels of tq_prologue_wide.cu and tq_prologue_fast.cu for the (rotation, K, dtype) combinations they are built for;
+// TQ_ERR_UNSUPPORTED otherwise.
+int run_prologue_wide(int kind, int K, int dtype, const PrologueParams& p, cudaStream_t st);
 int run_prologue_fast(int kind, int K, int dtype, const PrologueParams& p, cudaStream_t st);
 
 }  // namespace tq

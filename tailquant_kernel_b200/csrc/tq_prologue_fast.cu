@@ -1,5 +1,5 @@
-// Fused prologue of the split W4A4 + tail linear, the kernel for the layer widths of the benchmarked models
-// (K = 4096, 12288, 14336; sm_100a).  Same outputs, bit for bit, as the general kernel in tq_prologue.cu.
+// Fused prologue of the split W4A4 + tail linear, the kernel for many rows of the layer widths of the benchmarked models
+// (K = 4096, 12288, 14336; sm_100a).  Same outputs, bit for bit, as tq_prologue_wide.cu.
 //
 // One CTA of K/64 threads works on one row at a time (grid-stride over rows).
 //   * The row arrives by ONE tiled TMA load into shared memory ([K/64 rows of 64 elements], 128-byte swizzle), so a
@@ -699,17 +699,16 @@ prologue_fast_kernel(const __grid_constant__ CUtensorMap tmap_x, const PrologueP
       }
       if (p.tail_cnt) {
         p.tail_cnt[((size_t)(m >> 7) * NHS + tid) * 128 + (m & 127)] = (uint16_t)ntail;
-        if (m == p.M - 1) {
-          // the rows that pad M to a multiple of 256 (the CTA-pair GEMM's tile height) have no entries: the GEMM
-          // kernels rely on these zeros instead of checking rows
-          const int last = (p.M + 255) / 256 * 256;
-          for (int r = p.M; r < last; ++r) p.tail_cnt[((size_t)(r >> 7) * NHS + tid) * 128 + (r & 127)] = 0;
-        }
+        // the rows that pad M to a multiple of 256 (the CTA-pair GEMM's tile height) have no entries: the GEMM relies on
+        // these zeros instead of checking rows.  They are shared out over the rows: by the last row alone they cost up to
+        // 45 us (255 rows x 192 scattered stores at K = 12288)
+        for (int r = p.M + m; r < (p.M + 255) / 256 * 256; r += p.M)
+          p.tail_cnt[((size_t)(r >> 7) * NHS + tid) * 128 + (r & 127)] = 0;
       }
       // ---- tail entries: every thread writes the indices of its own entries to the row's list in shared memory
       // (ascending), then the threads share the list evenly -- entry r goes to thread r mod NT -- so that the global
       // stores of the lists are coalesced and no thread waits for the one with the most entries
-      {
+      if (p.tail_idx16 || p.tail_val || p.idx32 || p.top_q || p.tail_rec) {
         const smp list_s = sm + S::LIST_OFF;
         uint32_t* const hst = reinterpret_cast<uint32_t*>(sm + S::HST_OFF);
         hst[tid] = (uint32_t)tail_before;

@@ -351,8 +351,8 @@ def set_gemv_channel_tiles(tiles: int) -> None:
 
 
 def set_prologue_mode(mode: int) -> None:
-    """-1: the prologue kernel specialised for K = 4096 / 12288 / 14336 where it applies; 0: the general kernel only
-    (both give the same bits; a switch for comparisons)."""
+    """-1: by width and row count; 0: the kernel with 16 elements per thread always (both give the same bits; a switch
+    for comparisons)."""
     _lib.check(_lib.load().tq_set_prologue_mode(int(mode)), "set_prologue_mode")
 
 
