@@ -145,28 +145,34 @@ __global__ void dequant_finish_partials_kernel(const int32_t* __restrict__ P, in
 }
 
 // ------------------------------------------------------------------ T4 sparse term
-__device__ __forceinline__ int s4(uint32_t nib) { return (int)((nib & 0xfu) ^ 8u) - 8; }
+// sum_r tq[r] * q_w[idx[r], n0 .. n0 + 7], exact.  What bounds it is the integer work, so two channels share a 32-bit
+// multiply-add: the nibbles are biased to u = q + 8 (0 .. 15), the words (u_i | u_{i+4} << 16) are multiplied by tq, and the
+// bias comes off with 8 sum(tq).  16 entries of any int8 fit the 16-bit halves (16 * 128 * 15 < 2^15) before they are spread.
+constexpr int T4_CHUNK = 1024;   // entries staged at a time
 
-template <typename IdxT>
-__device__ __forceinline__ void sparse_sum8(const int8_t* __restrict__ tq_row, const IdxT* __restrict__ idx_row,
-                                            const uint8_t* __restrict__ b_row, int R, int N, int n0, int (&acc)[8]) {
+__device__ __forceinline__ void sparse_add(const uint2* __restrict__ list, int cnt, const uint8_t* __restrict__ b_row, int N,
+                                           int n0, int (&acc)[8]) {
+  for (int r0 = 0; r0 < cnt; r0 += 16) {
+    const int r1 = min(cnt, r0 + 16);
+    int p[4] = {0, 0, 0, 0}, bias = 0;
+#pragma unroll 8
+    for (int r = r0; r < r1; ++r) {
+      const uint2 e = list[r];
+      const uint32_t w = __ldg(reinterpret_cast<const uint32_t*>(b_row + ((size_t)e.x * N + n0) / 2));
+      const int a = (int)e.y;
+      bias += a;
 #pragma unroll
-  for (int i = 0; i < 8; ++i) acc[i] = 0;
-  for (int r = 0; r < R; ++r) {
-    const int k = (int)idx_row[r];
-    const int a = (int)tq_row[r];
-    const uint32_t w = *reinterpret_cast<const uint32_t*>(b_row + ((size_t)k * N + n0) / 2);
+      for (int i = 0; i < 4; ++i) p[i] += a * (int)(((w >> (4 * i)) & 0x000f000fu) ^ 0x00080008u);
+    }
 #pragma unroll
-    for (int i = 0; i < 8; ++i) acc[i] += a * s4(w >> (4 * i));
+    for (int i = 0; i < 4; ++i) {
+      const int lo = (int)(short)p[i];
+      acc[i] += lo - 8 * bias;
+      acc[i + 4] += ((p[i] - lo) >> 16) - 8 * bias;
+    }
   }
 }
 
-__device__ __forceinline__ void store16(void* out, size_t i, float v, int dtype) {
-  if (dtype == TQ_BF16)
-    reinterpret_cast<__nv_bfloat16*>(out)[i] = __float2bfloat16_rn(v);
-  else
-    reinterpret_cast<__half*>(out)[i] = __float2half_rn(v);
-}
 __device__ __forceinline__ float load16(const void* p, size_t i, int dtype) {
   return dtype == TQ_BF16 ? __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(p)[i])
                           : __half2float(reinterpret_cast<const __half*>(p)[i]);
@@ -176,28 +182,45 @@ __device__ __forceinline__ float load16(const void* p, size_t i, int dtype) {
 // mode 1: out = f16(float(out) + float(sum)*ts*ws)          (tools/sparse_correction_add_ext_v1.py:64-123)
 // mode 2: out = f16(float(sum)*ts*ws)                       (tools/split_sparse_idx16_ext_v1.py:50-109)
 template <typename IdxT>
-__global__ void t4_epilogue_kernel(int mode, const int32_t* __restrict__ C, const float* __restrict__ bs,
-                                   const int8_t* __restrict__ top_q, const IdxT* __restrict__ idx,
-                                   const uint8_t* __restrict__ b_row, const float* __restrict__ ts,
-                                   const void* __restrict__ ws, int ws_bf16, void* out, int out_dtype, int M, int N,
-                                   int R) {
+__global__ void __launch_bounds__(128) t4_epilogue_kernel(int mode, const int32_t* __restrict__ C, const float* __restrict__ bs,
+                                                          const int8_t* __restrict__ top_q, const IdxT* __restrict__ idx,
+                                                          const uint8_t* __restrict__ b_row, const float* __restrict__ ts,
+                                                          const void* __restrict__ ws, int ws_bf16, void* out, int out_dtype,
+                                                          int vec, int N, int R) {
+  __shared__ uint2 list[T4_CHUNK];   // (index, code) of the row's entries
   const int m = blockIdx.y;
   const int n0 = (blockIdx.x * blockDim.x + threadIdx.x) * 8;
-  if (m >= M || n0 >= N) return;
-  int acc[8];
-  sparse_sum8<IdxT>(top_q + (size_t)m * R, idx + (size_t)m * R, b_row, R, N, n0, acc);
+  const bool on = n0 < N;
+  int acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+  for (int c0 = 0; c0 < R; c0 += T4_CHUNK) {
+    const int cnt = min(R - c0, T4_CHUNK);
+    if (c0) __syncthreads();
+    for (int r = threadIdx.x; r < cnt; r += blockDim.x)
+      list[r] = make_uint2((uint32_t)idx[(size_t)m * R + c0 + r], (uint32_t)(int)top_q[(size_t)m * R + c0 + r]);
+    __syncthreads();
+    if (on) sparse_add(list, cnt, b_row, N, n0, acc);
+  }
+  if (!on) return;
   const float tsm = ts[m];
   const float bsm = (mode == 0) ? bs[m] : 0.0f;
+  const size_t o = (size_t)m * N + n0;
+  uint32_t r16[8];
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
-    const size_t o = (size_t)m * N + n0 + i;
     const float w = ws_bf16 ? __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(ws)[n0 + i])
                             : reinterpret_cast<const float*>(ws)[n0 + i];
     const float sparse = __fmul_rn(__fmul_rn((float)acc[i], tsm), w);
-    float v = sparse;
-    if (mode == 0) v = __fadd_rn(__fmul_rn(__fmul_rn((float)C[o], bsm), w), sparse);
-    if (mode == 1) v = __fadd_rn(load16(out, o, out_dtype), sparse);
-    store16(out, o, v, out_dtype);
+    float d = sparse;
+    if (mode == 0) d = __fadd_rn(__fmul_rn(__fmul_rn((float)C[o + i], bsm), w), sparse);
+    if (mode == 1) d = __fadd_rn(load16(out, o + i, out_dtype), sparse);
+    r16[i] = out_dtype == TQ_BF16 ? f32_to_bf16_bits(d) : (uint32_t)__half_as_ushort(__float2half_rn(d));
+  }
+  if (vec) {
+    *reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(out) + o) =
+        make_uint4(r16[0] | (r16[1] << 16), r16[2] | (r16[3] << 16), r16[4] | (r16[5] << 16), r16[6] | (r16[7] << 16));
+  } else {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) reinterpret_cast<uint16_t*>(out)[o + i] = (uint16_t)r16[i];
   }
 }
 
@@ -214,13 +237,14 @@ int t4_launch(int mode, const int32_t* C, const float* bs, const int8_t* top_q, 
   if (N % 8 != 0) return TQ_ERR_UNSUPPORTED;
   if (out_dtype != TQ_BF16 && out_dtype != TQ_FP16) return TQ_ERR_BAD_ARG;
   if (M == 0) return TQ_OK;
-  dim3 block(128), grid((N / 8 + 127) / 128, M);
+  const int vec = aligned16(out) ? 1 : 0;
+  const dim3 block(128), grid((N / 8 + 127) / 128, M);
   if (idx_u16)
-    t4_epilogue_kernel<uint16_t><<<grid, block, 0, st>>>(mode, C, bs, top_q, reinterpret_cast<const uint16_t*>(idx),
-                                                         b_row, ts, ws, ws_bf16, out, out_dtype, M, N, R);
+    t4_epilogue_kernel<uint16_t><<<grid, block, 0, st>>>(mode, C, bs, top_q, reinterpret_cast<const uint16_t*>(idx), b_row, ts,
+                                                         ws, ws_bf16, out, out_dtype, vec, N, R);
   else
-    t4_epilogue_kernel<int32_t><<<grid, block, 0, st>>>(mode, C, bs, top_q, reinterpret_cast<const int32_t*>(idx),
-                                                        b_row, ts, ws, ws_bf16, out, out_dtype, M, N, R);
+    t4_epilogue_kernel<int32_t><<<grid, block, 0, st>>>(mode, C, bs, top_q, reinterpret_cast<const int32_t*>(idx), b_row, ts,
+                                                        ws, ws_bf16, out, out_dtype, vec, N, R);
   return check_launch();
 }
 

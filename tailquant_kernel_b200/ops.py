@@ -51,10 +51,13 @@ def _check(cond: bool, msg: str) -> None:
 
 
 def _check_cuda(t: torch.Tensor, name: str, dtype=None) -> None:
-    _check(torch.is_tensor(t) and t.is_cuda, f"{name} must be a CUDA tensor")
-    _check(t.is_contiguous(), f"{name} must be contiguous")
-    if dtype is not None:
-        _check(t.dtype == dtype, f"{name} must be {dtype}")
+    # (messages are only put together where they are needed: these checks run for every tensor of every call)
+    if not (isinstance(t, torch.Tensor) and t.is_cuda):
+        raise RuntimeError(f"{name} must be a CUDA tensor")
+    if not t.is_contiguous():
+        raise RuntimeError(f"{name} must be contiguous")
+    if dtype is not None and t.dtype != dtype:
+        raise RuntimeError(f"{name} must be {dtype}")
 
 
 def _f16_code(dtype) -> int:
@@ -164,7 +167,8 @@ def split_prologue(x: torch.Tensor, had_kind: int, R: int, descending_rank: Opti
         _ptr(x), M, K, had_kind, R, descending_rank, eps, _ptr(out.a_pack), _ptr(out.a_q8), _ptr(out.body_scale),
         _ptr(out.top_scale), _ptr(out.tail_idx), _ptr(out.tail_val), ld, _ptr(out.tail_ptr), pld, _ptr(out.tail_rec),
         _ptr(out.tail_cnt), _ptr(out.tail_dense), _ptr(out.idx32), _ptr(out.top_q), _ptr(out.x_rot), _stream())
-    _lib.check(rc, f"split_prologue(M={M}, K={K}, had_kind={had_kind}, R={R})")
+    if rc:
+        _lib.check(rc, f"split_prologue(M={M}, K={K}, had_kind={had_kind}, R={R})")
     return out
 
 
@@ -186,7 +190,8 @@ def _topr_pack(name, A, R, descending_rank, A_pack, body_scale, top_scale, top_q
     rc = _lib.load().tq_topr_pack(_ptr(A), _f16_code(A.dtype), M, K, R, descending_rank, _ptr(A_pack),
                                   _ptr(body_scale), _ptr(top_scale), _ptr(top_q) if R else None,
                                   _ptr(idx) if R else None, float(eps), _stream())
-    _lib.check(rc, f"{name}(M={M}, K={K}, R={R}, descending_rank={descending_rank})")
+    if rc:
+        _lib.check(rc, f"{name}(M={M}, K={K}, R={R}, descending_rank={descending_rank})")
 
 
 def fused_topr_pack(A, R, descending_rank, A_pack, body_scale, top_scale, top_q, idx, eps) -> None:
@@ -230,7 +235,8 @@ def prepare_weight(W: torch.Tensor, had_kind: Optional[int] = None, eps: float =
     b_row = torch.empty((K, N // 2), dtype=torch.uint8, device=dev) if t4 else None
     rc = _lib.load().tq_prepare_weight(_ptr(Wb), N, K, had_kind, eps, _ptr(b_col), _ptr(w_scale), _ptr(w_rot),
                                        _ptr(b_row), _ptr(w_t), _stream())
-    _lib.check(rc, f"prepare_weight(N={N}, K={K}, had_kind={had_kind})")
+    if rc:
+        _lib.check(rc, f"prepare_weight(N={N}, K={K}, had_kind={had_kind})")
     b32 = None if bias is None else bias.detach().to(device=dev, dtype=torch.float32).contiguous()
     return PreparedWeight(N, K, had_kind, b_col, w_scale, w_t, b_row, w_rot if keep_w_rot else None, b32)
 
@@ -255,7 +261,8 @@ def matmul(A_pack: torch.Tensor, B_pack: torch.Tensor, M: Optional[int] = None, 
     M, N, K = _gemm_dims(A_pack, B_pack, M, N, K)
     C = torch.empty((M, N), dtype=torch.int32, device=A_pack.device)
     rc = _lib.load().tq_int4_matmul(_ptr(A_pack), _ptr(B_pack), _ptr(C), M, N, K, 1, _stream())
-    _lib.check(rc, f"matmul(M={M}, N={N}, K={K})")
+    if rc:
+        _lib.check(rc, f"matmul(M={M}, N={N}, K={K})")
     return C
 
 
@@ -267,7 +274,8 @@ def matmul_splitk(A_pack, B_pack, C: torch.Tensor, split_k: int, M=None, N=None,
     _check(C.numel() >= M * N, "C too small")
     C.zero_()
     rc = _lib.load().tq_int4_matmul(_ptr(A_pack), _ptr(B_pack), _ptr(C), M, N, K, int(split_k), _stream())
-    _lib.check(rc, f"matmul_splitk(M={M}, N={N}, K={K}, split_k={split_k})")
+    if rc:
+        _lib.check(rc, f"matmul_splitk(M={M}, N={N}, K={K}, split_k={split_k})")
     return C
 
 
@@ -285,7 +293,8 @@ def split_gemm_fused(A_pack, body_scale, B_pack, w_scale, out, tail=None, bias=N
         _check_cuda(bias, "bias", torch.float32)
     rc = _lib.load().tq_split_gemm_fused(_ptr(A_pack), _ptr(body_scale), _ptr(B_pack), _ptr(w_scale), _ptr(tail),
                                          _ptr(bias), _ptr(out), M, N, K, _stream())
-    _lib.check(rc, f"split_gemm_fused(M={M}, N={N}, K={K})")
+    if rc:
+        _lib.check(rc, f"split_gemm_fused(M={M}, N={N}, K={K})")
     return out
 
 
@@ -334,7 +343,8 @@ def split_gemm_mma(a_q8, body_scale, B_pack, w_scale, out, w_rot=None, pro: Opti
         rc = _lib.load().tq_split_gemm_mma_swiglu(*common, M, N, K, _stream())
     else:
         rc = _lib.load().tq_split_gemm_mma(*common, _ptr(dbg_acc), _ptr(dbg_tail), M, N, K, _stream())
-    _lib.check(rc, f"split_gemm_mma(M={M}, N={N}, K={K}, R={R}, act={act})")
+    if rc:
+        _lib.check(rc, f"split_gemm_mma(M={M}, N={N}, K={K}, R={R}, act={act})")
     return out
 
 
@@ -362,7 +372,8 @@ def dequant_finish(C, body_scale, w_scale, out, tail=None, bias=None):
     _check_cuda(out, "out", torch.bfloat16)
     rc = _lib.load().tq_dequant_finish(_ptr(C), _ptr(body_scale), _ptr(w_scale), _ptr(tail), _ptr(bias), _ptr(out),
                                        M, N, _stream())
-    _lib.check(rc, "dequant_finish")
+    if rc:
+        _lib.check(rc, "dequant_finish")
     return out
 
 
@@ -379,7 +390,8 @@ def gemv_splitk(A, B_pack, C: torch.Tensor, split_k: int = 0) -> torch.Tensor:
     _check(C.numel() >= M * N, "C too small")
     rc = _lib.load().tq_int4_gemv_splitk(None if a8 else _ptr(A), _ptr(A) if a8 else None, _ptr(B_pack), _ptr(C), M, N,
                                          K, int(split_k), _stream())
-    _lib.check(rc, f"gemv_splitk(M={M}, N={N}, K={K}, split_k={split_k})")
+    if rc:
+        _lib.check(rc, f"gemv_splitk(M={M}, N={N}, K={K}, split_k={split_k})")
     return C
 
 
@@ -404,7 +416,8 @@ def gemv_partials(A, B_pack, partials: torch.Tensor) -> torch.Tensor:
     _check(partials.dim() == 3 and tuple(partials.shape[1:]) == (M, N), "partials must be [splits, M, N]")
     rc = _lib.load().tq_int4_gemv_partials(None if a8 else _ptr(A), _ptr(A) if a8 else None, _ptr(B_pack),
                                            _ptr(partials), M, N, K, int(partials.shape[0]), _stream())
-    _lib.check(rc, f"gemv_partials(M={M}, N={N}, K={K}, splits={partials.shape[0]})")
+    if rc:
+        _lib.check(rc, f"gemv_partials(M={M}, N={N}, K={K}, splits={partials.shape[0]})")
     return partials
 
 
@@ -419,7 +432,8 @@ def dequant_finish_partials(partials, body_scale, w_scale, out, tail=None, bias=
     _check(out.numel() >= (M * N // 2 if act == "swiglu" else M * N), "out too small")
     rc = _lib.load().tq_dequant_finish_partials(_ptr(partials), int(S), _ptr(body_scale), _ptr(w_scale), _ptr(tail),
                                                 _ptr(bias), _ptr(out), M, N, 1 if act == "swiglu" else 0, _stream())
-    _lib.check(rc, f"dequant_finish_partials(S={S}, M={M}, N={N})")
+    if rc:
+        _lib.check(rc, f"dequant_finish_partials(S={S}, M={M}, N={N})")
     return out
 
 
@@ -435,7 +449,8 @@ def tail_gather_small(tail_idx, tail_val, w_t, tail_out, R: int):
     _check(tail_out.numel() >= M * N, "tail_out too small")
     rc = _lib.load().tq_tail_gather_small(_ptr(tail_idx), _ptr(tail_val), _ptr(w_t), _ptr(tail_out), M, N, K, int(R),
                                           ld, _stream())
-    _lib.check(rc, f"tail_gather_small(M={M}, N={N}, K={K}, R={R})")
+    if rc:
+        _lib.check(rc, f"tail_gather_small(M={M}, N={N}, K={K}, R={R})")
     return tail_out
 
 
@@ -455,7 +470,8 @@ def linear_splitk_noalloc(A_pack, body_scale, B_pack, w_scale, out, split_k: int
     rc = _lib.load().tq_int4_linear_splitk_noalloc(_ptr(A_pack), _ptr(body_scale), _ptr(B_pack), _ptr(w_scale),
                                                    _ptr(tail), _ptr(bias), _ptr(out), M, N, K, int(split_k),
                                                    _stream())
-    _lib.check(rc, f"linear_splitk_noalloc(M={M}, N={N}, K={K}, split_k={split_k})")
+    if rc:
+        _lib.check(rc, f"linear_splitk_noalloc(M={M}, N={N}, K={K}, split_k={split_k})")
     return out
 
 
@@ -471,7 +487,8 @@ def tail_gather(tail_idx, tail_val, w_t, tail_out, R: int):
     _check(tail_out.numel() >= M * N, "tail_out too small")
     rc = _lib.load().tq_tail_gather(_ptr(tail_idx), _ptr(tail_val), _ptr(w_t), _ptr(tail_out), M, N, K, int(R), ld,
                                     _stream())
-    _lib.check(rc, f"tail_gather(M={M}, N={N}, K={K}, R={R})")
+    if rc:
+        _lib.check(rc, f"tail_gather(M={M}, N={N}, K={K}, R={R})")
     return tail_out
 
 
@@ -503,7 +520,8 @@ def _scale_sparse_epilogue(name, C, body_scale, top_q, idx, B_row_pack, top_scal
     rc = _lib.load().tq_scale_sparse_epilogue(_ptr(C), _ptr(body_scale), _ptr(top_q), _ptr(idx), _ptr(B_row_pack),
                                               _ptr(top_scale), _ptr(w_scale), _ptr(out), _f16_code(out.dtype), M, N,
                                               K2, R, _stream())
-    _lib.check(rc, name)
+    if rc:
+        _lib.check(rc, name)
 
 
 def scale_sparse_epilogue_quad(C, body_scale, top_q, idx, B_row_pack, top_scale, w_scale, out, K) -> None:
@@ -527,7 +545,8 @@ def _sparse_correction_add(name, out, top_q, idx, B_row_pack, top_scale, w_scale
     rc = _lib.load().tq_sparse_correction_add(_ptr(out), _f16_code(out.dtype), _ptr(top_q), _ptr(idx),
                                               _ptr(B_row_pack), _ptr(top_scale), _ptr(w_scale),
                                               1 if ws_dtype == torch.bfloat16 else 0, M, N, K, R, _stream())
-    _lib.check(rc, name)
+    if rc:
+        _lib.check(rc, name)
 
 
 def sparse_correction_add_bf16_oct(out, top_q, idx, B_row_pack, top_scale, w_scale) -> None:
@@ -559,7 +578,8 @@ def sparse_top_write(top_q, idx, B_row_pack, top_scale, w_scale, out) -> None:
     rc = _lib.load().tq_sparse_top_write(_ptr(out), _f16_code(out.dtype), _ptr(top_q), _ptr(idx),
                                          0 if idx.dtype == torch.int32 else 1, _ptr(B_row_pack), _ptr(top_scale),
                                          _ptr(w_scale), M, N, K, R, _stream())
-    _lib.check(rc, "sparse_top_write")
+    if rc:
+        _lib.check(rc, "sparse_top_write")
 
 
 def idx_i32_to_u16(idx: torch.Tensor, out: torch.Tensor) -> None:
@@ -568,7 +588,8 @@ def idx_i32_to_u16(idx: torch.Tensor, out: torch.Tensor) -> None:
     _check_cuda(out, "out")
     _check(out.element_size() == 2 and out.numel() >= idx.numel(), "out must hold idx.numel() 16-bit values")
     rc = _lib.load().tq_idx_i32_to_u16(_ptr(idx), _ptr(out), idx.numel(), _stream())
-    _lib.check(rc, "idx_i32_to_u16")
+    if rc:
+        _lib.check(rc, "idx_i32_to_u16")
 
 
 def gemm_status() -> int:
