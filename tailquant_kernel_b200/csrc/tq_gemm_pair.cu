@@ -69,7 +69,11 @@ __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
   return *reinterpret_cast<const uint32_t*>(&v);
 }
 
-template <int ACT>  // 0: out [M, N]; 1: SwiGLU over interleaved (gate, up) channel pairs, out [M, N/2]
+// ACT 0: out [M, N]; 1: SwiGLU over interleaved (gate, up) channel pairs, out [M, N/2].  TAIL false compiles the tail away
+// (w4a4, M = 1000, N = 6144, K = 4096: 43 us -> 36 with the shared last tile).  In the instantiation with a tail `has_tail`
+// stays a run-time value: known at compile time, ptxas interleaved the builders' loops differently and spilled, and
+// 4096 x 28672 went from 1190 us to 1445.
+template <int ACT, bool TAIL>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(P_THREADS, 1)
 pair_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a8, const __grid_constant__ CUtensorMap tmap_b4,
                   const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_d,
@@ -100,7 +104,7 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a8, const __grid_const
   const int G = my_tiles * kbt;                     // K slices this pair goes through, over all its tiles
   const int look = kbt < P_LOOK ? kbt : P_LOOK;
   auto lead = [&](uint32_t bar) { return map_to_cta(bar, 0u); };  // the leader's barrier at this offset
-  const bool has_tail = p.has_tail != 0;
+  const bool has_tail = TAIL && p.has_tail != 0;
   const int uses = has_tail ? 3 : 1;                // slot uses per K slice: INT8 operands, then two bf16 halves
   constexpr uint32_t TMEM_COLS = 2 * BN;  // int32 accumulator, then fp32 tail accumulator
 
@@ -120,7 +124,7 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a8, const __grid_const
     for (int b = 0; b < 2; ++b) {
       mbar_init(acc_full(b), 1);
       // the epilogue warps of both CTAs (leader's copy is used): all twelve with a tail, warps 10..13 without
-      mbar_init(acc_empty(b), p.has_tail ? 2 * (4 + P_BUILD_WARPS) : 2 * 4);
+      mbar_init(acc_empty(b), has_tail ? 2 * (4 + P_BUILD_WARPS) : 2 * 4);
     }
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -221,17 +225,29 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a8, const __grid_const
     }
     tc_fence_before();
     __syncwarp();
-    if (lane == 0) mbar_arrive_cluster(lead(acc_empty(ab)));
+    // (nothing waits for the buffer of the last tile)
+    if (lane == 0 && (TAIL || i + 1 < my_tiles)) mbar_arrive_cluster(lead(acc_empty(ab)));
     return true;
   };
   // the eight 32-channel chunks of a tile are split 3 / 3 / 2 over the three warps of a lane quadrant
-  // (without a tail warps 10..13 take all eight chunks and the others none)
+  // (without a tail warps 10..13 take all eight chunks of every tile but the last one, under the next tile's main loop;
+  // the last tile has none to hide under and is shared like the others: 16 us -> 9 at M = 300)
   const int ethird = (warp - 2) >> 2;
-  const int c_lo = has_tail ? ethird * 3 : 0, c_hi = has_tail ? (ethird == 2 ? 8 : ethird * 3 + 3) : 8;
+  const int c_lo = ethird * 3, c_hi = ethird == 2 ? 8 : ethird * 3 + 3;
+  // (From four K slices per tile on: a widening warp has then seen slots released behind the previous use of the last
+  // tile's accumulator, so its first wait on that accumulator's barrier, by parity, cannot be a phase too early.)
+  const bool share_last = !TAIL && kbt >= 4;
   bool ok = true;
   int epi_done = 0;  // tiles whose epilogue share this warp has done
   auto catch_up = [&](int upto) {
-    while (ok && epi_done < upto) ok = epilogue(epi_done++, c_lo, c_hi);
+    while (ok && epi_done < upto) {
+      const bool all = !has_tail && !(share_last && epi_done + 1 == my_tiles);
+      ok = epilogue(epi_done++, all ? 0 : c_lo, all ? 8 : c_hi);
+    }
+  };
+  auto last_share = [&]() {  // without a tail: the share of a widening warp
+    epi_done = my_tiles - 1;
+    if (ok && share_last && my_tiles > 0) ok = epilogue(epi_done, c_lo, c_hi);
   };
   // INT4 -> INT8 (x16) of K slice g's weight tile by four warps (wtid = 0..127): staging buffer -> B region of
   // the slice's INT8 slot.  One group of four warps sees every phase of the staging barriers it waits on.
@@ -406,7 +422,10 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a8, const __grid_const
       const int i = g / kbt, kb = g - i * kbt;
       if (has_tail && (kb >= look - 1 || kb + step >= kbt)) catch_up(i);  // (second case: this group's last slice of the tile)
     }
-    if (has_tail) catch_up(my_tiles);
+    if (TAIL)
+      catch_up(my_tiles);
+    else
+      last_share();
   } else {
     // ------------------------------------------------------------------ tail builders (+ epilogue share)
     // 256 threads = 128 rows x the two 64-wide halves of a K slice: each builds its row of the zero-filled
@@ -554,6 +573,7 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a8, const __grid_const
         for (int g = 1; g < G && ok; g += 2) {
           if (!(ok = widen_one(g, wtid))) break;
         }
+        if (!TAIL) last_share();
       } else {
         catch_up(my_tiles);  // warps 10..13: the epilogues, each under the next tile's main loop
       }
@@ -568,7 +588,7 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a8, const __grid_const
   }
 }
 
-template <int ACT>
+template <int ACT, bool has_tail>
 int launch_pair_gemm(const int8_t* a_q8, const uint8_t* b_col, const void* w_rot, const void* tail_dense, PairGemmParams p,
                      cudaStream_t st) {
   using S = PS;
@@ -576,7 +596,7 @@ int launch_pair_gemm(const int8_t* a_q8, const uint8_t* b_col, const void* w_rot
   int dev = 0;
   cudaGetDevice(&dev);
   if (!(dev < 64 && configured[dev])) {
-    cudaError_t e = cudaFuncSetAttribute(pair_gemm_kernel<ACT>, cudaFuncAttributeMaxDynamicSharedMemorySize, S::DYN);
+    cudaError_t e = cudaFuncSetAttribute(pair_gemm_kernel<ACT, has_tail>, cudaFuncAttributeMaxDynamicSharedMemorySize, S::DYN);
     if (e != cudaSuccess) {
       set_last_cuda_error(e);
       return TQ_ERR_CUDA;
@@ -590,12 +610,12 @@ int launch_pair_gemm(const int8_t* a_q8, const uint8_t* b_col, const void* w_rot
   if (!make_tensor_map_2d(&mb, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, b_col, (uint64_t)(p.K / 2), (uint64_t)p.N,
                           (uint64_t)(p.K / 2), P_BK / 2, P_BH))
     return TQ_ERR_CUDA;
-  const void* wsrc = p.has_tail ? w_rot : (const void*)b_col;  // never loaded without a tail; kept valid
-  if (!make_tensor_map_2d(&mw, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, wsrc, (uint64_t)(p.has_tail ? p.K : p.K / 4),
-                          (uint64_t)p.N, (uint64_t)(p.has_tail ? p.K * 2 : p.K / 2), 64, P_BH, true))
+  const void* wsrc = has_tail ? w_rot : (const void*)b_col;  // never loaded without a tail; kept valid
+  if (!make_tensor_map_2d(&mw, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, wsrc, (uint64_t)(has_tail ? p.K : p.K / 4),
+                          (uint64_t)p.N, (uint64_t)(has_tail ? p.K * 2 : p.K / 2), 64, P_BH, true))
     return TQ_ERR_CUDA;
   // the zero-filled tail matrix, 32 rows x one 64-wide half slice per load (rows beyond M read as zeros)
-  p.dense = (p.has_tail && tail_dense) ? 1 : 0;
+  p.dense = (has_tail && tail_dense) ? 1 : 0;
   if (p.dense) {
     if (!make_tensor_map_2d(&md, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, tail_dense, (uint64_t)p.K, (uint64_t)p.M,
                             (uint64_t)p.K * 2, 64, 32, true))
@@ -610,7 +630,7 @@ int launch_pair_gemm(const int8_t* a_q8, const uint8_t* b_col, const void* w_rot
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const int total = p.tiles_m * p.tiles_n;
   const int pairs = total < sms / 2 ? total : sms / 2;
-  pair_gemm_kernel<ACT><<<2 * pairs, P_THREADS, S::DYN, st>>>(ma, mb, mw, md, p);
+  pair_gemm_kernel<ACT, has_tail><<<2 * pairs, P_THREADS, S::DYN, st>>>(ma, mb, mw, md, p);
   return check_launch();
 }
 
@@ -627,12 +647,12 @@ int run_pair_gemm(const int8_t* a_q8, const float* body_scale, const uint8_t* b_
   p.N = N;
   p.K = K;
   p.R = R;
+  p.has_tail = R > 0 ? 1 : 0;
   p.ld = tail_ld;
   p.ptr_ld = ptr_ld;
   p.ptr = tail_ptr;
   p.rec = tail_rec;
   p.cnt = tail_cnt;
-  p.has_tail = R > 0 ? 1 : 0;
   p.idx = tail_idx16;
   p.val = reinterpret_cast<const uint16_t*>(tail_val);
   p.sx = body_scale;
@@ -642,8 +662,11 @@ int run_pair_gemm(const int8_t* a_q8, const float* body_scale, const uint8_t* b_
   p.dbg_acc = dbg_acc;
   p.dbg_tail = dbg_tail;
   if (tail_dense && !aligned16(tail_dense)) return TQ_ERR_MISALIGNED;
-  return act ? launch_pair_gemm<1>(a_q8, b_col, w_rot, tail_dense, p, st)
-             : launch_pair_gemm<0>(a_q8, b_col, w_rot, tail_dense, p, st);
+  if (R > 0)
+    return act ? launch_pair_gemm<1, true>(a_q8, b_col, w_rot, tail_dense, p, st)
+               : launch_pair_gemm<0, true>(a_q8, b_col, w_rot, tail_dense, p, st);
+  return act ? launch_pair_gemm<1, false>(a_q8, b_col, w_rot, tail_dense, p, st)
+             : launch_pair_gemm<0, false>(a_q8, b_col, w_rot, tail_dense, p, st);
 }
 
 }  // namespace tq
