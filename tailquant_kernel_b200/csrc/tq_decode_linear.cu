@@ -40,6 +40,7 @@ struct DecodeLinearParams {
   uint16_t* out;            // [M, N], or [M, N/2] with act
   int M, N, K, R, ld, act;
   int nst;                  // stages of a warp's ring of weight blocks
+  int early;                // the weights may be read before the kernel in front has ended
 };
 
 // NT: tiles of eight token rows (M <= 8 NT).  CT: tiles of 16 output channels per CTA step.  The weights are the m16
@@ -119,6 +120,7 @@ decode_linear_kernel(const __grid_constant__ CUtensorMap tmap_b, const DecodeLin
       }
     }
   };
+  if (!p.early) pdl_wait();
   if (lane == 0)
     for (int s = 0; s < L.nst; ++s) request();
 

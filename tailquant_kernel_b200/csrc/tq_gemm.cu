@@ -2,10 +2,10 @@
 // int32 accumulators in tensor memory, operands staged by TMA as packed INT4 and widened to
 // INT8 in shared memory, dequant (+ tail + bias) fused into the epilogue.
 //
-// One persistent CTA per SM, 14 warps with fixed roles:
+// One persistent CTA per SM, 22 warps with fixed roles:
 //   warp 0        TMA producer: packed A [128 x 64 B] and B [BN x 64 B] tiles of one 128-wide
 //                 k-block into a ring of staging buffers (plain 2-D tiled loads, one CTA each)
-//   warps 6..13   unpackers: read 16 packed bytes, widen the 32 nibbles to INT8 (value x 16,
+//   warps 6..21   unpackers: read 16 packed bytes, widen the 32 nibbles to INT8 (value x 16,
 //                 sign kept in the top nibble, so no sign extension is needed) and store them
 //                 into the canonical K-major 128-byte-swizzled UMMA operand layout
 //   warp 1        MMA issuer: 4 x tcgen05.mma (M128 x BN x K32) per k-block into one of two
@@ -36,7 +36,7 @@ namespace {
 constexpr int BM = 128;
 constexpr int BK = 128;            // int8 elements per k-block = one 128-byte swizzle row
 constexpr int BKP = BK / 2;        // packed bytes per row per k-block
-constexpr int NUM_UNPACK_WARPS = 8;
+constexpr int NUM_UNPACK_WARPS = 16;
 constexpr int NUT = NUM_UNPACK_WARPS * 32;
 constexpr int NUM_THREADS = (6 + NUM_UNPACK_WARPS) * 32;
 constexpr int NUM_EPI_THREADS = 128;
@@ -135,7 +135,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
-    if (lane == 0) {
+    if (elect_one()) {
       int s = 0;
       uint32_t ph = 0;
       bool ok = true;
@@ -155,9 +155,13 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
       }
     }
   } else if (warp == 1) {
-    // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
+    // ------------------------------------------------------------------ MMA issuer (one elected thread, running
+    // descriptors: see tq_gemm_pair.cu)
+    if (elect_one()) {
       constexpr uint32_t idesc = make_idesc_i8<BN>();
+      constexpr uint64_t B = (uint64_t)(BM * BK) >> 4;
+      const uint64_t desc0 = make_smem_desc(base + S::OPER_OFF);
+      uint64_t d = desc0;
       int su = 0, as = 0;
       uint32_t phu = 0, pha = 0;
       bool ok = true;
@@ -166,19 +170,21 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
         if (!(ok = mbar_wait(acc_empty(as), pha ^ 1u, abort_flag, 0x2u))) break;
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + (uint32_t)(as * BN);
+        uint32_t acc = 0;
         for (int kb = 0; kb < c.nkb; ++kb) {
           if (!(ok = mbar_wait(full_u(su), phu, abort_flag, 0x4u))) break;
           tc_fence_after();
-          const uint32_t a_addr = base + S::OPER_OFF + su * S::OPER_STAGE;
-          const uint32_t b_addr = a_addr + BM * BK;
-#pragma unroll
-          for (int k = 0; k < BK / 32; ++k)
-            umma_i8(d_tmem, make_smem_desc(a_addr + k * 32), make_smem_desc(b_addr + k * 32), idesc,
-                    (kb > 0 || k > 0) ? 1u : 0u);
+          umma_i8(d_tmem, d, d + B, idesc, acc);
+          umma_i8(d_tmem, d + 2, d + B + 2, idesc, 1u);   // 32 bytes of K further: + 2
+          umma_i8(d_tmem, d + 4, d + B + 4, idesc, 1u);
+          umma_i8(d_tmem, d + 6, d + B + 6, idesc, 1u);
+          acc = 1u;
           umma_commit(empty_u(su));
+          d += S::OPER_STAGE >> 4;
           if (++su == S::SU) {
             su = 0;
             phu ^= 1u;
+            d = desc0;
           }
         }
         if (!ok) break;
@@ -353,8 +359,7 @@ int launch_gemm(const uint8_t* a_pack, const uint8_t* b_col, GemmParams p, cudaS
   if (p.split_k > p.kb_total) p.split_k = p.kb_total;
   p.kb_per_split = (p.kb_total + p.split_k - 1) / p.split_k;
   p.split_k = (p.kb_total + p.kb_per_split - 1) / p.kb_per_split;  // no empty split
-  int sms = 148;
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const int sms = current_device_sms();
   const int total = p.tiles_m * p.tiles_n * p.split_k;
   const int grid = total < sms ? total : sms;
   kern<<<grid, NUM_THREADS, S::DYN, st>>>(ma, mb, p);
@@ -366,8 +371,19 @@ int run_gemm(const uint8_t* a_pack, const uint8_t* b_col, GemmParams p, cudaStre
   if (p.K % BK != 0 || p.N % 8 != 0) return TQ_ERR_UNSUPPORTED;
   if (!aligned16(a_pack) || !aligned16(b_col)) return TQ_ERR_MISALIGNED;
   if (p.M == 0) return TQ_OK;
+  const int sms = current_device_sms();
   // wide tiles when they still fill the machine, narrow ones for small problems / split-K
   const long tiles256 = (long)((p.M + BM - 1) / BM) * ((p.N + 255) / 256) * (p.split_k > 0 ? p.split_k : 1);
+  if (p.mode != MODE_I32_ATOMIC && p.M <= 1024) {
+    // Few and medium row counts: tiles of 128 channels x up to 176 rows with the K range shared by a cluster, where that is
+    // estimated to be faster than this kernel's rounds (0.37 us per K slice of a 128 x 128 tile, 0.8 of a 128 x 256 one).
+    // N = K = 4096: 11.6 us against 18 at 256 rows, 8.3 / 17 at 64; the line is near 600 rows.
+    const long t128 = (long)((p.M + 127) / 128) * ((p.N + 127) / 128);
+    const float here = tiles256 >= 148 ? (float)((tiles256 + sms - 1) / sms) * (float)(p.K / BK) * 0.8f + 6.0f
+                                       : (float)((t128 + sms - 1) / sms) * (float)(p.K / BK) * 0.37f + 6.0f;
+    if (plan_stream(p.M, p.N, p.K, false).us < here)
+      return run_stream_packed(a_pack, b_col, p.C, p.sx, p.sw, p.tail, p.bias, p.out, p.M, p.N, p.K, st);
+  }
   if (tiles256 >= 148) return launch_gemm<256>(a_pack, b_col, p, st);
   return launch_gemm<128>(a_pack, b_col, p, st);
 }

@@ -26,22 +26,34 @@
 namespace tq {
 namespace {
 
-constexpr int ST_THREADS = 256;
-constexpr int ST_SP = 3;              // packed-weight staging buffers
+// operands of a call: INT8 codes + tail rows; INT8 codes alone; packed INT4 codes alone
+enum : int { ST_TAIL = 0, ST_INT8 = 1, ST_PACKED = 2 };
+// Four warps with other roles, then widening groups of four: a group takes about 700 cycles per slice whatever its size
+// (wait, load, store, proxy fence, arrival one after the other), which hides behind the bf16 MMAs of a tail; without one it
+// bounds the slice, so two groups take the even and the odd slices (and two more the packed token codes).
+__host__ __device__ constexpr int st_threads(int mode) { return mode == ST_TAIL ? 256 : mode == ST_INT8 ? 384 : 640; }
+// packed staging buffers; with two groups this and the number of INT8 slots are even: a buffer then always belongs to the
+// same group, and no group can fall two phases behind a barrier it waits on by parity
+__host__ __device__ constexpr int st_sp(int mode) { return mode == ST_TAIL ? 3 : 4; }
+constexpr int ST_MAX_SP = 4;
 constexpr int ST_STAGE = 128 * 64;    // [128 channels][128 k] INT4
 constexpr int ST_MAX_SLOTS = 8;       // slots of either ring
 constexpr int ST_MAX_T = 176;         // rows per tile (the exchange buffer of a tile must fit in the rings)
 constexpr int ST_SMEM = 222 * 1024;
+constexpr int ST_BARS = 4 * ST_MAX_SP + 4 * ST_MAX_SLOTS + 1;
 
 struct StreamParams {
-  int M, N, K, T, has_tail, act, tiles_n;
+  int M, N, K, T, act, tiles_n;
   int si, sb;   // INT8 slots, bf16 slots
+  int early;    // the weights may be read before the kernel in front has ended (it has waited for all others itself)
   const float* sx;
   const float* sw;
   const float* bias;
   uint16_t* out;
   int32_t* dbg_acc;
   float* dbg_tail;
+  const float* add;   // PK: [M, N] tail sums computed elsewhere, or NULL
+  int32_t* C;         // PK: [M, N] the int32 accumulators instead of `out`, or NULL
 };
 
 __device__ __forceinline__ void st_cluster_v4(uint32_t addr, const uint32_t* v) {
@@ -59,11 +71,36 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
-template <int HB>   // 64-wide halves per bf16 slot
-__global__ void __launch_bounds__(ST_THREADS, 1)
+// INT4 -> INT8 (x16) of `rows` rows of 64 packed bytes by 128 threads: staging -> 128-byte-swizzled operand tile
+__device__ __forceinline__ void widen_rows(const unsigned char* src, unsigned char* dst, int rows, int wtid) {
+#pragma unroll 4
+  for (int task = wtid; task < rows * 4; task += 128) {
+    const int row = task >> 2, pc = task & 3;
+    const uint4 w = *reinterpret_cast<const uint4*>(src + row * 64 + pc * 16);
+    unsigned char* drow = dst + (row >> 3) * 1024 + (row & 7) * 128;
+    uint4 lo, hi;
+    lo.x = (w.x << 4) & 0xf0f0f0f0u;
+    lo.y = w.x & 0xf0f0f0f0u;
+    lo.z = (w.y << 4) & 0xf0f0f0f0u;
+    lo.w = w.y & 0xf0f0f0f0u;
+    hi.x = (w.z << 4) & 0xf0f0f0f0u;
+    hi.y = w.z & 0xf0f0f0f0u;
+    hi.z = (w.w << 4) & 0xf0f0f0f0u;
+    hi.w = w.w & 0xf0f0f0f0u;
+    *reinterpret_cast<uint4*>(drow + (((2 * pc) ^ (row & 7)) << 4)) = lo;
+    *reinterpret_cast<uint4*>(drow + (((2 * pc + 1) ^ (row & 7)) << 4)) = hi;
+  }
+}
+
+// HB: 64-wide halves per bf16 slot.  ST_PACKED: `tmap_a8` covers the [M, K/2] packed bytes, and further warps widen the
+// token codes the way the weights are.
+template <int HB, int MODE>
+__global__ void __launch_bounds__(st_threads(MODE), 1)
 stream_gemm_kernel(const __grid_constant__ CUtensorMap tmap_b4, const __grid_constant__ CUtensorMap tmap_w,
                    const __grid_constant__ CUtensorMap tmap_a8, const __grid_constant__ CUtensorMap tmap_tail,
                    const StreamParams p) {
+  constexpr bool PK = MODE == ST_PACKED, has_tail = MODE == ST_TAIL;
+  constexpr int ST_SP = st_sp(MODE), GROUPS = has_tail ? 1 : 2;
   extern __shared__ unsigned char smem_dyn[];
   const uint32_t raw = smem_u32(smem_dyn);
   const uint32_t base = (raw + 1023u) & ~1023u;
@@ -74,7 +111,8 @@ stream_gemm_kernel(const __grid_constant__ CUtensorMap tmap_b4, const __grid_con
   const uint32_t bf_off = (uint32_t)SI * slot_bytes;
   const uint32_t bf_bytes = (uint32_t)HB * slot_bytes;   // [HB][128 rows] weights, then [HB][T rows] tail
   const uint32_t stage_off = bf_off + (uint32_t)SB * bf_bytes;
-  const uint32_t bar_off = stage_off + ST_SP * ST_STAGE;
+  const uint32_t tok_off = stage_off + ST_SP * ST_STAGE;   // PK: token staging buffers, [T rows][64 bytes]
+  const uint32_t bar_off = tok_off + (PK ? (uint32_t)(ST_SP * T * 64) : 0u);
   const uint32_t bars = base + bar_off;
   auto full_p = [&](int s) { return bars + 8u * s; };
   auto empty_p = [&](int s) { return bars + 8u * (ST_SP + s); };
@@ -83,16 +121,17 @@ stream_gemm_kernel(const __grid_constant__ CUtensorMap tmap_b4, const __grid_con
   auto full_b = [&](int s) { return bars + 8u * (2 * ST_SP + 2 * ST_MAX_SLOTS + s); };
   auto empty_b = [&](int s) { return bars + 8u * (2 * ST_SP + 3 * ST_MAX_SLOTS + s); };
   const uint32_t acc_full = bars + 8u * (2 * ST_SP + 4 * ST_MAX_SLOTS);
-  volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(sm + bar_off + 8 * (2 * ST_SP + 4 * ST_MAX_SLOTS + 1));
+  auto full_t = [&](int s) { return acc_full + 8u * (1 + s); };
+  auto empty_t = [&](int s) { return acc_full + 8u * (1 + ST_SP + s); };
+  volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(sm + bar_off + 8 * ST_BARS);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  float* s_sx = reinterpret_cast<float*>(sm + bar_off + 8 * (2 * ST_SP + 4 * ST_MAX_SLOTS + 1) + 16);   // [T]
+  float* s_sx = reinterpret_cast<float*>(sm + bar_off + 8 * ST_BARS + 16);   // [T]
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int S = (int)gridDim.x, rank = (int)blockIdx.x;   // the cluster spans blockIdx.x
   const int nt = (int)blockIdx.y % p.tiles_n, mt = (int)blockIdx.y / p.tiles_n;
   const int kb_total = p.K / 128;
   const int kb0 = rank * kb_total / S, kb1 = (rank + 1) * kb_total / S;
-  const bool has_tail = p.has_tail != 0;
   const uint32_t tmem_cols = 2 * T <= 32 ? 32u : 2 * T <= 64 ? 64u : 2 * T <= 128 ? 128u : 2 * T <= 256 ? 256u : 512u;
 
   if (tid == 0) {
@@ -105,13 +144,18 @@ stream_gemm_kernel(const __grid_constant__ CUtensorMap tmap_b4, const __grid_con
       mbar_init(empty_p(s), 4);
     }
     for (int s = 0; s < SI; ++s) {
-      mbar_init(full_i(s), 4 + 1);   // the widener warps + the token producer
+      mbar_init(full_i(s), PK ? 8 : 4 + 1);   // the widener warps of both operands, or those and the token producer
       mbar_init(empty_i(s), 1);
     }
     for (int s = 0; s < SB; ++s) {
       mbar_init(full_b(s), 2);       // the two producers
       mbar_init(empty_b(s), 1);
     }
+    if (PK)
+      for (int s = 0; s < ST_SP; ++s) {
+        mbar_init(full_t(s), 1);
+        mbar_init(empty_t(s), 4);
+      }
     mbar_init(acc_full, 1);
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -124,6 +168,7 @@ stream_gemm_kernel(const __grid_constant__ CUtensorMap tmap_b4, const __grid_con
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  if (!p.early) pdl_wait();
 
   if (warp == 0) {
     // ------------------------------------------------------------------ packed weights -> staging
@@ -151,6 +196,22 @@ stream_gemm_kernel(const __grid_constant__ CUtensorMap tmap_b4, const __grid_con
         tma_load_3d(base + bf_off + s * bf_bytes, &tmap_w, 0, nt * 128, k, full_b(s));
         if (++s == SB) {
           s = 0;
+          ph ^= 1u;
+        }
+      }
+    }
+  } else if (PK && warp == 3) {
+    // ------------------------------------------------------------------ packed token codes -> staging
+    if (lane == 0) {
+      int sp = 0;
+      uint32_t ph = 1;
+      pdl_wait();
+      for (int kb = kb0; kb < kb1; ++kb) {
+        if (!mbar_wait(empty_t(sp), ph, abort_flag, 0x40000u)) break;
+        mbar_arrive_expect_tx(full_t(sp), (uint32_t)T * 64u);
+        tma_load_2d(base + tok_off + (uint32_t)(sp * T * 64), &tmap_a8, kb * 64, mt * T, full_t(sp));
+        if (++sp == ST_SP) {
+          sp = 0;
           ph ^= 1u;
         }
       }
@@ -245,44 +306,32 @@ stream_gemm_kernel(const __grid_constant__ CUtensorMap tmap_b4, const __grid_con
       if (ok) umma_commit(acc_full);
     }
   } else if (warp >= 4) {
-    // ------------------------------------------------------------------ wideners
-    const int wtid = tid - 128;
-    int sp = 0, s = 0;
+    // ------------------------------------------------------------------ wideners: GROUPS groups of four warps for the
+    // weights, then (ST_PACKED) as many for the token codes; group g takes the slices g, g + GROUPS, ...
+    const int group = ((warp - 4) >> 2) % GROUPS;
+    const bool tokens = PK && warp >= 4 + 4 * GROUPS;
+    const int wtid = tid & 127;
+    int sp = group, s = group;
     uint32_t php = 0, phu = 1;
-    for (int kb = kb0; kb < kb1; ++kb) {
-      if (!mbar_wait(full_p(sp), php, abort_flag, 0x8000u)) break;
+    for (int kb = kb0 + group; kb < kb1; kb += GROUPS) {
+      if (!mbar_wait(tokens ? full_t(sp) : full_p(sp), php, abort_flag, 0x8000u)) break;
       if (!mbar_wait(empty_i(s), phu, abort_flag, 0x10000u)) break;
-      const unsigned char* src = sm + stage_off + sp * ST_STAGE;
-      unsigned char* dst = sm + s * slot_bytes;
-#pragma unroll
-      for (int task = wtid; task < 512; task += 128) {
-        const int row = task >> 2, pc = task & 3;
-        const uint4 w = *reinterpret_cast<const uint4*>(src + row * 64 + pc * 16);
-        unsigned char* drow = dst + (row >> 3) * 1024 + (row & 7) * 128;
-        uint4 lo, hi;
-        lo.x = (w.x << 4) & 0xf0f0f0f0u;
-        lo.y = w.x & 0xf0f0f0f0u;
-        lo.z = (w.y << 4) & 0xf0f0f0f0u;
-        lo.w = w.y & 0xf0f0f0f0u;
-        hi.x = (w.z << 4) & 0xf0f0f0f0u;
-        hi.y = w.z & 0xf0f0f0f0u;
-        hi.z = (w.w << 4) & 0xf0f0f0f0u;
-        hi.w = w.w & 0xf0f0f0f0u;
-        *reinterpret_cast<uint4*>(drow + (((2 * pc) ^ (row & 7)) << 4)) = lo;
-        *reinterpret_cast<uint4*>(drow + (((2 * pc + 1) ^ (row & 7)) << 4)) = hi;
-      }
+      if (tokens)
+        widen_rows(sm + tok_off + sp * T * 64, sm + s * slot_bytes + 16384, T, wtid);
+      else
+        widen_rows(sm + stage_off + sp * ST_STAGE, sm + s * slot_bytes, 128, wtid);
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       __syncwarp();
       if (lane == 0) {
         mbar_arrive(full_i(s));
-        mbar_arrive(empty_p(sp));
+        mbar_arrive(tokens ? empty_t(sp) : empty_p(sp));
       }
-      if (++sp == ST_SP) {
-        sp = 0;
+      if ((sp += GROUPS) >= ST_SP) {
+        sp -= ST_SP;
         php ^= 1u;
       }
-      if (++s == SI) {
-        s = 0;
+      if ((s += GROUPS) >= SI) {
+        s -= SI;
         phu ^= 1u;
       }
     }
@@ -295,11 +344,11 @@ stream_gemm_kernel(const __grid_constant__ CUtensorMap tmap_b4, const __grid_con
   // scales of the rows and of this thread's two channels (its column in the final loop), while the last MMAs run
   const int oc = (tid & 63) * 2, on = nt * 128 + oc;
   float2 sw = make_float2(0.0f, 0.0f), bias = make_float2(0.0f, 0.0f);
-  if (on < p.N) {
+  if (on < p.N && p.sw) {
     sw = *reinterpret_cast<const float2*>(p.sw + on);
     if (p.bias) bias = *reinterpret_cast<const float2*>(p.bias + on);
   }
-  if (warp < 4)
+  if (warp < 4 && p.sx)
     for (int t = tid; t < T; t += 128) s_sx[t] = mt * T + t < p.M ? p.sx[mt * T + t] : 0.0f;
   cluster_sync_all();   // every CTA's MMAs are done: the rings are free
 
@@ -307,7 +356,7 @@ stream_gemm_kernel(const __grid_constant__ CUtensorMap tmap_b4, const __grid_con
   // fp32 (128-bit stores of four rows of a channel: with one word per store the export took 1 us per 16 rows)
   const int TS = ((T + S - 1) / S + 3) & ~3;     // rows per CTA
   const uint32_t half = (uint32_t)(S * TS * 128) * 4u;
-  if (warp >= 4) {
+  if (warp >= 4 && warp < 8) {
     const int ch = (warp & 3) * 32 + lane;
     const uint32_t lane_addr = tmem_base + ((uint32_t)((warp & 3) * 32) << 16);
     const int rows = min(T, p.M - mt * T);   // (rows beyond M are not exported)
@@ -345,7 +394,7 @@ stream_gemm_kernel(const __grid_constant__ CUtensorMap tmap_b4, const __grid_con
   }
 
   // ---- rows [rank TS, (rank + 1) TS) of the tile: a thread takes two channels of four rows
-  for (int i = tid; i < (TS / 4) * 64; i += ST_THREADS) {
+  for (int i = tid; i < (TS / 4) * 64; i += st_threads(MODE)) {
     const int t = rank * TS + (i >> 6) * 4, row0 = mt * T + t;
     if (t >= T || row0 >= p.M || on >= p.N) continue;
     int a[2][4] = {};
@@ -372,18 +421,27 @@ stream_gemm_kernel(const __grid_constant__ CUtensorMap tmap_b4, const __grid_con
     for (int r = 0; r < 4; ++r) {
       const int row = row0 + r;
       if (row >= p.M) break;
+      const size_t o = (size_t)row * p.N + on;
+      const int a0 = a[0][r] >> (PK ? 8 : 4), a1 = a[1][r] >> (PK ? 8 : 4);   // (widened operands carry a factor 16)
+      if (PK && p.C) {
+        *reinterpret_cast<int2*>(p.C + o) = make_int2(a0, a1);
+        continue;
+      }
       const float sx = s_sx[t + r];
-      const int a0 = a[0][r] >> 4, a1 = a[1][r] >> 4;   // (the weights carried a factor 16)
       float d0 = __fmul_rn(__fmul_rn((float)a0, sx), sw.x), d1 = __fmul_rn(__fmul_rn((float)a1, sx), sw.y);
       if (has_tail) {
         d0 = __fadd_rn(d0, f[0][r]);
         d1 = __fadd_rn(d1, f[1][r]);
       }
+      if (PK && p.add) {
+        const float2 f2 = *reinterpret_cast<const float2*>(p.add + o);
+        d0 = __fadd_rn(d0, f2.x);
+        d1 = __fadd_rn(d1, f2.y);
+      }
       if (p.bias) {
         d0 = __fadd_rn(d0, bias.x);
         d1 = __fadd_rn(d1, bias.y);
       }
-      const size_t o = (size_t)row * p.N + on;
       if (p.act)
         p.out[o / 2] = (uint16_t)swiglu_bf16_bits(d0, d1);
       else
@@ -405,7 +463,7 @@ static int stream_active_clusters(int S) {
   if (S <= 1) return sms;
   if (dev < 64 && known[dev][S]) return known[dev][S];
   int n = 0;
-  if (cudaFuncSetAttribute(stream_gemm_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, ST_SMEM) == cudaSuccess) {
+  if (cudaFuncSetAttribute(stream_gemm_kernel<2, ST_TAIL>, cudaFuncAttributeMaxDynamicSharedMemorySize, ST_SMEM) == cudaSuccess) {
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeClusterDimension;
@@ -413,11 +471,11 @@ static int stream_active_clusters(int S) {
     at[0].val.clusterDim.y = 1;
     at[0].val.clusterDim.z = 1;
     cfg.gridDim = dim3((unsigned)S, 1024);
-    cfg.blockDim = dim3(ST_THREADS);
+    cfg.blockDim = dim3(st_threads(ST_TAIL));
     cfg.dynamicSmemBytes = ST_SMEM;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    if (cudaOccupancyMaxActiveClusters(&n, stream_gemm_kernel<2>, &cfg) != cudaSuccess) n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, stream_gemm_kernel<2, ST_TAIL>, &cfg) != cudaSuccess) n = 0;
   }
   cudaGetLastError();
   if (n < 1) n = sms / S > 1 ? sms / S - 1 : 1;
@@ -426,9 +484,9 @@ static int stream_active_clusters(int S) {
 }
 
 // Work split of a call and its estimated time.  The constants are a fit to timings at 8..512 rows of N = 1024..24576,
-// K = 1024..14336 (weights from HBM): a K slice of a tile of T rows takes 0.44 + 0.0024 T us with a tail and 0.36 without
-// (MMA issue and operand loads of one SM), a tile costs 2.4 + 0.045 T us around its main loop (launch, ring fill,
-// accumulator exchange, output), and the weights cannot arrive faster than 5.2 TB/s.
+// K = 1024..14336 (weights from HBM): a K slice of a tile of T rows takes 0.44 + 0.0024 T us with a tail and 0.28 + 0.0006 T
+// without (MMA issue, operand loads and widening of one SM), a tile costs 2.4 + 0.045 T (0.035 T) us around its main loop
+// (launch, ring fill, accumulator exchange, output), and the weights cannot arrive faster than 5.2 TB/s.
 struct StreamPlan {
   int T, tiles_m, tiles_n, S;
   float us;
@@ -441,7 +499,7 @@ static StreamPlan plan_stream(int M, int N, int K, bool tail) {
   const int tm0 = (M + ST_MAX_T - 1) / ST_MAX_T;
   for (int tm = tm0; tm <= tm0 + 2; ++tm) {
     const int T = ((M + tm - 1) / tm + 15) / 16 * 16;
-    const float slice = tail ? 0.44f + 0.0024f * T : 0.36f + 0.0003f * T, around = 2.4f + 0.045f * T;
+    const float slice = tail ? 0.44f + 0.0024f * T : 0.28f + 0.0006f * T, around = 2.4f + (tail ? 0.045f : 0.035f) * T;
     for (int S = 1; S <= 8 && S <= kb; ++S) {
       const int tiles = tm * tiles_n, fit = stream_active_clusters(S), waves = (tiles + fit - 1) / fit;
       const float one = (float)((kb + S - 1) / S) * slice + around + (S > 1 ? 0.8f : 0.0f);
@@ -460,18 +518,38 @@ static StreamPlan plan_stream(int M, int N, int K, bool tail) {
   return best;
 }
 
+template <int HB, int MODE>
+static int launch_stream(const StreamPlan& pl, const StreamParams& p, const CUtensorMap& mb, const CUtensorMap& mw,
+                         const CUtensorMap& ma, const CUtensorMap& mt, cudaStream_t st) {
+  auto kern = stream_gemm_kernel<HB, MODE>;
+  static bool configured[64] = {};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (!(dev < 64 && configured[dev])) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, ST_SMEM);
+    if (e != cudaSuccess) {
+      set_last_cuda_error(e);
+      return TQ_ERR_CUDA;
+    }
+    if (dev < 64) configured[dev] = true;
+  }
+  return launch_pdl(kern, dim3(pl.S, pl.tiles_n * pl.tiles_m), dim3(st_threads(MODE)), (size_t)ST_SMEM, st, pl.S,
+                    mb, mw, ma, mt, p);
+}
+
+// `early`: the kernel in front in the stream is the prologue of this call
 int run_stream_gemm(const int8_t* a_q8, const float* body_scale, const uint8_t* b_col, const float* w_scale,
                     const void* w_rot, const void* tail_dense, int R, const float* bias, void* out_bf16,
-                    int32_t* dbg_acc, float* dbg_tail, int M, int N, int K, int act, cudaStream_t st) {
+                    int32_t* dbg_acc, float* dbg_tail, int M, int N, int K, int act, bool early, cudaStream_t st) {
   const StreamPlan pl = plan_stream(M, N, K, R > 0);
   StreamParams p = {};
   p.M = M;
   p.N = N;
   p.K = K;
   p.T = pl.T;
-  p.has_tail = R > 0 ? 1 : 0;
   p.act = act;
   p.tiles_n = pl.tiles_n;
+  p.early = early ? 1 : 0;
   p.sx = body_scale;
   p.sw = w_scale;
   p.bias = bias;
@@ -481,8 +559,8 @@ int run_stream_gemm(const int8_t* a_q8, const float* body_scale, const uint8_t* 
   // Slots that fit beside the staging buffers: two bf16 slots of a whole slice and two INT8 slots up to 128 rows (half the
   // load instructions and waits), three of half a slice beyond; what is left goes to bf16, then INT8 slots.
   const int slot = (128 + pl.T) * 128;
-  const int fixed = ST_SP * ST_STAGE + 8 * (2 * ST_SP + 4 * ST_MAX_SLOTS + 1) + 16 + 4 * ST_MAX_T + 1024;
-  const int units = (ST_SMEM - fixed) / slot;   // 5 at T = 176, 10 at T = 16
+  const int fixed = st_sp(R > 0 ? ST_TAIL : ST_INT8) * ST_STAGE + 8 * ST_BARS + 16 + 4 * ST_MAX_T + 1024;
+  const int units = (ST_SMEM - fixed) / slot;   // with a tail 5 at T = 176, 10 at T = 16
   int hb = 1;
   if (R > 0) {
     hb = units >= 6 ? 2 : 1;
@@ -490,20 +568,8 @@ int run_stream_gemm(const int8_t* a_q8, const float* body_scale, const uint8_t* 
     p.sb = (units - p.si) / hb;
     if (p.sb > ST_MAX_SLOTS) p.sb = ST_MAX_SLOTS;
   } else {
-    p.si = units < ST_MAX_SLOTS ? units : ST_MAX_SLOTS;
+    p.si = units < ST_MAX_SLOTS ? units & ~1 : ST_MAX_SLOTS;
     p.sb = 0;
-  }
-  auto kern = hb == 2 ? stream_gemm_kernel<2> : stream_gemm_kernel<1>;
-  static bool configured[64][2] = {};
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (!(dev < 64 && configured[dev][hb - 1])) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, ST_SMEM);
-    if (e != cudaSuccess) {
-      set_last_cuda_error(e);
-      return TQ_ERR_CUDA;
-    }
-    if (dev < 64) configured[dev][hb - 1] = true;
   }
   CUtensorMap mb, mw, ma, mt;
   if (!make_tensor_map_2d(&mb, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, b_col, (uint64_t)(K / 2), (uint64_t)N, (uint64_t)(K / 2),
@@ -519,8 +585,38 @@ int run_stream_gemm(const int8_t* a_q8, const float* body_scale, const uint8_t* 
     mw = mb;   // never read
     mt = ma;
   }
-  return launch_pdl(kern, dim3(pl.S, pl.tiles_n * pl.tiles_m), dim3(ST_THREADS), (size_t)ST_SMEM, st, pl.S,
-                    mb, mw, ma, mt, p);
+  if (R == 0) return launch_stream<1, ST_INT8>(pl, p, mb, mw, ma, mt, st);
+  return hb == 2 ? launch_stream<2, ST_TAIL>(pl, p, mb, mw, ma, mt, st) : launch_stream<1, ST_TAIL>(pl, p, mb, mw, ma, mt, st);
+}
+
+// Packed activations and no tail operand: the int32 product into C, or (C == NULL) the dequantised bf16 result with the
+// optional tail sums `add`.
+int run_stream_packed(const uint8_t* a_pack, const uint8_t* b_col, int32_t* C, const float* body_scale, const float* w_scale,
+                      const float* add, const float* bias, void* out_bf16, int M, int N, int K, cudaStream_t st) {
+  const StreamPlan pl = plan_stream(M, N, K, false);
+  StreamParams p = {};
+  p.M = M;
+  p.N = N;
+  p.K = K;
+  p.T = pl.T;
+  p.tiles_n = pl.tiles_n;
+  p.sx = body_scale;
+  p.sw = w_scale;
+  p.bias = bias;
+  p.add = add;
+  p.C = C;
+  p.out = reinterpret_cast<uint16_t*>(out_bf16);
+  const int slot = (128 + pl.T) * 128;
+  const int fixed = st_sp(ST_PACKED) * (ST_STAGE + pl.T * 64) + 8 * ST_BARS + 16 + 4 * ST_MAX_T + 1024;
+  const int units = (ST_SMEM - fixed) / slot;   // 3 at T = 176
+  p.si = units < ST_MAX_SLOTS ? units & ~1 : ST_MAX_SLOTS;
+  CUtensorMap mb, ma;
+  if (!make_tensor_map_2d(&mb, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, b_col, (uint64_t)(K / 2), (uint64_t)N, (uint64_t)(K / 2),
+                          64, 128) ||
+      !make_tensor_map_2d(&ma, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, a_pack, (uint64_t)(K / 2), (uint64_t)M, (uint64_t)(K / 2),
+                          64, pl.T))
+    return TQ_ERR_CUDA;
+  return launch_stream<1, ST_PACKED>(pl, p, mb, mb, ma, ma, st);
 }
 
 }  // namespace tq

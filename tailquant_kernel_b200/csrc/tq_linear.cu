@@ -41,7 +41,8 @@ int linear_prologue(const tq_linear_call& c, const void* x, void* stream) {
                       nullptr, nullptr, nullptr, c.rms_weight, c.rms_eps, (cudaStream_t)stream, TQ_BF16, c.tail_dense);
 }
 
-int linear_compute(const tq_linear_call& c, void* out, void* stream) {
+// `early`: the prologue of this call is the kernel in front
+int linear_compute(const tq_linear_call& c, void* out, bool early, void* stream) {
   if (c.engine == TQ_LINEAR_DECODE) {
     if (!c.a_pack || !c.body_scale || !c.b_col || !c.w_scale || !out || c.M < 0 || c.M > 64 || c.R < 0 || c.R >= c.K)
       return TQ_ERR_BAD_ARG;
@@ -64,6 +65,7 @@ int linear_compute(const tq_linear_call& c, void* out, void* stream) {
     p.R = c.R;
     p.ld = c.tail_ld;
     p.act = c.act;
+    p.early = early ? 1 : 0;
     return run_decode_linear(p, c.tail, (cudaStream_t)stream);
   }
   if (c.engine == TQ_LINEAR_GATHER) {
@@ -77,7 +79,7 @@ int linear_compute(const tq_linear_call& c, void* out, void* stream) {
   if (c.engine != TQ_LINEAR_FUSED) return TQ_ERR_BAD_ARG;
   return run_split_gemm_mma(c.a_q8, c.body_scale, c.b_col, c.w_scale, c.w_rot, c.tail_idx16, c.tail_val, c.tail_ld,
                             c.tail_ptr, c.ptr_ld, c.tail_rec, c.tail_cnt, c.tail_dense, c.R, c.bias, out, nullptr, nullptr,
-                            c.M, c.N, c.K, c.act, stream);
+                            c.M, c.N, c.K, c.act, early, stream);
 }
 
 }  // namespace
@@ -87,7 +89,7 @@ extern "C" int tq_linear_forward(const tq_linear_call* call, const void* x, void
   if (!call) return TQ_ERR_BAD_ARG;
   const tq_linear_call own = tq::linear_own_part(*call);
   const int rc = tq::linear_prologue(own, x, stream);
-  return rc != TQ_OK ? rc : tq::linear_compute(own, out, stream);
+  return rc != TQ_OK ? rc : tq::linear_compute(own, out, true, stream);
 }
 
 extern "C" int tq_linear_prologue(const tq_linear_call* call, const void* x, void* stream) {
@@ -95,5 +97,5 @@ extern "C" int tq_linear_prologue(const tq_linear_call* call, const void* x, voi
 }
 
 extern "C" int tq_linear_compute(const tq_linear_call* call, void* out, void* stream) {
-  return call ? tq::linear_compute(*call, out, stream) : TQ_ERR_BAD_ARG;
+  return call ? tq::linear_compute(*call, out, false, stream) : TQ_ERR_BAD_ARG;
 }

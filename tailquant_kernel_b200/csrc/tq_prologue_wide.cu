@@ -139,13 +139,13 @@ __global__ void __launch_bounds__(K / 16, wide_min_ctas(K)) prologue_wide_kernel
   const int R = p.R;
   const smp my_row = rowbuf + tid * 32;
 
+  pdl_wait();   // the rows may come from the kernel in front
+  pdl_trigger();
   uint4 ga, gb;
-  if (NORM) {   // (a weight: nothing in front of this kernel writes it)
+  if (NORM) {
     ga = __ldg(reinterpret_cast<const uint4*>(p.gamma + 16 * tid));
     gb = __ldg(reinterpret_cast<const uint4*>(p.gamma + 16 * tid + 8));
   }
-  pdl_wait();   // the rows may come from the kernel in front
-  pdl_trigger();
   const uint4* xrow = reinterpret_cast<const uint4*>(p.x + (size_t)blockIdx.x * K + 16 * tid);
   uint4 xa = make_uint4(0u, 0u, 0u, 0u), xb = xa;
   if ((int)blockIdx.x < p.M) {

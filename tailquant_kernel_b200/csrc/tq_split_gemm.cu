@@ -98,15 +98,15 @@ namespace tq {
 
 // Which kernel a call takes: true = tq_gemm_stream.cu (128 channels x up to 176 rows per tile, K split over a cluster),
 // false = tq_gemm_pair.cu (256 x 256 tiles on CTA pairs).  Both estimates are fits to timings on the layer shapes; the
-// pair kernel goes through ceil(tiles / 74) rounds of 1.02 us per K slice with a tail (0.33 without) and about 12 us (16)
-// for the last tile's epilogue, launch and ring fill.  At N = K = 4096 the line lies between 512 and 1000 rows, at
+// pair kernel goes through ceil(tiles / 74) rounds of 1.02 us per K slice with a tail (0.33 without) and about 12 us for the
+// last tile's epilogue, launch and ring fill.  At N = K = 4096 the line lies between 512 and 1000 rows, at
 // N = 24576 between 160 and 200.
 static bool stream_is_faster(int M, int N, int K, int R) {
   if (g_gemm_pair_mode >= 0) return g_gemm_pair_mode == 0;
   if (M <= 64) return true;
   if (M > 1024) return false;
   const int tiles = ((M + 255) / 256) * ((N + 255) / 256), rounds = (tiles + 73) / 74;
-  const float pair = R > 0 ? rounds * (K / 128) * 1.02f + 12.0f : rounds * (K / 128) * 0.33f + 16.0f;
+  const float pair = R > 0 ? rounds * (K / 128) * 1.02f + 12.0f : rounds * (K / 128) * 0.33f + 12.0f;
   return plan_stream(M, N, K, R > 0).us < pair;
 }
 
@@ -115,7 +115,7 @@ static int run_split_gemm_mma(const int8_t* a_q8, const float* body_scale, const
                               const void* tail_val, int tail_ld, const uint16_t* tail_ptr, int ptr_ld,
                               const uint32_t* tail_rec, const uint16_t* tail_cnt, const void* tail_dense, int R,
                               const float* bias, void* out_bf16, int32_t* dbg_acc, float* dbg_tail, int M, int N, int K,
-                              int act, void* stream) {
+                              int act, bool early, void* stream) {
   if (!a_q8 || !body_scale || !b_col || !w_scale || !out_bf16 || M < 0 || N <= 0 || K <= 0 || R < 0 || R >= K)
     return TQ_ERR_BAD_ARG;
   const bool records = tail_idx16 && tail_val && tail_ld >= R && tail_ptr && ptr_ld >= K / 128 + 1 && tail_rec && tail_cnt;
@@ -129,7 +129,7 @@ static int run_split_gemm_mma(const int8_t* a_q8, const float* body_scale, const
   // (the stream kernel reads the tail from the zero-filled matrix, the pair kernel from the records)
   if (R > 0 ? (tail_dense && (!records || stream_is_faster(M, N, K, R))) : stream_is_faster(M, N, K, R))
     return run_stream_gemm(a_q8, body_scale, b_col, w_scale, w_rot, tail_dense, R, bias, out_bf16, dbg_acc, dbg_tail, M, N,
-                           K, act, (cudaStream_t)stream);
+                           K, act, early, (cudaStream_t)stream);
   return run_pair_gemm(a_q8, body_scale, b_col, w_scale, w_rot, tail_idx16, tail_val, tail_ld, tail_ptr, ptr_ld, tail_rec,
                        tail_cnt, tail_dense, R, bias, out_bf16, dbg_acc, dbg_tail, M, N, K, act, (cudaStream_t)stream);
 }
@@ -143,7 +143,7 @@ extern "C" int tq_split_gemm_mma(const int8_t* a_q8, const float* body_scale, co
                                  int32_t* dbg_acc, float* dbg_tail, int M, int N, int K, void* stream) {
   return tq::run_split_gemm_mma(a_q8, body_scale, b_col, w_scale, w_rot, tail_idx16, tail_val, tail_ld, tail_ptr,
                                 ptr_ld, tail_rec, tail_cnt, tail_dense, R, bias, out_bf16, dbg_acc, dbg_tail, M, N, K, 0,
-                                stream);
+                                false, stream);
 }
 
 extern "C" int tq_split_gemm_mma_swiglu(const int8_t* a_q8, const float* body_scale, const uint8_t* b_col,
@@ -153,5 +153,5 @@ extern "C" int tq_split_gemm_mma_swiglu(const int8_t* a_q8, const float* body_sc
                                         int R, const float* bias, void* out_bf16, int M, int N, int K, void* stream) {
   return tq::run_split_gemm_mma(a_q8, body_scale, b_col, w_scale, w_rot, tail_idx16, tail_val, tail_ld, tail_ptr,
                                 ptr_ld, tail_rec, tail_cnt, tail_dense, R, bias, out_bf16, nullptr, nullptr, M, N, K, 1,
-                                stream);
+                                false, stream);
 }

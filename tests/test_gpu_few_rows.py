@@ -82,3 +82,50 @@ def test_layers_on_different_kernels_share_a_prologue(M, ratio):
         ws = first.prologue(x)
         ya, yb = first.compute(ws, M), second.compute(ws, M)
         assert torch.equal(ya, want[a]) and torch.equal(yb, want[b])
+
+
+@pytest.mark.parametrize("M,N,K", [(16, 128, 128), (17, 136, 1152), (112, 4096, 640), (176, 264, 4096), (177, 1000, 2048),
+                                   (256, 4096, 4096), (353, 72, 384), (1000, 520, 12288), (1024, 6144, 256)])
+@pytest.mark.parametrize("fused", [False, True])
+def test_packed_matmul_exact(M, N, K, fused):
+    """INT4 x INT4 products on the kernel that shares the K range of a tile: odd slice counts, tile edges in rows and
+    channels, few slices per CTA; raw accumulators and the dequantised bf16 output, bit for bit."""
+    rng = np.random.default_rng(M + N + K)
+    qa, qw = (rng.integers(-8, 8, size=(r, K)).astype(np.int8) for r in (M, N))
+    acc = O.int_gemm(qa, qw)
+    A, B = (torch.from_numpy(O.pack_s4(q)).cuda() for q in (qa, qw))
+    if not fused:
+        assert np.array_equal(ops.matmul(A, B).cpu().numpy(), acc)
+        return
+    sx, sw = (rng.uniform(0.001, 0.02, r).astype(np.float32) for r in (M, N))
+    out = torch.empty((M, N), dtype=torch.bfloat16, device="cuda")
+    ops.split_gemm_fused(A, torch.from_numpy(sx).cuda(), B, torch.from_numpy(sw).cuda(), out)
+    assert np.array_equal(host(out), O.f32_to_bf16_bits(O.dequant(acc, sx, sw)))
+
+
+@pytest.mark.parametrize("M,N,K,R", [(1, 8, 64, 1), (3, 1032, 512, 16), (2, 72, 512, 17), (5, 136, 4096, 1024), (2, 16, 4096, 1025)])
+def test_t4_sparse_sum_exact(M, N, K, R):
+    """Sparse INT4 sums around the 16-entry groups and the staged 1024 entries, at the extreme codes; and an output that is
+    not 16-byte aligned."""
+    rng = np.random.default_rng(R)
+    qw = rng.integers(-8, 8, size=(N, K)).astype(np.int8)
+    top_q = rng.integers(-8, 8, size=(M, R)).astype(np.int8)
+    qw[0], top_q[0] = -8, -8
+    qw[-1] = 7
+    idx = np.sort(np.argsort(rng.random((M, K)), axis=1)[:, :R], axis=1).astype(np.int32)
+    ts, ws = rng.uniform(0.001, 0.02, M).astype(np.float32), rng.uniform(0.001, 0.02, N).astype(np.float32)
+    sp = O.sparse_int_t4(top_q, idx, qw).astype(np.float32)
+    want = ((sp * ts[:, None]).astype(np.float32) * ws[None, :]).astype(np.float32)
+    g = [torch.from_numpy(a).cuda() for a in (top_q, idx, O.pack_s4(np.ascontiguousarray(qw.T)), ts, ws)]
+    for shift in (0, 1):
+        out = torch.zeros(M * N + shift, dtype=torch.float16, device="cuda")[shift:].view(M, N)
+        ops.sparse_top_write(*g, out)
+        assert np.array_equal(out.cpu().numpy(), want.astype(np.float16))
+
+
+@pytest.mark.parametrize("M,N,K", [(257, 264, 128), (512, 512, 384), (1025, 2056, 512), (1100, 6144, 640)])
+def test_pair_kernel_without_a_tail(M, N, K):
+    """The paired-SM kernel without a tail: one tile or several per pair, fewer and more K slices than the shared epilogue of
+    the last tile needs."""
+    from test_gpu_parity import _run_split_gemm_mma
+    _run_split_gemm_mma(M, N, K, 0, bias=True, cluster=False, pair=1, dense=True)
