@@ -129,3 +129,22 @@ def test_pair_kernel_without_a_tail(M, N, K):
     the last tile needs."""
     from test_gpu_parity import _run_split_gemm_mma
     _run_split_gemm_mma(M, N, K, 0, bias=True, cluster=False, pair=1, dense=True)
+
+
+@pytest.mark.parametrize("M,N,K,R", [(1, 8, 128, 1), (5, 72, 512, 8), (128, 64, 640, 33), (129, 136, 1024, 64), (40, 4096, 4096, 7),
+                                     (300, 2056, 1536, 77), (17, 72, 14336, 3), (9, 16, 2048, 1500)])
+def test_gather_chunk_and_batch_edges(M, N, K, R):
+    """Ascending-order tail sums, bit for bit: one and few weight chunks, a ragged last chunk, batches of eight entries that
+    reach beyond the resident chunks, dense rows, several units of rows per CTA."""
+    rng = np.random.default_rng(M + K + R)
+    idx = np.sort(np.argsort(rng.random((M, K)), axis=1)[:, :R], axis=1).astype(np.int32)
+    idx[0] = np.arange(K - R, K)   # one run at the end of K
+    idx[-1] = np.arange(R)
+    val, w = O.round_bf16(rng.standard_normal((M, R), dtype=np.float32)), O.round_bf16(rng.standard_normal((K, N), dtype=np.float32))
+    want = np.zeros((M, N), np.float32)
+    for r in range(R):  # fp32 fma: the product of two bf16 is exact in fp64, and so is its sum up to one rounding
+        want = (want.astype(np.float64) + val[:, r:r + 1].astype(np.float64) * w[idx[:, r]]).astype(np.float32)
+    out = torch.zeros((M, N), device="cuda")
+    ops.tail_gather(torch.from_numpy(idx.astype(np.uint16).view(np.int16)).cuda(), dev(O.f32_to_bf16_bits(val)),
+                    dev(O.f32_to_bf16_bits(w)), out, R)
+    assert np.array_equal(out.cpu().numpy(), want)
