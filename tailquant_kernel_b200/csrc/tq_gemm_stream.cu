@@ -92,6 +92,34 @@ __device__ __forceinline__ void widen_rows(const unsigned char* src, unsigned ch
   }
 }
 
+__device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&r)[32]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,"
+      "%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};"
+      ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]),
+      "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]), "r"(r[17]), "r"(r[18]),
+      "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]),
+      "r"(r[29]), "r"(r[30]), "r"(r[31])
+      : "memory");
+  asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+}
+
+// INT4 -> INT8 (x16) of one channel's 64 packed bytes (64-byte swizzle: conflict-free) into its lane of tensor memory
+__device__ __forceinline__ void widen_row_tmem(const unsigned char* src, uint32_t taddr, int row) {
+  uint32_t r[32];
+#pragma unroll
+  for (int pc = 0; pc < 4; ++pc) {
+    const uint4 w = *reinterpret_cast<const uint4*>(src + row * 64 + ((pc ^ ((row >> 1) & 3)) << 4));
+    const uint32_t v[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      r[pc * 8 + 2 * i] = (v[i] << 4) & 0xf0f0f0f0u;
+      r[pc * 8 + 2 * i + 1] = v[i] & 0xf0f0f0f0u;
+    }
+  }
+  tmem_st32(taddr, r);
+}
+
 // HB: 64-wide halves per bf16 slot.  ST_PACKED: `tmap_a8` covers the [M, K/2] packed bytes, and further warps widen the
 // token codes the way the weights are.
 template <int HB, int MODE>
@@ -108,7 +136,8 @@ stream_gemm_kernel(const __grid_constant__ CUtensorMap tmap_b4, const __grid_con
 
   const int T = p.T, SI = p.si, SB = p.sb;
   const uint32_t slot_bytes = (uint32_t)(128 + T) * 128u;
-  const uint32_t bf_off = (uint32_t)SI * slot_bytes;
+  const uint32_t i8_bytes = (uint32_t)T * 128u;            // INT8 slots: tokens (the widened weights are in tensor memory)
+  const uint32_t bf_off = (uint32_t)SI * i8_bytes;
   const uint32_t bf_bytes = (uint32_t)HB * slot_bytes;   // [HB][128 rows] weights, then [HB][T rows] tail
   const uint32_t stage_off = bf_off + (uint32_t)SB * bf_bytes;
   const uint32_t tok_off = stage_off + ST_SP * ST_STAGE;   // PK: token staging buffers, [T rows][64 bytes]
@@ -132,7 +161,8 @@ stream_gemm_kernel(const __grid_constant__ CUtensorMap tmap_b4, const __grid_con
   const int nt = (int)blockIdx.y % p.tiles_n, mt = (int)blockIdx.y / p.tiles_n;
   const int kb_total = p.K / 128;
   const int kb0 = rank * kb_total / S, kb1 = (rank + 1) * kb_total / S;
-  const uint32_t tmem_cols = 2 * T <= 32 ? 32u : 2 * T <= 64 ? 64u : 2 * T <= 128 ? 128u : 2 * T <= 256 ? 256u : 512u;
+  const int w_col = has_tail ? 2 * T : T, cols = w_col + 32 * SI;   // accumulators, then the widened weights of the INT8 slots
+  const uint32_t tmem_cols = cols <= 32 ? 32u : cols <= 64 ? 64u : cols <= 128 ? 128u : cols <= 256 ? 256u : 512u;
 
   if (tid == 0) {
     asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tmap_b4)) : "memory");
@@ -228,7 +258,7 @@ stream_gemm_kernel(const __grid_constant__ CUtensorMap tmap_b4, const __grid_con
       for (int k = kb0 * 128; k < kb1 * 128 && ok; k += 128) {
         if (!(ok = mbar_wait(empty_i(si), phi, abort_flag, 0x40000u))) break;
         mbar_arrive_expect_tx(full_i(si), tok);
-        tma_load_2d(base + si * slot_bytes + 16384u, &tmap_a8, k, m0, full_i(si));
+        tma_load_2d(base + si * i8_bytes, &tmap_a8, k, m0, full_i(si));
         if (++si == SI) {
           si = 0;
           phi ^= 1u;
@@ -256,6 +286,8 @@ stream_gemm_kernel(const __grid_constant__ CUtensorMap tmap_b4, const __grid_con
       const uint64_t tok_rows = (uint64_t)(T * 128) >> 4;
       uint32_t phi = 0, phb = 0, acc = 0;
       uint32_t fi = full_i(0), fb = full_b(0);
+      const uint32_t ta0 = tmem_base + (uint32_t)w_col;
+      uint32_t ta = ta0;
       uint64_t di = desc0, db = desc0 + (bf_off >> 4);
       const uint32_t fi_end = full_i(SI), fb_end = full_b(SB);
       constexpr uint32_t TO_EMPTY = 8u * ST_MAX_SLOTS;
@@ -263,16 +295,18 @@ stream_gemm_kernel(const __grid_constant__ CUtensorMap tmap_b4, const __grid_con
       for (int kb = kb0; kb < kb1; ++kb) {
         if (!(ok = mbar_wait(fi, phi, abort_flag, 0x4000u))) break;
         tc_fence_after();
-        umma_i8(tmem_base, di, di + 1024, idesc_i8, acc);
-        umma_i8(tmem_base, di + 2, di + 1026, idesc_i8, 1u);   // 32 bytes of K further: + 2
-        umma_i8(tmem_base, di + 4, di + 1028, idesc_i8, 1u);
-        umma_i8(tmem_base, di + 6, di + 1030, idesc_i8, 1u);
+        umma_i8_ta(tmem_base, ta, di, idesc_i8, acc);
+        umma_i8_ta(tmem_base, ta + 8, di + 2, idesc_i8, 1u);   // 32 bytes of K further: + 8 columns, + 2
+        umma_i8_ta(tmem_base, ta + 16, di + 4, idesc_i8, 1u);
+        umma_i8_ta(tmem_base, ta + 24, di + 6, idesc_i8, 1u);
         umma_commit(fi + TO_EMPTY);
         fi += 8u;
-        di += slot_bytes >> 4;
+        di += i8_bytes >> 4;
+        ta += 32u;
         if (fi == fi_end) {
           fi = full_i(0);
           di = desc0;
+          ta = ta0;
           phi ^= 1u;
         }
         if (has_tail) {
@@ -314,13 +348,17 @@ stream_gemm_kernel(const __grid_constant__ CUtensorMap tmap_b4, const __grid_con
     int sp = group, s = group;
     uint32_t php = 0, phu = 1;
     for (int kb = kb0 + group; kb < kb1; kb += GROUPS) {
-      if (!mbar_wait(tokens ? full_t(sp) : full_p(sp), php, abort_flag, 0x8000u)) break;
-      if (!mbar_wait(empty_i(s), phu, abort_flag, 0x10000u)) break;
-      if (tokens)
-        widen_rows(sm + tok_off + sp * T * 64, sm + s * slot_bytes + 16384, T, wtid);
-      else
-        widen_rows(sm + stage_off + sp * ST_STAGE, sm + s * slot_bytes, 128, wtid);
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      bool ok = mbar_wait(tokens ? full_t(sp) : full_p(sp), php, abort_flag, 0x8000u);
+      ok = ok && mbar_wait(empty_i(s), phu, abort_flag, 0x10000u);
+      if (!__all_sync(0xffffffffu, ok)) break;
+      if (tokens) {
+        widen_rows(sm + tok_off + sp * T * 64, sm + s * i8_bytes, T, wtid);
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      } else {
+        tc_fence_after();
+        widen_row_tmem(sm + stage_off + sp * ST_STAGE, tmem_base + (uint32_t)(w_col + 32 * s) + ((uint32_t)(wtid & 96) << 16), wtid);
+        tc_fence_before();
+      }
       __syncwarp();
       if (lane == 0) {
         mbar_arrive(full_i(s));
@@ -556,24 +594,26 @@ int run_stream_gemm(const int8_t* a_q8, const float* body_scale, const uint8_t* 
   p.out = reinterpret_cast<uint16_t*>(out_bf16);
   p.dbg_acc = dbg_acc;
   p.dbg_tail = dbg_tail;
-  // Slots that fit beside the staging buffers: two bf16 slots of a whole slice and two INT8 slots up to 128 rows (half the
-  // load instructions and waits), three of half a slice beyond; what is left goes to bf16, then INT8 slots.
+  // What fits beside the staging buffers.  With a tail: bf16 slots beside two INT8 slots (of tokens: the widened weights are
+  // in tensor memory), two or more of a whole slice up to 160 rows (half the load instructions and waits), three of half a
+  // slice beyond; what is left goes to INT8 slots.
   const int slot = (128 + pl.T) * 128;
-  const int fixed = st_sp(R > 0 ? ST_TAIL : ST_INT8) * ST_STAGE + 8 * ST_BARS + 16 + 4 * ST_MAX_T + 1024;
-  const int units = (ST_SMEM - fixed) / slot;   // with a tail 5 at T = 176, 10 at T = 16
+  const int room = ST_SMEM - (st_sp(R > 0 ? ST_TAIL : ST_INT8) * ST_STAGE + 8 * ST_BARS + 16 + 4 * ST_MAX_T + 1024);
   int hb = 1;
   if (R > 0) {
-    hb = units >= 6 ? 2 : 1;
-    p.si = units >= 9 ? 3 : 2;
-    p.sb = (units - p.si) / hb;
-    if (p.sb > ST_MAX_SLOTS) p.sb = ST_MAX_SLOTS;
+    const int units = (room - 2 * pl.T * 128) / slot;   // 3 at T = 176, 10 at T = 16
+    hb = units >= 4 ? 2 : 1;
+    p.sb = units / hb < ST_MAX_SLOTS ? units / hb : ST_MAX_SLOTS;
+    p.si = (room - p.sb * hb * slot) / (pl.T * 128);
+    if (p.si > 4) p.si = 4;
   } else {
+    const int units = room / (pl.T * 128);
     p.si = units < ST_MAX_SLOTS ? units & ~1 : ST_MAX_SLOTS;
     p.sb = 0;
   }
   CUtensorMap mb, mw, ma, mt;
   if (!make_tensor_map_2d(&mb, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, b_col, (uint64_t)(K / 2), (uint64_t)N, (uint64_t)(K / 2),
-                          64, 128) ||
+                          64, 128, 64) ||
       !make_tensor_map_2d(&ma, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, a_q8, (uint64_t)K, (uint64_t)M, (uint64_t)K, 128, pl.T,
                           true))
     return TQ_ERR_CUDA;
@@ -606,13 +646,12 @@ int run_stream_packed(const uint8_t* a_pack, const uint8_t* b_col, int32_t* C, c
   p.add = add;
   p.C = C;
   p.out = reinterpret_cast<uint16_t*>(out_bf16);
-  const int slot = (128 + pl.T) * 128;
   const int fixed = st_sp(ST_PACKED) * (ST_STAGE + pl.T * 64) + 8 * ST_BARS + 16 + 4 * ST_MAX_T + 1024;
-  const int units = (ST_SMEM - fixed) / slot;   // 3 at T = 176
+  const int units = (ST_SMEM - fixed) / (pl.T * 128);   // 6 at T = 176
   p.si = units < ST_MAX_SLOTS ? units & ~1 : ST_MAX_SLOTS;
   CUtensorMap mb, ma;
   if (!make_tensor_map_2d(&mb, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, b_col, (uint64_t)(K / 2), (uint64_t)N, (uint64_t)(K / 2),
-                          64, 128) ||
+                          64, 128, 64) ||
       !make_tensor_map_2d(&ma, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, a_pack, (uint64_t)(K / 2), (uint64_t)M, (uint64_t)(K / 2),
                           64, pl.T))
     return TQ_ERR_CUDA;

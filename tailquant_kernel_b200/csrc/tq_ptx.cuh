@@ -93,6 +93,15 @@ __device__ __forceinline__ void umma_i8(uint32_t d_tmem, uint64_t adesc, uint64_
       ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
+// the 128-row operand in tensor memory (row = lane, four codes per 32-bit column)
+__device__ __forceinline__ void umma_i8_ta(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::i8 [%0], [%1], %2, %3, p;\n\t}"
+      ::"r"(d_tmem), "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
 __device__ __forceinline__ void umma_bf16(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
@@ -224,7 +233,7 @@ inline EncodeTiledFn encode_fn() {
 // be 128 bytes); out-of-range parts of a box read as zero.
 inline bool make_tensor_map_2d(CUtensorMap* map, CUtensorMapDataType dt, int esize, const void* ptr,
                                uint64_t inner, uint64_t outer, uint64_t pitch_bytes, int box_inner, int box_outer,
-                               bool swizzle128 = false) {
+                               int swizzle = 0) {  // 64: 64-byte swizzle, true: 128-byte
   EncodeTiledFn fn = encode_fn();
   if (!fn) {
     set_last_error_text("cuTensorMapEncodeTiled is not available from this driver");
@@ -236,7 +245,8 @@ inline bool make_tensor_map_2d(CUtensorMap* map, CUtensorMapDataType dt, int esi
   cuuint32_t estr[2] = {1, 1};
   (void)esize;
   CUresult r = fn(map, dt, 2, const_cast<void*>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                  swizzle128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
+                  swizzle == 64 ? CU_TENSOR_MAP_SWIZZLE_64B
+                                : swizzle ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
                   CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS)
     set_last_error_text("cuTensorMapEncodeTiled rejected a tensor map (base address, pitch or box of an operand)");
