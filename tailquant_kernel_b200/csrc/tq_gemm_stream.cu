@@ -522,9 +522,9 @@ static int stream_active_clusters(int S) {
 }
 
 // Work split of a call and its estimated time.  The constants are a fit to timings at 8..512 rows of N = 1024..24576,
-// K = 1024..14336 (weights from HBM): a K slice of a tile of T rows takes 0.44 + 0.0024 T us with a tail and 0.28 + 0.0006 T
-// without (MMA issue, operand loads and widening of one SM), a tile costs 2.4 + 0.045 T (0.035 T) us around its main loop
-// (launch, ring fill, accumulator exchange, output), and the weights cannot arrive faster than 5.2 TB/s.
+// K = 1024..14336: a K slice of a tile of T rows takes 0.42 + 0.0023 T us with a tail and 0.17 + 0.0005 T without (MMA issue,
+// operand loads and widening of one SM), a tile costs 2.4 + 0.042 T (2 + 0.012 T) us around its main loop (launch, ring
+// fill, accumulator exchange, output), and the weights cannot arrive faster than 5.2 TB/s.
 struct StreamPlan {
   int T, tiles_m, tiles_n, S;
   float us;
@@ -537,13 +537,13 @@ static StreamPlan plan_stream(int M, int N, int K, bool tail) {
   const int tm0 = (M + ST_MAX_T - 1) / ST_MAX_T;
   for (int tm = tm0; tm <= tm0 + 2; ++tm) {
     const int T = ((M + tm - 1) / tm + 15) / 16 * 16;
-    const float slice = tail ? 0.44f + 0.0024f * T : 0.28f + 0.0006f * T, around = 2.4f + (tail ? 0.045f : 0.035f) * T;
+    const float slice = tail ? 0.42f + 0.0023f * T : 0.17f + 0.0005f * T, around = tail ? 2.4f + 0.042f * T : 2.0f + 0.012f * T;
     for (int S = 1; S <= 8 && S <= kb; ++S) {
       const int tiles = tm * tiles_n, fit = stream_active_clusters(S), waves = (tiles + fit - 1) / fit;
       const float one = (float)((kb + S - 1) / S) * slice + around + (S > 1 ? 0.8f : 0.0f);
       float us = waves * one;
       if (us < hbm + waves * around) us = hbm + waves * around;
-      if (waves > 1) us *= 1.2f;
+      if (waves > 1) us *= 1.1f;
       if (us < best.us) {
         best.T = T;
         best.tiles_m = tm;

@@ -98,15 +98,15 @@ namespace tq {
 
 // Which kernel a call takes: true = tq_gemm_stream.cu (128 channels x up to 176 rows per tile, K split over a cluster),
 // false = tq_gemm_pair.cu (256 x 256 tiles on CTA pairs).  Both estimates are fits to timings on the layer shapes; the
-// pair kernel goes through ceil(tiles / 74) rounds of 1.02 us per K slice with a tail (0.33 without) and about 12 us for the
-// last tile's epilogue, launch and ring fill.  At N = K = 4096 the line lies between 512 and 1000 rows, at
-// N = 24576 between 160 and 200.
+// pair kernel goes through ceil(tiles / 74) rounds of 1.02 us per K slice and 5 us with a tail (0.34 and 3.5 without), and
+// takes about 5 us for the launch and ring fill.  At N = K = 4096 the line lies between 700 and 1000 rows, at
+// N = 28672 between 100 and 176.
 static bool stream_is_faster(int M, int N, int K, int R) {
   if (g_gemm_pair_mode >= 0) return g_gemm_pair_mode == 0;
   if (M <= 64) return true;
-  if (M > 1024) return false;
+  if (M > 1024 && R > 0) return false;   // (its dense tail matrix is not worth its memory there)
   const int tiles = ((M + 255) / 256) * ((N + 255) / 256), rounds = (tiles + 73) / 74;
-  const float pair = R > 0 ? rounds * (K / 128) * 1.02f + 12.0f : rounds * (K / 128) * 0.33f + 12.0f;
+  const float pair = R > 0 ? rounds * ((K / 128) * 1.02f + 5.0f) + 5.0f : rounds * ((K / 128) * 0.34f + 3.5f) + 6.0f;
   return plan_stream(M, N, K, R > 0).us < pair;
 }
 
