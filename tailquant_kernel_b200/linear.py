@@ -167,19 +167,23 @@ class SplitLinear:
                                  rms_eps=float(h.get("rms_eps") or 1e-6))
 
     def _use_mma(self, M: int) -> bool:
-        # The decode kernel reads only the M R tail rows it needs, the fused kernels stream all of the bf16 weights: from a
-        # few rows on the second is faster (N = K = 4096, ratio 0.05: 8.8 us against 11.3 at 4 rows, 15.5 against 11.2
-        # at 8; N = 24576: 31 / 52 and 59 / 51; ratio 0.01: 9.2 / 11.2 at 8 rows).  Without a tail the GEMV holds out to 32
-        # rows (N = 24576: 27 us against 35), and narrow projections stay on it up to `small_m`.
+        # The decode kernel reads only the M R tail rows it needs, the fused kernel streams all of the bf16 weights.  Estimates
+        # in us of the whole linear, fits to timings at 1..64 rows of N = 256..28672, K = 4096..14336, R = 0..0.1 K: a start-up
+        # that grows with K, the weight bytes, and in the decode kernel the entries, per 4096 channels (in a kernel of their
+        # own beyond eight rows).  N = K = 4096, R = 205: decode / fused 10.4 / 12.0 at 2 rows, 19.0 / 12.1 at 8; N = 28672:
+        # 39 / 54 at 4, 73 / 54 at 8.
         if self.tail_engine != "mma":
             return False
-        if M > self.small_m:
+        if M > min(self.small_m, 32):
             return True
-        if self.N <= 1024:
-            return False
-        if not self.R:
-            return M > 32
-        return M > 8 or (M > 2 and M * self.R > 0.22 * self.K)
+        N, K, R = self.N, self.K, self.R
+        if not R:  # 7.2 / 7.3 at 16 rows of N = 256, K = 4096; 12.9 / 11.4 at 8, 9.8 / 11.3 at 4 of N = 12288
+            return M > (16 if N <= 4096 and K <= 4096 else 8)
+        wide = max(1.0, N / 4096)
+        decode = 5.9 + 7e-4 * K + 5e-8 * N * K + ((0.3 * M + 0.0038 * M * R) * wide if M <= 8 else
+                                                  3.0 + (0.17 * M + 0.001 * M * R) * wide)
+        fused = 7e-4 * K + max(7.2, 2.7 + 4.1e-7 * N * K) + 0.1 * M
+        return fused < decode
 
     @property
     def N_out(self) -> int:
