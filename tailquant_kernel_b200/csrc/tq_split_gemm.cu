@@ -104,7 +104,8 @@ namespace tq {
 static bool stream_is_faster(int M, int N, int K, int R) {
   if (g_gemm_pair_mode >= 0) return g_gemm_pair_mode == 0;
   if (M <= 64) return true;
-  if (M > 1024 && R > 0) return false;   // (its dense tail matrix is not worth its memory there)
+  // (the zero-filled tail matrix is worth its memory for narrow layers only: 1174 x 1200 x 14336 takes 63 us instead of 120)
+  if (M > 1024 && R > 0 && (long)M * N > (1 << 21)) return false;
   const int tiles = ((M + 255) / 256) * ((N + 255) / 256), rounds = (tiles + 73) / 74;
   const float pair = R > 0 ? rounds * ((K / 128) * 1.02f + 5.0f) + 5.0f : rounds * ((K / 128) * 0.34f + 3.5f) + 6.0f;
   return plan_stream(M, N, K, R > 0).us < pair;

@@ -191,8 +191,10 @@ class SplitLinear:
 
     def _new_workspace(self, M: int, with_pro: bool) -> _Workspace:
         mma = self._use_mma(M)
+        # the row counts for which the GEMM that reads the zero-filled tail matrix can be the faster one
+        dense = M <= 1024 or (M <= 4096 and M * self.N <= 1 << 21)
         return _Workspace(M, self.K, self.N, self.R, self.w.b_col.device, mma, not mma and M <= self.small_m, self.N_out,
-                          with_pro=with_pro, dense=self.w.had_kind == ops.TQ_HAD_BLOCK128 or M <= 1024,
+                          with_pro=with_pro, dense=dense or self.w.had_kind == ops.TQ_HAD_BLOCK128,
                           both=self.tail_engine == "mma" and M <= min(self.small_m, 64))
 
     def workspace(self, M: int) -> _Workspace:

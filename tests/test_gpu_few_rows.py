@@ -57,7 +57,7 @@ def test_decode_linear_exact(M, N, K, kind, ratio):
         assert np.array_equal(host(lin(dev(xb))), ref)
 
 
-@pytest.mark.parametrize("M,N", [(1, 2056), (2, 6152), (3, 2056), (8, 2056), (40, 2056)])
+@pytest.mark.parametrize("M,N", [(1, 2056), (2, 6152), (3, 2056), (8, 2056), (40, 2056), (1100, 136)])
 def test_few_rows_on_wider_layers(M, N):
     """Widths on which the dispatch between the decode and the fused kernels depends on rows x tail entries."""
     from tailquant_kernel_b200 import SplitLinear
