@@ -381,7 +381,7 @@ int run_gemm(const uint8_t* a_pack, const uint8_t* b_col, GemmParams p, cudaStre
     const long t128 = (long)((p.M + 127) / 128) * ((p.N + 127) / 128);
     const float here = tiles256 >= 148 ? (float)((tiles256 + sms - 1) / sms) * (float)(p.K / BK) * 0.8f + 6.0f
                                        : (float)((t128 + sms - 1) / sms) * (float)(p.K / BK) * 0.37f + 6.0f;
-    if (plan_stream(p.M, p.N, p.K, false).us < here)
+    if (plan_stream(p.M, p.N, p.K, ST_PACKED).us < here)
       return run_stream_packed(a_pack, b_col, p.C, p.sx, p.sw, p.tail, p.bias, p.out, p.M, p.N, p.K, st);
   }
   if (tiles256 >= 148) return launch_gemm<256>(a_pack, b_col, p, st);

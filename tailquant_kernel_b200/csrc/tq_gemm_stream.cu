@@ -1,5 +1,6 @@
 // Split GEMM for few and medium row counts (sm_100a): the computation of tq_gemm_pair.cu on tiles of 128 output channels
-// x T token rows (T a multiple of 16, at most 176), the K range of a tile shared by a CLUSTER of S CTAs.
+// x T token rows (T a multiple of 16, at most 176, or 256 for INT8 activations without a tail), the K range of a tile
+// shared by a CLUSTER of S CTAs.
 //
 // What bounds it: up to a few hundred rows every weight byte (N K / 2 packed INT4 + 2 N K bf16) is used for so few rows
 // that the weight stream is the floor, and 256 x 256 or 128 x 256 tiles leave most of the chip without work (32 tiles
@@ -38,7 +39,10 @@ __host__ __device__ constexpr int st_sp(int mode) { return mode == ST_TAIL ? 3 :
 constexpr int ST_MAX_SP = 4;
 constexpr int ST_STAGE = 128 * 64;    // [128 channels][128 k] INT4
 constexpr int ST_MAX_SLOTS = 8;       // slots of either ring
-constexpr int ST_MAX_T = 176;         // rows per tile (the exchange buffer of a tile must fit in the rings)
+// rows per tile: with a tail the exchange buffer (8 bytes per accumulator pair) must fit in the rings, packed tokens need
+// staging buffers besides
+__host__ __device__ constexpr int st_max_t(int mode) { return mode == ST_INT8 ? 256 : 176; }
+constexpr int ST_MAX_T = 256;
 constexpr int ST_SMEM = 222 * 1024;
 constexpr int ST_BARS = 4 * ST_MAX_SP + 4 * ST_MAX_SLOTS + 1;
 
@@ -521,23 +525,24 @@ static int stream_active_clusters(int S) {
   return n;
 }
 
-// Work split of a call and its estimated time.  The constants are a fit to timings at 8..512 rows of N = 1024..24576,
-// K = 1024..14336: a K slice of a tile of T rows takes 0.42 + 0.0023 T us with a tail and 0.17 + 0.0005 T without (MMA issue,
-// operand loads and widening of one SM), a tile costs 2.4 + 0.042 T (2 + 0.012 T) us around its main loop (launch, ring
-// fill, accumulator exchange, output), and the weights cannot arrive faster than 5.2 TB/s.
+// Work split of a call and its estimated time.  The constants are a fit to timings at 16..4000 rows of N = 1024..28672,
+// K = 4096..14336: a K slice of a tile of T rows takes 0.42 + 0.0023 T us with a tail and 0.17 + 0.0005 T without (MMA issue,
+// operand loads and widening of one SM), a tile costs 2.4 + 0.042 T (2 + 0.012 T, and 0.042 for each row beyond 160) us
+// around its main loop (launch, ring fill, accumulator exchange, output), and the weights cannot arrive faster than 5.2 TB/s.
 struct StreamPlan {
   int T, tiles_m, tiles_n, S;
   float us;
 };
-static StreamPlan plan_stream(int M, int N, int K, bool tail) {
+static StreamPlan plan_stream(int M, int N, int K, int mode) {
+  const bool tail = mode == ST_TAIL;
   StreamPlan best = {};
   best.us = 1e30f;
   const int tiles_n = (N + 127) / 128, kb = K / 128;
   const float hbm = (float)N * (float)K * (tail ? 2.5f : 0.5f) / 5.2e6f;
-  const int tm0 = (M + ST_MAX_T - 1) / ST_MAX_T;
-  for (int tm = tm0; tm <= tm0 + 2; ++tm) {
+  const int tm0 = (M + st_max_t(mode) - 1) / st_max_t(mode);
+  for (int tm = tm0; tm <= tm0 + 3; ++tm) {
     const int T = ((M + tm - 1) / tm + 15) / 16 * 16;
-    const float slice = tail ? 0.42f + 0.0023f * T : 0.17f + 0.0005f * T, around = tail ? 2.4f + 0.042f * T : 2.0f + 0.012f * T;
+    const float slice = tail ? 0.42f + 0.0023f * T : 0.17f + 0.0005f * T, around = tail ? 2.4f + 0.042f * T : 2.0f + 0.012f * T + (T > 160 ? 0.042f * (T - 160) : 0.0f);
     for (int S = 1; S <= 8 && S <= kb; ++S) {
       const int tiles = tm * tiles_n, fit = stream_active_clusters(S), waves = (tiles + fit - 1) / fit;
       const float one = (float)((kb + S - 1) / S) * slice + around + (S > 1 ? 0.8f : 0.0f);
@@ -579,7 +584,7 @@ static int launch_stream(const StreamPlan& pl, const StreamParams& p, const CUte
 int run_stream_gemm(const int8_t* a_q8, const float* body_scale, const uint8_t* b_col, const float* w_scale,
                     const void* w_rot, const void* tail_dense, int R, const float* bias, void* out_bf16,
                     int32_t* dbg_acc, float* dbg_tail, int M, int N, int K, int act, bool early, cudaStream_t st) {
-  const StreamPlan pl = plan_stream(M, N, K, R > 0);
+  const StreamPlan pl = plan_stream(M, N, K, R > 0 ? ST_TAIL : ST_INT8);
   StreamParams p = {};
   p.M = M;
   p.N = N;
@@ -633,7 +638,7 @@ int run_stream_gemm(const int8_t* a_q8, const float* body_scale, const uint8_t* 
 // optional tail sums `add`.
 int run_stream_packed(const uint8_t* a_pack, const uint8_t* b_col, int32_t* C, const float* body_scale, const float* w_scale,
                       const float* add, const float* bias, void* out_bf16, int M, int N, int K, cudaStream_t st) {
-  const StreamPlan pl = plan_stream(M, N, K, false);
+  const StreamPlan pl = plan_stream(M, N, K, ST_PACKED);
   StreamParams p = {};
   p.M = M;
   p.N = N;

@@ -108,7 +108,7 @@ static bool stream_is_faster(int M, int N, int K, int R) {
   if (M > 1024 && R > 0 && (long)M * N > (1 << 21)) return false;
   const int tiles = ((M + 255) / 256) * ((N + 255) / 256), rounds = (tiles + 73) / 74;
   const float pair = R > 0 ? rounds * ((K / 128) * 1.02f + 5.0f) + 5.0f : rounds * ((K / 128) * 0.34f + 3.5f) + 6.0f;
-  return plan_stream(M, N, K, R > 0).us < pair;
+  return plan_stream(M, N, K, R > 0 ? ST_TAIL : ST_INT8).us < pair;
 }
 
 static int run_split_gemm_mma(const int8_t* a_q8, const float* body_scale, const uint8_t* b_col,

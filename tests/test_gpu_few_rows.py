@@ -32,7 +32,8 @@ def host(t):
 
 @pytest.mark.parametrize("M,N,K,R", [(16, 128, 256, 13), (17, 136, 512, 26), (64, 1032, 4096, 205), (65, 264, 1024, 0),
                                      (112, 4096, 512, 60), (176, 256, 4096, 205), (177, 264, 2048, 1), (300, 520, 14336, 717),
-                                     (61, 4096, 12288, 615), (353, 128, 1152, 40), (1, 8, 128, 5)])
+                                     (61, 4096, 12288, 615), (353, 128, 1152, 40), (1, 8, 128, 5), (241, 136, 4096, 0), (256, 264, 384, 0),
+                                     (1000, 4096, 512, 0)])
 def test_shared_k_range_gemm(M, N, K, R):
     """128-channel tiles with the K range of a tile shared by a cluster: accumulators exact, tail sums and outputs inside
     the bounds, at row counts around the 16-row steps and the 176-row tile."""
