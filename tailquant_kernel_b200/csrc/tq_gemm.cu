@@ -374,13 +374,13 @@ int run_gemm(const uint8_t* a_pack, const uint8_t* b_col, GemmParams p, cudaStre
   const int sms = current_device_sms();
   // wide tiles when they still fill the machine, narrow ones for small problems / split-K
   const long tiles256 = (long)((p.M + BM - 1) / BM) * ((p.N + 255) / 256) * (p.split_k > 0 ? p.split_k : 1);
-  if (p.mode != MODE_I32_ATOMIC && p.M <= 1024) {
-    // Few and medium row counts: tiles of 128 channels x up to 176 rows with the K range shared by a cluster, where that is
-    // estimated to be faster than this kernel's rounds (0.37 us per K slice of a 128 x 128 tile, 0.8 of a 128 x 256 one).
-    // N = K = 4096: 11.6 us against 18 at 256 rows, 8.3 / 17 at 64; the line is near 600 rows.
+  if (p.mode != MODE_I32_ATOMIC && p.M <= 2048) {
+    // Tiles of 128 channels x up to 176 rows with the K range shared by a cluster, where that is estimated to be faster than
+    // this kernel's rounds (fits: 0.38 us per K slice and 5.2 us per round of 128 x 128 tiles, 0.55 and 7 of 128 x 256 ones).
+    // N = K = 4096: 11.2 us against 18 at 256 rows, 30 / 35 at 1000, 34 / 49 at 1300; N = 8192: the line is near 900 rows.
     const long t128 = (long)((p.M + 127) / 128) * ((p.N + 127) / 128);
-    const float here = tiles256 >= 148 ? (float)((tiles256 + sms - 1) / sms) * (float)(p.K / BK) * 0.8f + 6.0f
-                                       : (float)((t128 + sms - 1) / sms) * (float)(p.K / BK) * 0.37f + 6.0f;
+    const float here = tiles256 >= 148 ? (float)((tiles256 + sms - 1) / sms) * ((float)(p.K / BK) * 0.55f + 7.0f)
+                                       : (float)((t128 + sms - 1) / sms) * ((float)(p.K / BK) * 0.38f + 5.2f);
     if (plan_stream(p.M, p.N, p.K, ST_PACKED).us < here)
       return run_stream_packed(a_pack, b_col, p.C, p.sx, p.sw, p.tail, p.bias, p.out, p.M, p.N, p.K, st);
   }

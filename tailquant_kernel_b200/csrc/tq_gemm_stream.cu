@@ -528,7 +528,8 @@ static int stream_active_clusters(int S) {
 // Work split of a call and its estimated time.  The constants are a fit to timings at 16..4000 rows of N = 1024..28672,
 // K = 4096..14336: a K slice of a tile of T rows takes 0.42 + 0.0023 T us with a tail and 0.17 + 0.0005 T without (MMA issue,
 // operand loads and widening of one SM), a tile costs 2.4 + 0.042 T (2 + 0.012 T, and 0.042 for each row beyond 160) us
-// around its main loop (launch, ring fill, accumulator exchange, output), and the weights cannot arrive faster than 5.2 TB/s.
+// around its main loop (launch, ring fill, accumulator exchange, output); packed tokens take 0.16 + 0.001 T a slice and 1.5 us
+// more around it; and the weights cannot arrive faster than 5.2 TB/s.
 struct StreamPlan {
   int T, tiles_m, tiles_n, S;
   float us;
@@ -542,13 +543,15 @@ static StreamPlan plan_stream(int M, int N, int K, int mode) {
   const int tm0 = (M + st_max_t(mode) - 1) / st_max_t(mode);
   for (int tm = tm0; tm <= tm0 + 3; ++tm) {
     const int T = ((M + tm - 1) / tm + 15) / 16 * 16;
-    const float slice = tail ? 0.42f + 0.0023f * T : 0.17f + 0.0005f * T, around = tail ? 2.4f + 0.042f * T : 2.0f + 0.012f * T + (T > 160 ? 0.042f * (T - 160) : 0.0f);
+    const float slice = tail ? 0.42f + 0.0023f * T : mode == ST_PACKED ? 0.16f + 0.001f * T : 0.17f + 0.0005f * T;
+    const float around = tail ? 2.4f + 0.042f * T
+                              : (mode == ST_PACKED ? 3.5f : 2.0f) + 0.012f * T + (T > 160 ? 0.042f * (T - 160) : 0.0f);
     for (int S = 1; S <= 8 && S <= kb; ++S) {
       const int tiles = tm * tiles_n, fit = stream_active_clusters(S), waves = (tiles + fit - 1) / fit;
       const float one = (float)((kb + S - 1) / S) * slice + around + (S > 1 ? 0.8f : 0.0f);
       float us = waves * one;
       if (us < hbm + waves * around) us = hbm + waves * around;
-      if (waves > 1) us *= 1.1f;
+      if (mode == ST_PACKED ? waves > 2 : waves > 1) us *= mode == ST_PACKED ? 1.05f : 1.1f;
       if (us < best.us) {
         best.T = T;
         best.tiles_m = tm;
