@@ -6,7 +6,7 @@ tools/profile_multimodel_split_components_v34.py:93-272):
     prologue (rotation + select + pack)  ->  tail gather (R > 0)  ->  GEMM with fused dequant,
     tail add and bias.  Rows M <= `small_m` take the decode kernel instead.
 The kernels of a forward are enqueued by one native call (`tq_linear_forward`) on a description that is filled in once
-per row count.  Everything runs on the current CUDA stream out of per-(M) workspaces that are allocated once, so
+per row count, and again when a weight, the bias or the norm was replaced.  Everything runs on the current CUDA stream out of per-(M) workspaces that are allocated once, so
 a forward is capturable in a CUDA graph after its first call, as the reference's benches require
 (tools/bench_hadamard_three_schemes_quarot_dense_sharedqkv_inplace_fusedtopr_v43.py:105-123).
 """
@@ -62,8 +62,9 @@ class _Workspace:
         self.tail = torch.empty((M, N), dtype=torch.float32, device=device) if (R and not mma and (M > 8 or not small)) else None
         self.out = torch.empty((M, N if n_out is None else n_out), dtype=torch.bfloat16, device=device)
         self.engine = _lib.TQ_LINEAR_FUSED if mma else _lib.TQ_LINEAR_DECODE if small else _lib.TQ_LINEAR_GATHER
-        self.call = None   # the native description of a forward out of these buffers, and the prologue outputs it names
+        self.call = None   # the native description of a forward out of these buffers, and what it was filled in from
         self.call_pro = None
+        self.call_src = ()
 
 
 class SplitLinear:
@@ -220,14 +221,28 @@ class SplitLinear:
         if self.R and self.w.w_t is None:
             self.w.w_t = self.w.w_rot.t().contiguous()
 
+    def _described(self, own: _Workspace) -> bool:
+        """Whether `own.call` still names what this layer consists of.  All of it can be replaced between two forwards, and a
+        tensor's storage can move under it (`.data = ...`, offloading): objects and addresses are compared on every call,
+        half a microsecond where filling the description in again takes ten."""
+        w = self.w
+        b, c, r, t, i, g, kind, rank, eps, act, pb, pc, pr, pt, pi, pg = own.call_src
+        return (b is w.b_col and b.data_ptr() == pb and c is w.w_scale and c.data_ptr() == pc
+                and r is w.w_rot and (r is None or r.data_ptr() == pr) and t is w.w_t and (t is None or t.data_ptr() == pt)
+                and i is w.bias and (i is None or i.data_ptr() == pi)
+                and g is self.rms_weight and (g is None or g.data_ptr() == pg)
+                and kind == w.had_kind and rank == self.descending_rank and eps == self.rms_eps and act == self.epilogue)
+
     def _call(self, own: _Workspace, pro: "ops.PrologueOut") -> "_lib.LinearCall":
         """Description of this layer's forward: prologue outputs `pro` (own or another layer's), output side `own`."""
-        if own.call is not None and own.call_pro is pro:
+        if own.call is not None and own.call_pro is pro and self._described(own):
             return own.call
         if own.engine == _lib.TQ_LINEAR_DECODE:
             self.prepare_decode()
         w, p = self.w, ops._ptr
         own.call_pro = pro
+        src = (w.b_col, w.w_scale, w.w_rot, w.w_t, w.bias, self.rms_weight)
+        own.call_src = (*src, w.had_kind, self.descending_rank, self.rms_eps, self.epilogue, *map(p, src))
         own.call = _lib.LinearCall(
             M=own.M, N=self.N, K=self.K, R=self.R, had_kind=w.had_kind, descending_rank=self.descending_rank,
             engine=own.engine, act=1 if self.epilogue == "swiglu" else 0,
@@ -277,7 +292,7 @@ class SplitLinear:
         ws = self._ws.get(M)
         if ws is None:
             ws = self.workspace(M)
-        call = ws.call if ws.call is not None else self._call(ws, ws.pro)
+        call = self._call(ws, ws.pro)
         y = ws.out if self.reuse_output else torch.empty_like(ws.out)
         rc = _lib.load().tq_linear_forward(ctypes.byref(call), x.data_ptr(), y.data_ptr(), ops._stream())
         if rc:

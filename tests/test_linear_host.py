@@ -1,0 +1,86 @@
+"""Host side of `SplitLinear` without a GPU: what the native description of a forward names.  The library is replaced by a
+stand-in that records the descriptions; tensors live on the CPU and only claim to be CUDA tensors."""
+import dataclasses
+
+import pytest
+import torch
+
+from tailquant_kernel_b200 import _lib, ops
+from tailquant_kernel_b200.linear import SplitLinear
+
+FORWARD, PROLOGUE, COMPUTE = "tq_linear_forward", "tq_linear_prologue", "tq_linear_compute"
+
+
+class Claimed(torch.Tensor):
+    """A CPU tensor that passes for a CUDA one (views and copies of it too)."""
+    is_cuda = property(lambda self: True)
+
+
+def claimed(*shape, dtype):
+    return torch.zeros(*shape, dtype=dtype).as_subclass(Claimed)
+
+
+class FakeLibrary:
+    def __init__(self, real):
+        self.real, self.calls = real, []
+
+    def __getattr__(self, name):
+        if name not in (FORWARD, PROLOGUE, COMPUTE):
+            return getattr(self.real, name)
+
+        def record(call, *rest):
+            c = call._obj
+            self.calls.append((name, {f: getattr(c, f) for f, _ in c._fields_}))
+            return 0
+        return record
+
+
+@pytest.fixture
+def fake(monkeypatch):
+    lib = FakeLibrary(_lib.load())
+    monkeypatch.setattr(_lib, "load", lambda: lib)
+    monkeypatch.setattr(ops, "_stream", lambda: 0)
+    return lib
+
+
+def weight(N, K, bias=True):
+    kind = ops.default_had_kind(K)
+    return ops.PreparedWeight(N, K, kind, claimed(N, K // 2, dtype=torch.uint8), claimed(N, dtype=torch.float32),
+                              claimed(K, N, dtype=torch.bfloat16), None, claimed(N, K, dtype=torch.bfloat16),
+                              claimed(N, dtype=torch.float32) if bias else None)
+
+
+def layer(N=256, K=512, **kw):
+    kw.setdefault("rms_weight", claimed(K, dtype=torch.bfloat16))
+    return SplitLinear.from_prepared(weight(N, K), **kw)
+
+
+def _replace(lin, what):
+    if what == "rms_weight":
+        lin.rms_weight = claimed(lin.K, dtype=torch.bfloat16)
+    elif what == "w":
+        lin.w = weight(lin.N, lin.K)
+    elif what == "storage":   # as `.to()` or an offloader moves it: the tensor object stays, its memory does not
+        lin.w.bias.data = torch.ones(lin.N)
+    elif what == "rms_eps":
+        lin.rms_eps = 0.25
+    else:
+        setattr(lin.w, what, torch.clone(getattr(lin.w, what)).as_subclass(Claimed))
+
+
+@pytest.mark.parametrize("what", ["rms_weight", "bias", "b_col", "w_scale", "w_rot", "w_t", "w", "storage", "rms_eps"])
+@pytest.mark.parametrize("M,engine", [(1, "mma"), (20, "mma"), (300, "mma"), (70, "gather")])
+def test_a_replaced_part_is_used_by_the_next_call(fake, what, M, engine):
+    """No call reads the memory of a weight, bias or norm that the layer no longer holds."""
+    lin = layer(tail_engine=engine)
+    x = claimed(M, lin.K, dtype=torch.bfloat16)
+    for run in (lambda: lin(x), lambda: lin.prologue(x), lambda: lin.compute(lin.workspace(M), M)):
+        run()
+        _replace(lin, what)
+        run()
+        c = fake.calls[-1][1]
+        w = lin.w
+        for field, t in (("b_col", w.b_col), ("w_scale", w.w_scale), ("w_rot", w.w_rot), ("w_t", w.w_t), ("bias", w.bias),
+                         ("rms_weight", lin.rms_weight)):
+            assert c[field] == t.data_ptr(), field
+        assert c["rms_eps"] == lin.rms_eps or what != "rms_eps"
