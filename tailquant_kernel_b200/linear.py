@@ -233,12 +233,34 @@ class SplitLinear:
                 and g is self.rms_weight and (g is None or g.data_ptr() == pg)
                 and kind == w.had_kind and rank == self.descending_rank and eps == self.rms_eps and act == self.epilogue)
 
+    def _check_parts(self, engine: int) -> None:
+        """Types, layout and sizes of what a forward reads: the kernels take all of it for granted."""
+        w, N, K = self.w, self.N, self.K
+        ops._check_cuda(w.b_col, "b_col", torch.uint8)
+        ops._check(tuple(w.b_col.shape) == (N, K // 2), "b_col must be [N, K/2]")
+        ops._check_cuda(w.w_scale, "w_scale", torch.float32)
+        ops._check(w.w_scale.numel() >= N, "w_scale must have N elements")
+        if self.R and engine == _lib.TQ_LINEAR_FUSED:
+            ops._check_cuda(w.w_rot, "w_rot", torch.bfloat16)
+            ops._check(tuple(w.w_rot.shape) == (N, K), "w_rot must be [N, K]")
+        elif self.R:
+            ops._check_cuda(w.w_t, "w_t", torch.bfloat16)
+            ops._check(tuple(w.w_t.shape) == (K, N), "w_t must be [K, N]")
+        if w.bias is not None:
+            ops._check_cuda(w.bias, "bias", torch.float32)
+            ops._check(w.bias.numel() >= N, "bias must have N elements")
+        if self.rms_weight is not None:
+            ops._check_cuda(self.rms_weight, "rms_weight", torch.bfloat16)
+            ops._check(self.rms_weight.numel() == K, "rms_weight must have K elements")
+
     def _call(self, own: _Workspace, pro: "ops.PrologueOut") -> "_lib.LinearCall":
         """Description of this layer's forward: prologue outputs `pro` (own or another layer's), output side `own`."""
         if own.call is not None and own.call_pro is pro and self._described(own):
             return own.call
         if own.engine == _lib.TQ_LINEAR_DECODE:
             self.prepare_decode()
+        own.call = None   # (a part that is refused must not leave the former description in force)
+        self._check_parts(own.engine)
         w, p = self.w, ops._ptr
         own.call_pro = pro
         src = (w.b_col, w.w_scale, w.w_rot, w.w_t, w.bias, self.rms_weight)
@@ -275,6 +297,9 @@ class SplitLinear:
         own = self._own_buffers(ws, M)
         if out is None:
             out = own.out
+        else:
+            ops._check_cuda(out, "out", torch.bfloat16)
+            ops._check(out.numel() >= M * self.N_out, "out too small")
         rc = _lib.load().tq_linear_compute(ctypes.byref(self._call(own, ws.pro)), out.data_ptr(), ops._stream())
         if rc:
             _lib.check(rc, self._what(M))

@@ -84,3 +84,39 @@ def test_a_replaced_part_is_used_by_the_next_call(fake, what, M, engine):
                          ("rms_weight", lin.rms_weight)):
             assert c[field] == t.data_ptr(), field
         assert c["rms_eps"] == lin.rms_eps or what != "rms_eps"
+
+
+@pytest.mark.parametrize("M,engine,what,bad", [
+    (1, "mma", "rms_weight", torch.zeros(512, dtype=torch.bfloat16)),   # on the CPU
+    (300, "mma", "rms_weight", claimed(512, dtype=torch.float32)),
+    (300, "mma", "rms_weight", claimed(256, dtype=torch.bfloat16)),
+    (1, "mma", "bias", claimed(256, dtype=torch.float64)),
+    (1, "mma", "bias", claimed(128, dtype=torch.float32)),
+    (300, "mma", "w_rot", claimed(256, 256, dtype=torch.bfloat16)),
+    (300, "mma", "w_rot", claimed(512, 256, dtype=torch.bfloat16).t()),
+    (1, "mma", "w_t", claimed(256, 512, dtype=torch.bfloat16)),
+    (70, "gather", "w_t", claimed(512, 256, dtype=torch.float16)),
+    (70, "gather", "b_col", claimed(256, 128, dtype=torch.uint8)),
+    (70, "gather", "w_scale", claimed(128, dtype=torch.float32))])
+def test_a_part_of_the_wrong_kind_is_refused(fake, M, engine, what, bad):
+    """Wrong device, type, layout or size: an error, and no native call, from the first forward and from a later one."""
+    x = claimed(M, 512, dtype=torch.bfloat16)
+    first, later = layer(tail_engine=engine), layer(tail_engine=engine)
+    later(x)
+    fake.calls.clear()
+    for lin in (first, later):
+        setattr(lin if what == "rms_weight" else lin.w, what, bad)
+        for _ in range(2):
+            with pytest.raises(RuntimeError, match=what):
+                lin(x)
+    assert not fake.calls
+
+
+def test_an_output_of_the_wrong_kind_is_refused(fake):
+    lin = layer()
+    ws = lin.prologue(claimed(9, 512, dtype=torch.bfloat16))
+    fake.calls.clear()
+    for out in (claimed(9, 255, dtype=torch.bfloat16), claimed(9, 256, dtype=torch.float32), torch.zeros(9, 256, dtype=torch.bfloat16)):
+        with pytest.raises(RuntimeError, match="out"):
+            lin.compute(ws, 9, out)
+    assert not fake.calls
