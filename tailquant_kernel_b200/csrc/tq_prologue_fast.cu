@@ -358,7 +358,7 @@ prologue_fast_kernel(const __grid_constant__ CUtensorMap tmap_x, const PrologueP
         const uint4* gp = reinterpret_cast<const uint4*>(p.gamma + 64 * tid);
 #pragma unroll
         for (int c = 0; c < 8; ++c) {
-          const uint4 g4 = __ldg(gp + c);
+          const uint4 g4 = gp[c];
           const uint32_t gw[4] = {g4.x, g4.y, g4.z, g4.w};
 #pragma unroll
           for (int i = 0; i < 4; ++i) {

@@ -143,22 +143,22 @@ __global__ void __launch_bounds__(K / 16, wide_min_ctas(K)) prologue_wide_kernel
   pdl_trigger();
   uint4 ga, gb;
   if (NORM) {
-    ga = __ldg(reinterpret_cast<const uint4*>(p.gamma + 16 * tid));
-    gb = __ldg(reinterpret_cast<const uint4*>(p.gamma + 16 * tid + 8));
+    ga = *reinterpret_cast<const uint4*>(p.gamma + 16 * tid);
+    gb = *reinterpret_cast<const uint4*>(p.gamma + 16 * tid + 8);
   }
   const uint4* xrow = reinterpret_cast<const uint4*>(p.x + (size_t)blockIdx.x * K + 16 * tid);
   uint4 xa = make_uint4(0u, 0u, 0u, 0u), xb = xa;
   if ((int)blockIdx.x < p.M) {
-    xa = ldg_nc_128(xrow);
-    xb = ldg_nc_128(xrow + 1);
+    xa = ldg_na_128(xrow);
+    xb = ldg_na_128(xrow + 1);
   }
 
   for (int m = blockIdx.x; m < p.M; m += gridDim.x) {
     uint32_t w[8] = {xa.x, xa.y, xa.z, xa.w, xb.x, xb.y, xb.z, xb.w};
     if (m + (int)gridDim.x < p.M) {   // the next row, while this one is worked on
       xrow += (size_t)gridDim.x * (K / 8);
-      xa = ldg_nc_128(xrow);
-      xb = ldg_nc_128(xrow + 1);
+      xa = ldg_na_128(xrow);
+      xb = ldg_na_128(xrow + 1);
     }
     for (int i = tid; i < 256; i += NT) hist[i] = 0u;
 

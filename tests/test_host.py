@@ -45,6 +45,19 @@ def test_argument_errors_need_no_gpu():
         _lib.check(-2, "x")
 
 
+def test_kernels_that_start_early_read_coherently():
+    """A kernel that starts under its predecessor (it calls pdl_wait) may read what that one is still writing, where the
+    non-coherent load path is undefined: none of its sources may use it, directly or through `const __restrict__`."""
+    csrc = os.path.join(ROOT, "tailquant_kernel_b200", "csrc")
+    early = 0
+    for name in sorted(os.listdir(csrc)):
+        code = re.sub(r"//[^\n]*", "", open(os.path.join(csrc, name)).read())
+        if name.endswith(".cu") and "pdl_wait()" in code:
+            early += 1
+            assert not re.search(r"__ldg\s*\(|\bldg_nc_\w+|\.global\.nc|__restrict__", code), name
+    assert early >= 4
+
+
 def test_missing_library_fails_loudly(monkeypatch):
     from tailquant_kernel_b200 import _lib
     monkeypatch.setattr(_lib, "_lib", None)
