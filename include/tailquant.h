@@ -311,6 +311,17 @@ typedef struct tq_linear_call {
   void* tail_dense;
   float* tail;
 } tq_linear_call;
+/* Prologue outputs that the workspace of a call should hold, as a sum of these; reads M, N, K, R, had_kind and engine of
+ * `call` only.  shared = 0: what tq_linear_forward of this call reads and writes.  shared = 1: what tq_linear_prologue should
+ * leave for linears of any width (a wide and a narrow layer can be on different kernels; up to 64 rows also on the decode
+ * and on the fused engine).  A fused call takes its kernel by shape AND by what it finds: without tail_dense the CTA pairs,
+ * without the records the other one.  Negative = error code. */
+#define TQ_OUT_PACK 1    /* a_pack */
+#define TQ_OUT_Q8 2      /* a_q8 */
+#define TQ_OUT_LISTS 4   /* tail_idx16, tail_val */
+#define TQ_OUT_RECORDS 8 /* tail_ptr, tail_rec, tail_cnt */
+#define TQ_OUT_DENSE 16  /* tail_dense */
+int tq_linear_outputs(const tq_linear_call* call, int shared);
 int tq_linear_forward(const tq_linear_call* call, const void* x, void* out, void* stream);
 int tq_linear_prologue(const tq_linear_call* call, const void* x, void* stream);
 int tq_linear_compute(const tq_linear_call* call, void* out, void* stream);

@@ -15,6 +15,7 @@ TQ_HAD_NONE, TQ_HAD_WHT, TQ_HAD_KRON12, TQ_HAD_BLOCK128 = 0, 1, 2, 3
 TQ_BF16, TQ_FP16 = 0, 1
 
 TQ_LINEAR_DECODE, TQ_LINEAR_FUSED, TQ_LINEAR_GATHER = 0, 1, 2
+TQ_OUT_PACK, TQ_OUT_Q8, TQ_OUT_LISTS, TQ_OUT_RECORDS, TQ_OUT_DENSE = 1, 2, 4, 8, 16
 
 _P, _I, _F, _LL = C.c_void_p, C.c_int, C.c_float, C.c_longlong
 
@@ -57,6 +58,7 @@ SIGNATURES = {
     "tq_tail_gather_small": [_P, _P, _P, _P, _I, _I, _I, _I, _I, _P],
     "tq_set_gemm_pair_mode": [_I],
     "tq_set_prologue_mode": [_I],
+    "tq_linear_outputs": [_P, _I],
     "tq_linear_forward": [_P, _P, _P, _P],
     "tq_linear_prologue": [_P, _P, _P],
     "tq_linear_compute": [_P, _P, _P],

@@ -7,15 +7,33 @@
 namespace tq {
 namespace {
 
-// The part of a workspace that a forward of this call fills and reads; a prologue on its own fills all of it, since
-// another linear, of another width and hence perhaps on another kernel, may run on it.  The sorted tail lists and the
-// records cost a small call about 3 us, the zero-filled matrix a large one 2 bytes per element.
-//
 // Whether the fused engine of this call runs the stream kernel (which reads the tail from the zero-filled matrix).
 bool linear_streams(const tq_linear_call& c) {
   return c.engine == TQ_LINEAR_FUSED && c.M > 0 && (c.R == 0 || c.tail_dense) && stream_is_faster(c.M, c.N, c.K, c.R);
 }
 
+// Rows beyond which the zero-filled matrix is not kept whatever it would save (layers whose pair kernel reads it excepted).
+constexpr int DENSE_MAX_ROWS = 4096;
+
+// THE rule for the buffers of a workspace (see tailquant.h); which kernel then runs follows from what is there.
+int linear_outputs(const tq_linear_call& c, bool shared) {
+  const bool fused = c.engine == TQ_LINEAR_FUSED;
+  int o = fused ? TQ_OUT_Q8 : TQ_OUT_PACK;
+  const bool few = shared && c.engine != TQ_LINEAR_GATHER && c.M <= 64;   // decode or fused, either may come
+  if (few) o = TQ_OUT_Q8 | TQ_OUT_PACK;
+  if (c.R == 0) return o;
+  const bool pair_dense = c.had_kind == TQ_HAD_BLOCK128;   // (the pair kernel loads long runs from it)
+  if (few) return o | TQ_OUT_LISTS | TQ_OUT_DENSE;
+  if (!fused) return o | TQ_OUT_LISTS;
+  const bool streams = c.M <= DENSE_MAX_ROWS && stream_is_faster(c.M, c.N, c.K, c.R);
+  if (shared || !streams) o |= TQ_OUT_LISTS | TQ_OUT_RECORDS;
+  if (streams || pair_dense || (shared && c.M <= DENSE_ROWS)) o |= TQ_OUT_DENSE;
+  return o;
+}
+
+// The part of a workspace that a forward of this call fills and reads; a prologue on its own fills all of it, since
+// another linear, of another width and hence perhaps on another kernel, may run on it.  The sorted tail lists and the
+// records cost a small call about 3 us, the zero-filled matrix a large one 2 bytes per element.
 tq_linear_call linear_own_part(tq_linear_call c) {
   const bool fused = c.engine == TQ_LINEAR_FUSED, streams = linear_streams(c);
   if (fused)
@@ -84,6 +102,13 @@ int linear_compute(const tq_linear_call& c, void* out, bool early, void* stream)
 
 }  // namespace
 }  // namespace tq
+
+extern "C" int tq_linear_outputs(const tq_linear_call* call, int shared) {
+  if (!call || call->M < 0 || call->N <= 0 || call->K <= 0 || call->R < 0 || call->R >= call->K ||
+      call->engine < TQ_LINEAR_DECODE || call->engine > TQ_LINEAR_GATHER)
+    return TQ_ERR_BAD_ARG;
+  return tq::linear_outputs(*call, shared != 0);
+}
 
 extern "C" int tq_linear_forward(const tq_linear_call* call, const void* x, void* out, void* stream) {
   if (!call) return TQ_ERR_BAD_ARG;

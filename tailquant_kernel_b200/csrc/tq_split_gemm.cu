@@ -96,7 +96,13 @@ extern "C" int tq_set_gemm_pair_mode(int mode) {
 
 namespace tq {
 
-// Which kernel a call takes: true = tq_gemm_stream.cu (128 channels x up to 176 rows per tile, K split over a cluster),
+// The zero-filled tail matrix (2 M K bytes) is worth its memory up to this many rows, and beyond them for narrow layers
+// only, up to this many outputs: 1174 x 1200 x 14336 takes 63 us instead of 120.
+constexpr int DENSE_ROWS = 1024;
+constexpr long DENSE_OUTPUTS = 1 << 21;
+
+// Which kernel a call takes: true = tq_gemm_stream.cu (128 channels x up to 176 rows per tile, 256 without a tail, K
+// split over a cluster),
 // false = tq_gemm_pair.cu (256 x 256 tiles on CTA pairs).  Both estimates are fits to timings on the layer shapes; the
 // pair kernel goes through ceil(tiles / 74) rounds of 1.02 us per K slice and 5 us with a tail (0.34 and 3.5 without), and
 // takes about 5 us for the launch and ring fill.  At N = K = 4096 the line lies between 700 and 1000 rows, at
@@ -104,8 +110,7 @@ namespace tq {
 static bool stream_is_faster(int M, int N, int K, int R) {
   if (g_gemm_pair_mode >= 0) return g_gemm_pair_mode == 0;
   if (M <= 64) return true;
-  // (the zero-filled tail matrix is worth its memory for narrow layers only: 1174 x 1200 x 14336 takes 63 us instead of 120)
-  if (M > 1024 && R > 0 && (long)M * N > (1 << 21)) return false;
+  if (M > DENSE_ROWS && R > 0 && (long)M * N > DENSE_OUTPUTS) return false;
   const int tiles = ((M + 255) / 256) * ((N + 255) / 256), rounds = (tiles + 73) / 74;
   const float pair = R > 0 ? rounds * ((K / 128) * 1.02f + 5.0f) + 5.0f : rounds * ((K / 128) * 0.34f + 3.5f) + 6.0f;
   return plan_stream(M, N, K, R > 0 ? ST_TAIL : ST_INT8).us < pair;

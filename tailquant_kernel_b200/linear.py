@@ -34,34 +34,31 @@ class _Workspace:
     """Buffers of one (layer, M): the prologue outputs (`pro`; absent in the workspace a layer uses when it runs on
     another layer's prologue) and the layer's own output and scratch."""
 
-    def __init__(self, M: int, K: int, N: int, R: int, device, mma: bool, small: bool, n_out: Optional[int] = None,
-                 with_pro: bool = True, dense: bool = False, both: bool = False):
-        """`mma` / `small`: the fused kernels / the decode kernel run on this; `both`: room for the prologue outputs of
-        either, since layers that share one prologue may differ in which one they take (few rows)."""
-        ld = (R + 7) // 8 * 8
-        q8 = mma or both
+    def __init__(self, M: int, N: int, K: int, R: int, device, engine: int, n_out: int, outputs: Optional[int]):
+        """`outputs`: the prologue outputs to hold (TQ_OUT_* bits; None: another layer's are used)."""
         empty = lambda shape, dtype: torch.empty(shape, dtype=dtype, device=device)  # noqa: E731
-        half_slices = (2 * ((M + 255) // 256), K // 64, 128)
-        self.M, self.K, self.R = M, K, R
-        self.pro = None if not with_pro else ops.PrologueOut(
-            a_pack=None if mma and not both else empty((M, K // 2), torch.uint8),
-            a_q8=empty((M, K), torch.int8) if q8 else None,
-            # what the pair kernel reads (few rows never take it)
-            tail_ptr=empty((M, K // 128 + 1), torch.int16) if (mma and not both and R) else None,
-            tail_rec=empty((*half_slices, ops.TAIL_REC_CAP), torch.int32) if (mma and not both and R) else None,
-            tail_cnt=torch.zeros(half_slices, dtype=torch.int16, device=device) if (mma and not both and R) else None,
-            body_scale=empty(M, torch.float32),
-            top_scale=empty(M, torch.float32),
-            tail_idx=torch.zeros((M, ld), dtype=torch.int16, device=device) if R else None,
-            tail_val=torch.zeros((M, ld), dtype=torch.bfloat16, device=device) if R else None,
-            # the operand of the kernel for few and medium row counts; and block-diagonal rotations leave the tail
-            # concentrated in a few 128-blocks: the pair kernel then loads whole operand rows of this matrix instead
-            # of walking long runs entry by entry
-            tail_dense=empty((M, K), torch.bfloat16) if (dense and q8 and R) else None,
-            R=R)
-        self.tail = torch.empty((M, N), dtype=torch.float32, device=device) if (R and not mma and (M > 8 or not small)) else None
-        self.out = torch.empty((M, N if n_out is None else n_out), dtype=torch.bfloat16, device=device)
-        self.engine = _lib.TQ_LINEAR_FUSED if mma else _lib.TQ_LINEAR_DECODE if small else _lib.TQ_LINEAR_GATHER
+        self.M, self.K, self.R, self.engine = M, K, R, engine
+        self.pro = None
+        if outputs is not None:
+            q8, lists, records = (outputs & b for b in (_lib.TQ_OUT_Q8, _lib.TQ_OUT_LISTS, _lib.TQ_OUT_RECORDS))
+            ld = (R + 7) // 8 * 8
+            half_slices = (2 * ((M + 255) // 256), K // 64, 128)
+            self.pro = ops.PrologueOut(
+                a_pack=empty((M, K // 2), torch.uint8) if outputs & _lib.TQ_OUT_PACK else None,
+                a_q8=empty((M, K), torch.int8) if q8 else None,
+                tail_ptr=empty((M, K // 128 + 1), torch.int16) if records else None,
+                tail_rec=empty((*half_slices, ops.TAIL_REC_CAP), torch.int32) if records else None,
+                tail_cnt=torch.zeros(half_slices, dtype=torch.int16, device=device) if records else None,
+                body_scale=empty(M, torch.float32),
+                top_scale=empty(M, torch.float32),
+                tail_idx=torch.zeros((M, ld), dtype=torch.int16, device=device) if lists else None,
+                tail_val=torch.zeros((M, ld), dtype=torch.bfloat16, device=device) if lists else None,
+                tail_dense=empty((M, K), torch.bfloat16) if outputs & _lib.TQ_OUT_DENSE else None,
+                R=R)
+        # sums of a tail kernel of its own (the decode kernel makes them itself up to eight rows)
+        apart = R and (engine == _lib.TQ_LINEAR_GATHER or (engine == _lib.TQ_LINEAR_DECODE and M > 8))
+        self.tail = empty((M, N), torch.float32) if apart else None
+        self.out = empty((M, n_out), torch.bfloat16)
         self.call = None   # the native description of a forward out of these buffers, and what it was filled in from
         self.call_pro = None
         self.call_src = ()
@@ -190,13 +187,23 @@ class SplitLinear:
     def N_out(self) -> int:
         return self.N // 2 if self.epilogue == "swiglu" else self.N
 
+    def _engine(self, M: int) -> int:
+        if self._use_mma(M):
+            return _lib.TQ_LINEAR_FUSED
+        return _lib.TQ_LINEAR_DECODE if M <= self.small_m else _lib.TQ_LINEAR_GATHER
+
+    def _outputs(self, M: int, engine: int) -> int:
+        """Prologue outputs to keep for `M` rows.  A layer with the exact-order engine only shares with its like."""
+        c = _lib.LinearCall(M=M, N=self.N, K=self.K, R=self.R, had_kind=self.w.had_kind, engine=engine)
+        bits = _lib.load().tq_linear_outputs(ctypes.byref(c), int(self.tail_engine == "mma"))
+        if bits < 0:
+            _lib.check(bits, self._what(M))
+        return bits
+
     def _new_workspace(self, M: int, with_pro: bool) -> _Workspace:
-        mma = self._use_mma(M)
-        # the row counts for which the GEMM that reads the zero-filled tail matrix can be the faster one
-        dense = M <= 1024 or (M <= 4096 and M * self.N <= 1 << 21)
-        return _Workspace(M, self.K, self.N, self.R, self.w.b_col.device, mma, not mma and M <= self.small_m, self.N_out,
-                          with_pro=with_pro, dense=dense or self.w.had_kind == ops.TQ_HAD_BLOCK128,
-                          both=self.tail_engine == "mma" and M <= min(self.small_m, 64))
+        engine = self._engine(M)
+        return _Workspace(M, self.N, self.K, self.R, self.w.b_col.device, engine, self.N_out,
+                          self._outputs(M, engine) if with_pro else None)
 
     def workspace(self, M: int) -> _Workspace:
         ws = self._ws.get(M)

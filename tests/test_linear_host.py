@@ -120,3 +120,66 @@ def test_an_output_of_the_wrong_kind_is_refused(fake):
         with pytest.raises(RuntimeError, match="out"):
             lin.compute(ws, 9, out)
     assert not fake.calls
+
+
+def _held(pro):
+    bits = {_lib.TQ_OUT_PACK: [pro.a_pack], _lib.TQ_OUT_Q8: [pro.a_q8], _lib.TQ_OUT_LISTS: [pro.tail_idx, pro.tail_val],
+            _lib.TQ_OUT_RECORDS: [pro.tail_ptr, pro.tail_rec, pro.tail_cnt], _lib.TQ_OUT_DENSE: [pro.tail_dense]}
+    for b, ts in bits.items():
+        assert len({t is None for t in ts}) == 1, b
+    return sum(b for b, ts in bits.items() if ts[0] is not None)
+
+
+def _asked(M, N, K, R, kind, engine, shared):
+    import ctypes
+    call = _lib.LinearCall(M=M, N=N, K=K, R=R, had_kind=kind, engine=engine)
+    return _lib.load().tq_linear_outputs(ctypes.byref(call), shared)
+
+
+@pytest.mark.parametrize("R", [0, 26])
+@pytest.mark.parametrize("kind,K", [(1, 512), (3, 2048)])
+@pytest.mark.parametrize("M", [0, 1, 8, 33, 64, 65, 300, 1024, 1025, 1100, 4096, 4097, 9000])
+def test_buffers_of_a_prologue_serve_every_width(M, kind, K, R):
+    """Whichever kernel a linear on shared prologue outputs would take on its own, it finds that kernel's operands, or (the
+    zero-filled matrix of many rows, kept by narrow layers only) those of the other fused kernel."""
+    fused, decode = _lib.TQ_LINEAR_FUSED, _lib.TQ_LINEAR_DECODE
+    for n in (8, 136, 1024, 28672):
+        held = [_asked(M, n, K, R, kind, e, 1) for e in ((fused, decode) if M <= 64 else (fused,))]
+        for h in held:
+            for other in (8, 136, 1024, 28672):
+                need = _asked(M, other, K, R, kind, fused, 0)
+                if M > 1024 and R:
+                    need = need & ~_lib.TQ_OUT_DENSE | (need & _lib.TQ_OUT_DENSE and _lib.TQ_OUT_LISTS | _lib.TQ_OUT_RECORDS)
+                assert need & ~h == 0, (n, other)
+                if M <= 64:
+                    assert _asked(M, other, K, R, kind, decode, 0) & ~h == 0
+            if kind == 3 and R:
+                assert h & _lib.TQ_OUT_DENSE   # long runs of the block rotation
+
+
+@pytest.mark.parametrize("mode", [-1, 0, 1])
+@pytest.mark.parametrize("M", [1, 20, 64, 100, 1000, 1500, 5000])
+def test_workspaces_hold_what_the_library_asks_for(fake, M, mode):
+    ops.set_gemm_pair_mode(mode)
+    try:
+        for lin in (layer(), layer(N=24576, K=512, rms_weight=None), layer(ratio=0.0), layer(K=2048), layer(tail_engine="gather")):
+            ws = lin.workspace(M)
+            assert _held(ws.pro) == _asked(M, lin.N, lin.K, lin.R, lin.w.had_kind, ws.engine, int(lin.tail_engine == "mma"))
+    finally:
+        ops.set_gemm_pair_mode(-1)
+
+
+def test_what_a_forward_alone_reads():
+    """One format of the codes, and the tail in the one form that the kernel of this shape reads."""
+    P, Q, L, T, D = _lib.TQ_OUT_PACK, _lib.TQ_OUT_Q8, _lib.TQ_OUT_LISTS, _lib.TQ_OUT_RECORDS, _lib.TQ_OUT_DENSE
+    decode, fused, gather = _lib.TQ_LINEAR_DECODE, _lib.TQ_LINEAR_FUSED, _lib.TQ_LINEAR_GATHER
+    assert _asked(4, 4096, 4096, 205, 1, decode, 0) == P | L
+    assert _asked(4, 4096, 4096, 0, 1, decode, 0) == P
+    assert _asked(300, 4096, 4096, 205, 1, gather, 0) == P | L
+    assert _asked(40, 4096, 4096, 205, 1, fused, 0) == Q | D       # 128-channel tiles
+    assert _asked(1000, 28672, 4096, 205, 1, fused, 0) == Q | L | T   # CTA pairs
+    assert _asked(1000, 28672, 14336, 717, 3, fused, 0) == Q | L | T | D
+    assert _asked(1000, 28672, 4096, 0, 1, fused, 0) == Q
+    assert _asked(1200, 1200, 14336, 717, 1, fused, 0) == Q | D
+    assert _asked(9000, 136, 4096, 205, 1, fused, 0) == Q | L | T
+    assert _asked(4, 4096, 4096, 4096, 1, fused, 0) == -1 and _asked(4, 4096, 4096, 5, 1, 3, 0) == -1
