@@ -13,6 +13,7 @@ a forward is capturable in a CUDA graph after its first call, as the reference's
 from __future__ import annotations
 
 import ctypes
+import dataclasses
 import weakref
 from collections import OrderedDict
 from typing import Dict, Optional, Tuple
@@ -32,29 +33,17 @@ def interleave_gate_up(w_gate: torch.Tensor, w_up: torch.Tensor) -> torch.Tensor
 
 class _Workspace:
     """Buffers of one (layer, M): the prologue outputs (`pro`; absent in the workspace a layer uses when it runs on
-    another layer's prologue) and the layer's own output and scratch."""
+    another layer's prologue) and the layer's own output and scratch.  They stay for as long as the layer does and are
+    only ever added to, since captured graphs name them: a row count that is seen once costs what its forward reads."""
 
-    def __init__(self, M: int, N: int, K: int, R: int, device, engine: int, n_out: int, outputs: Optional[int]):
-        """`outputs`: the prologue outputs to hold (TQ_OUT_* bits; None: another layer's are used)."""
+    def __init__(self, M: int, N: int, K: int, R: int, device, engine: int, n_out: int, with_pro: bool):
         empty = lambda shape, dtype: torch.empty(shape, dtype=dtype, device=device)  # noqa: E731
         self.M, self.K, self.R, self.engine = M, K, R, engine
         self.pro = None
-        if outputs is not None:
-            q8, lists, records = (outputs & b for b in (_lib.TQ_OUT_Q8, _lib.TQ_OUT_LISTS, _lib.TQ_OUT_RECORDS))
-            ld = (R + 7) // 8 * 8
-            half_slices = (2 * ((M + 255) // 256), K // 64, 128)
-            self.pro = ops.PrologueOut(
-                a_pack=empty((M, K // 2), torch.uint8) if outputs & _lib.TQ_OUT_PACK else None,
-                a_q8=empty((M, K), torch.int8) if q8 else None,
-                tail_ptr=empty((M, K // 128 + 1), torch.int16) if records else None,
-                tail_rec=empty((*half_slices, ops.TAIL_REC_CAP), torch.int32) if records else None,
-                tail_cnt=torch.zeros(half_slices, dtype=torch.int16, device=device) if records else None,
-                body_scale=empty(M, torch.float32),
-                top_scale=empty(M, torch.float32),
-                tail_idx=torch.zeros((M, ld), dtype=torch.int16, device=device) if lists else None,
-                tail_val=torch.zeros((M, ld), dtype=torch.bfloat16, device=device) if lists else None,
-                tail_dense=empty((M, K), torch.bfloat16) if outputs & _lib.TQ_OUT_DENSE else None,
-                R=R)
+        self.outputs, self.asked = 0, (-1, -1)   # TQ_OUT_* bits held; for what (see SplitLinear._provide)
+        if with_pro:
+            self.pro = ops.PrologueOut(a_pack=None, body_scale=empty(M, torch.float32), top_scale=empty(M, torch.float32),
+                                       tail_idx=None, tail_val=None, R=R)
         # sums of a tail kernel of its own (the decode kernel makes them itself up to eight rows)
         apart = R and (engine == _lib.TQ_LINEAR_GATHER or (engine == _lib.TQ_LINEAR_DECODE and M > 8))
         self.tail = empty((M, N), torch.float32) if apart else None
@@ -62,6 +51,30 @@ class _Workspace:
         self.call = None   # the native description of a forward out of these buffers, and what it was filled in from
         self.call_pro = None
         self.call_src = ()
+
+    def hold(self, outputs: int) -> None:
+        """Adds the prologue outputs of `outputs` (TQ_OUT_* bits) that are not there yet."""
+        new = outputs & ~self.outputs
+        if not new:
+            return
+        p = self.pro = dataclasses.replace(self.pro)   # (descriptions that name the old one are filled in again)
+        M, K, R, device = self.M, self.K, self.R, self.out.device
+        empty = lambda shape, dtype: torch.empty(shape, dtype=dtype, device=device)  # noqa: E731
+        if new & _lib.TQ_OUT_PACK:
+            p.a_pack = empty((M, K // 2), torch.uint8)
+        if new & _lib.TQ_OUT_Q8:
+            p.a_q8 = empty((M, K), torch.int8)
+        if new & _lib.TQ_OUT_LISTS:
+            p.tail_idx = torch.zeros((M, (R + 7) // 8 * 8), dtype=torch.int16, device=device)
+            p.tail_val = torch.zeros((M, (R + 7) // 8 * 8), dtype=torch.bfloat16, device=device)
+        if new & _lib.TQ_OUT_RECORDS:
+            half_slices = (2 * ((M + 255) // 256), K // 64, 128)
+            p.tail_ptr = empty((M, K // 128 + 1), torch.int16)
+            p.tail_rec = empty((*half_slices, ops.TAIL_REC_CAP), torch.int32)
+            p.tail_cnt = torch.zeros(half_slices, dtype=torch.int16, device=device)
+        if new & _lib.TQ_OUT_DENSE:
+            p.tail_dense = empty((M, K), torch.bfloat16)
+        self.outputs |= new
 
 
 class SplitLinear:
@@ -192,24 +205,30 @@ class SplitLinear:
             return _lib.TQ_LINEAR_FUSED
         return _lib.TQ_LINEAR_DECODE if M <= self.small_m else _lib.TQ_LINEAR_GATHER
 
-    def _outputs(self, M: int, engine: int) -> int:
-        """Prologue outputs to keep for `M` rows.  A layer with the exact-order engine only shares with its like."""
-        c = _lib.LinearCall(M=M, N=self.N, K=self.K, R=self.R, had_kind=self.w.had_kind, engine=engine)
-        bits = _lib.load().tq_linear_outputs(ctypes.byref(c), int(self.tail_engine == "mma"))
+    def _provide(self, ws: _Workspace, shared: bool) -> None:
+        """Has `ws` hold what this layer's forward reads, or with `shared` what any layer on the same prologue may read (a
+        layer with the exact-order engine only shares with its like).  Asked once, and again under another forced kernel."""
+        c = _lib.LinearCall(M=ws.M, N=self.N, K=self.K, R=self.R, had_kind=self.w.had_kind, engine=ws.engine)
+        bits = _lib.load().tq_linear_outputs(ctypes.byref(c), int(shared and self.tail_engine == "mma"))
         if bits < 0:
-            _lib.check(bits, self._what(M))
-        return bits
+            _lib.check(bits, self._what(ws.M))
+        ws.hold(bits)
+        ws.asked = (ops.gemm_pair_mode_changes, int(shared))
 
     def _new_workspace(self, M: int, with_pro: bool) -> _Workspace:
-        engine = self._engine(M)
-        return _Workspace(M, self.N, self.K, self.R, self.w.b_col.device, engine, self.N_out,
-                          self._outputs(M, engine) if with_pro else None)
+        return _Workspace(M, self.N, self.K, self.R, self.w.b_col.device, self._engine(M), self.N_out, with_pro)
 
-    def workspace(self, M: int) -> _Workspace:
+    def _workspace(self, M: int, shared: bool) -> _Workspace:
         ws = self._ws.get(M)
         if ws is None:
             ws = self._ws[M] = self._new_workspace(M, True)
+        if ws.asked[0] != ops.gemm_pair_mode_changes or shared > ws.asked[1]:
+            self._provide(ws, shared or ws.asked[1] > 0)
         return ws
+
+    def workspace(self, M: int) -> _Workspace:
+        """The buffers for `M` rows, with room for every prologue output that a layer on them may read."""
+        return self._workspace(M, True)
 
     def _own_buffers(self, ws: _Workspace, M: int) -> _Workspace:
         """Output and scratch of THIS layer for a prologue workspace that may belong to another layer."""
@@ -321,9 +340,7 @@ class SplitLinear:
         if not x.is_cuda:
             raise RuntimeError("x must be a CUDA tensor")
         M = x.numel() // self.K
-        ws = self._ws.get(M)
-        if ws is None:
-            ws = self.workspace(M)
+        ws = self._workspace(M, False)
         call = self._call(ws, ws.pro)
         y = ws.out if self.reuse_output else torch.empty_like(ws.out)
         rc = _lib.load().tq_linear_forward(ctypes.byref(call), x.data_ptr(), y.data_ptr(), ops._stream())

@@ -348,10 +348,15 @@ def split_gemm_mma(a_q8, body_scale, B_pack, w_scale, out, w_rot=None, pro: Opti
     return out
 
 
+gemm_pair_mode_changes = 0  # of the kernel of split_gemm_mma: operands that were chosen before one are asked for again
+
+
 def set_gemm_pair_mode(mode: int) -> None:
     """-1: split_gemm_mma picks its kernel by problem size; 0: 128-channel tiles with the K range shared by a cluster,
     wherever that kernel can run (with a tail it needs `tail_dense`); 1: CTA pairs (256 x 256 tiles)."""
+    global gemm_pair_mode_changes
     _lib.check(_lib.load().tq_set_gemm_pair_mode(int(mode)), "set_gemm_pair_mode")
+    gemm_pair_mode_changes += 1
 
 
 def set_gemv_channel_tiles(tiles: int) -> None:

@@ -169,6 +169,39 @@ def test_workspaces_hold_what_the_library_asks_for(fake, M, mode):
         ops.set_gemm_pair_mode(-1)
 
 
+@pytest.mark.parametrize("M", [1, 20, 64, 200, 1000, 1500])
+def test_a_forward_allocates_what_it_reads(fake, M):
+    """No operand of a kernel or a format that the call does not take; what a shared prologue needs beside it comes with the
+    first one, and leaves the buffers that a captured graph may name where they are."""
+    for lin in (layer(), layer(N=24576, K=512, rms_weight=None), layer(ratio=0.0), layer(K=2048), layer(tail_engine="gather")):
+        x = claimed(M, lin.K, dtype=torch.bfloat16)
+        lin(x)
+        ws = lin._ws[M]
+        assert _held(ws.pro) == _asked(M, lin.N, lin.K, lin.R, lin.w.had_kind, ws.engine, 0)
+        before = {f.name: getattr(ws.pro, f.name) for f in dataclasses.fields(ws.pro)}
+        assert lin.prologue(x) is ws
+        assert _held(ws.pro) == _asked(M, lin.N, lin.K, lin.R, lin.w.had_kind, ws.engine, int(lin.tail_engine == "mma"))
+        assert all(v is None or getattr(ws.pro, n) is v for n, v in before.items())
+        name, c = fake.calls[-1]
+        assert name == PROLOGUE and c["a_q8"] == (ws.pro.a_q8.data_ptr() if ws.pro.a_q8 is not None else None)
+        assert c["tail_dense"] == (ws.pro.tail_dense.data_ptr() if ws.pro.tail_dense is not None else None)
+        lin(x)
+        assert lin._ws[M] is ws and _held(ws.pro) == ws.outputs
+
+
+def test_a_forced_kernel_finds_its_operands(fake):
+    lin = layer()
+    x = claimed(300, lin.K, dtype=torch.bfloat16)
+    lin(x)
+    assert not lin._ws[300].outputs & _lib.TQ_OUT_RECORDS
+    ops.set_gemm_pair_mode(1)
+    try:
+        lin(x)
+    finally:
+        ops.set_gemm_pair_mode(-1)
+    assert lin._ws[300].outputs & _lib.TQ_OUT_RECORDS and fake.calls[-1][1]["tail_rec"]
+
+
 def test_what_a_forward_alone_reads():
     """One format of the codes, and the tail in the one form that the kernel of this shape reads."""
     P, Q, L, T, D = _lib.TQ_OUT_PACK, _lib.TQ_OUT_Q8, _lib.TQ_OUT_LISTS, _lib.TQ_OUT_RECORDS, _lib.TQ_OUT_DENSE
