@@ -36,7 +36,8 @@ class _Workspace:
     another layer's prologue) and the layer's own output and scratch.  They stay for as long as the layer does and are
     only ever added to, since captured graphs name them: a row count that is seen once costs what its forward reads."""
 
-    def __init__(self, M: int, N: int, K: int, R: int, device, engine: int, n_out: int, with_pro: bool):
+    def __init__(self, M: int, N: int, K: int, R: int, device, engine: int, n_out: int, with_pro: bool,
+                 with_tail: bool):
         empty = lambda shape, dtype: torch.empty(shape, dtype=dtype, device=device)  # noqa: E731
         self.M, self.K, self.R, self.engine = M, K, R, engine
         self.pro = None
@@ -44,9 +45,7 @@ class _Workspace:
         if with_pro:
             self.pro = ops.PrologueOut(a_pack=None, body_scale=empty(M, torch.float32), top_scale=empty(M, torch.float32),
                                        tail_idx=None, tail_val=None, R=R)
-        # sums of a tail kernel of its own (the decode kernel makes them itself up to eight rows)
-        apart = R and (engine == _lib.TQ_LINEAR_GATHER or (engine == _lib.TQ_LINEAR_DECODE and M > 8))
-        self.tail = empty((M, N), torch.float32) if apart else None
+        self.tail = empty((M, N), torch.float32) if with_tail else None   # sums of a tail kernel of its own
         self.out = empty((M, n_out), torch.bfloat16)
         self.call = None   # the native description of a forward out of these buffers, and what it was filled in from
         self.call_pro = None
@@ -177,24 +176,37 @@ class SplitLinear:
                                  rms_weight=weights_io.load_extra(path, "rms_weight", device),
                                  rms_eps=float(h.get("rms_eps") or 1e-6))
 
+    # Estimates in us of the whole linear at few rows, by engine.  The decode kernel reads only the M R tail rows it needs, the
+    # fused kernel streams all of the bf16 weights.  Fits to 2880 timings at 1..32 rows of N = 256..28672, K = 512..14336,
+    # R = 0.01..0.1 K, half of them with the weights in L2; each grows faster with M than the one after it, so a layer goes
+    # from the one kernel over the two to the fused one and never back.  The choice is 0.6 % behind the best on average.
+    def _decode_us(self, M: int, apart: bool) -> float:
+        """`apart`: the tail sums in a kernel of their own, which reads 512 bytes of a weight row at a time where the decode
+        kernel's CTAs read 32 or 64: ahead once the row pieces outweigh a launch and the entries one CTA goes through
+        (N = 24576, R = 205: 29 / 28 us at 2 rows, 64 / 36 at 8; N = K = 4096: 14 / 18 at 4, 20 / 18 at 8)."""
+        N, K, R, wide = self.N, self.K, self.R, max(1.0, self.N / 4096)
+        if apart:
+            return 7.14 + 4.79e-4 * K + 9.66e-8 * N * K + 0.0206 * R + (0.14 * M + 6.06e-4 * M * R) * wide
+        return 5.87 + 4.72e-4 * K + 5.87e-8 * N * K + (0.342 * M + 0.00374 * M * R) * wide
+
+    def _fused_us(self, M: int) -> float:
+        return 5.83e-4 * self.K + max(7.34, 3.46 + 3.73e-7 * self.N * self.K) + 0.0209 * M
+
+    def _tail_apart(self, M: int) -> bool:
+        """Whether the decode engine sums the tails in their own kernel (the one kernel takes eight rows with a tail, the
+        other one 8192 entries; same bits)."""
+        if M > 8 or self.R > 8192:
+            return M > 8
+        return self._decode_us(M, True) < self._decode_us(M, False)
+
     def _use_mma(self, M: int) -> bool:
-        # The decode kernel reads only the M R tail rows it needs, the fused kernel streams all of the bf16 weights.  Estimates
-        # in us of the whole linear, fits to timings at 1..64 rows of N = 256..28672, K = 4096..14336, R = 0..0.1 K: a start-up
-        # that grows with K, the weight bytes, and in the decode kernel the entries, per 4096 channels (in a kernel of their
-        # own beyond eight rows).  N = K = 4096, R = 205: decode / fused 10.4 / 12.0 at 2 rows, 19.0 / 12.1 at 8; N = 28672:
-        # 39 / 54 at 4, 73 / 54 at 8.
         if self.tail_engine != "mma":
             return False
         if M > min(self.small_m, 32):
             return True
-        N, K, R = self.N, self.K, self.R
-        if not R:  # 7.2 / 7.3 at 16 rows of N = 256, K = 4096; 12.9 / 11.4 at 8, 9.8 / 11.3 at 4 of N = 12288
-            return M > (16 if N <= 4096 and K <= 4096 else 8)
-        wide = max(1.0, N / 4096)
-        decode = 5.9 + 7e-4 * K + 5e-8 * N * K + ((0.3 * M + 0.0038 * M * R) * wide if M <= 8 else
-                                                  3.0 + (0.17 * M + 0.001 * M * R) * wide)
-        fused = 7e-4 * K + max(7.2, 2.7 + 4.1e-7 * N * K) + 0.1 * M
-        return fused < decode
+        if not self.R:  # 7.2 / 7.3 us at 16 rows of N = 256, K = 4096; 12.9 / 11.4 at 8, 9.8 / 11.3 at 4 of N = 12288
+            return M > (16 if self.N <= 4096 and self.K <= 4096 else 8)
+        return self._fused_us(M) < self._decode_us(M, self._tail_apart(M))
 
     @property
     def N_out(self) -> int:
@@ -216,7 +228,10 @@ class SplitLinear:
         ws.asked = (ops.gemm_pair_mode_changes, int(shared))
 
     def _new_workspace(self, M: int, with_pro: bool) -> _Workspace:
-        return _Workspace(M, self.N, self.K, self.R, self.w.b_col.device, self._engine(M), self.N_out, with_pro)
+        engine = self._engine(M)
+        with_tail = self.R > 0 and (engine == _lib.TQ_LINEAR_GATHER or
+                                    (engine == _lib.TQ_LINEAR_DECODE and self._tail_apart(M)))
+        return _Workspace(M, self.N, self.K, self.R, self.w.b_col.device, engine, self.N_out, with_pro, with_tail)
 
     def _workspace(self, M: int, shared: bool) -> _Workspace:
         ws = self._ws.get(M)

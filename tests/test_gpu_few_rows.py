@@ -58,6 +58,26 @@ def test_decode_linear_exact(M, N, K, kind, ratio):
         assert np.array_equal(host(lin(dev(xb))), ref)
 
 
+@pytest.mark.parametrize("M,N,K,ratio,act", [(1, 1000, 512, 0.05, False), (2, 48, 4096, 0.05, True), (5, 72, 4096, 0.4, False),
+                                             (8, 272, 2048, 0.01, True), (8, 2056, 1024, 0.002, False)])
+def test_decode_tail_sums_apart_or_not(M, N, K, ratio, act):
+    """Up to eight rows the tail sums come from the decode kernel or from their own: the bits of the eight-chain order."""
+    from tailquant_kernel_b200 import SplitLinear
+    kind = O.HAD_WHT
+    xb, wb = O.make_activations(M, K, seed=M, n_outlier=2), O.make_weights(N, K, seed=N)
+    b = np.random.default_rng(3).standard_normal(N, dtype=np.float32)
+    got = []
+    for apart in (True, False):
+        lin = SplitLinear(dev(wb), torch.from_numpy(b).cuda(), ratio=ratio, had_kind=kind, epilogue="swiglu" if act else "none")
+        lin._use_mma, lin._tail_apart = lambda M: False, lambda M: apart
+        got.append(host(lin(dev(xb))))
+        assert (lin._ws[M].tail is not None) == apart
+    assert np.array_equal(got[0], got[1])
+    if not act:
+        R = O.ceil_ratio_count(K, ratio)
+        assert np.array_equal(got[0], O.split_linear_t16(xb, O.prepare_weight(wb, kind), kind, R, bias=b, tail_chains=8)[0])
+
+
 @pytest.mark.parametrize("M,N", [(1, 2056), (2, 6152), (3, 2056), (8, 2056), (40, 2056), (1100, 136)])
 def test_few_rows_on_wider_layers(M, N):
     """Widths on which the dispatch between the decode and the fused kernels depends on rows x tail entries."""

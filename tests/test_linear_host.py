@@ -216,3 +216,28 @@ def test_what_a_forward_alone_reads():
     assert _asked(1200, 1200, 14336, 717, 1, fused, 0) == Q | D
     assert _asked(9000, 136, 4096, 205, 1, fused, 0) == Q | L | T
     assert _asked(4, 4096, 4096, 4096, 1, fused, 0) == -1 and _asked(4, 4096, 4096, 5, 1, 3, 0) == -1
+
+
+@pytest.mark.parametrize("K", [1024, 4096, 12288, 14336])
+@pytest.mark.parametrize("ratio", [0.0, 0.01, 0.05, 0.1, 0.4])
+def test_one_line_between_decode_and_fused(K, ratio):
+    """With more rows a layer goes from the decode kernel over the decode kernel with the tails apart to the fused kernel, and
+    never back; rows beyond the single kernel's eight always have the scratch for the tail sums."""
+    for N in (8, 256, 1024, 4096, 6144, 12288, 24576, 28672, 65536):
+        lin = SplitLinear.__new__(SplitLinear)
+        lin.N, lin.K, lin.R, lin.small_m, lin.tail_engine = N, K, ops.ceil_ratio_count(K, ratio), 64, "mma"
+        steps = [2 if lin._use_mma(M) else int(lin.R > 0 and lin._tail_apart(M)) for M in range(1, 70)]
+        assert steps == sorted(steps), (N, steps)
+        assert steps[-1] == 2
+        lin.tail_engine = "gather"
+        assert not any(lin._use_mma(M) for M in range(1, 70))
+        if lin.R:
+            assert all(lin._tail_apart(M) for M in range(9, 65))
+
+
+@pytest.mark.parametrize("N,M,apart", [(24576, 8, True), (24576, 1, False), (256, 4, False), (256, 9, True)])
+def test_the_scratch_for_tail_sums_says_where_they_are_made(fake, N, M, apart):
+    lin = layer(N=N, K=4096, rms_weight=None, tail_engine="gather")   # (its few rows take the decode engine)
+    lin(claimed(M, 4096, dtype=torch.bfloat16))
+    c = fake.calls[-1][1]
+    assert c["engine"] == _lib.TQ_LINEAR_DECODE and (c["tail"] is not None) == apart
