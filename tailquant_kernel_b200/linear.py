@@ -355,7 +355,9 @@ class SplitLinear:
         if not x.is_cuda:
             raise RuntimeError("x must be a CUDA tensor")
         M = x.numel() // self.K
-        ws = self._workspace(M, False)
+        ws = self._ws.get(M)
+        if ws is None or ws.asked[0] != ops.gemm_pair_mode_changes:
+            ws = self._workspace(M, False)
         call = self._call(ws, ws.pro)
         y = ws.out if self.reuse_output else torch.empty_like(ws.out)
         rc = _lib.load().tq_linear_forward(ctypes.byref(call), x.data_ptr(), y.data_ptr(), ops._stream())
