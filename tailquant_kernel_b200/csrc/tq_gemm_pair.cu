@@ -298,9 +298,12 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a8, const __grid_const
       for (int i = 0; ok && i < my_tiles; ++i) {
         const int nrow = tile_nt(i) * BN + (int)rank * P_BH;
         for (int kb = 0; kb < kbt; ++kb) {
+          TQ_TRACE(6, (i * kbt + kb) * uses, 0);
           if (!(ok = TQ_WAIT(0, mbar_wait(empty_p(sp), ph, abort_flag, 0x1000u)))) break;
+          TQ_TRACE(6, (i * kbt + kb) * uses, 1);
           mbar_arrive_expect_tx(full_p(sp), S::STAGE);
           tma_load_2d(base + S::STAGE_OFF + sp * S::STAGE, &tmap_b4, kb * (P_BK / 2), nrow, full_p(sp));
+          TQ_TRACE(6, (i * kbt + kb) * uses, 2);
           if (++sp == S::SP) {
             sp = 0;
             ph ^= 1u;
@@ -317,9 +320,12 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a8, const __grid_const
       for (int i = 0; ok && i < my_tiles; ++i) {
         const int mrow = (2 * tile_mt(i) + (int)rank) * P_BM;
         for (int kb = 0; kb < kbt; ++kb) {
+          TQ_TRACE(1, (i * kbt + kb) * uses, 0);
           if (!(ok = TQ_WAIT(1, mbar_wait(empty_u(s), ph, abort_flag, 0x2000u)))) break;
+          TQ_TRACE(1, (i * kbt + kb) * uses, 1);
           if (rank == 0) mbar_arrive_expect_tx(full_u(s), 2 * P_BM * 128);  // the A tiles of both CTAs
           tma_load_2d_pair(base + s * S::SLOT, &tmap_a8, kb * P_BK, mrow, lead(full_u(s)));
+          TQ_TRACE(1, (i * kbt + kb) * uses, 2);
           s += uses;
           if (s >= S::SU) {
             s -= S::SU;
@@ -339,9 +345,12 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a8, const __grid_const
         for (int kb = 0; kb < kbt && ok; ++kb) {
 #pragma unroll
           for (int h = 0; h < 2; ++h) {   // (six slots, three uses per slice: both halves lie in front of the wrap)
+            TQ_TRACE(2, 3 * (i * kbt + kb) + 1 + h, 0);
             if (!(ok = TQ_WAIT(2, mbar_wait(empty_u(s + h), ph, abort_flag, 0x4000u)))) break;
+            TQ_TRACE(2, 3 * (i * kbt + kb) + 1 + h, 1);
             if (rank == 0) mbar_arrive_expect_tx(full_u(s + h), BN * 128);  // both halves of the bf16 B tile
             tma_load_2d_pair(base + (s + h) * S::SLOT + S::B_OFF, &tmap_w, kb * P_BK + h * 64, nrow, lead(full_u(s + h)));
+            TQ_TRACE(2, 3 * (i * kbt + kb) + 1 + h, 2);
           }
           s += 3;
           if (s >= S::SU) {
@@ -373,6 +382,7 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a8, const __grid_const
           ph ^= 1u;
         }
       };
+      TQ_TRACE_ONLY(int q = 0;)
       bool ok = true;
       for (int i = 0; ok && i < my_tiles; ++i) {
         const int ab = acc_buf(i);
@@ -381,24 +391,32 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a8, const __grid_const
         tc_fence_after();
         uint32_t acc = 0;
         for (int kb = 0; kb < kbt; ++kb) {
+          TQ_TRACE(0, q, 0);
           if (!(ok = TQ_WAIT(4, mbar_wait(fb, ph, abort_flag, 0x10000u)))) break;
+          TQ_TRACE(0, q, 1);
           tc_fence_after();
           umma_i8_pair(acc_tmem, d, d + B, idesc_i8, acc);
           umma_i8_pair(acc_tmem, d + 2, d + B + 2, idesc_i8, 1u);   // 32 bytes of K further: + 2
           umma_i8_pair(acc_tmem, d + 4, d + B + 4, idesc_i8, 1u);
           umma_i8_pair(acc_tmem, d + 6, d + B + 6, idesc_i8, 1u);
           umma_commit_pair(fb + TO_EMPTY);
+          TQ_TRACE(0, q, 2);
+          TQ_TRACE_ONLY(++q;)
           next();
           if (has_tail) {
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
+              TQ_TRACE(0, q, 0);
               if (!(ok = TQ_WAIT(5, mbar_wait(fb, ph, abort_flag, 0x20000u)))) break;
+              TQ_TRACE(0, q, 1);
               tc_fence_after();
               umma_bf16_pair(tmem_base + BN, d, d + B, idesc_bf, h > 0 ? 1u : acc);
               umma_bf16_pair(tmem_base + BN, d + 2, d + B + 2, idesc_bf, 1u);
               umma_bf16_pair(tmem_base + BN, d + 4, d + B + 4, idesc_bf, 1u);
               umma_bf16_pair(tmem_base + BN, d + 6, d + B + 6, idesc_bf, 1u);
               umma_commit_pair(fb + TO_EMPTY);
+              TQ_TRACE(0, q, 2);
+              TQ_TRACE_ONLY(++q;)
               next();
             }
             if (!ok) break;

@@ -36,8 +36,12 @@ __device__ unsigned long long g_wait_cycles[16];
 #define TQ_WAIT(slot, call) (call)
 #endif
 
-// Diagnostic build (-DTQ_GEMM_TRACE): clock64 stamps of CTA 0's roles for slot uses [TQ_TRACE_Q0, +128), in
-// g_trace[role][use][event]; read back with tq_gemm_trace().  Compiled out otherwise.
+// Diagnostic build (-DTQ_GEMM_TRACE): clock64 stamps of CTA 0's roles in the pair kernel for slot uses [TQ_TRACE_Q0, +128),
+// in g_trace[role][use][event]; read back with tq_gemm_trace().  Compiled out otherwise.
+//   role 0 MMA issuer, 1 INT8 activations, 2 bf16 weight rows, 6 packed weights: 0 = wait begun, 1 = wait over, 2 = issued
+//   role 3 wideners: 0 / 1 / 2 = before and after the wait for the staging buffer, after that for the slot, 3 = done
+//   role 4 builders: 0 / 1 = before and after the wait for the slot, 3 = records scattered, 2 = arrived; role 5: 2 = zeroed,
+//   0 / 1 = before and after the proxy fence
 #ifdef TQ_GEMM_TRACE
 #ifndef TQ_TRACE_Q0
 #define TQ_TRACE_Q0 30
@@ -48,8 +52,10 @@ __device__ unsigned long long g_trace[8][128][4];
     if (blockIdx.x == 0 && (q) >= TQ_TRACE_Q0 && (q) < TQ_TRACE_Q0 + 128)                  \
       g_trace[role][(q) - TQ_TRACE_Q0][ev] = (unsigned long long)clock64();                \
   } while (0)
+#define TQ_TRACE_ONLY(...) __VA_ARGS__
 #else
 #define TQ_TRACE(role, q, ev) do { } while (0)
+#define TQ_TRACE_ONLY(...)
 #endif
 
 }  // namespace

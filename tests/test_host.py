@@ -58,6 +58,14 @@ def test_kernels_that_start_early_read_coherently():
     assert early >= 4
 
 
+def test_every_role_of_the_pair_kernel_is_stamped():
+    """The diagnostic build (-DTQ_GEMM_TRACE) records what its legend in tq_split_gemm.cu names."""
+    csrc = os.path.join(ROOT, "tailquant_kernel_b200", "csrc")
+    stamps = set(re.findall(r"TQ_TRACE\((\d), [^;]*?, (\d)\);", open(os.path.join(csrc, "tq_gemm_pair.cu")).read()))
+    want = {0: 3, 1: 3, 2: 3, 6: 3, 3: 4, 4: 4, 5: 3}
+    assert stamps == {(str(r), str(e)) for r, n in want.items() for e in range(n)}
+
+
 def test_missing_library_fails_loudly(monkeypatch):
     from tailquant_kernel_b200 import _lib
     monkeypatch.setattr(_lib, "_lib", None)
