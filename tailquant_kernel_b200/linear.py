@@ -4,7 +4,7 @@ reference's drop-in adapter discovers.
 Forward of one linear (mirrors the step list of `RealPolicyLinear.forward` as restated in
 tools/profile_multimodel_split_components_v34.py:93-272):
     prologue (rotation + select + pack)  ->  tail gather (R > 0)  ->  GEMM with fused dequant,
-    tail add and bias.  Rows M <= `small_m` take the decode kernel instead.
+    tail add and bias.  A few rows take the decode kernel instead (see `SplitLinear`).
 The kernels of a forward are enqueued by one native call (`tq_linear_forward`) on a description that is filled in once
 per row count, and again when a weight, the bias or the norm was replaced.  Everything runs on the current CUDA stream out of per-(M) workspaces that are allocated once, so
 a forward is capturable in a CUDA graph after its first call, as the reference's benches require
@@ -84,8 +84,13 @@ class SplitLinear:
                  split_k: int = 0, tail_engine: str = "mma", epilogue: str = "none",
                  rms_weight: Optional[torch.Tensor] = None, rms_eps: float = 1e-6, reuse_output: bool = True):
         """tail_engine: "mma" = tail on the tensor cores inside the GEMM kernel (default, fastest at
-        ratios of a few percent); "gather" = exact-order fp32 fma chain on the CUDA cores (bit-exact
-        against the CPU oracle, and the engine of the small-M path).
+        ratios of a few percent); a few rows take the decode kernel where that is faster.  The order of a tail sum, and
+        with it the last place of an output now and then, then depends on how many rows come together.  "gather" = fp32
+        fma chains in a stated order on the CUDA cores, bit-exact against the CPU oracle: one ascending chain per output
+        beyond `small_m` rows, eight interleaved ones (the decode kernel's) up to `small_m`.  With small_m=0 the bits of
+        a row do not depend on the rows that come with it.
+        small_m: rows up to which the decode kernel is considered (at most 64; with the "mma" engine at most 32 count).
+        split_k: without effect, kept for existing calls: the integer sums are exact however K is split.
         epilogue: "swiglu" = `weight` is a fused gate_up matrix with interleaved rows (`interleave_gate_up`) and the
         layer returns bf16(bf16(silu(gate)) * up), [.., N/2], without writing the [.., N] intermediate.
         rms_weight: [K] bf16 weight of an RMSNorm that precedes this linear: the layer then takes the UN-normalised

@@ -170,3 +170,19 @@ def test_gather_chunk_and_batch_edges(M, N, K, R):
     ops.tail_gather(torch.from_numpy(idx.astype(np.uint16).view(np.int16)).cuda(), dev(O.f32_to_bf16_bits(val)),
                     dev(O.f32_to_bf16_bits(w)), out, R)
     assert np.array_equal(out.cpu().numpy(), want)
+
+
+@pytest.mark.parametrize("N,K,kind,ratio", [(520, 1024, O.HAD_WHT, 0.05), (72, 2048, O.HAD_BLOCK128, 0.1), (136, 6144, O.HAD_KRON12, 0.01)])
+def test_bits_of_a_row_do_not_depend_on_the_others(N, K, kind, ratio):
+    """The exact-order engine without the decode kernel: one row alone, in a few and among many, and the oracle's chain."""
+    from tailquant_kernel_b200 import SplitLinear
+    M = 300
+    xb, wb = O.make_activations(M, K, seed=7, n_outlier=4), O.make_weights(N, K, seed=N)
+    b = np.random.default_rng(3).standard_normal(N, dtype=np.float32)
+    lin = SplitLinear(dev(wb), torch.from_numpy(b).cuda(), ratio=ratio, had_kind=kind, tail_engine="gather", small_m=0)
+    x = dev(xb)
+    want = lin(x).clone()
+    R = O.ceil_ratio_count(K, ratio)
+    assert np.array_equal(host(want[:4]), O.split_linear_t16(xb[:4], O.prepare_weight(wb, kind), kind, R, bias=b)[0])
+    for first, rows in ((0, 1), (299, 1), (1, 3), (0, 16), (17, 47), (3, 64), (100, 65), (20, 130)):
+        assert torch.equal(lin(x[first:first + rows]), want[first:first + rows]), rows
