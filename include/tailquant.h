@@ -194,8 +194,9 @@ int tq_split_gemm_mma_swiglu(const int8_t* a_q8, const float* body_scale, const 
                              const uint32_t* tail_rec, const uint16_t* tail_cnt, const void* tail_dense, int R,
                              const float* bias, void* out_bf16, int M, int N, int K, void* stream);
 
-/* tq_split_gemm_mma has two kernels: tiles of 128 channels x up to 176 rows whose K range a cluster of CTAs shares (for
- * few and medium row counts; with a tail it needs tail_dense), and CTA pairs on 256 x 256 tiles (tcgen05 cta_group::2).
+/* tq_split_gemm_mma has two kernels: tiles of 128 channels x up to 176 rows (256 without a tail) whose K range a cluster of
+ * CTAs shares (for few and medium row counts; with a tail it needs tail_dense), and CTA pairs on 256 x 256 tiles (tcgen05
+ * cta_group::2).
  * mode -1 (default) chooses by shape, 0 takes the first wherever it can run, 1 the second always.  A tuning knob
  * without a reference counterpart. */
 int tq_set_gemm_pair_mode(int mode);

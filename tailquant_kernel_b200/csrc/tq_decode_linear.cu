@@ -1,17 +1,18 @@
-// The whole linear behind the prologue for few token rows (M <= 64), ONE launch: INT4 x INT4 dense part, exact-order
-// tail correction, dequantisation, bias / SwiGLU, bf16 out.
+// The whole linear behind the prologue for few token rows (M <= 64), ONE launch up to eight rows: INT4 x INT4 dense part,
+// exact-order tail correction, dequantisation, bias / SwiGLU, bf16 out.  Beyond that, and on wide layers before, the tail
+// sums come from tail_small_kernel (see run_decode_linear).
 //
 // What bounds it: at one row the latency of a few dependent memory round trips, from a few rows on the weight bytes
-// (N K / 2 packed + the bf16 rows that the tails name).  A CTA owns 8 CT output channels and its eight WARPS are the
+// (N K / 2 packed + the bf16 rows that the tails name).  A CTA owns 16 CT output channels and its eight WARPS are the
 // eight K ranges and the eight tail chains, so everything between the prologue's lists and the bf16 results stays in
 // one CTA and no warp waits for another before the final sum:
-//   * warp w streams K range w of the packed weights -- the first 16 128-bit loads per lane are issued before the
-//     wait for the prologue (this kernel is its programmatic dependent) -- and multiplies with mma.sync m16n8k32 s8,
-//     both operands widened with the same nibble order;
+//   * warp w streams K range w of the packed weights through a ring of its own (TMA blocks of 256 K, at most 8 KB a warp;
+//     the first ones are requested before the wait for the prologue, whose programmatic dependent this kernel is) and
+//     multiplies with mma.sync m16n8k32 s8, both operands widened with the same nibble order;
 //   * the tail sum of an output is eight interleaved fp32 fma chains (entry r on chain r mod 8), combined as
 //     ((c0+c1)+(c2+c3))+((c4+c5)+(c6+c7)): warp w evaluates chain w.  The weight-row pieces of its entries arrive by
-//     cp.async in a buffer of the warp's own, 4 KB at a time and two buffers deep, so a chain costs a memory latency
-//     per buffer instead of one per batch of registers;
+//     cp.async in buffers of the warp's own, two or three of 2 KB, so a chain costs a memory latency per buffer
+//     instead of one per batch of registers;
 //   * the partials meet in shared memory once, at the end.
 // A cluster of eight CTAs per 64 channels (ranges = CTAs, partials over distributed shared memory) was measured first:
 // as fast at N = 4096, but 27 us against 12 for the average projection at N = 24576, where thousands of small CTAs

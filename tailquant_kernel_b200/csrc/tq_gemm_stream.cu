@@ -1,6 +1,6 @@
 // Split GEMM for few and medium row counts (sm_100a): the computation of tq_gemm_pair.cu on tiles of 128 output channels
-// x T token rows (T a multiple of 16, at most 176, or 256 for INT8 activations without a tail), the K range of a tile
-// shared by a CLUSTER of S CTAs.
+// x T token rows (T a multiple of 16, at most 176; 256 for INT8 codes without a tail), the K range of a tile shared by a
+// CLUSTER of S CTAs.
 //
 // What bounds it: up to a few hundred rows every weight byte (N K / 2 packed INT4 + 2 N K bf16) is used for so few rows
 // that the weight stream is the floor, and 256 x 256 or 128 x 256 tiles leave most of the chip without work (32 tiles
@@ -13,11 +13,13 @@
 //     builder warps, and the cost does not depend on how the tail entries are distributed;
 //   * the kernel is a programmatic dependent of the prologue: its weight loads fill the ring while the prologue runs.
 //
-// Operand slots are [128 rows x 128 B weights | T rows x 128 B tokens], in two rings: INT8 slots (a 128-wide K slice; the
-// weights arrive as INT4 by TMA in a staging buffer and are widened x16 by four warps) and bf16 slots (HB 64-wide halves
-// of a slice, one tiled load per operand for all of them).
+// Operands come in two rings.  INT8 slots hold the T x 128 B token codes of a 128-wide K slice; its weights arrive as INT4
+// by TMA in a staging buffer and are widened x16 by four warps (eight without a tail) into 32 columns of tensor memory,
+// where the MMA reads them.  bf16 slots hold [128 rows x 128 B weights | T rows x 128 B tail] for HB 64-wide halves of a
+// slice, one tiled load per operand for all of them.
 // Warp roles: 0 = producer of packed weights, 1 = MMA issuer (+ tensor memory), 2 = producer of the bf16 weight rows,
-// 3 = producer of the token operands, 4..7 = wideners, then accumulator export; all warps share the final reduction.
+// 3 = producer of the token operands, 4.. = wideners, of which 4..7 then export the accumulators; all warps share the final
+// reduction.
 // (One thread that waits for a slot, announces its bytes and issues its loads takes about 400 cycles per load: with one
 // producer for everything a K slice took 2700 cycles however few rows there were.)
 // Every mbarrier wait is bounded (see mbar_wait).
