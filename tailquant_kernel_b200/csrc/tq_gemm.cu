@@ -381,7 +381,10 @@ int run_gemm(const uint8_t* a_pack, const uint8_t* b_col, GemmParams p, cudaStre
     const long t128 = (long)((p.M + 127) / 128) * ((p.N + 127) / 128);
     const float here = tiles256 >= 148 ? (float)((tiles256 + sms - 1) / sms) * ((float)(p.K / BK) * 0.55f + 7.0f)
                                        : (float)((t128 + sms - 1) / sms) * ((float)(p.K / BK) * 0.38f + 5.2f);
-    if (plan_stream(p.M, p.N, p.K, ST_PACKED).us < here)
+    // (Where the 256-wide tiles fill the chip, the dequantised output costs the narrow tiles more than the int32 one that the
+    // fits were made with: 6144 x 4096 at 2048 rows 81 us against 73, 12288 x 4096 163 / 134; int32 70 / 78 and 143 / 149.)
+    const float out = tiles256 >= 148 && p.mode == MODE_FUSED ? 1.12f : 1.0f;
+    if (out * plan_stream(p.M, p.N, p.K, ST_PACKED).us < here)
       return run_stream_packed(a_pack, b_col, p.C, p.sx, p.sw, p.tail, p.bias, p.out, p.M, p.N, p.K, st);
   }
   if (tiles256 >= 148) return launch_gemm<256>(a_pack, b_col, p, st);
