@@ -16,8 +16,8 @@
 //
 // What bounds it: for few rows the latency of one row, i.e. the instructions a thread issues one after the other, which is
 // why a thread has so few elements (one row of K = 4096, R = 205, with RMSNorm: 5.9 us; 9.5 with 64 elements per thread,
-// 7.4 without norm in the 256-thread kernel with three exchanges that this one replaces); with many rows instruction
-// issue, where the 64-element kernel of tq_prologue_fast.cu (K = 4096, 12288, 14336) is ahead: 25 against 30 us at 2048 rows.
+// 7.4 without norm in the 256-thread kernel with three exchanges that this one replaces); with many rows the
+// instructions per element, where the 64-element kernel of tq_prologue_fast.cu (K = 4096, 12288, 14336) is ahead: 25 against 30 us at 2048 rows.
 //
 // Reference behaviour covered: tools/fused_threshold_topr_pack_ext_v57.py:96-194 (select, scales, pack),
 // tools/fused_topr_pack_ext_v55.py:21-26,73-109 (clamp_s4, scale = max(key, eps)/7, body nibble 0 at tail positions, nibble

@@ -441,10 +441,10 @@ def split_linear_forward(x: torch.Tensor, weight: torch.Tensor, bias: Optional[t
     if hit is not None and hit[0]() is x:
         ws = hit[1]
     else:
-        ws = lin.prologue(x2d)
+        _SHARED.clear()   # one entry: the prologue outputs live in a workspace that the next prologue of that layer
+        ws = lin.prologue(x2d)                    # overwrites, whatever its input
         if x2d.data_ptr() == x.data_ptr():  # only inputs that were used as they are can be recognised again
-            _SHARED.clear()                  # one entry: the prologue outputs live in a workspace that the next
-            _SHARED[skey] = (weakref.ref(x), ws)  # prologue of that layer overwrites
+            _SHARED[skey] = (weakref.ref(x), ws)
     y = lin.compute(ws, M, torch.empty((M, lin.N_out), dtype=torch.bfloat16, device=x2d.device))
     y = y.view(*x.shape[:-1], lin.N_out)
     return y if y.dtype == x.dtype else y.to(x.dtype)

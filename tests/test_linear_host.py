@@ -241,3 +241,34 @@ def test_the_scratch_for_tail_sums_says_where_they_are_made(fake, N, M, apart):
     lin(claimed(M, 4096, dtype=torch.bfloat16))
     c = fake.calls[-1][1]
     assert c["engine"] == _lib.TQ_LINEAR_DECODE and (c["tail"] is not None) == apart
+
+
+@pytest.fixture
+def adapter(fake, monkeypatch):
+    """`split_linear_forward` on two prepared layers, reporting which layers ran a prologue."""
+    from tailquant_kernel_b200 import linear
+    layers, ran = {}, []
+    monkeypatch.setattr(linear, "_cached_layer", lambda w, b, r: layers[id(w)])
+    monkeypatch.setattr(ops, "_check_cuda", lambda *a, **k: None)
+    weights = [claimed(n, 512, dtype=torch.bfloat16) for n in (256, 128)]
+    for w in weights:
+        lin = layers[id(w)] = layer(N=w.shape[0], rms_weight=None)
+        lin.prologue = lambda x, lin=lin: ran.append(lin.N) or SplitLinear.prologue(lin, x)
+    linear.clear_cache()
+
+    def call(x, i):
+        ran.clear()
+        linear.split_linear_forward(x, weights[i])
+        return list(ran)
+    yield call
+    linear.clear_cache()
+
+
+def test_a_shared_prologue_ends_with_the_next_one(adapter):
+    """An input that has to be converted runs a prologue of its own in the layer's buffers: what an earlier input left there
+    must not be taken for its prologue any more."""
+    x, other = claimed(100, 512, dtype=torch.bfloat16), claimed(100, 512, dtype=torch.float32)
+    assert adapter(x, 0) == [256] and adapter(x, 1) == []
+    assert adapter(other, 0) == [256]
+    assert adapter(x, 1) == [128]
+    assert adapter(x, 0) == []
