@@ -329,6 +329,10 @@ int tq_linear_forward(const tq_linear_call* call, const void* x, void* out, void
 int tq_linear_prologue(const tq_linear_call* call, const void* x, void* stream);
 int tq_linear_compute(const tq_linear_call* call, void* out, void* stream);
 
+/* Number of the stream capture that `stream` is part of, 0 when it is not being captured: what one capture enqueued is not
+ * there for another, nor for work outside of it. */
+long long tq_stream_capture_id(void* stream);
+
 /* Split-K linear for callers that cannot allocate device memory: the same computation as
  * tq_int4_matmul(split_k) followed by tq_dequant_finish,
  *   out[m,n] = bf16((float(sum_k qa qw) * body_scale[m]) * w_scale[n] + tail[m,n] + bias[n]),

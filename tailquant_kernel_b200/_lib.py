@@ -62,6 +62,7 @@ SIGNATURES = {
     "tq_linear_forward": [_P, _P, _P, _P],
     "tq_linear_prologue": [_P, _P, _P],
     "tq_linear_compute": [_P, _P, _P],
+    "tq_stream_capture_id": [_P],
     "tq_gemm_status": [_P],
 }
 _CHAR_P_RETURNS = {"tq_error_string", "tq_last_cuda_error"}
@@ -81,7 +82,7 @@ def load() -> C.CDLL:
     for name, argtypes in SIGNATURES.items():
         fn = getattr(lib, name)  # AttributeError if the symbol is not exported
         fn.argtypes = argtypes
-        fn.restype = C.c_char_p if name in _CHAR_P_RETURNS else C.c_int
+        fn.restype = C.c_char_p if name in _CHAR_P_RETURNS else _LL if name == "tq_stream_capture_id" else C.c_int
     _lib = lib
     return lib
 

@@ -47,6 +47,16 @@ extern "C" const char* tq_error_string(int code) {
 
 extern "C" const char* tq_last_cuda_error(void) { return tq::g_cuda_error; }
 
+extern "C" long long tq_stream_capture_id(void* stream) {
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  unsigned long long id = 0;
+  if (cudaStreamGetCaptureInfo((cudaStream_t)stream, &status, &id) != cudaSuccess) {
+    cudaGetLastError();   // (no device, or the legacy stream while another thread captures)
+    return 0;
+  }
+  return status == cudaStreamCaptureStatusActive ? (long long)id : 0;
+}
+
 // Rotation + RTN quantisation of a weight matrix is the pure (R = 0) prologue applied to the
 // rows of W with the weight flavour of the scale clamp; the two tail layouts are re-layouts
 // of its outputs.

@@ -380,7 +380,7 @@ class _Entry:
 
 _CACHE: "OrderedDict[Tuple, _Entry]" = OrderedDict()
 _CACHE_MAX = 1024        # prepared layers kept (a 36-layer model has 252 target linears)
-_SHARED: Dict[Tuple, Tuple] = {}  # (device, x ptr, x version, M, K, R, rank, rotation) -> (x weakref, workspace)
+_SHARED: Dict[Tuple, Tuple] = {}  # (input, shape of the split, stream, capture) -> (x weakref, workspace)
 
 
 def _drop(key) -> None:
@@ -435,8 +435,10 @@ def split_linear_forward(x: torch.Tensor, weight: torch.Tensor, bias: Optional[t
         x2d = x2d.to(torch.bfloat16)
     x2d = x2d.contiguous()
     M = x2d.shape[0]
-    skey = (x.device.index, x2d.data_ptr(), x._version, M, lin.K, lin.R, lin.descending_rank, lin.w.had_kind,
-            ops._stream())
+    stream = ops._stream()
+    # (a graph has to contain the prologue of its linears: one that ran before the capture, or in another, is none of it)
+    skey = (x.device.index, x2d.data_ptr(), x._version, M, lin.K, lin.R, lin.descending_rank, lin.w.had_kind, stream,
+            _lib.load().tq_stream_capture_id(stream))
     hit = _SHARED.get(skey) if x2d.data_ptr() == x.data_ptr() else None
     if hit is not None and hit[0]() is x:
         ws = hit[1]

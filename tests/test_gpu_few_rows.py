@@ -186,3 +186,28 @@ def test_bits_of_a_row_do_not_depend_on_the_others(N, K, kind, ratio):
     assert np.array_equal(host(want[:4]), O.split_linear_t16(xb[:4], O.prepare_weight(wb, kind), kind, R, bias=b)[0])
     for first, rows in ((0, 1), (299, 1), (1, 3), (0, 16), (17, 47), (3, 64), (100, 65), (20, 130)):
         assert torch.equal(lin(x[first:first + rows]), want[first:first + rows]), rows
+
+
+def test_adapter_in_two_captures():
+    """Two graphs captured one after the other on the same static input: each follows the input on its own."""
+    from tailquant_kernel_b200 import linear, split_linear_forward
+    M, K = 100, 1024
+    x = dev(O.make_activations(M, K, seed=1, n_outlier=4))
+    ws = [dev(O.make_weights(n, K, seed=n)) for n in (512, 136)]
+    linear.clear_cache()
+    inputs = [x.clone(), dev(O.make_activations(M, K, seed=2, n_outlier=4))]
+    want = [[split_linear_forward(i, w).clone() for w in ws] for i in inputs]
+    side = torch.cuda.Stream()
+    graphs, outs = [], []
+    with torch.cuda.stream(side):
+        [split_linear_forward(x, w) for w in ws]
+    torch.cuda.synchronize()
+    for _ in range(2):
+        graphs.append(torch.cuda.CUDAGraph())
+        with torch.cuda.graph(graphs[-1], stream=side):
+            outs.append([split_linear_forward(x, w) for w in ws])
+    for i in (1, 0):
+        x.copy_(inputs[i])
+        graphs[i].replay()
+        torch.cuda.synchronize()
+        assert all(torch.equal(a, b) for a, b in zip(outs[i], want[i]))

@@ -22,9 +22,11 @@ def claimed(*shape, dtype):
 
 class FakeLibrary:
     def __init__(self, real):
-        self.real, self.calls = real, []
+        self.real, self.calls, self.capture = real, [], 0
 
     def __getattr__(self, name):
+        if name == "tq_stream_capture_id":
+            return lambda stream: self.capture
         if name not in (FORWARD, PROLOGUE, COMPUTE):
             return getattr(self.real, name)
 
@@ -272,3 +274,11 @@ def test_a_shared_prologue_ends_with_the_next_one(adapter):
     assert adapter(other, 0) == [256]
     assert adapter(x, 1) == [128]
     assert adapter(x, 0) == []
+
+
+def test_a_capture_contains_the_prologue_of_its_linears(adapter, fake):
+    """A replay must not run on what was left by a prologue outside of the graph, nor eager work on a captured one."""
+    x = claimed(100, 512, dtype=torch.bfloat16)
+    assert adapter(x, 0) == [256] and adapter(x, 1) == []
+    for fake.capture in (7, 8, 0):
+        assert adapter(x, 0) == [256] and adapter(x, 1) == []
