@@ -47,7 +47,7 @@ class _Workspace:
                                        tail_idx=None, tail_val=None, R=R)
         self.tail = empty((M, N), torch.float32) if with_tail else None   # sums of a tail kernel of its own
         self.out = empty((M, n_out), torch.bfloat16)
-        self.call = None   # the native description of a forward out of these buffers, and what it was filled in from
+        self.call = None   # (a reference to) the native description of a forward out of these buffers; what it was filled in from
         self.call_pro = None
         self.call_src = ()
 
@@ -299,8 +299,9 @@ class SplitLinear:
             ops._check_cuda(self.rms_weight, "rms_weight", torch.bfloat16)
             ops._check(self.rms_weight.numel() == K, "rms_weight must have K elements")
 
-    def _call(self, own: _Workspace, pro: "ops.PrologueOut") -> "_lib.LinearCall":
-        """Description of this layer's forward: prologue outputs `pro` (own or another layer's), output side `own`."""
+    def _call(self, own: _Workspace, pro: "ops.PrologueOut"):
+        """Reference to the description of this layer's forward: prologue outputs `pro` (own or another layer's), output side
+        `own`."""
         if own.call is not None and own.call_pro is pro and self._described(own):
             return own.call
         if own.engine == _lib.TQ_LINEAR_DECODE:
@@ -311,7 +312,7 @@ class SplitLinear:
         own.call_pro = pro
         src = (w.b_col, w.w_scale, w.w_rot, w.w_t, w.bias, self.rms_weight)
         own.call_src = (*src, w.had_kind, self.descending_rank, self.rms_eps, self.epilogue, *map(p, src))
-        own.call = _lib.LinearCall(
+        own.call = ctypes.byref(_lib.LinearCall(
             M=own.M, N=self.N, K=self.K, R=self.R, had_kind=w.had_kind, descending_rank=self.descending_rank,
             engine=own.engine, act=1 if self.epilogue == "swiglu" else 0,
             tail_ld=pro.tail_idx.shape[1] if pro.tail_idx is not None else 0,
@@ -319,7 +320,7 @@ class SplitLinear:
             b_col=p(w.b_col), w_scale=p(w.w_scale), w_rot=p(w.w_rot), w_t=p(w.w_t), bias=p(w.bias),
             rms_weight=p(self.rms_weight), a_pack=p(pro.a_pack), a_q8=p(pro.a_q8), body_scale=p(pro.body_scale),
             top_scale=p(pro.top_scale), tail_idx16=p(pro.tail_idx), tail_val=p(pro.tail_val), tail_ptr=p(pro.tail_ptr),
-            tail_rec=p(pro.tail_rec), tail_cnt=p(pro.tail_cnt), tail_dense=p(pro.tail_dense), tail=p(own.tail))
+            tail_rec=p(pro.tail_rec), tail_cnt=p(pro.tail_cnt), tail_dense=p(pro.tail_dense), tail=p(own.tail)))
         return own.call
 
     def _what(self, M: int) -> str:
@@ -329,7 +330,7 @@ class SplitLinear:
         ops._check_cuda(x2d, "x", torch.bfloat16)
         ops._check(x2d.dim() == 2 and x2d.shape[1] == self.K, "x must be [M, K]")
         ws = self.workspace(x2d.shape[0])
-        rc = _lib.load().tq_linear_prologue(ctypes.byref(self._call(ws, ws.pro)), x2d.data_ptr(), ops._stream())
+        rc = _lib.load().tq_linear_prologue(self._call(ws, ws.pro), x2d.data_ptr(), ops._stream())
         if rc:
             _lib.check(rc, self._what(ws.M))
         return ws
@@ -346,7 +347,7 @@ class SplitLinear:
         else:
             ops._check_cuda(out, "out", torch.bfloat16)
             ops._check(out.numel() >= M * self.N_out, "out too small")
-        rc = _lib.load().tq_linear_compute(ctypes.byref(self._call(own, ws.pro)), out.data_ptr(), ops._stream())
+        rc = _lib.load().tq_linear_compute(self._call(own, ws.pro), out.data_ptr(), ops._stream())
         if rc:
             _lib.check(rc, self._what(M))
         return out
@@ -363,9 +364,11 @@ class SplitLinear:
         ws = self._ws.get(M)
         if ws is None or ws.asked[0] != ops.gemm_pair_mode_changes:
             ws = self._workspace(M, False)
-        call = self._call(ws, ws.pro)
+        call = ws.call
+        if call is None or ws.call_pro is not ws.pro or not self._described(ws):
+            call = self._call(ws, ws.pro)
         y = ws.out if self.reuse_output else torch.empty_like(ws.out)
-        rc = _lib.load().tq_linear_forward(ctypes.byref(call), x.data_ptr(), y.data_ptr(), ops._stream())
+        rc = _lib.load().tq_linear_forward(call, x.data_ptr(), y.data_ptr(), ops._stream())
         if rc:
             _lib.check(rc, self._what(M))
         return y.view(*shape[:-1], self.N_out)
