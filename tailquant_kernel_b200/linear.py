@@ -439,16 +439,19 @@ def split_linear_forward(x: torch.Tensor, weight: torch.Tensor, bias: Optional[t
     x2d = x2d.contiguous()
     M = x2d.shape[0]
     stream = ops._stream()
+    # Only an input that is used as it is can be recognised again, and only one whose in-place changes are counted (those
+    # made in inference mode are not).
+    known = x2d.data_ptr() == x.data_ptr() and not x.is_inference()
     # (a graph has to contain the prologue of its linears: one that ran before the capture, or in another, is none of it)
-    skey = (x.device.index, x2d.data_ptr(), x._version, M, lin.K, lin.R, lin.descending_rank, lin.w.had_kind, stream,
+    skey = (x.device.index, x2d.data_ptr(), x._version if known else 0, M, lin.K, lin.R, lin.descending_rank, lin.w.had_kind, stream,
             _lib.load().tq_stream_capture_id(stream))
-    hit = _SHARED.get(skey) if x2d.data_ptr() == x.data_ptr() else None
+    hit = _SHARED.get(skey) if known else None
     if hit is not None and hit[0]() is x:
         ws = hit[1]
     else:
         _SHARED.clear()   # one entry: the prologue outputs live in a workspace that the next prologue of that layer
         ws = lin.prologue(x2d)                    # overwrites, whatever its input
-        if x2d.data_ptr() == x.data_ptr():  # only inputs that were used as they are can be recognised again
+        if known:
             _SHARED[skey] = (weakref.ref(x), ws)
     y = lin.compute(ws, M, torch.empty((M, lin.N_out), dtype=torch.bfloat16, device=x2d.device))
     y = y.view(*x.shape[:-1], lin.N_out)

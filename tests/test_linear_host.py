@@ -282,3 +282,10 @@ def test_a_capture_contains_the_prologue_of_its_linears(adapter, fake):
     assert adapter(x, 0) == [256] and adapter(x, 1) == []
     for fake.capture in (7, 8, 0):
         assert adapter(x, 0) == [256] and adapter(x, 1) == []
+
+
+def test_inputs_made_in_inference_mode(adapter):
+    """Their in-place changes are not counted: every layer runs its own prologue on them."""
+    with torch.inference_mode():
+        x = claimed(100, 512, dtype=torch.bfloat16)
+        assert adapter(x, 0) == [256] and adapter(x, 1) == [128]
