@@ -279,7 +279,7 @@ int tq_idx_i32_to_u16(const int32_t* idx, uint16_t* out, long long n, void* stre
  * workspace, options -- is described once by a tq_linear_call; x [M,K] bf16 and out ([M,N] bf16, [M,N/2] with act = 1)
  * come with each call.  tq_linear_forward enqueues the prologue and the linear; tq_linear_prologue and tq_linear_compute
  * are its two halves (linears that share one input run tq_linear_compute on one set of prologue outputs).
- *   engine TQ_LINEAR_DECODE  M <= 64: one kernel behind the prologue, or with `tail` (needed beyond 8 rows) one for the
+ *   engine TQ_LINEAR_DECODE  M <= 64: one kernel behind the prologue, or with `tail` (needed beyond 8 rows; R <= 8192) one for the
  *                            tail sums and one for the rest; sums as tq_int4_gemv_splitk + tq_tail_gather_small +
  *                            tq_dequant_finish either way (needs a_pack, w_t, tail_idx16 / tail_val)
  *          TQ_LINEAR_FUSED   as tq_split_gemm_mma (needs a_q8, w_rot and the tail arrays)

@@ -356,8 +356,8 @@ int run_decode_linear(DecodeLinearParams p, float* tail_scratch, cudaStream_t st
   // Beyond eight rows the tail sums come from their own kernel, up to eight where the caller brings the scratch: a CTA's 16
   // or 32 channels make 32- or 64-byte pieces of the weight rows, and with many rows or channels the pieces, not the
   // latency, are what takes time (512 bytes each there; N = 24576, R = 205: 64 us in this kernel at 8 rows, 36 in two; at
-  // one row 19 and 25.  `SplitLinear._tail_apart` draws the line).
-  if (p.R > 0 && (p.M > 8 || tail_scratch)) {
+  // one row 19 and 25.  `SplitLinear._tail_apart` draws the line; that kernel takes 8192 entries).
+  if (p.R > 0 && (p.M > 8 || (tail_scratch && p.R <= 8192))) {
     if (!tail_scratch) return TQ_ERR_BAD_ARG;
     const int rc = tq_tail_gather_small(p.idx, p.val, p.w_t, tail_scratch, p.M, p.N, p.K, p.R, p.ld, st);
     if (rc != TQ_OK) return rc;

@@ -59,11 +59,12 @@ def test_decode_linear_exact(M, N, K, kind, ratio):
 
 
 @pytest.mark.parametrize("M,N,K,ratio,act", [(1, 1000, 512, 0.05, False), (2, 48, 4096, 0.05, True), (5, 72, 4096, 0.4, False),
-                                             (8, 272, 2048, 0.01, True), (8, 2056, 1024, 0.002, False)])
+                                             (8, 272, 2048, 0.01, True), (8, 2056, 1024, 0.002, False),
+                                             (2, 16, 14336, 0.6, False)])   # more entries than the tail kernel takes
 def test_decode_tail_sums_apart_or_not(M, N, K, ratio, act):
     """Up to eight rows the tail sums come from the decode kernel or from their own: the bits of the eight-chain order."""
     from tailquant_kernel_b200 import SplitLinear
-    kind = O.HAD_WHT
+    kind = O.HAD_WHT if K <= 8192 else O.HAD_BLOCK128
     xb, wb = O.make_activations(M, K, seed=M, n_outlier=2), O.make_weights(N, K, seed=N)
     b = np.random.default_rng(3).standard_normal(N, dtype=np.float32)
     got = []
