@@ -188,7 +188,7 @@ class SplitLinear:
     def _decode_us(self, M: int, apart: bool) -> float:
         """`apart`: the tail sums in a kernel of their own, which reads 512 bytes of a weight row at a time where the decode
         kernel's CTAs read 32 or 64: ahead once the row pieces outweigh a launch and the entries one CTA goes through
-        (N = 24576, R = 205: 29 / 28 us at 2 rows, 64 / 36 at 8; N = K = 4096: 14 / 18 at 4, 20 / 18 at 8)."""
+        (N = 24576, R = 205: 28 / 29 us at 2 rows, 64 / 36 at 8; N = K = 4096: 14 / 18 at 4, 20 / 18 at 8)."""
         N, K, R, wide = self.N, self.K, self.R, max(1.0, self.N / 4096)
         if apart:
             return 7.14 + 4.79e-4 * K + 9.66e-8 * N * K + 0.0206 * R + (0.14 * M + 6.06e-4 * M * R) * wide
@@ -199,8 +199,9 @@ class SplitLinear:
 
     def _tail_apart(self, M: int) -> bool:
         """Whether the decode engine sums the tails in their own kernel (the one kernel takes eight rows with a tail, the
-        other one 8192 entries; same bits)."""
-        if M > 8 or self.R > 8192:
+        other one 8192 entries; same bits).  At two rows the third launch costs what it saves: N = 28672, R = 205 30.3 us
+        either way in a graph, a layer called launch by launch 2 % slower."""
+        if M > 8 or M <= 2 or self.R > 8192:
             return M > 8
         return self._decode_us(M, True) < self._decode_us(M, False)
 
@@ -211,7 +212,8 @@ class SplitLinear:
             return True
         if not self.R:  # 7.2 / 7.3 us at 16 rows of N = 256, K = 4096; 12.9 / 11.4 at 8, 9.8 / 11.3 at 4 of N = 12288
             return M > (16 if self.N <= 4096 and self.K <= 4096 else 8)
-        return self._fused_us(M) < self._decode_us(M, self._tail_apart(M))
+        decode = self._decode_us(M, True)
+        return self._fused_us(M) < (decode if M > 8 else min(decode, self._decode_us(M, False)))
 
     @property
     def N_out(self) -> int:
