@@ -194,6 +194,16 @@ int tq_split_gemm_mma_swiglu(const int8_t* a_q8, const float* body_scale, const 
                              const uint32_t* tail_rec, const uint16_t* tail_cnt, const void* tail_dense, int R,
                              const float* bias, void* out_bf16, int M, int N, int K, void* stream);
 
+/* The same linear from the 2:4-sparse form of the tail that tq_linear_prologue / tq_linear_forward leave in the sp_* arrays of a
+ * tq_linear_call: sp_val has the first two entries of each group of four (zeros where there are fewer), sp_meta their places,
+ * four bits per group (the lower place, the higher one << 2); sp_over the entries beyond two of a group (index | bf16 << 16,
+ * ascending), sp_over_cnt how many there are.
+ * w_t may be NULL (the left-over entries then read w_rot, slower); act = 1: SwiGLU, out [M, N/2]. */
+int tq_split_gemm_sparse(const int8_t* a_q8, const float* body_scale, const uint8_t* b_col, const float* w_scale,
+                         const void* w_rot, const void* w_t, int R, void* sp_val, uint32_t* sp_meta, uint16_t* sp_over_cnt, uint32_t* sp_over, int sp_over_ld,
+                         const float* bias, void* out_bf16,
+                         int32_t* dbg_acc, float* dbg_tail, int M, int N, int K, int act, void* stream);
+
 /* tq_split_gemm_mma has two kernels: tiles of 128 channels x up to 176 rows (256 without a tail) whose K range a cluster of
  * CTAs shares (for few and medium row counts; with a tail it needs tail_dense), and CTA pairs on 256 x 256 tiles (tcgen05
  * cta_group::2).
@@ -313,7 +323,14 @@ typedef struct tq_linear_call {
   uint16_t* tail_cnt;
   void* tail_dense;
   float* tail;
+  /* operands of the kernel for a 2:4-sparse tail (see tq_linear_sparse); all or none */
+  void* sp_val;           /* [M,K/2] bf16 */
+  uint32_t* sp_meta;      /* [M,K/32] */
+  uint16_t* sp_over_cnt;  /* [M] */
+  uint32_t* sp_over;      /* [M,sp_over_ld] */
+  int sp_over_ld;         /* at least (R + 1) / 2 */
 } tq_linear_call;
+
 /* Prologue outputs that the workspace of a call should hold, as a sum of these; reads M, N, K, R, had_kind and engine of
  * `call` only.  shared = 0: what tq_linear_forward of this call reads and writes.  shared = 1: what tq_linear_prologue should
  * leave for linears of any width (a wide and a narrow layer can be on different kernels; up to 64 rows also on the decode
@@ -325,6 +342,12 @@ typedef struct tq_linear_call {
 #define TQ_OUT_RECORDS 8 /* tail_ptr, tail_rec, tail_cnt */
 #define TQ_OUT_DENSE 16  /* tail_dense */
 int tq_linear_outputs(const tq_linear_call* call, int shared);
+/* 1 where a fused forward of this call (shared = 1: of a linear of some width on the same prologue) takes the tail as a
+ * 2:4-sparse operand once its workspace holds the sp_* arrays beside those of tq_linear_outputs, else 0; reads the same fields.
+ * A forward on the sparse form writes no records, and neither does tq_linear_prologue where tail_dense is there too. */
+int tq_linear_sparse(const tq_linear_call* call, int shared);
+/* out [K,N] = in [N,K] transposed, bf16 (the w_t of rotated weights). */
+int tq_transpose_bf16(const void* in, void* out, int N, int K, void* stream);
 int tq_linear_forward(const tq_linear_call* call, const void* x, void* out, void* stream);
 int tq_linear_prologue(const tq_linear_call* call, const void* x, void* stream);
 int tq_linear_compute(const tq_linear_call* call, void* out, void* stream);

@@ -26,7 +26,8 @@ class LinearCall(C.Structure):
                 + [(n, _F) for n in ("eps", "rms_eps")]
                 + [(n, _P) for n in ("b_col", "w_scale", "w_rot", "w_t", "bias", "rms_weight", "a_pack", "a_q8", "body_scale",
                                      "top_scale", "tail_idx16", "tail_val", "tail_ptr", "tail_rec", "tail_cnt", "tail_dense",
-                                     "tail")])
+                                     "tail", "sp_val", "sp_meta", "sp_over_cnt", "sp_over")]
+                + [("sp_over_ld", _I)])
 
 
 # name -> argument types; must list every function declared in include/tailquant.h
@@ -40,6 +41,8 @@ SIGNATURES = {
     "tq_set_gemv_channel_tiles": [_I],
     "tq_split_gemm_mma": [_P, _P, _P, _P, _P, _P, _P, _I, _P, _I, _P, _P, _P, _I, _P, _P, _P, _P, _I, _I, _I, _P],
     "tq_split_gemm_mma_swiglu": [_P, _P, _P, _P, _P, _P, _P, _I, _P, _I, _P, _P, _P, _I, _P, _P, _I, _I, _I, _P],
+    # ..., w_rot, w_t, R, sp_val, sp_meta, sp_over_cnt, sp_over, ld, bias, out, dbg_acc, dbg_tail, M, N, K, act, stream
+    "tq_split_gemm_sparse": [_P] * 6 + [_I] + [_P] * 4 + [_I] + [_P] * 4 + [_I, _I, _I, _I, _P],
     "tq_topr_pack": [_P, _I, _I, _I, _I, _I, _P, _P, _P, _P, _P, _F, _P],
     "tq_prepare_weight": [_P, _I, _I, _I, _F, _P, _P, _P, _P, _P, _P],
     "tq_int4_matmul": [_P, _P, _P, _I, _I, _I, _I, _P],
@@ -59,6 +62,8 @@ SIGNATURES = {
     "tq_set_gemm_pair_mode": [_I],
     "tq_set_prologue_mode": [_I],
     "tq_linear_outputs": [_P, _I],
+    "tq_linear_sparse": [_P, _I],
+    "tq_transpose_bf16": [_P, _P, _I, _I, _P],
     "tq_linear_forward": [_P, _P, _P, _P],
     "tq_linear_prologue": [_P, _P, _P],
     "tq_linear_compute": [_P, _P, _P],

@@ -15,6 +15,24 @@ bool linear_streams(const tq_linear_call& c) {
 // Rows beyond which the zero-filled matrix is not kept whatever it would save (layers whose pair kernel reads it excepted).
 constexpr int DENSE_MAX_ROWS = 4096;
 
+// Whether a linear can take its tail as a 2:4-sparse operand: a full rotation, which spreads the entries over K, and few enough of
+// them that a group of four rarely holds more than two.  (At R = 0.1 K the left-over entries outweigh what the sparse product
+// saves, and rows with a few large channels have twice as many.)
+bool tail_can_be_sparse(const tq_linear_call& c) {
+  return c.engine == TQ_LINEAR_FUSED && (c.had_kind == TQ_HAD_WHT || c.had_kind == TQ_HAD_KRON12) && c.R > 0 && c.K % 512 == 0 &&
+         c.N % 8 == 0 && (long)c.R * 100 <= 7l * c.K;
+}
+
+// Whether the sparse form is the fastest for this call.
+bool linear_sparse(const tq_linear_call& c) { return tail_can_be_sparse(c) && sparse_is_faster(c.M, c.N, c.K, c.R); }
+// Whether the buffers of a call hold the sparse form and the zero-filled matrix: between them they serve every fused kernel (the
+// CTA pairs then load all of their tail operand from the matrix), so the records are left out.
+bool sparse_and_dense(const tq_linear_call& c) { return c.sp_val && c.tail_dense && tail_can_be_sparse(c); }
+
+SparseTail linear_sparse_tail(const tq_linear_call& c) {
+  return SparseTail{reinterpret_cast<uint16_t*>(c.sp_val), c.sp_meta, c.sp_over_cnt, c.sp_over, c.sp_over_ld};
+}
+
 // THE rule for the buffers of a workspace (see tailquant.h); which kernel then runs follows from what is there.
 int linear_outputs(const tq_linear_call& c, bool shared) {
   const bool fused = c.engine == TQ_LINEAR_FUSED;
@@ -35,15 +53,24 @@ int linear_outputs(const tq_linear_call& c, bool shared) {
 // another linear, of another width and hence perhaps on another kernel, may run on it.  The sorted tail lists and the
 // records cost a small call about 3 us, the zero-filled matrix a large one 2 bytes per element.
 tq_linear_call linear_own_part(tq_linear_call c) {
-  const bool fused = c.engine == TQ_LINEAR_FUSED, streams = linear_streams(c);
+  const bool fused = c.engine == TQ_LINEAR_FUSED;
   if (fused)
     c.a_pack = nullptr;
   else
     c.a_q8 = nullptr;
+  if (c.sp_val && linear_sparse(c)) {
+    c.tail_dense = nullptr;
+    c.tail_ptr = nullptr;
+    c.tail_rec = nullptr;
+    c.tail_cnt = nullptr;
+    return c;
+  }
+  const bool streams = linear_streams(c);
   if (streams) {
     c.tail_idx16 = nullptr;
     c.tail_val = nullptr;
   }
+  c.sp_val = nullptr;
   if (!fused || streams) {
     c.tail_ptr = nullptr;
     c.tail_rec = nullptr;
@@ -54,9 +81,12 @@ tq_linear_call linear_own_part(tq_linear_call c) {
 }
 
 int linear_prologue(const tq_linear_call& c, const void* x, void* stream) {
+  const SparseTail sp = linear_sparse_tail(c);
+  const bool records = !sparse_and_dense(c);
   return run_prologue(x, c.M, c.K, c.had_kind, c.R, c.descending_rank, c.eps, 0, c.a_pack, c.a_q8, c.body_scale,
-                      c.top_scale, c.tail_idx16, c.tail_val, c.tail_ld, c.tail_ptr, c.ptr_ld, c.tail_rec, c.tail_cnt,
-                      nullptr, nullptr, nullptr, c.rms_weight, c.rms_eps, (cudaStream_t)stream, TQ_BF16, c.tail_dense);
+                      c.top_scale, c.tail_idx16, c.tail_val, c.tail_ld, records ? c.tail_ptr : nullptr, c.ptr_ld,
+                      records ? c.tail_rec : nullptr, records ? c.tail_cnt : nullptr,
+                      nullptr, nullptr, nullptr, c.rms_weight, c.rms_eps, (cudaStream_t)stream, TQ_BF16, c.tail_dense, sp.val ? &sp : nullptr);
 }
 
 // `early`: the prologue of this call is the kernel in front
@@ -95,9 +125,20 @@ int linear_compute(const tq_linear_call& c, void* out, bool early, void* stream)
                                c.N, c.K, stream);
   }
   if (c.engine != TQ_LINEAR_FUSED) return TQ_ERR_BAD_ARG;
+  if (c.sp_val && c.M > 0 && linear_sparse(c)) {
+    if (!c.a_q8 || !c.body_scale || !c.b_col || !c.w_scale || !c.w_rot || !out || !c.sp_meta || !c.sp_over_cnt ||
+        !c.sp_over || c.sp_over_ld < (c.R + 1) / 2 || c.N <= 0 || c.K <= 0 || c.R >= c.K)
+      return TQ_ERR_BAD_ARG;
+    if (c.N % 8 != 0 || c.K > 65536) return TQ_ERR_UNSUPPORTED;
+    if (!aligned16(c.a_q8) || !aligned16(c.b_col) || !aligned16(out) || !aligned16(c.w_scale) || !aligned16(c.w_rot) ||
+        !aligned16(c.w_t) || !aligned16(c.sp_over_cnt) || (c.bias && !aligned16(c.bias)))
+      return TQ_ERR_MISALIGNED;
+    return run_sparse_gemm(c.a_q8, c.body_scale, c.b_col, c.w_scale, c.w_rot, c.w_t, linear_sparse_tail(c), c.bias, out, nullptr,
+                           nullptr, c.M, c.N, c.K, c.act, early, (cudaStream_t)stream);
+  }
   return run_split_gemm_mma(c.a_q8, c.body_scale, c.b_col, c.w_scale, c.w_rot, c.tail_idx16, c.tail_val, c.tail_ld,
                             c.tail_ptr, c.ptr_ld, c.tail_rec, c.tail_cnt, c.tail_dense, c.R, c.bias, out, nullptr, nullptr,
-                            c.M, c.N, c.K, c.act, early, stream);
+                            c.M, c.N, c.K, c.act, early, stream, !sparse_and_dense(c));
 }
 
 }  // namespace
@@ -108,6 +149,11 @@ extern "C" int tq_linear_outputs(const tq_linear_call* call, int shared) {
       call->engine < TQ_LINEAR_DECODE || call->engine > TQ_LINEAR_GATHER)
     return TQ_ERR_BAD_ARG;
   return tq::linear_outputs(*call, shared != 0);
+}
+
+extern "C" int tq_linear_sparse(const tq_linear_call* call, int shared) {
+  if (!call || call->M < 0 || call->N <= 0 || call->K <= 0 || call->R < 0 || call->R >= call->K) return TQ_ERR_BAD_ARG;
+  return (shared ? tq::tail_can_be_sparse(*call) && tq::g_gemm_pair_mode < 0 && call->M > 64 : tq::linear_sparse(*call)) ? 1 : 0;
 }
 
 extern "C" int tq_linear_forward(const tq_linear_call* call, const void* x, void* out, void* stream) {

@@ -274,6 +274,12 @@ int run_col_to_row_s4(const uint8_t* b_col, uint8_t* b_row, int N, int K, cudaSt
 
 }  // namespace tq
 
+extern "C" int tq_transpose_bf16(const void* in, void* out, int N, int K, void* stream) {
+  if (!in || !out || N < 0 || K < 0) return TQ_ERR_BAD_ARG;
+  if (N == 0 || K == 0) return TQ_OK;
+  return tq::run_transpose_bf16(in, out, N, K, (cudaStream_t)stream);
+}
+
 extern "C" int tq_dequant_finish(const int32_t* C, const float* body_scale, const float* w_scale, const float* tail,
                                  const float* bias, void* out_bf16, int M, int N, void* stream) {
   if (!C || !body_scale || !w_scale || !out_bf16 || M < 0 || N <= 0) return TQ_ERR_BAD_ARG;

@@ -22,7 +22,7 @@ int run_prologue(const void* x, int M, int K, int had_kind, int R, int dr, float
                  uint8_t* a_pack, int8_t* a_q8, float* body_scale, float* top_scale, uint16_t* tail_idx16,
                  void* tail_val, int tail_ld, uint16_t* tail_ptr, int ptr_ld, uint32_t* tail_rec, uint16_t* tail_cnt,
                  int32_t* idx32, int8_t* top_q, void* x_rot, const void* gamma, float rms_eps, cudaStream_t st,
-                 int dtype, void* tail_dense) {
+                 int dtype, void* tail_dense, const SparseTail* sparse) {
   if ((tail_idx16 || tail_val) && tail_ld < R) return TQ_ERR_BAD_ARG;
   if (gamma && !aligned16(gamma)) return TQ_ERR_MISALIGNED;
   if (tail_ptr && (ptr_ld < K / 128 + 1 || K % 128 != 0)) return TQ_ERR_BAD_ARG;
@@ -30,7 +30,8 @@ int run_prologue(const void* x, int M, int K, int had_kind, int R, int dr, float
   if (!x || (!a_pack && !a_q8) || !body_scale || M < 0 || K <= 0 || R < 0 || R >= K) return TQ_ERR_BAD_ARG;
   if (dr < 1 || dr > K) return TQ_ERR_BAD_ARG;
   if (!aligned16(x) || (a_pack && !aligned16(a_pack)) || (a_q8 && !aligned16(a_q8)) || (x_rot && !aligned16(x_rot)) ||
-      (tail_dense && !aligned16(tail_dense)))
+      (tail_dense && !aligned16(tail_dense)) ||
+      (sparse && ((reinterpret_cast<uintptr_t>(sparse->val) & 31) || !aligned16(sparse->meta))))
     return TQ_ERR_MISALIGNED;
   if (M == 0) return TQ_OK;
   PrologueParams p;
@@ -58,6 +59,11 @@ int run_prologue(const void* x, int M, int K, int had_kind, int R, int dr, float
   p.tail_dense = reinterpret_cast<uint16_t*>(tail_dense);
   p.gamma = reinterpret_cast<const uint16_t*>(gamma);
   p.rms_eps = rms_eps;
+  p.sp = SparseTail{};
+  if (sparse && R > 0) {
+    if (!sparse->val || !sparse->meta || !sparse->over_cnt || !sparse->over || sparse->over_ld < (R + 1) / 2) return TQ_ERR_BAD_ARG;
+    p.sp = *sparse;
+  }
   // 64 elements per thread issue fewer instructions per element, 16 give a row a quarter of the latency: the lines lie where
   // the rows no longer fit the chip at once (K = 4096: 9.2 against 9.8 us at 300 rows, 7.8 / 5.7 at 64; K = 12288, one
   // CTA of 768 threads per SM: 16.9 / 23.7 at 300, 10.0 / 9.2 at 61).

@@ -254,13 +254,16 @@ struct FS {
   static constexpr int RED_OFF = HIST_OFF + 1024;          // 16 words: block max / sums
   static constexpr int RES_OFF = RED_OFF + 64;             // 8 words: select result
   static constexpr int SCAN_OFF = RES_OFF + 32;            // 8 words: warp totals of the scan
-  static constexpr int BAR_OFF = SCAN_OFF + 32;            // mbarrier (8 B) + abort flag
+  static constexpr int OVER_OFF = SCAN_OFF + 32;           // 8 words: entries beyond two of a group, by warp
+  static constexpr int TAB_OFF = OVER_OFF + 32;            // group table
+  static constexpr int BAR_OFF = TAB_OFF + 128;            // mbarrier (8 B) + abort flag
   static constexpr int DYN = BAR_OFF + 16 + 1024;          // + alignment slack
 };
 
 constexpr int fast_min_ctas(int K) { return K <= 4096 ? 10 : (K <= 12288 ? 3 : 2); }
 
-template <int KIND, int K, int DT, bool NORM>
+// SP: the tail in its 2:4-sparse form too (p.sp)
+template <int KIND, int K, int DT, bool NORM, bool SP>
 __global__ void __launch_bounds__(K / 64, fast_min_ctas(K))
 prologue_fast_kernel(const __grid_constant__ CUtensorMap tmap_x, const PrologueParams p) {
   using S = FS<KIND, K>;
@@ -286,8 +289,11 @@ prologue_fast_kernel(const __grid_constant__ CUtensorMap tmap_x, const PrologueP
   uint32_t* scanw = reinterpret_cast<uint32_t*>(sm + S::SCAN_OFF);
   const uint32_t bar = base + S::BAR_OFF;
   volatile int* abort_flag = reinterpret_cast<volatile int*>(sm + S::BAR_OFF + 8);
+  uint32_t* const overw = reinterpret_cast<uint32_t*>(sm + S::OVER_OFF);
+  uint2* const table = reinterpret_cast<uint2*>(sm + S::TAB_OFF);
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  if (SP && tid < 16) table[tid] = GROUP_TABLE.e[tid];
   const int R = p.R;
   const smp my_row = rowbuf + tid * 128;
   const uint32_t my_sw = (uint32_t)(tid & 7) << 4;
@@ -626,6 +632,7 @@ prologue_fast_kernel(const __grid_constant__ CUtensorMap tmap_x, const PrologueP
     // word i), bit 16 + i = element 2 i + 1.
     uint32_t tm[2] = {0u, 0u};
     int tail_before = 0;  // tail entries of the row in front of this thread's elements
+    int n_over = 0;       // this thread's entries beyond two of a group of four
     if (R > 0) {
       const uint32_t T2 = (uint32_t)Tkp | ((uint32_t)Tkp << 16);
       const uint32_t c_le = 0x80008000u + T2, c_lt = 0x7fff7fffu + T2;  // per half: top bit set <=> d <= T, d < T
@@ -755,6 +762,33 @@ prologue_fast_kernel(const __grid_constant__ CUtensorMap tmap_x, const PrologueP
           }
         }
       }
+      if (SP) {
+        if ((uint32_t)Tkp == kmax) {   // the threshold is zero: entries that are add nothing
+#pragma unroll
+          for (int j = 0; j < 32; ++j) {
+            if (!(w[j] & 0x7fffu)) tm[j >> 4] &= ~(1u << (j & 15));
+            if (!(w[j] & 0x7fff0000u)) tm[j >> 4] &= ~(0x10000u << (j & 15));
+          }
+        }
+        // ---- 2:4-sparse operand: a byte permutation per group of four, picked by a table
+        uint32_t v[16], places[2] = {0u, 0u};
+#pragma unroll
+        for (int g = 0; g < 16; ++g) {
+          const uint2 e = table[group_index(tm[g >> 3], (2 * g) & 15)];
+          v[g] = prmt(w[2 * g], w[2 * g + 1], e.x) & e.y;
+          places[g >> 3] |= (e.x >> 16) << (4 * (g & 7));
+        }
+        uint16_t* const dst = p.sp.val + (size_t)m * (K / 2) + 32 * tid;
+        st_global_v8(dst, v);
+        st_global_v8(dst + 16, v + 8);
+        *reinterpret_cast<uint2*>(p.sp.meta + (size_t)m * (K / 32) + 2 * tid) = make_uint2(places[0], places[1]);
+        int x0, x1;
+        over_groups(tm[0], x0);
+        over_groups(tm[1], x1);
+        n_over = x0 + x1;
+        const int w_over = __reduce_add_sync(FM, n_over);
+        if (lane == 0) overw[warp] = (uint32_t)w_over;
+      }
     }
 
     // ---- INT4 codes of the body: t = x * (1 / scale), rounded by adding 1.5 * 2^23 (the low byte of the sum is the
@@ -845,14 +879,43 @@ prologue_fast_kernel(const __grid_constant__ CUtensorMap tmap_x, const PrologueP
       p.body_scale[m] = bscale;
       if (p.top_scale) p.top_scale[m] = tscale;
     }
+    if (SP) {   // (R > 0) the list of the entries beyond two of a group, in index order
+      __syncthreads();
+      int total = 0, pos = 0;
+#pragma unroll
+      for (int q = 0; q < NW; ++q) {
+        if (q == warp) pos = total;
+        total += (int)overw[q];
+      }
+      if (tid == 0) p.sp.over_cnt[m] = (uint16_t)total;
+      if (overw[warp]) {   // (uniform over the warp)
+        int incl = n_over;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const int t = __shfl_up_sync(FM, incl, o);
+          if (lane >= o) incl += t;
+        }
+        pos += incl - n_over;
+        if (n_over) {
+#pragma unroll
+          for (int h = 0; h < 2; ++h)
+            for_each_over(tm[h], over_groups(tm[h], incl), [&](int e0) {
+              const int e = 32 * h + e0;
+              const uint32_t vb = lds16(my_row + ((((uint32_t)e >> 3) << 4) ^ my_sw) + ((uint32_t)e & 7u) * 2u);
+              p.sp.over[(size_t)m * p.sp.over_ld + pos] = (uint32_t)(64 * tid + e) | (vb << 16);
+              ++pos;
+            });
+        }
+      }
+    }
     __syncthreads();  // the next row's load overwrites the row buffer; hist / res / red / scanw start over
   }
 }
 
-template <int KIND, int K, int DT, bool NORM>
+template <int KIND, int K, int DT, bool NORM, bool SP = false>
 int launch_fast(const PrologueParams& p, cudaStream_t st) {
   using S = FS<KIND, K>;
-  auto kern = prologue_fast_kernel<KIND, K, DT, NORM>;
+  auto kern = prologue_fast_kernel<KIND, K, DT, NORM, SP>;
   static bool configured[64] = {};
   static int grid_per_dev[64] = {};
   int dev = 0;
@@ -889,6 +952,15 @@ int run_prologue_fast(int kind, int K, int dtype, const PrologueParams& p, cudaS
     if (kind != TQ_HAD_NONE || norm) return TQ_ERR_UNSUPPORTED;
     if (K == 4096) return launch_fast<TQ_HAD_NONE, 4096, TQ_FP16, false>(p, st);
     if (K == 12288) return launch_fast<TQ_HAD_NONE, 12288, TQ_FP16, false>(p, st);
+    return TQ_ERR_UNSUPPORTED;
+  }
+  if (p.sp.val) {   // (full rotations only)
+#define TQ_FAST_SP(KIND, KK)                     \
+  if (kind == KIND && K == KK)                   \
+    return norm ? launch_fast<KIND, KK, TQ_BF16, true, true>(p, st) : launch_fast<KIND, KK, TQ_BF16, false, true>(p, st);
+    TQ_FAST_SP(TQ_HAD_WHT, 4096)
+    TQ_FAST_SP(TQ_HAD_KRON12, 12288)
+#undef TQ_FAST_SP
     return TQ_ERR_UNSUPPORTED;
   }
 #define TQ_FAST(KIND, KK)                        \

@@ -39,7 +39,9 @@ struct WS {
   static constexpr int RED_OFF = HIST_OFF + 1024;               // [32] warp maxima
   static constexpr int SCAN_OFF = RED_OFF + 128;                // [32] warp totals
   static constexpr int SUM_OFF = SCAN_OFF + 128;                // [256] sums of squares
-  static constexpr int BYTES = SUM_OFF + 1024;
+  static constexpr int OVER_OFF = SUM_OFF + 1024;               // [32] entries beyond two of a group, by warp
+  static constexpr int TAB_OFF = OVER_OFF + 128;                // group table
+  static constexpr int BYTES = TAB_OFF + 128;
 };
 
 // rank is 1-based in (key descending) order; dd[j] holds the distances kmax - key of elements 2j (low half) and 2j + 1 (high
@@ -123,7 +125,8 @@ __device__ __forceinline__ Sel select_rank_wide(const uint32_t (&dd)[W], int ran
 // register budgets: 64 up to 4096 and at 8192, 72 .. 85 for the others
 constexpr int wide_min_ctas(int K) { return K <= 1024 ? 16 : K == 2048 ? 8 : K == 4096 ? 4 : K <= 8192 ? 2 : 1; }
 
-template <int KIND, int K, int DT, bool NORM>
+// SP: the tail in its 2:4-sparse form too (p.sp)
+template <int KIND, int K, int DT, bool NORM, bool SP>
 __global__ void __launch_bounds__(K / 16, wide_min_ctas(K)) prologue_wide_kernel(const PrologueParams p) {
   using S = WS<KIND, K>;
   constexpr int NT = S::NT, NW = S::NW;
@@ -135,9 +138,12 @@ __global__ void __launch_bounds__(K / 16, wide_min_ctas(K)) prologue_wide_kernel
   uint32_t* const red = reinterpret_cast<uint32_t*>(sm + S::RED_OFF);
   uint32_t* const scanw = reinterpret_cast<uint32_t*>(sm + S::SCAN_OFF);
   float* const sums = reinterpret_cast<float*>(sm + S::SUM_OFF);
+  uint32_t* const overw = reinterpret_cast<uint32_t*>(sm + S::OVER_OFF);
+  uint2* const table = reinterpret_cast<uint2*>(sm + S::TAB_OFF);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int R = p.R;
   const smp my_row = rowbuf + tid * 32;
+  if (SP && tid < 16) table[tid] = GROUP_TABLE.e[tid];   // (read behind the barriers of the selection)
 
   pdl_wait();   // the rows may come from the kernel in front
   pdl_trigger();
@@ -443,6 +449,7 @@ __global__ void __launch_bounds__(K / 16, wide_min_ctas(K)) prologue_wide_kernel
 
     // ---- tail membership.  Mask layout: bit i = element 2 i (low half of word i), bit 16 + i = element 2 i + 1.
     uint32_t tm = 0u;
+    int n_over = 0;   // this thread's entries beyond two of a group of four
     if (R > 0) {
       const uint32_t T2 = (uint32_t)Tkp | ((uint32_t)Tkp << 16);
       const uint32_t c_le = 0x80008000u + T2, c_lt = 0x7fff7fffu + T2;   // per half: top bit set <=> d <= T, d < T
@@ -551,6 +558,27 @@ __global__ void __launch_bounds__(K / 16, wide_min_ctas(K)) prologue_wide_kernel
           ++r;
         }
       }
+      if (SP) {   // 2:4-sparse operand (see the 64-element kernel)
+        if ((uint32_t)Tkp == kmax) {   // the threshold is zero: entries that are add nothing
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            if (!(w[j] & 0x7fffu)) tm &= ~(1u << j);
+            if (!(w[j] & 0x7fff0000u)) tm &= ~(0x10000u << j);
+          }
+        }
+        uint32_t v[4], places = 0u;
+#pragma unroll
+        for (int g = 0; g < 4; ++g) {
+          const uint2 e = table[group_index(tm, 2 * g)];
+          v[g] = prmt(w[2 * g], w[2 * g + 1], e.x) & e.y;
+          places |= (e.x >> 16) << (4 * g);
+        }
+        *reinterpret_cast<uint4*>(p.sp.val + (size_t)m * (K / 2) + 8 * tid) = make_uint4(v[0], v[1], v[2], v[3]);
+        reinterpret_cast<uint16_t*>(p.sp.meta)[(size_t)m * (K / 16) + tid] = (uint16_t)places;
+        over_groups(tm, n_over);
+        const int w_over = __reduce_add_sync(FM, n_over);
+        if (lane == 0) overw[warp] = (uint32_t)w_over;
+      }
     }
 
     // ---- INT4 codes of the body (see the 64-element kernel): reciprocal product, magic-number rounding, IEEE division
@@ -616,14 +644,35 @@ __global__ void __launch_bounds__(K / 16, wide_min_ctas(K)) prologue_wide_kernel
       p.body_scale[m] = bscale;
       if (p.top_scale) p.top_scale[m] = tscale;
     }
+    if (SP) {   // (R > 0) the list of the entries beyond two of a group, in index order
+      __syncthreads();
+      const int cw = lane < NW ? (int)overw[lane] : 0;
+      const int total = __reduce_add_sync(FM, cw);
+      int pos = __reduce_add_sync(FM, lane < warp ? cw : 0);
+      if (tid == 0) p.sp.over_cnt[m] = (uint16_t)total;
+      if (overw[warp]) {   // (uniform over the warp)
+        int incl = n_over;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const int t = __shfl_up_sync(FM, incl, o);
+          if (lane >= o) incl += t;
+        }
+        pos += incl - n_over;
+        if (n_over)
+          for_each_over(tm, over_groups(tm, incl), [&](int e) {
+            p.sp.over[(size_t)m * p.sp.over_ld + pos] = (uint32_t)(16 * tid + e) | (lds16(my_row + 2 * e) << 16);
+            ++pos;
+          });
+      }
+    }
     if (m + (int)gridDim.x < p.M) __syncthreads();   // the next row starts over on all buffers
   }
 }
 
-template <int KIND, int K, int DT, bool NORM>
+template <int KIND, int K, int DT, bool NORM, bool SP = false>
 int launch_wide(const PrologueParams& p, cudaStream_t st) {
   using S = WS<KIND, K>;
-  auto kern = prologue_wide_kernel<KIND, K, DT, NORM>;
+  auto kern = prologue_wide_kernel<KIND, K, DT, NORM, SP>;
   static int grid_per_dev[64] = {};
   int dev = 0;
   const int sms = current_device_sms(&dev);
@@ -651,6 +700,20 @@ int run_prologue_wide(int kind, int K, int dtype, const PrologueParams& p, cudaS
     if (kind != TQ_HAD_NONE || norm) return TQ_ERR_UNSUPPORTED;
     if (K == 4096) return launch_wide<TQ_HAD_NONE, 4096, TQ_FP16, false>(p, st);
     if (K == 12288) return launch_wide<TQ_HAD_NONE, 12288, TQ_FP16, false>(p, st);
+    return TQ_ERR_UNSUPPORTED;
+  }
+  if (p.sp.val) {   // (full rotations only)
+#define TQ_WIDE_SP(KIND, KK)                     \
+  if (kind == KIND && K == KK)                   \
+    return norm ? launch_wide<KIND, KK, TQ_BF16, true, true>(p, st) : launch_wide<KIND, KK, TQ_BF16, false, true>(p, st);
+    TQ_WIDE_SP(TQ_HAD_WHT, 512)
+    TQ_WIDE_SP(TQ_HAD_WHT, 1024)
+    TQ_WIDE_SP(TQ_HAD_WHT, 2048)
+    TQ_WIDE_SP(TQ_HAD_WHT, 4096)
+    TQ_WIDE_SP(TQ_HAD_WHT, 8192)
+    TQ_WIDE_SP(TQ_HAD_KRON12, 6144)
+    TQ_WIDE_SP(TQ_HAD_KRON12, 12288)
+#undef TQ_WIDE_SP
     return TQ_ERR_UNSUPPORTED;
   }
 #define TQ_WIDE(KIND, KK)                        \

@@ -67,7 +67,10 @@ int run_pair_gemm(const int8_t* a_q8, const float* body_scale, const uint8_t* b_
                   const void* w_rot, const uint16_t* tail_idx16, const void* tail_val, int tail_ld,
                   const uint16_t* tail_ptr, int ptr_ld, const uint32_t* tail_rec, const uint16_t* tail_cnt,
                   const void* tail_dense, int R, const float* bias, void* out_bf16, int32_t* dbg_acc, float* dbg_tail,
-                  int M, int N, int K, int act, cudaStream_t st);
+                  int M, int N, int K, int act, bool records_filled, cudaStream_t st);
+int run_sparse_gemm(const int8_t* a_q8, const float* body_scale, const uint8_t* b_col, const float* w_scale, const void* w_rot,
+                    const void* w_t, const SparseTail& sp, const float* bias, void* out_bf16, int32_t* dbg_acc, float* dbg_tail,
+                    int M, int N, int K, int act, bool early, cudaStream_t st);
 }  // namespace tq
 
 #ifdef TQ_GEMM_PROFILE
@@ -113,13 +116,31 @@ constexpr long DENSE_OUTPUTS = 1 << 21;
 // pair kernel goes through ceil(tiles / 74) rounds of 1.02 us per K slice and 5 us with a tail (0.34 and 3.5 without), and
 // takes about 5 us for the launch and ring fill.  At N = K = 4096 the line lies between 700 and 1000 rows, at
 // N = 28672 between 100 and 176.
+static float pair_us(int M, int N, int K, int R) {
+  const int tiles = ((M + 255) / 256) * ((N + 255) / 256), rounds = (tiles + 73) / 74;
+  return R > 0 ? rounds * ((K / 128) * 1.02f + 5.0f) + 5.0f : rounds * ((K / 128) * 0.34f + 3.5f) + 6.0f;
+}
+static bool stream_can(int M, int N, int R) { return M <= DENSE_ROWS || R == 0 || (long)M * N <= DENSE_OUTPUTS; }
 static bool stream_is_faster(int M, int N, int K, int R) {
   if (g_gemm_pair_mode >= 0) return g_gemm_pair_mode == 0;
   if (M <= 64) return true;
-  if (M > DENSE_ROWS && R > 0 && (long)M * N > DENSE_OUTPUTS) return false;
-  const int tiles = ((M + 255) / 256) * ((N + 255) / 256), rounds = (tiles + 73) / 74;
-  const float pair = R > 0 ? rounds * ((K / 128) * 1.02f + 5.0f) + 5.0f : rounds * ((K / 128) * 0.34f + 3.5f) + 6.0f;
-  return plan_stream(M, N, K, R > 0 ? ST_TAIL : ST_INT8).us < pair;
+  return stream_can(M, N, R) && plan_stream(M, N, K, R > 0 ? ST_TAIL : ST_INT8).us < pair_us(M, N, K, R);
+}
+
+// The kernel with the 2:4-sparse tail (tq_gemm_sparse.cu): ceil(tiles / 74) rounds of 0.55 us per K slice and 3.7 us (narrow last
+// tiles take as long as full ones), a share of the weight stream, and 0.08 us for each left-over entry among four rows of a
+// tile; 5.5 us around it, 1.5 of them in the prologue.  `e`: left-over entries of a row whose R entries lie independently.  Fit
+// to 200 shapes (80..2048 rows, N = 1024..28672, K = 1024, 4096, 12288, R = 0.05 K): 5 % off on average, 0.4 % lost by the
+// choice.  300 x 24576 x 4096: 88 us, 118 and 122 on the other two; 2048 x 4096 x 4096: 68 against 81 on pairs.
+static float sparse_us(int M, int N, int K, int R) {
+  const int rounds = (((M + 255) / 256) * ((N + 223) / 224) + 73) / 74;
+  const float q = (float)R / (float)K, e = (float)K * q * q * q * (1.0f - 0.5f * q);
+  return rounds * ((K / 128) * 0.55f + 3.7f + 5.2f * e) + 5.5f + 1.25e-7f * (float)N * (float)K;
+}
+static bool sparse_is_faster(int M, int N, int K, int R) {
+  if (g_gemm_pair_mode >= 0 || M <= 64) return false;
+  const float us = sparse_us(M, N, K, R);
+  return us < pair_us(M, N, K, R) && (!stream_can(M, N, R) || us < plan_stream(M, N, K, ST_TAIL).us);
 }
 
 static int run_split_gemm_mma(const int8_t* a_q8, const float* body_scale, const uint8_t* b_col,
@@ -127,7 +148,7 @@ static int run_split_gemm_mma(const int8_t* a_q8, const float* body_scale, const
                               const void* tail_val, int tail_ld, const uint16_t* tail_ptr, int ptr_ld,
                               const uint32_t* tail_rec, const uint16_t* tail_cnt, const void* tail_dense, int R,
                               const float* bias, void* out_bf16, int32_t* dbg_acc, float* dbg_tail, int M, int N, int K,
-                              int act, bool early, void* stream) {
+                              int act, bool early, void* stream, bool records_filled = true) {
   if (!a_q8 || !body_scale || !b_col || !w_scale || !out_bf16 || M < 0 || N <= 0 || K <= 0 || R < 0 || R >= K)
     return TQ_ERR_BAD_ARG;
   const bool records = tail_idx16 && tail_val && tail_ld >= R && tail_ptr && ptr_ld >= K / 128 + 1 && tail_rec && tail_cnt;
@@ -143,7 +164,7 @@ static int run_split_gemm_mma(const int8_t* a_q8, const float* body_scale, const
     return run_stream_gemm(a_q8, body_scale, b_col, w_scale, w_rot, tail_dense, R, bias, out_bf16, dbg_acc, dbg_tail, M, N,
                            K, act, early, (cudaStream_t)stream);
   return run_pair_gemm(a_q8, body_scale, b_col, w_scale, w_rot, tail_idx16, tail_val, tail_ld, tail_ptr, ptr_ld, tail_rec,
-                       tail_cnt, tail_dense, R, bias, out_bf16, dbg_acc, dbg_tail, M, N, K, act, (cudaStream_t)stream);
+                       tail_cnt, tail_dense, R, bias, out_bf16, dbg_acc, dbg_tail, M, N, K, act, records_filled, (cudaStream_t)stream);
 }
 }  // namespace tq
 

@@ -23,6 +23,9 @@ import torch
 from . import _lib, ops
 
 
+SPARSE_FIELDS = ("sp_val", "sp_meta", "sp_over_cnt", "sp_over")
+
+
 def interleave_gate_up(w_gate: torch.Tensor, w_up: torch.Tensor) -> torch.Tensor:
     """[2 I, K] weight of a fused gate_up projection with rows (gate_0, up_0, gate_1, up_1, ...): the layout
     `SplitLinear(..., epilogue="swiglu")` expects."""
@@ -42,6 +45,7 @@ class _Workspace:
         self.M, self.K, self.R, self.engine = M, K, R, engine
         self.pro = None
         self.outputs, self.asked = 0, (-1, -1)   # TQ_OUT_* bits held; for what (see SplitLinear._provide)
+        self.sparse = None   # the tail in its 2:4-sparse form
         if with_pro:
             self.pro = ops.PrologueOut(a_pack=None, body_scale=empty(M, torch.float32), top_scale=empty(M, torch.float32),
                                        tail_idx=None, tail_val=None, R=R)
@@ -50,6 +54,7 @@ class _Workspace:
         self.call = None   # (a reference to) the native description of a forward out of these buffers; what it was filled in from
         self.call_pro = None
         self.call_src = ()
+        self.rot_version = None   # of w_rot, where the description rests on its transpose
 
     def hold(self, outputs: int) -> None:
         """Adds the prologue outputs of `outputs` (TQ_OUT_* bits) that are not there yet."""
@@ -74,6 +79,17 @@ class _Workspace:
         if new & _lib.TQ_OUT_DENSE:
             p.tail_dense = empty((M, K), torch.bfloat16)
         self.outputs |= new
+
+    def use_sparse(self, use: bool) -> None:
+        """Whether the prologue fills the tail in its 2:4-sparse form."""
+        if use == (self.pro.sparse is not None):
+            return
+        if use and self.sparse is None:
+            M, K = self.M, self.K
+            self.sparse = tuple(torch.empty(s, dtype=t, device=self.out.device) for s, t in (
+                ((M, K // 2), torch.bfloat16), ((M, K // 32), torch.int32), ((M,), torch.int16),
+                ((M, (self.R + 1) // 2), torch.int32)))
+        self.pro = dataclasses.replace(self.pro, sparse=self.sparse if use else None)
 
 
 class SplitLinear:
@@ -130,6 +146,7 @@ class SplitLinear:
         self.reuse_output = bool(reuse_output)
         self._ws: Dict[int, _Workspace] = {}
         self._ws_shared: Dict[int, _Workspace] = {}
+        self._t_of = (None, None, None)   # a transpose, the w_rot and the version of it that it belongs to
 
     @classmethod
     def from_prepared(cls, w: "ops.PreparedWeight", ratio: float = 0.05, activation_percentile: float = 100.0,
@@ -232,6 +249,7 @@ class SplitLinear:
         if bits < 0:
             _lib.check(bits, self._what(ws.M))
         ws.hold(bits)
+        ws.use_sparse(_lib.load().tq_linear_sparse(ctypes.byref(c), int(shared and self.tail_engine == "mma")) > 0)
         ws.asked = (ops.gemm_pair_mode_changes, int(shared))
 
     def _new_workspace(self, M: int, with_pro: bool) -> _Workspace:
@@ -267,7 +285,23 @@ class SplitLinear:
         """Builds the [K, N] transpose of the rotated weights that the small-M tail reads, ahead of the first small-M
         forward (which otherwise builds it: an allocation inside that call)."""
         if self.R and self.w.w_t is None:
-            self.w.w_t = self.w.w_rot.t().contiguous()
+            r = self.w.w_rot
+            self.w.w_t = ops.transpose_bf16(r) if r.device.type == "cuda" and r.is_contiguous() else r.t().contiguous()
+
+    def _rot_version(self) -> int:
+        r = self.w.w_rot
+        return -1 if r is None or r.is_inference() else r._version
+
+    def _prepare_sparse(self, own: _Workspace) -> None:
+        """The transpose that the left-over entries of the sparse tail are read from.  A layer that had none did not ask for it
+        and is not expected to keep it in line: it is made again when `w_rot` was replaced or changed in place since."""
+        w, version = self.w, self._rot_version()
+        t, rot, v = self._t_of
+        if w.w_t is not None and w.w_t is t and (w.w_rot is not rot or version != v):
+            w.w_t = None
+        self.prepare_decode()
+        self._t_of = (w.w_t, w.w_rot, version)
+        own.rot_version = version
 
     def _described(self, own: _Workspace) -> bool:
         """Whether `own.call` still names what this layer consists of.  All of it can be replaced between two forwards, and a
@@ -279,6 +313,7 @@ class SplitLinear:
                 and r is w.w_rot and (r is None or r.data_ptr() == pr) and t is w.w_t and (t is None or t.data_ptr() == pt)
                 and i is w.bias and (i is None or i.data_ptr() == pi)
                 and g is self.rms_weight and (g is None or g.data_ptr() == pg)
+                and (own.rot_version is None or own.rot_version == self._rot_version())
                 and kind == w.had_kind and rank == self.descending_rank and eps == self.rms_eps and act == self.epilogue)
 
     def _check_parts(self, engine: int) -> None:
@@ -306,8 +341,12 @@ class SplitLinear:
         `own`."""
         if own.call is not None and own.call_pro is pro and self._described(own):
             return own.call
+        own.rot_version = None
         if own.engine == _lib.TQ_LINEAR_DECODE:
             self.prepare_decode()
+        elif own.engine == _lib.TQ_LINEAR_FUSED and pro.sparse is not None and \
+                ops.takes_sparse(own.M, self.N, self.K, self.R, self.w.had_kind):
+            self._prepare_sparse(own)
         own.call = None   # (a part that is refused must not leave the former description in force)
         self._check_parts(own.engine)
         w, p = self.w, ops._ptr
@@ -322,7 +361,8 @@ class SplitLinear:
             b_col=p(w.b_col), w_scale=p(w.w_scale), w_rot=p(w.w_rot), w_t=p(w.w_t), bias=p(w.bias),
             rms_weight=p(self.rms_weight), a_pack=p(pro.a_pack), a_q8=p(pro.a_q8), body_scale=p(pro.body_scale),
             top_scale=p(pro.top_scale), tail_idx16=p(pro.tail_idx), tail_val=p(pro.tail_val), tail_ptr=p(pro.tail_ptr),
-            tail_rec=p(pro.tail_rec), tail_cnt=p(pro.tail_cnt), tail_dense=p(pro.tail_dense), tail=p(own.tail)))
+            tail_rec=p(pro.tail_rec), tail_cnt=p(pro.tail_cnt), tail_dense=p(pro.tail_dense), tail=p(own.tail),
+            **({} if pro.sparse is None else dict(zip(SPARSE_FIELDS, map(p, pro.sparse)), sp_over_ld=pro.sparse[3].shape[1]))))
         return own.call
 
     def _what(self, M: int) -> str:

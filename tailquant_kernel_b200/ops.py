@@ -18,9 +18,10 @@ PyTorch is used for device memory and streams only.  Nothing here computes on th
 """
 from __future__ import annotations
 
+import ctypes
 import math
 from dataclasses import dataclass
-from typing import Optional
+from typing import Optional, Tuple
 
 import torch
 
@@ -115,6 +116,9 @@ class PrologueOut:
     tail_rec: Optional[torch.Tensor] = None  # [2 ceil(M/256), K/64, 128, TAIL_REC_CAP] int32: tile position | bf16 << 16
     tail_cnt: Optional[torch.Tensor] = None  # [2 ceil(M/256), K/64, 128] int16: entries per (row, 64-wide half slice)
     tail_dense: Optional[torch.Tensor] = None  # [M, K] bf16: the rotated row, zero outside the tail (R > 0)
+    # the tail as a 2:4-sparse operand (tq_split_gemm_sparse): sp_val [M, K/2] bf16, sp_meta [M, K/32] int32,
+    # sp_over_cnt [M] int16, sp_over [M, (R + 1) / 2] int32
+    sparse: Optional[Tuple[torch.Tensor, ...]] = None
 
 
 def split_prologue(x: torch.Tensor, had_kind: int, R: int, descending_rank: Optional[int] = None,
@@ -241,6 +245,14 @@ def prepare_weight(W: torch.Tensor, had_kind: Optional[int] = None, eps: float =
     return PreparedWeight(N, K, had_kind, b_col, w_scale, w_t, b_row, w_rot if keep_w_rot else None, b32)
 
 
+def transpose_bf16(w: torch.Tensor) -> torch.Tensor:
+    """[K, N] transpose of a bf16 matrix [N, K] (rotated weights -> `w_t`)."""
+    _check_cuda(w, "w", torch.bfloat16)
+    out = torch.empty((w.shape[1], w.shape[0]), dtype=torch.bfloat16, device=w.device)
+    _lib.check(_lib.load().tq_transpose_bf16(_ptr(w), _ptr(out), w.shape[0], w.shape[1], _stream()), "transpose_bf16")
+    return out
+
+
 # --------------------------------------------------------------------------- GEMM
 def _gemm_dims(A_pack, B_pack, M, N, K):
     _check_cuda(A_pack, "A_pack", torch.uint8)
@@ -298,6 +310,12 @@ def split_gemm_fused(A_pack, body_scale, B_pack, w_scale, out, tail=None, bias=N
     return out
 
 
+def takes_sparse(M: int, N: int, K: int, R: int, had_kind: int = TQ_HAD_WHT) -> bool:
+    """Whether a fused linear reads the tail in its 2:4-sparse form where it finds it (the rule of tq_linear_compute)."""
+    c = _lib.LinearCall(M=M, N=N, K=K, R=R, had_kind=had_kind, engine=_lib.TQ_LINEAR_FUSED)
+    return _lib.load().tq_linear_sparse(ctypes.byref(c), 0) > 0
+
+
 def split_gemm_mma(a_q8, body_scale, B_pack, w_scale, out, w_rot=None, pro: Optional[PrologueOut] = None,
                    R: int = 0, bias=None, dbg_acc=None, dbg_tail=None, act: str = "none"):
     """One kernel: dense INT4 x INT4 part on tcgen05 kind::i8 plus the tail as a bf16 tensor-core product
@@ -334,6 +352,16 @@ def split_gemm_mma(a_q8, body_scale, B_pack, w_scale, out, w_rot=None, pro: Opti
             _check(tuple(pro.tail_dense.shape) == (M, K), "tail_dense must be [M, K]")
     if bias is not None:
         _check_cuda(bias, "bias", torch.float32)
+    if R and pro.sparse is not None:
+        if takes_sparse(M, N, K, R):
+            _check(tuple(pro.sparse[0].shape) == (M, K // 2), "the sparse tail operand has the wrong shape")
+            rc = _lib.load().tq_split_gemm_sparse(
+                _ptr(a_q8), _ptr(body_scale), _ptr(B_pack), _ptr(w_scale), _ptr(w_rot), None, int(R), *map(_ptr, pro.sparse),
+                pro.sparse[3].shape[1], _ptr(bias), _ptr(out), _ptr(dbg_acc), _ptr(dbg_tail), M, N, K, int(act == "swiglu"), _stream())
+            _lib.check(rc, f"split_gemm_mma(M={M}, N={N}, K={K}, R={R})")
+            return out
+        if pro.tail_dense is not None:   # (the records are not filled where both of the others are)
+            tail_rec = tail_cnt = None
     common = (_ptr(a_q8), _ptr(body_scale), _ptr(B_pack), _ptr(w_scale),
               _ptr(w_rot) if R else None, _ptr(tail_idx) if R else None,
               _ptr(tail_val) if R else None, ld, _ptr(tail_ptr) if R else None,

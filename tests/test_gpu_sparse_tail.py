@@ -1,0 +1,169 @@
+"""The tail as a 2:4-sparse operand: what the prologue writes, and the GEMM that reads it.  The dense part is exact; a tail sum is
+an fp32 tensor-core sum of R products, so it differs from the exact one by at most about R roundings of the partial sums, which
+|x| |w| R bounds: 1e-5 of that, as for the other fused kernels."""
+import ctypes
+
+import numpy as np
+import pytest
+import torch
+
+from oracle import oracle as O
+from tailquant_kernel_b200 import _lib, ops
+
+pytestmark = pytest.mark.gpu
+KINDS = {O.HAD_WHT: _lib.TQ_HAD_WHT, O.HAD_KRON12: _lib.TQ_HAD_KRON12}
+
+
+def dev(bits):
+    return torch.from_numpy(np.ascontiguousarray(bits).view(np.int16)).cuda().view(torch.bfloat16)
+
+
+def activations(what, M, K, seed):
+    g = torch.Generator().manual_seed(seed)
+    x = torch.randn(M, K, generator=g)
+    if what == "hot":
+        x[:, torch.randperm(K, generator=g)[:max(1, K // 256)]] *= 50
+    elif what == "few_levels":     # channels of equal size: entries come in whole groups
+        x[:, [0, 4, 16, 64]] = 300.0
+    elif what == "one_row":        # one row of them, and one that is all ties
+        x[M // 2, :] = 0.01 * x[M // 2, :]
+        x[M // 2, [0, 4]] = 500.0
+        x[M // 3, :] = 0.0
+        x[M // 3, 5] = 3.0
+    elif what == "zeros":          # rotated rows of zeros, and of one value and zeros
+        x[::2] = 0.0
+        x[1::2] = 1.0
+    return x.to(torch.bfloat16).cuda()
+
+
+def prologue(x, K, R, wide=False):
+    """All tail forms of one prologue call, through the native description."""
+    M = x.shape[0]
+    kind = ops.default_had_kind(K)
+    e = lambda *s, t: torch.empty(s, dtype=t, device="cuda")  # noqa: E731
+    out = dict(a_q8=e(M, K, t=torch.int8), body_scale=e(M, t=torch.float32), top_scale=e(M, t=torch.float32),
+               tail_idx16=e(M, (R + 7) // 8 * 8, t=torch.int16), tail_val=e(M, (R + 7) // 8 * 8, t=torch.bfloat16),
+               tail_dense=e(M, K, t=torch.bfloat16), sp_val=e(M, K // 2, t=torch.bfloat16), sp_meta=e(M, K // 32, t=torch.int32),
+               sp_over_cnt=e(M, t=torch.int16), sp_over=e(M, (R + 1) // 2, t=torch.int32))
+    c = _lib.LinearCall(M=M, N=8, K=K, R=R, had_kind=kind, descending_rank=ops.split_select_params(K, R)[1],
+                        engine=_lib.TQ_LINEAR_FUSED, eps=ops.EPS, tail_ld=out["tail_idx16"].shape[1],
+                        sp_over_ld=out["sp_over"].shape[1], **{k: v.data_ptr() for k, v in out.items()})
+    lib = _lib.load()
+    lib.tq_set_prologue_mode(0 if wide else -1)
+    try:
+        _lib.check(lib.tq_linear_prologue(ctypes.byref(c), x.data_ptr(), ops._stream()), "prologue")
+    finally:
+        lib.tq_set_prologue_mode(-1)
+    torch.cuda.synchronize()
+    return out
+
+
+CASES = [("plain", 3, 512, 26), ("hot", 300, 4096, 205), ("few_levels", 130, 4096, 287), ("one_row", 300, 4096, 205),
+         ("zeros", 20, 1024, 52), ("plain", 9, 2048, 1), ("hot", 140, 12288, 615), ("one_row", 33, 6144, 400),
+         ("few_levels", 40, 8192, 410)]
+
+
+@pytest.mark.parametrize("what,M,K,R", CASES)
+@pytest.mark.parametrize("wide", [False, True])
+def test_prologue_writes_the_tail_in_sparse_form(what, M, K, R, wide):
+    """The first two entries of each group in order with their places, all others in the row's list; only zeros are left out."""
+    o = prologue(activations(what, M, K, 11), K, R, wide)
+    want = o["tail_dense"].view(torch.int16).cpu().numpy().astype(np.int64) & 0xffff
+    member = np.zeros((M, K), bool)
+    np.put_along_axis(member, o["tail_idx16"].cpu().numpy()[:, :R].astype(np.int64) & 0xffff, True, 1)
+    val = (o["sp_val"].view(torch.int16).cpu().numpy().astype(np.int64) & 0xffff).reshape(M, K // 4, 2)
+    meta = o["sp_meta"].cpu().numpy().view(np.uint32).astype(np.int64)
+    nib = ((meta[:, :, None] >> (4 * np.arange(8))) & 15).reshape(M, K // 4)
+    lo, hi = nib & 3, nib >> 2
+    assert (lo < hi).all(), "places in order"
+    got = np.zeros((M, K // 4, 4), np.int64)
+    np.put_along_axis(got, np.stack((lo, hi), -1), val, -1)
+    cnt, over = o["sp_over_cnt"].cpu().numpy().astype(np.int64), o["sp_over"].cpu().numpy().view(np.uint32).astype(np.int64)
+    assert (cnt >= 0).all() and (cnt <= (R + 1) // 2).all()
+    flat = got.reshape(M, K)
+    for m in range(M):
+        k, v = over[m, :cnt[m]] & 0xffff, over[m, :cnt[m]] >> 16
+        assert (np.diff(k) > 0).all()
+        nz = (want[m] & 0x7fff) != 0
+        tail = member[m] & nz if (want[m][member[m]] & 0x7fff).min() == 0 else member[m]
+        rank = np.cumsum(tail.reshape(-1, 4), 1).reshape(-1)
+        assert np.array_equal(k, np.flatnonzero(tail & (rank > 2))), "entries beyond two of a group"
+        assert (flat[m][k] == 0).all()
+        flat[m][k] = v
+    assert np.array_equal(flat, want)
+
+
+@pytest.mark.parametrize("what,M,N,K,ratio", [
+    ("plain", 1, 8, 512, 0.05), ("plain", 129, 232, 512, 0.05), ("hot", 257, 456, 1024, 0.05), ("hot", 300, 264, 4096, 0.05),
+    ("few_levels", 300, 240, 2048, 0.05), ("one_row", 520, 224, 4096, 0.05), ("zeros", 64, 40, 1024, 0.05),
+    ("hot", 200, 72, 12288, 0.05), ("plain", 2000, 4096, 512, 0.07), ("plain", 300, 1000, 6144, 0.001)])
+@pytest.mark.parametrize("with_t", [True, False])
+def test_gemm_on_the_sparse_tail(what, M, N, K, ratio, with_t):
+    """Rows and channels that do not fill a tile, several tiles per pair, many and no left-over entries, with and without the
+    transposed weights: accumulators bit for bit, tail sums and outputs inside the bound."""
+    R = ops.ceil_ratio_count(K, ratio)
+    o = prologue(activations(what, M, K, 5), K, R)
+    g = torch.Generator().manual_seed(N)
+    w = ops.prepare_weight((torch.randn(N, K, generator=g) * 0.02).to(torch.bfloat16).cuda(), t16=True, keep_w_rot=True)
+    bias = torch.randn(N, generator=g).cuda()
+    out = torch.empty((M, N), dtype=torch.bfloat16, device="cuda")
+    acc, tail = torch.empty((M, N), dtype=torch.int32, device="cuda"), torch.empty((M, N), device="cuda")
+    p = lambda t: None if t is None else t.data_ptr()  # noqa: E731
+    _lib.check(_lib.load().tq_split_gemm_sparse(
+        p(o["a_q8"]), p(o["body_scale"]), p(w.b_col), p(w.w_scale), p(w.w_rot), p(w.w_t) if with_t else None, R, p(o["sp_val"]),
+        p(o["sp_meta"]), p(o["sp_over_cnt"]), p(o["sp_over"]), o["sp_over"].shape[1], p(bias), p(out), p(acc), p(tail), M, N, K, 0,
+        ops._stream()), "sparse gemm")
+    torch.cuda.synchronize()
+    assert ops.gemm_status() == 0
+    codes = o["a_q8"].cpu().numpy().reshape(M, K // 8, 8)[:, :, [0, 4, 1, 5, 2, 6, 3, 7]].reshape(M, K).astype(np.float64)
+    qw = O.unpack_s4(w.b_col.cpu().numpy()).astype(np.float64)
+    assert np.array_equal(acc.cpu().numpy(), (codes @ qw.T).astype(np.int64))
+    wr, d = w.w_rot.double(), o["tail_dense"].double()
+    exact = (d @ wr.T).cpu().numpy()
+    bound = 1e-5 * R * float(d.abs().max()) * float(wr.abs().max())
+    assert np.abs(tail.cpu().numpy() - exact).max() <= bound
+    y = (acc.float() * o["body_scale"][:, None]) * w.w_scale[None] + tail + bias[None]
+    assert torch.equal(out, y.to(torch.bfloat16)), "dequantised, tail and bias added, rounded once"
+
+
+@pytest.mark.parametrize("M,N,K", [(700, 8192, 1024), (1500, 4096, 4096)])
+def test_layer_with_swiglu_on_the_sparse_tail(M, N, K):
+    """The layer object takes the sparse operand at this size; SwiGLU in the epilogue against the plain layer's outputs."""
+    from tailquant_kernel_b200 import SplitLinear, interleave_gate_up
+    x = activations("hot", M, K, 3)
+    g = torch.Generator().manual_seed(9)
+    wg, wu = ((torch.randn(N // 2, K, generator=g) * 0.02).to(torch.bfloat16).cuda() for _ in range(2))
+    W = interleave_gate_up(wg, wu)
+    plain, fused = SplitLinear(W), SplitLinear(W, epilogue="swiglu")
+    y, h = plain(x), fused(x)
+    assert plain._ws[M].pro.sparse is not None and fused._ws[M].pro.sparse is not None
+    want = (torch.nn.functional.silu(y[:, 0::2].float()).to(torch.bfloat16).float() * y[:, 1::2].float()).to(torch.bfloat16)
+    diff = want.float() - h.float()
+    assert (diff != 0).float().mean() < 2e-3 and bool((diff.abs() <= want.float().abs() * 2.0 ** -7 + 1e-30).all())
+    ops.set_gemm_pair_mode(1)
+    try:
+        ref = SplitLinear(W)(x).float()
+    finally:
+        ops.set_gemm_pair_mode(-1)
+    d = (y.float() - ref).abs()
+    assert float((d != 0).float().mean()) < 1e-3 and bool((d <= ref.abs() * 2.0 ** -7 + 1e-4).all())
+
+
+def test_weights_changed_in_place_reach_the_left_over_entries():
+    """The transposed weights are a copy that the layer made: it follows `w_rot`."""
+    from tailquant_kernel_b200 import SplitLinear
+    M, N, K = 1100, 4096, 1024
+    x = activations("few_levels", M, K, 1)
+    g = torch.Generator().manual_seed(2)
+    w = (torch.randn(N, K, generator=g) * 0.02).to(torch.bfloat16).cuda()
+    lin = SplitLinear(w)
+    lin(x)
+    assert lin._ws[M].pro.sparse is not None
+    other = SplitLinear(2 * w)
+    lin.w.w_rot.copy_(other.w.w_rot)
+    lin.w.b_col.copy_(other.w.b_col)
+    lin.w.w_scale.copy_(other.w.w_scale)
+    assert torch.equal(lin(x), other(x))
+    lin.w.w_rot = SplitLinear(w).w.w_rot
+    other.w.w_rot, other.w.w_t = lin.w.w_rot, None
+    assert torch.equal(lin(x), other(x))

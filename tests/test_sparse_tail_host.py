@@ -1,0 +1,74 @@
+"""When a layer takes its tail as a 2:4-sparse operand, and what it holds for it (no GPU; see test_linear_host.py)."""
+import ctypes
+
+import pytest
+import torch
+
+from tailquant_kernel_b200 import _lib, ops
+from test_linear_host import claimed, fake, layer  # noqa: F401
+
+
+def sparse(M, N, K, R, kind=1, engine=_lib.TQ_LINEAR_FUSED, shared=0):
+    c = _lib.LinearCall(M=M, N=N, K=K, R=R, had_kind=kind, engine=engine)
+    return _lib.load().tq_linear_sparse(ctypes.byref(c), shared)
+
+
+def test_rule():
+    assert sparse(2048, 4096, 4096, 205) == 1 and sparse(2048, 4096, 12288, 615, kind=2) == 1
+    assert sparse(2048, 4096, 4096, 410) == 0                                 # many entries: groups hold more than two
+    assert sparse(2048, 4096, 14336, 717, kind=3) == sparse(2048, 4096, 4096, 205, kind=0) == 0   # not spread over K
+    assert sparse(2048, 4096, 4096, 0) == 0 and sparse(2048, 4096, 4096, 205, engine=_lib.TQ_LINEAR_GATHER) == 0
+    assert sparse(40, 4096, 4096, 205) == 0 and sparse(300, 1024, 4096, 205) == 0                  # the kernel for few rows
+    ops.set_gemm_pair_mode(1)
+    try:
+        assert sparse(2048, 4096, 4096, 205) == 0
+    finally:
+        ops.set_gemm_pair_mode(-1)
+    assert sparse(2048, 4096, 4096, 4096) == -1
+
+
+@pytest.mark.parametrize("M", [300, 777, 1500])
+def test_a_linear_of_another_width_on_the_same_prologue(fake, M):  # noqa: F811
+    """Whichever layer runs the prologue, the others find the operand that they take on their own."""
+    lins = [layer(N=n, K=4096, rms_weight=None) for n in (24576, 1024, 4096)]
+    for first in lins:
+        ws = first.prologue(claimed(M, 4096, dtype=torch.bfloat16))
+        assert ws.pro.sparse is not None and (ws.pro.tail_dense is not None or M > 1024)
+        for lin in lins:
+            lin.w.w_t = None
+            lin.compute(ws, M)
+            c = fake.calls[-1][1]
+            assert c["sp_val"] == ws.pro.sparse[0].data_ptr()
+            assert bool(c["w_t"]) == (sparse(M, lin.N, 4096, lin.R) == 1)
+
+
+@pytest.mark.parametrize("M", [64, 300, 1500])
+def test_a_layer_holds_and_names_the_sparse_operand(fake, M):  # noqa: F811
+    lin = layer(N=24576, K=512, rms_weight=None)
+    lin(claimed(M, 512, dtype=torch.bfloat16))
+    pro, c = lin._ws[M].pro, fake.calls[-1][1]
+    if not sparse(M, 24576, 512, lin.R, kind=lin.w.had_kind):
+        assert pro.sparse is None and not c["sp_val"]
+        return
+    assert [t.data_ptr() for t in pro.sparse] == [c[f] for f in ("sp_val", "sp_meta", "sp_over_cnt", "sp_over")]
+    assert c["sp_over_ld"] >= (lin.R + 1) // 2 and c["w_t"]
+
+
+@pytest.mark.parametrize("change", ["replaced", "in_place", "both"])
+def test_the_layers_own_transpose_follows_w_rot(fake, change):  # noqa: F811
+    lin = layer(N=24576, K=512, rms_weight=None)
+    lin.w.w_t = None
+    x = claimed(1500, 512, dtype=torch.bfloat16)
+    lin(x)
+    first = lin.w.w_t
+    lin(x)
+    assert first is not None and lin.w.w_t is first
+    if change == "in_place":
+        lin.w.w_rot.fill_(2.0)
+    else:
+        lin.w.w_rot = torch.full_like(lin.w.w_rot, 2.0)
+    if change == "both":
+        lin.w.w_t = mine = torch.full_like(first, 2.0)
+    lin(x)
+    assert float(lin.w.w_t[3, 5]) == 2.0 and fake.calls[-1][1]["w_t"] == lin.w.w_t.data_ptr()
+    assert change != "both" or lin.w.w_t is mine
