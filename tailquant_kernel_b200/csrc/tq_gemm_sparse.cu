@@ -46,7 +46,7 @@ struct SG {
   static constexpr int BSLOT = A + 2 * B;                 // tail values, bf16 weights of the two 64-wide halves
   static constexpr int B_OFF = SI * ISLOT;
   static constexpr int BAR_OFF = B_OFF + SB * BSLOT;
-  static constexpr int NUM_BARS = 2 * SI + 2 * SB + 6 + LISTS;
+  static constexpr int NUM_BARS = 2 * SI + 2 * SB + 6 + 2 * LISTS;
   static constexpr int LIST_OFF = (BAR_OFF + NUM_BARS * 8 + 16 + 15) / 16 * 16;
   static constexpr int SCALE_OFF = (LIST_OFF + LISTS * LIST * 4 + 1024 + 8 + 15) / 16 * 16;   // channel scales and bias
   static constexpr int DYN = SCALE_OFF + 2 * SPG_BN * 4 + 1024;
@@ -117,6 +117,8 @@ struct SparseBars {
   __device__ __forceinline__ uint32_t over_known(int b) const { return acc_full() + 32u + 8u * b; }
   // the entries of a dense slice are in their buffer
   __device__ __forceinline__ uint32_t listed(int b) const { return acc_full() + 48u + 8u * b; }
+  // and so is its operand A
+  __device__ __forceinline__ uint32_t built(int b) const { return acc_full() + 48u + 8u * (SG::LISTS + b); }
 };
 
 // The tiles of a pair: pair, pair + npairs, ..., row tiles first
@@ -275,7 +277,10 @@ sparse_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a8, const __grid_con
       mbar_init(b.over_known(k), 1);
       mbar_init(b.last_placed(k), 4);
     }
-    for (int k = 0; k < S::LISTS; ++k) mbar_init(b.listed(k), 1);
+    for (int k = 0; k < S::LISTS; ++k) {
+      mbar_init(b.listed(k), 1);
+      mbar_init(b.built(k), 1);
+    }
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -491,7 +496,7 @@ sparse_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a8, const __grid_con
         }
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncwarp();
-        if (lane == 0) mbar_arrive_cluster_n(lead(b.full_b(s)), 4u);   // (for the four warps that place metadata)
+        if (lane == 0) mbar_arrive(b.built(l));
         load(64 * (q + 1) + lane, v[0], r[0]);
         load(64 * (q + 1) + lane + 32, v[1], r[1]);
       }
@@ -626,7 +631,7 @@ sparse_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a8, const __grid_con
     const uint32_t taddr = tmem_base + S::T_META + ((uint32_t)(quad * 32) << 16);
     const uint32_t sel = h ? 0x7632u : 0x5410u;
     const size_t meta_ld = (size_t)(p.K / 32);
-    int s = 0;          // bf16 slot and the parity of the release that its next use waits for
+    int s = 0, slices = 0;   // bf16 slot and the parity of the release that its next use waits for; dense slices so far
     uint32_t ph = 1;
     auto next_slot = [&]() {
       if (++s == S::SB) {
@@ -689,7 +694,14 @@ sparse_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a8, const __grid_con
       if (lane == 0) mbar_arrive(b.last_placed(i & 1));
       const int ex = extra_of(i);
       if (!(ok = __all_sync(0xffffffffu, ok))) break;
-      for (int q = 0; q < ex && wait_slot(); ++q) next_slot();   // (warp 0's)
+      // dense slices: these warps pass on that warp 0 has built A.  (Every role takes part in every use of a slot: one that only
+      // watched could find the slot released twice and wait, by parity, for a release that needs it.)
+      for (int q = 0; q < ex && wait_slot(); ++q, ++slices) {
+        ok = __all_sync(0xffffffffu, mbar_wait(b.built(slices % S::LISTS), (uint32_t)((slices / S::LISTS) & 1), abort_flag, 0x8000000u));
+        if (!ok) break;
+        if (lane == 0) mbar_arrive_cluster(lead(b.full_b(s)));
+        next_slot();
+      }
     }
     catch_up(my_tiles);
   }
