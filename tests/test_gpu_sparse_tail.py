@@ -167,3 +167,22 @@ def test_weights_changed_in_place_reach_the_left_over_entries():
     lin.w.w_rot = SplitLinear(w).w.w_rot
     other.w.w_rot, other.w.w_t = lin.w.w_rot, None
     assert torch.equal(lin(x), other(x))
+
+
+def test_swiglu_of_every_gate():
+    """The quotient of the epilogue rounds like a division: all 2^16 gates (through the finisher of the split-K path), against
+    fp64 rounded once to fp32 and then to bf16."""
+    g = torch.arange(65536, dtype=torch.int32).to(torch.int16).view(torch.bfloat16).float()
+    g = g[torch.isfinite(g) & (g.abs() < 3e38)]
+    n = g.numel() // 8 * 8
+    g = g[:n].cuda()
+    y = torch.stack((g, torch.ones_like(g)), 1).reshape(1, -1).contiguous()
+    acc, one = torch.zeros((1, 1, 2 * n), dtype=torch.int32, device="cuda"), torch.ones(2 * n, device="cuda")
+    out = torch.empty((1, n), dtype=torch.bfloat16, device="cuda")
+    _lib.check(_lib.load().tq_dequant_finish_partials(acc.data_ptr(), 1, one.data_ptr(), one.data_ptr(), y.data_ptr(), None,
+                                                      out.data_ptr(), 1, 2 * n, 1, ops._stream()), "finish")
+    e = torch.exp(-g)                                        # (fp32, as the kernel's)
+    want = (g.double() / (1.0 + e).double()).float().to(torch.bfloat16)
+    # torch's exp may differ from the kernel's by an ulp or two, which moves a bf16 result now and then
+    d = (out[0].float() - want.float()).abs()
+    assert float((d > 0).float().mean()) < 2e-3 and bool((d <= want.float().abs() * 2.0 ** -7).all())
