@@ -31,7 +31,7 @@ int run_prologue(const void* x, int M, int K, int had_kind, int R, int dr, float
   if (dr < 1 || dr > K) return TQ_ERR_BAD_ARG;
   if (!aligned16(x) || (a_pack && !aligned16(a_pack)) || (a_q8 && !aligned16(a_q8)) || (x_rot && !aligned16(x_rot)) ||
       (tail_dense && !aligned16(tail_dense)) ||
-      (sparse && ((reinterpret_cast<uintptr_t>(sparse->val) & 31) || !aligned16(sparse->meta))))
+      (sparse && !(aligned16(sparse->val) && aligned16(sparse->meta))))
     return TQ_ERR_MISALIGNED;
   if (M == 0) return TQ_OK;
   PrologueParams p;
@@ -64,6 +64,8 @@ int run_prologue(const void* x, int M, int K, int had_kind, int R, int dr, float
     if (!sparse->val || !sparse->meta || !sparse->over_cnt || !sparse->over || sparse->over_ld < (R + 1) / 2) return TQ_ERR_BAD_ARG;
     p.sp = *sparse;
   }
+  p.wide = ((reinterpret_cast<uintptr_t>(a_q8) | reinterpret_cast<uintptr_t>(x_rot) | reinterpret_cast<uintptr_t>(tail_dense) |
+             reinterpret_cast<uintptr_t>(p.sp.val)) & 31) == 0;
   // 64 elements per thread issue fewer instructions per element, 16 give a row a quarter of the latency: the lines lie where
   // the rows no longer fit the chip at once (K = 4096: 9.2 against 9.8 us at 300 rows, 7.8 / 5.7 at 64; K = 12288, one
   // CTA of 768 threads per SM: 16.9 / 23.7 at 300, 10.0 / 9.2 at 61).

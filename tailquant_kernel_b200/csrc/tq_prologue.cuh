@@ -31,6 +31,7 @@ struct PrologueParams {
   const uint16_t* gamma;  // [K] bf16 RMSNorm weight, or NULL: x is used as it is
   float rms_eps;
   SparseTail sp;          // (val == NULL: not asked for)
+  bool wide;              // a_q8, x_rot, tail_dense, sp.val are 32-byte aligned
 };
 
 // What to do with a group of four, by which of its elements are tail entries (bit 0 = element 0, 1 = element 2, 2 = element 1,

@@ -85,6 +85,17 @@ __device__ __forceinline__ void sts32(unsigned char* a, uint32_t v) { *reinterpr
 __device__ __forceinline__ void sts16(unsigned char* a, uint32_t v) { *reinterpret_cast<unsigned short*>(a) = (unsigned short)v; }
 __device__ __forceinline__ uint32_t lds16(const unsigned char* a) { return (uint32_t)*reinterpret_cast<const unsigned short*>(a); }
 
+// 32 bytes of a thread's row piece, as one store where every output row starts on 32 bytes: as two the sectors are written in
+// halves (weights of 24576 x 4096, rotated and packed: 147 -> 135 us)
+__device__ __forceinline__ void store32(void* dst, const uint32_t* v, bool wide) {
+  if (wide) {
+    st_global_v8(dst, v);
+  } else {
+    reinterpret_cast<uint4*>(dst)[0] = make_uint4(v[0], v[1], v[2], v[3]);
+    reinterpret_cast<uint4*>(dst)[1] = make_uint4(v[4], v[5], v[6], v[7]);
+  }
+}
+
 // 64-point Walsh-Hadamard butterflies, strides 1, 2, ..., 32 in that order, on 32 packed pairs (elements 2j, 2j+1)
 __device__ __forceinline__ void wht64(u64 (&v)[32]) {
 #pragma unroll
@@ -260,7 +271,9 @@ struct FS {
   static constexpr int DYN = BAR_OFF + 16 + 1024;          // + alignment slack
 };
 
-constexpr int fast_min_ctas(int K) { return K <= 4096 ? 10 : (K <= 12288 ? 3 : 2); }
+// CTAs per SM.  K = 14336: 80 registers and a few spills, 2048 rows 109 -> 100 us against two CTAs with 125, 300 rows, which two
+// would take in two rounds, 17 -> 15.  K = 4096: 12 CTAs (80 registers) 31.6 against 29.1 us at 2048 rows.
+constexpr int fast_min_ctas(int K) { return K <= 4096 ? 10 : 3; }
 
 // SP: the tail in its 2:4-sparse form too (p.sp)
 template <int KIND, int K, int DT, bool NORM, bool SP>
@@ -573,9 +586,8 @@ prologue_fast_kernel(const __grid_constant__ CUtensorMap tmap_x, const PrologueP
 
     // =============================================================== thread t owns elements [64 t, 64 t + 64)
     if (p.x_rot) {
-      uint4* dst = reinterpret_cast<uint4*>(p.x_rot + (size_t)m * K + 64 * tid);
 #pragma unroll
-      for (int c = 0; c < 8; ++c) dst[c] = make_uint4(w[4 * c], w[4 * c + 1], w[4 * c + 2], w[4 * c + 3]);
+      for (int c = 0; c < 4; ++c) store32(p.x_rot + (size_t)m * K + 64 * tid + 16 * c, w + 8 * c, p.wide);
     }
     // ---- row maximum of the 15-bit magnitude keys
     uint32_t kmax;
@@ -688,16 +700,15 @@ prologue_fast_kernel(const __grid_constant__ CUtensorMap tmap_x, const PrologueP
       if (p.tail_dense) {
         // the row with everything outside the tail zeroed: the operand rows that the fused GEMM loads by TMA where a
         // half slice holds more entries than a record
-        uint4* dst = reinterpret_cast<uint4*>(p.tail_dense + (size_t)m * K + 64 * tid);
 #pragma unroll
-        for (int c = 0; c < 8; ++c) {
-          uint32_t o[4];
+        for (int c = 0; c < 4; ++c) {
+          uint32_t o[8];
 #pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            const int j = 4 * c + i;
+          for (int i = 0; i < 8; ++i) {
+            const int j = 8 * c + i;
             o[i] = w[j] & (((tm[j >> 4] >> (j & 15)) & 0x00010001u) * 0xffffu);
           }
-          dst[c] = make_uint4(o[0], o[1], o[2], o[3]);
+          store32(p.tail_dense + (size_t)m * K + 64 * tid + 16 * c, o, p.wide);
         }
       }
       if (p.tail_ptr) {  // run boundaries of the row's ascending index list at multiples of 128
@@ -779,8 +790,8 @@ prologue_fast_kernel(const __grid_constant__ CUtensorMap tmap_x, const PrologueP
           places[g >> 3] |= (e.x >> 16) << (4 * (g & 7));
         }
         uint16_t* const dst = p.sp.val + (size_t)m * (K / 2) + 32 * tid;
-        st_global_v8(dst, v);
-        st_global_v8(dst + 16, v + 8);
+        store32(dst, v, p.wide);
+        store32(dst + 16, v + 8, p.wide);
         *reinterpret_cast<uint2*>(p.sp.meta + (size_t)m * (K / 32) + 2 * tid) = make_uint2(places[0], places[1]);
         int x0, x1;
         over_groups(tm[0], x0);
@@ -836,9 +847,8 @@ prologue_fast_kernel(const __grid_constant__ CUtensorMap tmap_x, const PrologueP
         if (p.a_q8) {
           // INT8 form: even elements of the group first, then the odd ones -- the order in which the GEMM's
           // widening of the packed INT4 weights lays out K
-          uint4* dst = reinterpret_cast<uint4*>(p.a_q8 + (size_t)m * K + 64 * tid + 32 * g4);
-          dst[0] = make_uint4(ev[0], od[0], ev[1], od[1]);
-          dst[1] = make_uint4(ev[2], od[2], ev[3], od[3]);
+          const uint32_t o[8] = {ev[0], od[0], ev[1], od[1], ev[2], od[2], ev[3], od[3]};
+          store32(p.a_q8 + (size_t)m * K + 64 * tid + 32 * g4, o, p.wide);
         }
         if (p.a_pack) {
           // packed form: byte k of a group's word = nibbles of elements (2 k, 2 k + 1)
