@@ -333,8 +333,7 @@ def run_ours(args) -> None:
 
     def gemm_call(lin, ws):
         if mma:
-            return lambda: ops.split_gemm_mma(ws.pro.a_q8, ws.pro.body_scale, lin.w.b_col, lin.w.w_scale, ws.out,
-                                              w_rot=lin.w.w_rot, pro=ws.pro, R=lin.R)
+            return lambda: lin.compute(ws, M_TOKENS)   # (the kernel that a forward takes)
         return lambda: ops.split_gemm_fused(ws.pro.a_pack, ws.pro.body_scale, lin.w.b_col, lin.w.w_scale, ws.out,
                                             tail=ws.tail)
 
@@ -492,18 +491,20 @@ def run_ours(args) -> None:
     pro_gbs = pro_bytes / (t_pro * 1e-3) / 1e9
     tail_flops = sum(2.0 * M_TOKENS * lin.R * N for (_, K, N), lin in zip(LAYER, lins))
     # tensor-pipe time the kernel's MMAs need at the measured library rates: the int8 product, plus (tensor-core
-    # tail) a dense bf16 product of the same shape over the zero-filled tail matrix
+    # tail) a bf16 product of the same shape over the tail, at the dense rate (the sparse operand takes half of that)
     pipe_ms = ops_step / (int8_peak * 1e12) * 1e3 + (ops_step / (peaks["bf16"] * 1e12) * 1e3 if mma else 0.0)
     t_sum = t_gemm + t_tail + t_pro
 
     h2d = sum(int(h.numel() * h.element_size()) for h in host_x)
     d2h = sum(int(h.numel() * h.element_size()) for h in host_y)
-    # The dominant kernel: with the tensor-core tail all four projections of the layer run on CTA pairs
-    # (pair_gemm_kernel); the roofline entry sums its four launches of a step.
+    # The dominant kernel: with the tensor-core tail all four projections of the layer run on CTA pairs, the tail as a
+    # 2:4-sparse operand (sparse_gemm_kernel); the roofline entry sums its four launches of a step.
     if mma:
         dom = [n for (n, K, N) in LAYER]
-        kname = ("pair_gemm_kernel (tcgen05 cta_group::2: kind::i8 dense + kind::f16 tail, fused dequant); launches: "
-                 + ", ".join(dom))
+        sparse = all(ops.takes_sparse(M_TOKENS, lin.N, lin.K, lin.R, lin.w.had_kind) for lin in lins)
+        kernel = "sparse_gemm_kernel" if sparse else "pair_gemm_kernel"
+        kname = (kernel + " (tcgen05 cta_group::2: kind::i8 dense + kind::f16 " + ("2:4-sparse " if sparse else "") +
+                 "tail, fused dequant); launches: " + ", ".join(dom))
     else:
         dom = [n for (n, K, N) in LAYER]
         kname = "gemm_kernel<256> (tcgen05 kind::i8, fused dequant + tail add)"
@@ -540,7 +541,7 @@ def run_ours(args) -> None:
         "roofline": {"kernel": kname, "bound": "tensor",
                      "achieved": dom_tops, "peak": int8_peak, "unit": "TFLOP/s", "frac": dom_tops / int8_peak,
                      "ms_per_step_in_kernel": dom_ms,
-                     "traffic": measured_dram_traffic("pair_gemm_kernel") if mma else None,
+                     "traffic": measured_dram_traffic(kernel) if mma else None,
                      "peak_note": f"2 x burst bf16 cuBLAS figure ({peaks['source']}; the kernel is timed alone); nominal dense INT8 {NOMINAL_INT8_TOPS}; "
                                   "achieved counts the algorithmic 2*M*N*K of the INT4 product only",
                      "frac_of_nominal_int8": dom_tops / NOMINAL_INT8_TOPS,
