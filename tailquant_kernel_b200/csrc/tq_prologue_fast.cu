@@ -373,6 +373,7 @@ prologue_fast_kernel(const __grid_constant__ CUtensorMap tmap_x, const PrologueP
         for (int q = 1; q < NW; ++q) tot = __fadd_rn(tot, redf[q]);
         __syncthreads();  // (red is reused by the block maximum)
         const float rms_inv = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(tot, (float)K), p.rms_eps)));
+        const u64 inv2 = pk2(rms_inv, rms_inv);
         // y = bf16(bf16(x * inv) * gamma), as a bf16 framework's RMSNorm rounds
         const uint4* gp = reinterpret_cast<const uint4*>(p.gamma + 64 * tid);
 #pragma unroll
@@ -382,12 +383,11 @@ prologue_fast_kernel(const __grid_constant__ CUtensorMap tmap_x, const PrologueP
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
             float lo, hi, gl, gh;
-            up2(v[4 * c + i], lo, hi);
+            up2(mul2(v[4 * c + i], inv2), lo, hi);   // (both elements of a pair per instruction: 36.5 -> 35.6 us at 2048 x 4096)
+            unpack_word<TQ_BF16>(cvt_bf16x2(lo, hi), lo, hi);
             unpack_word<TQ_BF16>(gw[i], gl, gh);
-            lo = bf16_bits_to_f32(f32_to_bf16_bits(__fmul_rn(lo, rms_inv)));
-            hi = bf16_bits_to_f32(f32_to_bf16_bits(__fmul_rn(hi, rms_inv)));
-            lo = bf16_bits_to_f32(f32_to_bf16_bits(__fmul_rn(lo, gl)));
-            hi = bf16_bits_to_f32(f32_to_bf16_bits(__fmul_rn(hi, gh)));
+            up2(mul2(pk2(lo, hi), pk2(gl, gh)), lo, hi);
+            unpack_word<TQ_BF16>(cvt_bf16x2(lo, hi), lo, hi);
             v[4 * c + i] = pk2(lo, hi);
           }
         }
