@@ -316,8 +316,8 @@ class SplitLinear:
                 and (own.rot_version is None or own.rot_version == self._rot_version())
                 and kind == w.had_kind and rank == self.descending_rank and eps == self.rms_eps and act == self.epilogue)
 
-    def _check_parts(self, engine: int) -> None:
-        """Types, layout and sizes of what a forward reads: the kernels take all of it for granted."""
+    def _check_parts(self, engine: int, transposed: bool = False) -> None:
+        """Types, layout and sizes of what a forward reads (`transposed`: w_t beside w_rot): the kernels take it for granted."""
         w, N, K = self.w, self.N, self.K
         ops._check_cuda(w.b_col, "b_col", torch.uint8)
         ops._check(tuple(w.b_col.shape) == (N, K // 2), "b_col must be [N, K/2]")
@@ -326,7 +326,7 @@ class SplitLinear:
         if self.R and engine == _lib.TQ_LINEAR_FUSED:
             ops._check_cuda(w.w_rot, "w_rot", torch.bfloat16)
             ops._check(tuple(w.w_rot.shape) == (N, K), "w_rot must be [N, K]")
-        elif self.R:
+        if self.R and (transposed or engine != _lib.TQ_LINEAR_FUSED):
             ops._check_cuda(w.w_t, "w_t", torch.bfloat16)
             ops._check(tuple(w.w_t.shape) == (K, N), "w_t must be [K, N]")
         if w.bias is not None:
@@ -348,7 +348,7 @@ class SplitLinear:
                 ops.takes_sparse(own.M, self.N, self.K, self.R, self.w.had_kind):
             self._prepare_sparse(own)
         own.call = None   # (a part that is refused must not leave the former description in force)
-        self._check_parts(own.engine)
+        self._check_parts(own.engine, own.rot_version is not None)
         w, p = self.w, ops._ptr
         own.call_pro = pro
         src = (w.b_col, w.w_scale, w.w_rot, w.w_t, w.bias, self.rms_weight)

@@ -72,3 +72,18 @@ def test_the_layers_own_transpose_follows_w_rot(fake, change):  # noqa: F811
     lin(x)
     assert float(lin.w.w_t[3, 5]) == 2.0 and fake.calls[-1][1]["w_t"] == lin.w.w_t.data_ptr()
     assert change != "both" or lin.w.w_t is mine
+
+
+@pytest.mark.parametrize("bad", [claimed(512, 24576, dtype=torch.float16), claimed(24576, 512, dtype=torch.bfloat16),
+                                 claimed(24576, 512, dtype=torch.bfloat16).t(), torch.zeros(512, 24576, dtype=torch.bfloat16)])
+def test_a_transpose_of_the_wrong_kind_is_refused(fake, bad):  # noqa: F811
+    x = claimed(1500, 512, dtype=torch.bfloat16)
+    first, later = layer(N=24576, K=512, rms_weight=None), layer(N=24576, K=512, rms_weight=None)
+    later(x)
+    fake.calls.clear()
+    for lin in (first, later):
+        lin.w.w_t = bad
+        for _ in range(2):
+            with pytest.raises(RuntimeError, match="w_t"):
+                lin(x)
+    assert not fake.calls
