@@ -146,7 +146,7 @@ class SplitLinear:
         self.reuse_output = bool(reuse_output)
         self._ws: Dict[int, _Workspace] = {}
         self._ws_shared: Dict[int, _Workspace] = {}
-        self._t_of = (None, None, None)   # a transpose, the w_rot and the version of it that it belongs to
+        self._t_of = (None, None, None, None)   # a transpose; the w_rot, its version and place that it belongs to
 
     @classmethod
     def from_prepared(cls, w: "ops.PreparedWeight", ratio: float = 0.05, activation_percentile: float = 100.0,
@@ -285,8 +285,13 @@ class SplitLinear:
         """Builds the [K, N] transpose of the rotated weights that the small-M tail reads, ahead of the first small-M
         forward (which otherwise builds it: an allocation inside that call)."""
         if self.R and self.w.w_t is None:
-            r = self.w.w_rot
-            self.w.w_t = ops.transpose_bf16(r) if r.device.type == "cuda" and r.is_contiguous() else r.t().contiguous()
+            self.w.w_t = self._transposed()
+
+    def _transposed(self, into: Optional[torch.Tensor] = None) -> torch.Tensor:
+        r = self.w.w_rot
+        if r.device.type == "cuda" and r.is_contiguous():
+            return ops.transpose_bf16(r, into)
+        return r.t().contiguous() if into is None else into.copy_(r.t())
 
     def _rot_version(self) -> int:
         r = self.w.w_rot
@@ -294,13 +299,20 @@ class SplitLinear:
 
     def _prepare_sparse(self, own: _Workspace) -> None:
         """The transpose that the left-over entries of the sparse tail are read from.  A layer that had none did not ask for it
-        and is not expected to keep it in line: it is made again when `w_rot` was replaced or changed in place since."""
-        w, version = self.w, self._rot_version()
-        t, rot, v = self._t_of
-        if w.w_t is not None and w.w_t is t and (w.w_rot is not rot or version != v):
-            w.w_t = None
+        and is not expected to keep it in line: it is made again when `w_rot` was replaced or changed since, in the same memory
+        where `w_rot` is the same tensor (a graph captured before names both)."""
+        w = self.w
+        if w.w_rot is None:
+            return   # (refused with the other parts)
+        version = self._rot_version()
+        t, rot, v, place = self._t_of
+        if w.w_t is not None and w.w_t is t and (w.w_rot is not rot or (version, rot.data_ptr()) != (v, place)):
+            if w.w_rot is rot and tuple(t.shape) == tuple(reversed(rot.shape)) and t.dtype == rot.dtype and t.device == rot.device:
+                self._transposed(t)
+            else:
+                w.w_t = None
         self.prepare_decode()
-        self._t_of = (w.w_t, w.w_rot, version)
+        self._t_of = (w.w_t, w.w_rot, version, w.w_rot.data_ptr())
         own.rot_version = version
 
     def _described(self, own: _Workspace) -> bool:

@@ -245,10 +245,14 @@ def prepare_weight(W: torch.Tensor, had_kind: Optional[int] = None, eps: float =
     return PreparedWeight(N, K, had_kind, b_col, w_scale, w_t, b_row, w_rot if keep_w_rot else None, b32)
 
 
-def transpose_bf16(w: torch.Tensor) -> torch.Tensor:
-    """[K, N] transpose of a bf16 matrix [N, K] (rotated weights -> `w_t`)."""
+def transpose_bf16(w: torch.Tensor, out: Optional[torch.Tensor] = None) -> torch.Tensor:
+    """[K, N] transpose of a bf16 matrix [N, K] (rotated weights -> `w_t`), into `out` where that is given."""
     _check_cuda(w, "w", torch.bfloat16)
-    out = torch.empty((w.shape[1], w.shape[0]), dtype=torch.bfloat16, device=w.device)
+    if out is None:
+        out = torch.empty((w.shape[1], w.shape[0]), dtype=torch.bfloat16, device=w.device)
+    _check_cuda(out, "out", torch.bfloat16)
+    _check(w.dim() == 2 and tuple(out.shape) == (w.shape[1], w.shape[0]), "transpose_bf16: out must be [K, N] for w [N, K]")
+    _check(out.device == w.device, "transpose_bf16: w and out must be on one device")
     _lib.check(_lib.load().tq_transpose_bf16(_ptr(w), _ptr(out), w.shape[0], w.shape[1], _stream()), "transpose_bf16")
     return out
 

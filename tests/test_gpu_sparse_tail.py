@@ -160,10 +160,11 @@ def test_weights_changed_in_place_reach_the_left_over_entries():
     lin(x)
     assert lin._ws[M].pro.sparse is not None
     other = SplitLinear(2 * w)
+    t = lin.w.w_t
     lin.w.w_rot.copy_(other.w.w_rot)
     lin.w.b_col.copy_(other.w.b_col)
     lin.w.w_scale.copy_(other.w.w_scale)
-    assert torch.equal(lin(x), other(x))
+    assert torch.equal(lin(x), other(x)) and lin.w.w_t is t and torch.equal(t, lin.w.w_rot.t())
     lin.w.w_rot = SplitLinear(w).w.w_rot
     other.w.w_rot, other.w.w_t = lin.w.w_rot, None
     assert torch.equal(lin(x), other(x))

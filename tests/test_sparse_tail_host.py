@@ -74,6 +74,28 @@ def test_the_layers_own_transpose_follows_w_rot(fake, change):  # noqa: F811
     assert change != "both" or lin.w.w_t is mine
 
 
+def test_a_transpose_is_refreshed_where_it_is(fake):  # noqa: F811
+    """A graph captured before still names it."""
+    lin = layer(N=24576, K=512, rms_weight=None)
+    lin.w.w_t = None
+    x = claimed(1500, 512, dtype=torch.bfloat16)
+    lin(x)
+    first, at = lin.w.w_t, lin.w.w_t.data_ptr()
+    lin.w.w_rot.fill_(2.0)
+    lin(x)
+    assert lin.w.w_t is first and lin.w.w_t.data_ptr() == at and float(first[3, 5]) == 2.0
+
+
+def test_a_transpose_follows_data_put_under_w_rot(fake):  # noqa: F811
+    lin = layer(N=24576, K=512, rms_weight=None)
+    lin.w.w_t = None
+    x = claimed(1500, 512, dtype=torch.bfloat16)
+    lin(x)
+    lin.w.w_rot.data = torch.full_like(lin.w.w_rot, 2.0)
+    lin(x)
+    assert float(lin.w.w_t[3, 5]) == 2.0
+
+
 @pytest.mark.parametrize("bad", [claimed(512, 24576, dtype=torch.float16), claimed(24576, 512, dtype=torch.bfloat16),
                                  claimed(24576, 512, dtype=torch.bfloat16).t(), torch.zeros(512, 24576, dtype=torch.bfloat16)])
 def test_a_transpose_of_the_wrong_kind_is_refused(fake, bad):  # noqa: F811
@@ -86,4 +108,12 @@ def test_a_transpose_of_the_wrong_kind_is_refused(fake, bad):  # noqa: F811
         for _ in range(2):
             with pytest.raises(RuntimeError, match="w_t"):
                 lin(x)
+    assert not fake.calls
+
+
+def test_a_layer_without_w_rot_is_refused(fake):  # noqa: F811
+    lin = layer(N=24576, K=512, rms_weight=None)
+    lin.w.w_rot = None
+    with pytest.raises(RuntimeError):
+        lin(claimed(1500, 512, dtype=torch.bfloat16))
     assert not fake.calls
