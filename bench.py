@@ -491,8 +491,10 @@ def run_ours(args) -> None:
     pro_gbs = pro_bytes / (t_pro * 1e-3) / 1e9
     tail_flops = sum(2.0 * M_TOKENS * lin.R * N for (_, K, N), lin in zip(LAYER, lins))
     # tensor-pipe time the kernel's MMAs need at the measured library rates: the int8 product, plus (tensor-core
-    # tail) a bf16 product of the same shape over the tail, at the dense rate (the sparse operand takes half of that)
-    pipe_ms = ops_step / (int8_peak * 1e12) * 1e3 + (ops_step / (peaks["bf16"] * 1e12) * 1e3 if mma else 0.0)
+    # tail) a bf16 product of the same shape over the tail; the 2:4-sparse operand counts at twice the bf16 rate
+    sparse = mma and all(ops.takes_sparse(M_TOKENS, lin.N, lin.K, lin.R, lin.w.had_kind) for lin in lins)
+    bf16_part = (0.5 if sparse else 1.0) if mma else 0.0
+    pipe_ms = (ops_step / int8_peak + bf16_part * ops_step / peaks["bf16"]) / 1e12 * 1e3
     t_sum = t_gemm + t_tail + t_pro
 
     h2d = sum(int(h.numel() * h.element_size()) for h in host_x)
@@ -501,7 +503,6 @@ def run_ours(args) -> None:
     # 2:4-sparse operand (sparse_gemm_kernel); the roofline entry sums its four launches of a step.
     if mma:
         dom = [n for (n, K, N) in LAYER]
-        sparse = all(ops.takes_sparse(M_TOKENS, lin.N, lin.K, lin.R, lin.w.had_kind) for lin in lins)
         kernel = "sparse_gemm_kernel" if sparse else "pair_gemm_kernel"
         kname = (kernel + " (tcgen05 cta_group::2: kind::i8 dense + kind::f16 " + ("2:4-sparse " if sparse else "") +
                  "tail, fused dequant); launches: " + ", ".join(dom))
