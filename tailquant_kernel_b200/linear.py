@@ -23,9 +23,6 @@ import torch
 from . import _lib, ops
 
 
-SPARSE_FIELDS = ("sp_val", "sp_meta", "sp_over_cnt", "sp_over")
-
-
 def interleave_gate_up(w_gate: torch.Tensor, w_up: torch.Tensor) -> torch.Tensor:
     """[2 I, K] weight of a fused gate_up projection with rows (gate_0, up_0, gate_1, up_1, ...): the layout
     `SplitLinear(..., epilogue="swiglu")` expects."""
@@ -374,7 +371,7 @@ class SplitLinear:
             rms_weight=p(self.rms_weight), a_pack=p(pro.a_pack), a_q8=p(pro.a_q8), body_scale=p(pro.body_scale),
             top_scale=p(pro.top_scale), tail_idx16=p(pro.tail_idx), tail_val=p(pro.tail_val), tail_ptr=p(pro.tail_ptr),
             tail_rec=p(pro.tail_rec), tail_cnt=p(pro.tail_cnt), tail_dense=p(pro.tail_dense), tail=p(own.tail),
-            **({} if pro.sparse is None else dict(zip(SPARSE_FIELDS, map(p, pro.sparse)), sp_over_ld=pro.sparse[3].shape[1]))))
+            **({} if pro.sparse is None else dict(zip(ops.SPARSE_FIELDS, map(p, pro.sparse)), sp_over_ld=pro.sparse[3].shape[1]))))
         return own.call
 
     def _what(self, M: int) -> str:

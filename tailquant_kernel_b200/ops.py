@@ -30,6 +30,7 @@ from ._lib import TQ_BF16, TQ_FP16, TQ_HAD_BLOCK128, TQ_HAD_KRON12, TQ_HAD_NONE,
 
 EPS = 1e-8
 TAIL_REC_CAP = 12  # TQ_TAIL_REC_CAP of include/tailquant.h
+SPARSE_FIELDS = ("sp_val", "sp_meta", "sp_over_cnt", "sp_over")  # of a tq_linear_call, in the order of PrologueOut.sparse
 
 
 # --------------------------------------------------------------------------- helpers
@@ -160,6 +161,22 @@ def split_prologue(x: torch.Tensor, had_kind: int, R: int, descending_rank: Opti
         _check_cuda(rms_weight, "rms_weight", torch.bfloat16)
         _check(rms_weight.numel() == K, "rms_weight must have K elements")
         _check(out.idx32 is None and out.top_q is None, "the fused RMSNorm prologue has no T4 outputs")
+    if out.sparse is not None:   # (a linear prefers it to the other forms of the tail, so it must not keep an earlier input's)
+        _check(out.idx32 is None and out.top_q is None and out.x_rot is None,
+               "the sparse tail operand comes without T4 outputs and without x_rot")
+        val, meta, over_cnt, over = out.sparse
+        _check(R > 0 and tuple(val.shape) == (M, K // 2) and tuple(meta.shape) == (M, K // 32) and over_cnt.numel() == M and
+               over.shape[0] == M, "the sparse tail operand has the wrong shape")
+        c = _lib.LinearCall(
+            M=M, N=8, K=K, R=R, had_kind=had_kind, descending_rank=descending_rank, engine=_lib.TQ_LINEAR_FUSED, tail_ld=ld,
+            ptr_ld=pld, eps=eps, rms_eps=float(rms_eps), rms_weight=_ptr(rms_weight), a_pack=_ptr(out.a_pack), a_q8=_ptr(out.a_q8),
+            body_scale=_ptr(out.body_scale), top_scale=_ptr(out.top_scale), tail_idx16=_ptr(out.tail_idx),
+            tail_val=_ptr(out.tail_val), tail_ptr=_ptr(out.tail_ptr), tail_rec=_ptr(out.tail_rec), tail_cnt=_ptr(out.tail_cnt),
+            tail_dense=_ptr(out.tail_dense), sp_over_ld=over.shape[1], **dict(zip(SPARSE_FIELDS, map(_ptr, out.sparse))))
+        _lib.check(_lib.load().tq_linear_prologue(ctypes.byref(c), _ptr(x), _stream()),
+                   f"split_prologue(M={M}, K={K}, had_kind={had_kind}, R={R})")
+        return out
+    if rms_weight is not None:
         rc = _lib.load().tq_split_prologue_rmsnorm(
             _ptr(x), _ptr(rms_weight), float(rms_eps), M, K, had_kind, R, descending_rank, eps, _ptr(out.a_pack),
             _ptr(out.a_q8), _ptr(out.body_scale), _ptr(out.top_scale), _ptr(out.tail_idx), _ptr(out.tail_val), ld,

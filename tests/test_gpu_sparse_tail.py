@@ -170,6 +170,25 @@ def test_weights_changed_in_place_reach_the_left_over_entries():
     assert torch.equal(lin(x), other(x))
 
 
+@pytest.mark.parametrize("M", [700, 1500])
+def test_a_prologue_into_a_used_workspace(M):
+    """Another input through `split_prologue`, then the GEMM by either entry point: the outputs of a layer that never saw the first."""
+    from tailquant_kernel_b200 import SplitLinear
+    N, K = 8192, 1024
+    g = torch.Generator().manual_seed(4)
+    w = (torch.randn(N, K, generator=g) * 0.02).to(torch.bfloat16).cuda()
+    lin, fresh = SplitLinear(w), SplitLinear(w)
+    lin(activations("few_levels", M, K, 1))
+    assert lin._ws[M].pro.sparse is not None
+    x = activations("hot", M, K, 2)
+    ws = lin.workspace(M)
+    ops.split_prologue(x, lin.w.had_kind, lin.R, lin.descending_rank, out=ws.pro)
+    out = torch.empty((M, N), dtype=torch.bfloat16, device="cuda")
+    ops.split_gemm_mma(ws.pro.a_q8, ws.pro.body_scale, lin.w.b_col, lin.w.w_scale, out, w_rot=lin.w.w_rot, pro=ws.pro, R=lin.R)
+    y = fresh(x)
+    assert torch.equal(out, y) and torch.equal(lin.compute(ws, M), y)
+
+
 def test_swiglu_of_every_gate():
     """The quotient of the epilogue rounds like a division: all 2^16 gates (through the finisher of the split-K path), against
     fp64 rounded once to fp32 and then to bf16."""

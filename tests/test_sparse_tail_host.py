@@ -117,3 +117,30 @@ def test_a_layer_without_w_rot_is_refused(fake):  # noqa: F811
     with pytest.raises(RuntimeError):
         lin(claimed(1500, 512, dtype=torch.bfloat16))
     assert not fake.calls
+
+
+@pytest.mark.parametrize("norm", [False, True])
+def test_a_prologue_into_a_workspace_fills_its_sparse_operand(fake, norm):  # noqa: F811
+    """The linears on it prefer that operand: one that the prologue left out would be an earlier input's."""
+    lin = layer(N=24576, K=512, rms_weight=None)
+    x = claimed(1500, 512, dtype=torch.bfloat16)
+    lin(x)
+    pro = lin.workspace(1500).pro
+    assert pro.sparse is not None
+    fake.calls.clear()
+    gamma = claimed(512, dtype=torch.bfloat16) if norm else None
+    assert ops.split_prologue(x, lin.w.had_kind, lin.R, lin.descending_rank, out=pro, rms_weight=gamma) is pro
+    (name, c), = fake.calls
+    assert name == "tq_linear_prologue" and [t.data_ptr() for t in pro.sparse] == [c[f] for f in ops.SPARSE_FIELDS]
+    assert c["a_q8"] == pro.a_q8.data_ptr() and c["rms_weight"] == (gamma.data_ptr() if norm else None)
+    assert c["sp_over_ld"] == pro.sparse[3].shape[1]
+
+
+def test_a_sparse_operand_of_another_size_is_refused(fake):  # noqa: F811
+    lin = layer(N=24576, K=512, rms_weight=None)
+    lin(claimed(1500, 512, dtype=torch.bfloat16))
+    fake.calls.clear()
+    with pytest.raises(RuntimeError, match="sparse"):
+        ops.split_prologue(claimed(900, 512, dtype=torch.bfloat16), lin.w.had_kind, lin.R, lin.descending_rank,
+                           out=lin.workspace(1500).pro)
+    assert not fake.calls
