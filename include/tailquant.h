@@ -332,10 +332,11 @@ typedef struct tq_linear_call {
 } tq_linear_call;
 
 /* Prologue outputs that the workspace of a call should hold, as a sum of these; reads M, N, K, R, had_kind and engine of
- * `call` only.  shared = 0: what tq_linear_forward of this call reads and writes.  shared = 1: what tq_linear_prologue should
+ * `call`, and whether sp_val is NULL: with sp_val the answer is what is needed beside the sp_* arrays, where tq_linear_sparse
+ * says 1.  shared = 0: what tq_linear_forward of this call reads and writes.  shared = 1: what tq_linear_prologue should
  * leave for linears of any width (a wide and a narrow layer can be on different kernels; up to 64 rows also on the decode
  * and on the fused engine).  A fused call takes its kernel by shape AND by what it finds: without tail_dense the CTA pairs,
- * without the records the other one.  Negative = error code. */
+ * without the records the other one, with neither the 2:4-sparse form.  Negative = error code. */
 #define TQ_OUT_PACK 1    /* a_pack */
 #define TQ_OUT_Q8 2      /* a_q8 */
 #define TQ_OUT_LISTS 4   /* tail_idx16, tail_val */
@@ -344,7 +345,7 @@ typedef struct tq_linear_call {
 int tq_linear_outputs(const tq_linear_call* call, int shared);
 /* 1 where a fused forward of this call (shared = 1: of a linear of some width on the same prologue) takes the tail as a
  * 2:4-sparse operand once its workspace holds the sp_* arrays beside those of tq_linear_outputs, else 0; reads the same fields.
- * A forward on the sparse form writes no records, and neither does tq_linear_prologue where tail_dense is there too. */
+ * A forward on the sparse form writes no other operand of the tail; tq_linear_prologue writes every array that is there. */
 int tq_linear_sparse(const tq_linear_call* call, int shared);
 /* out [K,N] = in [N,K] transposed, bf16 (the w_t of rotated weights). */
 int tq_transpose_bf16(const void* in, void* out, int N, int K, void* stream);

@@ -34,8 +34,7 @@ constexpr int P_LOOK = 2;  // K slices of the next tile prepared before a tile's
 struct PairGemmParams {
   int M, N, K, R, ld, ptr_ld;
   int tiles_m, tiles_n, kb_total, has_tail;
-  int dense;             // the zero-filled tail matrix is available (tmap_d): half slices with long runs load it,
-  int rec_cap;           // those with more entries than this (the record's capacity; -1: all, the records are not filled)
+  int dense;             // the zero-filled tail matrix is available (tmap_d): half slices with long runs load it
   const uint16_t* idx;   // [M, ld] ascending tail indices (only read for runs longer than the record capacity)
   const uint16_t* val;   // [M, ld] tail values
   const uint16_t* ptr;   // [M, ptr_ld] ptr[m][j] = entries of row m with index < 128 j
@@ -502,7 +501,7 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a8, const __grid_const
         if (brow == 0) TQ_TRACE(4, q, 1);
         tc_fence_after();
         const int nwmax = __reduce_max_sync(0xffffffffu, n);
-        if (p.dense && nwmax > p.rec_cap) {
+        if (p.dense && nwmax > C) {
           // a run longer than the record among the warp's 32 rows and the zero-filled tail matrix at hand: its 32 x 64
           // block is the operand itself -- one tiled load (same 128-byte swizzle as the tile), whose bytes the slot's
           // barrier counts on top of this warp's arrival
@@ -660,9 +659,8 @@ int run_pair_gemm(const int8_t* a_q8, const float* body_scale, const uint8_t* b_
                   const void* w_rot, const uint16_t* tail_idx16, const void* tail_val, int tail_ld,
                   const uint16_t* tail_ptr, int ptr_ld, const uint32_t* tail_rec, const uint16_t* tail_cnt,
                   const void* tail_dense, int R, const float* bias, void* out_bf16, int32_t* dbg_acc, float* dbg_tail,
-                  int M, int N, int K, int act, bool records_filled, cudaStream_t st) {
+                  int M, int N, int K, int act, cudaStream_t st) {
   PairGemmParams p = {};
-  p.rec_cap = records_filled ? TQ_TAIL_REC_CAP : -1;
   p.M = M;
   p.N = N;
   p.K = K;

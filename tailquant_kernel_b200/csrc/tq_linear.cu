@@ -7,9 +7,13 @@
 namespace tq {
 namespace {
 
+// Whether the operands of the pair kernel's tail are there.
+bool has_records(const tq_linear_call& c) { return c.tail_idx16 && c.tail_val && c.tail_ptr && c.tail_rec && c.tail_cnt; }
+
 // Whether the fused engine of this call runs the stream kernel (which reads the tail from the zero-filled matrix).
 bool linear_streams(const tq_linear_call& c) {
-  return c.engine == TQ_LINEAR_FUSED && c.M > 0 && (c.R == 0 || c.tail_dense) && stream_is_faster(c.M, c.N, c.K, c.R);
+  if (c.engine != TQ_LINEAR_FUSED || c.M <= 0) return false;
+  return c.R == 0 ? stream_is_faster(c.M, c.N, c.K, 0) : c.tail_dense && (!has_records(c) || stream_is_faster(c.M, c.N, c.K, c.R));
 }
 
 // Rows beyond which the zero-filled matrix is not kept whatever it would save (layers whose pair kernel reads it excepted).
@@ -25,9 +29,18 @@ bool tail_can_be_sparse(const tq_linear_call& c) {
 
 // Whether the sparse form is the fastest for this call.
 bool linear_sparse(const tq_linear_call& c) { return tail_can_be_sparse(c) && sparse_is_faster(c.M, c.N, c.K, c.R); }
-// Whether the buffers of a call hold the sparse form and the zero-filled matrix: between them they serve every fused kernel (the
-// CTA pairs then load all of their tail operand from the matrix), so the records are left out.
-bool sparse_and_dense(const tq_linear_call& c) { return c.sp_val && c.tail_dense && tail_can_be_sparse(c); }
+
+// Whether a linear of some width on the prologue of this call may take it.
+bool shared_sparse(const tq_linear_call& c) { return tail_can_be_sparse(c) && g_gemm_pair_mode < 0 && c.M > 64; }
+
+// Whether a fused call runs on the sparse form that it holds: where that is the fastest, and where nothing faster is there (the
+// prologue filled what the kernel of ANOTHER width reads).
+bool takes_sparse(const tq_linear_call& c) {
+  if (!c.sp_val || c.M == 0 || c.R == 0) return false;
+  if (linear_sparse(c)) return true;
+  if (has_records(c)) return false;
+  return !c.tail_dense || (shared_sparse(c) && sparse_us(c.M, c.N, c.K, c.R) < plan_stream(c.M, c.N, c.K, ST_TAIL).us);
+}
 
 SparseTail linear_sparse_tail(const tq_linear_call& c) {
   return SparseTail{reinterpret_cast<uint16_t*>(c.sp_val), c.sp_meta, c.sp_over_cnt, c.sp_over, c.sp_over_ld};
@@ -43,14 +56,18 @@ int linear_outputs(const tq_linear_call& c, bool shared) {
   const bool pair_dense = c.had_kind == TQ_HAD_BLOCK128;   // (the pair kernel loads long runs from it)
   if (few) return o | TQ_OUT_LISTS | TQ_OUT_DENSE;
   if (!fused) return o | TQ_OUT_LISTS;
+  if (c.sp_val && !shared && linear_sparse(c)) return o | TQ_OUT_LISTS;
+  // (the sparse form and the zero-filled matrix serve every width between them)
+  if (c.sp_val && shared && shared_sparse(c) && c.M <= DENSE_ROWS)
+    return o | TQ_OUT_LISTS | TQ_OUT_DENSE | linear_outputs(c, false);
   const bool streams = c.M <= DENSE_MAX_ROWS && stream_is_faster(c.M, c.N, c.K, c.R);
   if (shared || !streams) o |= TQ_OUT_LISTS | TQ_OUT_RECORDS;
   if (streams || pair_dense || (shared && c.M <= DENSE_ROWS)) o |= TQ_OUT_DENSE;
   return o;
 }
 
-// The part of a workspace that a forward of this call fills and reads; a prologue on its own fills all of it, since
-// another linear, of another width and hence perhaps on another kernel, may run on it.  The sorted tail lists and the
+// The part of a workspace that a forward of this call fills and reads; a prologue on its own fills every array that is there,
+// since another linear, of another width and hence perhaps on another kernel, may run on it.  The sorted tail lists and the
 // records cost a small call about 3 us, the zero-filled matrix a large one 2 bytes per element.
 tq_linear_call linear_own_part(tq_linear_call c) {
   const bool fused = c.engine == TQ_LINEAR_FUSED;
@@ -58,7 +75,7 @@ tq_linear_call linear_own_part(tq_linear_call c) {
     c.a_pack = nullptr;
   else
     c.a_q8 = nullptr;
-  if (c.sp_val && linear_sparse(c)) {
+  if (fused && takes_sparse(c)) {
     c.tail_dense = nullptr;
     c.tail_ptr = nullptr;
     c.tail_rec = nullptr;
@@ -82,11 +99,10 @@ tq_linear_call linear_own_part(tq_linear_call c) {
 
 int linear_prologue(const tq_linear_call& c, const void* x, void* stream) {
   const SparseTail sp = linear_sparse_tail(c);
-  const bool records = !sparse_and_dense(c);
   return run_prologue(x, c.M, c.K, c.had_kind, c.R, c.descending_rank, c.eps, 0, c.a_pack, c.a_q8, c.body_scale,
-                      c.top_scale, c.tail_idx16, c.tail_val, c.tail_ld, records ? c.tail_ptr : nullptr, c.ptr_ld,
-                      records ? c.tail_rec : nullptr, records ? c.tail_cnt : nullptr,
-                      nullptr, nullptr, nullptr, c.rms_weight, c.rms_eps, (cudaStream_t)stream, TQ_BF16, c.tail_dense, sp.val ? &sp : nullptr);
+                      c.top_scale, c.tail_idx16, c.tail_val, c.tail_ld, c.tail_ptr, c.ptr_ld, c.tail_rec, c.tail_cnt,
+                      nullptr, nullptr, nullptr, c.rms_weight, c.rms_eps, (cudaStream_t)stream, TQ_BF16, c.tail_dense,
+                      sp.val ? &sp : nullptr);
 }
 
 // `early`: the prologue of this call is the kernel in front
@@ -125,11 +141,11 @@ int linear_compute(const tq_linear_call& c, void* out, bool early, void* stream)
                                c.N, c.K, stream);
   }
   if (c.engine != TQ_LINEAR_FUSED) return TQ_ERR_BAD_ARG;
-  if (c.sp_val && c.M > 0 && linear_sparse(c)) {
+  if (takes_sparse(c)) {
     if (!c.a_q8 || !c.body_scale || !c.b_col || !c.w_scale || !c.w_rot || !out || !c.sp_meta || !c.sp_over_cnt ||
         !c.sp_over || c.sp_over_ld < (c.R + 1) / 2 || c.N <= 0 || c.K <= 0 || c.R >= c.K)
       return TQ_ERR_BAD_ARG;
-    if (c.N % 8 != 0 || c.K > 65536) return TQ_ERR_UNSUPPORTED;
+    if (c.K % 512 != 0 || c.N % 8 != 0 || c.K > 65536) return TQ_ERR_UNSUPPORTED;
     if (!aligned16(c.a_q8) || !aligned16(c.b_col) || !aligned16(out) || !aligned16(c.w_scale) || !aligned16(c.w_rot) ||
         !aligned16(c.w_t) || !aligned16(c.sp_over_cnt) || (c.bias && !aligned16(c.bias)))
       return TQ_ERR_MISALIGNED;
@@ -138,7 +154,7 @@ int linear_compute(const tq_linear_call& c, void* out, bool early, void* stream)
   }
   return run_split_gemm_mma(c.a_q8, c.body_scale, c.b_col, c.w_scale, c.w_rot, c.tail_idx16, c.tail_val, c.tail_ld,
                             c.tail_ptr, c.ptr_ld, c.tail_rec, c.tail_cnt, c.tail_dense, c.R, c.bias, out, nullptr, nullptr,
-                            c.M, c.N, c.K, c.act, early, stream, !sparse_and_dense(c));
+                            c.M, c.N, c.K, c.act, early, stream);
 }
 
 }  // namespace
@@ -153,7 +169,7 @@ extern "C" int tq_linear_outputs(const tq_linear_call* call, int shared) {
 
 extern "C" int tq_linear_sparse(const tq_linear_call* call, int shared) {
   if (!call || call->M < 0 || call->N <= 0 || call->K <= 0 || call->R < 0 || call->R >= call->K) return TQ_ERR_BAD_ARG;
-  return (shared ? tq::tail_can_be_sparse(*call) && tq::g_gemm_pair_mode < 0 && call->M > 64 : tq::linear_sparse(*call)) ? 1 : 0;
+  return (shared ? tq::shared_sparse(*call) : tq::linear_sparse(*call)) ? 1 : 0;
 }
 
 extern "C" int tq_linear_forward(const tq_linear_call* call, const void* x, void* out, void* stream) {

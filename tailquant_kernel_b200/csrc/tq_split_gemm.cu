@@ -67,7 +67,7 @@ int run_pair_gemm(const int8_t* a_q8, const float* body_scale, const uint8_t* b_
                   const void* w_rot, const uint16_t* tail_idx16, const void* tail_val, int tail_ld,
                   const uint16_t* tail_ptr, int ptr_ld, const uint32_t* tail_rec, const uint16_t* tail_cnt,
                   const void* tail_dense, int R, const float* bias, void* out_bf16, int32_t* dbg_acc, float* dbg_tail,
-                  int M, int N, int K, int act, bool records_filled, cudaStream_t st);
+                  int M, int N, int K, int act, cudaStream_t st);
 int run_sparse_gemm(const int8_t* a_q8, const float* body_scale, const uint8_t* b_col, const float* w_scale, const void* w_rot,
                     const void* w_t, const SparseTail& sp, const float* bias, void* out_bf16, int32_t* dbg_acc, float* dbg_tail,
                     int M, int N, int K, int act, bool early, cudaStream_t st);
@@ -148,7 +148,7 @@ static int run_split_gemm_mma(const int8_t* a_q8, const float* body_scale, const
                               const void* tail_val, int tail_ld, const uint16_t* tail_ptr, int ptr_ld,
                               const uint32_t* tail_rec, const uint16_t* tail_cnt, const void* tail_dense, int R,
                               const float* bias, void* out_bf16, int32_t* dbg_acc, float* dbg_tail, int M, int N, int K,
-                              int act, bool early, void* stream, bool records_filled = true) {
+                              int act, bool early, void* stream) {
   if (!a_q8 || !body_scale || !b_col || !w_scale || !out_bf16 || M < 0 || N <= 0 || K <= 0 || R < 0 || R >= K)
     return TQ_ERR_BAD_ARG;
   const bool records = tail_idx16 && tail_val && tail_ld >= R && tail_ptr && ptr_ld >= K / 128 + 1 && tail_rec && tail_cnt;
@@ -164,7 +164,7 @@ static int run_split_gemm_mma(const int8_t* a_q8, const float* body_scale, const
     return run_stream_gemm(a_q8, body_scale, b_col, w_scale, w_rot, tail_dense, R, bias, out_bf16, dbg_acc, dbg_tail, M, N,
                            K, act, early, (cudaStream_t)stream);
   return run_pair_gemm(a_q8, body_scale, b_col, w_scale, w_rot, tail_idx16, tail_val, tail_ld, tail_ptr, ptr_ld, tail_rec,
-                       tail_cnt, tail_dense, R, bias, out_bf16, dbg_acc, dbg_tail, M, N, K, act, records_filled, (cudaStream_t)stream);
+                       tail_cnt, tail_dense, R, bias, out_bf16, dbg_acc, dbg_tail, M, N, K, act, (cudaStream_t)stream);
 }
 }  // namespace tq
 

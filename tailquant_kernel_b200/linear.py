@@ -13,7 +13,6 @@ a forward is capturable in a CUDA graph after its first call, as the reference's
 from __future__ import annotations
 
 import ctypes
-import dataclasses
 import weakref
 from collections import OrderedDict
 from typing import Dict, Optional, Tuple
@@ -32,20 +31,24 @@ def interleave_gate_up(w_gate: torch.Tensor, w_up: torch.Tensor) -> torch.Tensor
 
 
 class _Workspace:
-    """Buffers of one (layer, M): the prologue outputs (`pro`; absent in the workspace a layer uses when it runs on
-    another layer's prologue) and the layer's own output and scratch.  They stay for as long as the layer does and are
-    only ever added to, since captured graphs name them: a row count that is seen once costs what its forward reads."""
+    """Buffers of one (layer, M): the prologue outputs (absent in the workspace a layer uses when it runs on another layer's
+    prologue) and the layer's own output and scratch.  They stay for as long as the layer does and are only ever added to,
+    since captured graphs name them: a row count that is seen once costs what its forward reads.  `pro` shows those of the
+    prologue outputs that are filled together, by a forward or by a prologue for several linears: a kernel chooses its
+    operand by what it finds, and must not find what another call left."""
 
     def __init__(self, M: int, N: int, K: int, R: int, device, engine: int, n_out: int, with_pro: bool,
                  with_tail: bool):
         empty = lambda shape, dtype: torch.empty(shape, dtype=dtype, device=device)  # noqa: E731
         self.M, self.K, self.R, self.engine = M, K, R, engine
-        self.pro = None
-        self.outputs, self.asked = 0, (-1, -1)   # TQ_OUT_* bits held; for what (see SplitLinear._provide)
-        self.sparse = None   # the tail in its 2:4-sparse form
+        self.held = None   # all prologue outputs
+        self.pro = None    # the ones in use, `outputs` and `sparse` of show()
+        self.outputs = 0
+        self.forward_for = self.shared_for = -1   # forced-kernel state (see ops) that `pro` was chosen under, -1: not `pro`
+        self._views: Dict[Tuple[int, bool], ops.PrologueOut] = {}
         if with_pro:
-            self.pro = ops.PrologueOut(a_pack=None, body_scale=empty(M, torch.float32), top_scale=empty(M, torch.float32),
-                                       tail_idx=None, tail_val=None, R=R)
+            self.held = ops.PrologueOut(a_pack=None, body_scale=empty(M, torch.float32), top_scale=empty(M, torch.float32),
+                                        tail_idx=None, tail_val=None, R=R)
         self.tail = empty((M, N), torch.float32) if with_tail else None   # sums of a tail kernel of its own
         self.out = empty((M, n_out), torch.bfloat16)
         self.call = None   # (a reference to) the native description of a forward out of these buffers; what it was filled in from
@@ -53,40 +56,44 @@ class _Workspace:
         self.call_src = ()
         self.rot_version = None   # of w_rot, where the description rests on its transpose
 
-    def hold(self, outputs: int) -> None:
-        """Adds the prologue outputs of `outputs` (TQ_OUT_* bits) that are not there yet."""
-        new = outputs & ~self.outputs
-        if not new:
-            return
-        p = self.pro = dataclasses.replace(self.pro)   # (descriptions that name the old one are filled in again)
-        M, K, R, device = self.M, self.K, self.R, self.out.device
+    _FIELDS = {_lib.TQ_OUT_PACK: ("a_pack",), _lib.TQ_OUT_Q8: ("a_q8",), _lib.TQ_OUT_LISTS: ("tail_idx", "tail_val"),
+               _lib.TQ_OUT_RECORDS: ("tail_ptr", "tail_rec", "tail_cnt"), _lib.TQ_OUT_DENSE: ("tail_dense",)}
+
+    def show(self, outputs: int, sparse: bool) -> None:
+        """Has `pro` be the prologue outputs of `outputs` (TQ_OUT_* bits) and, with `sparse`, the 2:4-sparse form of the tail,
+        making those that are not there yet."""
+        view = self._views.get((outputs, sparse))
+        if view is None:
+            self._make(outputs, sparse)
+            h = self.held
+            view = ops.PrologueOut(a_pack=None, body_scale=h.body_scale, top_scale=h.top_scale, tail_idx=None, tail_val=None,
+                                   R=h.R, sparse=h.sparse if sparse else None)
+            for bit, names in self._FIELDS.items():
+                for name in names if outputs & bit else ():
+                    setattr(view, name, getattr(h, name))
+            self._views[outputs, sparse] = view
+        self.pro, self.outputs = view, outputs
+
+    def _make(self, outputs: int, sparse: bool) -> None:
+        p, M, K, R, device = self.held, self.M, self.K, self.R, self.out.device
         empty = lambda shape, dtype: torch.empty(shape, dtype=dtype, device=device)  # noqa: E731
-        if new & _lib.TQ_OUT_PACK:
+        if outputs & _lib.TQ_OUT_PACK and p.a_pack is None:
             p.a_pack = empty((M, K // 2), torch.uint8)
-        if new & _lib.TQ_OUT_Q8:
+        if outputs & _lib.TQ_OUT_Q8 and p.a_q8 is None:
             p.a_q8 = empty((M, K), torch.int8)
-        if new & _lib.TQ_OUT_LISTS:
+        if outputs & _lib.TQ_OUT_LISTS and p.tail_idx is None:
             p.tail_idx = torch.zeros((M, (R + 7) // 8 * 8), dtype=torch.int16, device=device)
             p.tail_val = torch.zeros((M, (R + 7) // 8 * 8), dtype=torch.bfloat16, device=device)
-        if new & _lib.TQ_OUT_RECORDS:
+        if outputs & _lib.TQ_OUT_RECORDS and p.tail_ptr is None:
             half_slices = (2 * ((M + 255) // 256), K // 64, 128)
             p.tail_ptr = empty((M, K // 128 + 1), torch.int16)
             p.tail_rec = empty((*half_slices, ops.TAIL_REC_CAP), torch.int32)
             p.tail_cnt = torch.zeros(half_slices, dtype=torch.int16, device=device)
-        if new & _lib.TQ_OUT_DENSE:
+        if outputs & _lib.TQ_OUT_DENSE and p.tail_dense is None:
             p.tail_dense = empty((M, K), torch.bfloat16)
-        self.outputs |= new
-
-    def use_sparse(self, use: bool) -> None:
-        """Whether the prologue fills the tail in its 2:4-sparse form."""
-        if use == (self.pro.sparse is not None):
-            return
-        if use and self.sparse is None:
-            M, K = self.M, self.K
-            self.sparse = tuple(torch.empty(s, dtype=t, device=self.out.device) for s, t in (
-                ((M, K // 2), torch.bfloat16), ((M, K // 32), torch.int32), ((M,), torch.int16),
-                ((M, (self.R + 1) // 2), torch.int32)))
-        self.pro = dataclasses.replace(self.pro, sparse=self.sparse if use else None)
+        if sparse and p.sparse is None:
+            p.sparse = (empty((M, K // 2), torch.bfloat16), empty((M, K // 32), torch.int32), empty((M,), torch.int16),
+                        empty((M, (R + 1) // 2), torch.int32))
 
 
 class SplitLinear:
@@ -239,15 +246,19 @@ class SplitLinear:
         return _lib.TQ_LINEAR_DECODE if M <= self.small_m else _lib.TQ_LINEAR_GATHER
 
     def _provide(self, ws: _Workspace, shared: bool) -> None:
-        """Has `ws` hold what this layer's forward reads, or with `shared` what any layer on the same prologue may read (a
-        layer with the exact-order engine only shares with its like).  Asked once, and again under another forced kernel."""
+        """Has `ws` show what this layer's forward reads, or with `shared` what any layer on the same prologue may read (a
+        layer with the exact-order engine only shares with its like).  Asked when the one follows the other, and again under
+        another forced kernel."""
+        lib, any_width = _lib.load(), int(shared and self.tail_engine == "mma")
         c = _lib.LinearCall(M=ws.M, N=self.N, K=self.K, R=self.R, had_kind=self.w.had_kind, engine=ws.engine)
-        bits = _lib.load().tq_linear_outputs(ctypes.byref(c), int(shared and self.tail_engine == "mma"))
+        sparse = lib.tq_linear_sparse(ctypes.byref(c), any_width) > 0
+        c.sp_val = 1 if sparse else None   # (asks for what is needed beside it)
+        bits = lib.tq_linear_outputs(ctypes.byref(c), any_width)
         if bits < 0:
             _lib.check(bits, self._what(ws.M))
-        ws.hold(bits)
-        ws.use_sparse(_lib.load().tq_linear_sparse(ctypes.byref(c), int(shared and self.tail_engine == "mma")) > 0)
-        ws.asked = (ops.gemm_pair_mode_changes, int(shared))
+        ws.show(bits, sparse)
+        now = ops.gemm_pair_mode_changes
+        ws.forward_for, ws.shared_for = (-1, now) if shared else (now, -1)
 
     def _new_workspace(self, M: int, with_pro: bool) -> _Workspace:
         engine = self._engine(M)
@@ -259,8 +270,8 @@ class SplitLinear:
         ws = self._ws.get(M)
         if ws is None:
             ws = self._ws[M] = self._new_workspace(M, True)
-        if ws.asked[0] != ops.gemm_pair_mode_changes or shared > ws.asked[1]:
-            self._provide(ws, shared or ws.asked[1] > 0)
+        if (ws.shared_for if shared else ws.forward_for) != ops.gemm_pair_mode_changes:
+            self._provide(ws, shared)
         return ws
 
     def workspace(self, M: int) -> _Workspace:
@@ -413,7 +424,7 @@ class SplitLinear:
             raise RuntimeError("x must be a CUDA tensor")
         M = x.numel() // self.K
         ws = self._ws.get(M)
-        if ws is None or ws.asked[0] != ops.gemm_pair_mode_changes:
+        if ws is None or ws.forward_for != ops.gemm_pair_mode_changes:
             ws = self._workspace(M, False)
         call = ws.call
         if call is None or ws.call_pro is not ws.pro or not self._described(ws):

@@ -353,40 +353,39 @@ def split_gemm_mma(a_q8, body_scale, B_pack, w_scale, out, w_rot=None, pro: Opti
     _check(B_pack.shape[1] * 2 == K, "a_q8 and B_pack disagree on K")
     _check(out.numel() >= (M * N // 2 if act == "swiglu" else M * N), "out too small")
     _check(act == "none" or (dbg_acc is None and dbg_tail is None), "no debug outputs with a fused activation")
-    ld = 0
+    ld = ptr_ld = 0
+    if bias is not None:
+        _check_cuda(bias, "bias", torch.float32)
     if R:
         _check_cuda(w_rot, "w_rot", torch.bfloat16)
         _check(tuple(w_rot.shape) == (N, K), "w_rot must be [N, K]")
         _check(pro is not None, "the prologue outputs are needed when R > 0")
-        tail_idx, tail_val, tail_ptr, tail_rec, tail_cnt = pro.tail_idx, pro.tail_val, pro.tail_ptr, pro.tail_rec, pro.tail_cnt
-        _check_cuda(tail_idx, "tail_idx", torch.int16)
-        _check_cuda(tail_val, "tail_val", torch.bfloat16)
-        _check_cuda(tail_ptr, "tail_ptr", torch.int16)
-        _check_cuda(tail_rec, "tail_rec", torch.int32)
-        _check_cuda(tail_cnt, "tail_cnt", torch.int16)
-        _check(tail_ptr.shape[0] == M and tail_ptr.shape[1] >= K // 128 + 1, "tail_ptr must be [M, K/128 + 1]")
-        _check(tuple(tail_rec.shape) == (2 * ((M + 255) // 256), K // 64, 128, TAIL_REC_CAP), "tail_rec has the wrong shape")
-        _check(tuple(tail_cnt.shape) == (2 * ((M + 255) // 256), K // 64, 128), "tail_cnt has the wrong shape")
-        ld = tail_idx.shape[1]
-        if pro.tail_dense is not None:
-            _check_cuda(pro.tail_dense, "tail_dense", torch.bfloat16)
-            _check(tuple(pro.tail_dense.shape) == (M, K), "tail_dense must be [M, K]")
-    if bias is not None:
-        _check_cuda(bias, "bias", torch.float32)
-    if R and pro.sparse is not None:
-        if takes_sparse(M, N, K, R):
+        # (what the prologue of another kernel left unfilled is not in `pro`: its sparse form serves where nothing else is there)
+        if pro.sparse is not None and (takes_sparse(M, N, K, R) or (pro.tail_rec is None and pro.tail_dense is None)):
             _check(tuple(pro.sparse[0].shape) == (M, K // 2), "the sparse tail operand has the wrong shape")
             rc = _lib.load().tq_split_gemm_sparse(
                 _ptr(a_q8), _ptr(body_scale), _ptr(B_pack), _ptr(w_scale), _ptr(w_rot), None, int(R), *map(_ptr, pro.sparse),
                 pro.sparse[3].shape[1], _ptr(bias), _ptr(out), _ptr(dbg_acc), _ptr(dbg_tail), M, N, K, int(act == "swiglu"), _stream())
             _lib.check(rc, f"split_gemm_mma(M={M}, N={N}, K={K}, R={R})")
             return out
-        if pro.tail_dense is not None:   # (the records are not filled where both of the others are)
-            tail_rec = tail_cnt = None
+        tail_idx, tail_val, tail_ptr, tail_rec, tail_cnt = pro.tail_idx, pro.tail_val, pro.tail_ptr, pro.tail_rec, pro.tail_cnt
+        if pro.sparse is None or tail_rec is not None:
+            _check_cuda(tail_idx, "tail_idx", torch.int16)
+            _check_cuda(tail_val, "tail_val", torch.bfloat16)
+            _check_cuda(tail_ptr, "tail_ptr", torch.int16)
+            _check_cuda(tail_rec, "tail_rec", torch.int32)
+            _check_cuda(tail_cnt, "tail_cnt", torch.int16)
+            _check(tail_ptr.shape[0] == M and tail_ptr.shape[1] >= K // 128 + 1, "tail_ptr must be [M, K/128 + 1]")
+            _check(tuple(tail_rec.shape) == (2 * ((M + 255) // 256), K // 64, 128, TAIL_REC_CAP), "tail_rec has the wrong shape")
+            _check(tuple(tail_cnt.shape) == (2 * ((M + 255) // 256), K // 64, 128), "tail_cnt has the wrong shape")
+            ld, ptr_ld = tail_idx.shape[1], tail_ptr.shape[1]
+        if pro.tail_dense is not None:
+            _check_cuda(pro.tail_dense, "tail_dense", torch.bfloat16)
+            _check(tuple(pro.tail_dense.shape) == (M, K), "tail_dense must be [M, K]")
     common = (_ptr(a_q8), _ptr(body_scale), _ptr(B_pack), _ptr(w_scale),
               _ptr(w_rot) if R else None, _ptr(tail_idx) if R else None,
               _ptr(tail_val) if R else None, ld, _ptr(tail_ptr) if R else None,
-              tail_ptr.shape[1] if R else 0, _ptr(tail_rec) if R else None,
+              ptr_ld, _ptr(tail_rec) if R else None,
               _ptr(tail_cnt) if R else None, _ptr(pro.tail_dense) if R else None, int(R), _ptr(bias), _ptr(out))
     if act == "swiglu":
         rc = _lib.load().tq_split_gemm_mma_swiglu(*common, M, N, K, _stream())

@@ -189,6 +189,56 @@ def test_a_prologue_into_a_used_workspace(M):
     assert torch.equal(out, y) and torch.equal(lin.compute(ws, M), y)
 
 
+def outputs(pro):
+    return [t for t in (pro.a_pack, pro.a_q8, pro.body_scale, pro.tail_idx, pro.tail_val, pro.tail_ptr, pro.tail_rec, pro.tail_cnt,
+                        pro.tail_dense, *(pro.sparse or ())) if t is not None]
+
+
+@pytest.mark.parametrize("M,N,K", [(3, 512, 1024), (40, 512, 1024), (200, 8192, 1024), (1000, 4096, 1024), (1000, 4096, 4096),
+                                   (1500, 8192, 1024), (1500, 4096, 2048)])
+def test_every_output_shown_is_written(M, N, K):
+    """By a forward and by a prologue for several linears, in turn on inputs of their own: whatever a kernel finds there is of
+    this input, and the results are those of a fresh layer."""
+    from tailquant_kernel_b200 import SplitLinear
+    g = torch.Generator().manual_seed(6)
+    w = (torch.randn(N, K, generator=g) * 0.02).to(torch.bfloat16).cuda()
+    lin = SplitLinear(w, had_kind=3 if K == 2048 else None)
+    for seed, run in enumerate((lin.forward, lin.prologue, lin.forward, lin.prologue)):
+        x = activations("few_levels", M, K, seed)
+        lin.workspace(M)
+        if run == lin.forward:
+            lin._workspace(M, False)
+        shown = outputs(lin._ws[M].pro)
+        for t in shown:
+            t.view(torch.uint8).fill_(0x5b)
+        run(x)
+        assert [t.data_ptr() for t in outputs(lin._ws[M].pro)] == [t.data_ptr() for t in shown]
+        for t in shown:
+            assert not bool((t.view(torch.uint8) == 0x5b).all())
+        y = lin.compute(lin._ws[M], M).clone()
+        fresh = SplitLinear.from_prepared(lin.w)
+        assert torch.equal(y, fresh(x))
+
+
+@pytest.mark.parametrize("mode", [0, 1])
+def test_another_kernel_after_a_forward_on_the_sparse_form(mode):
+    """It finds the sparse form and nothing else of the tail, and takes that."""
+    from tailquant_kernel_b200 import SplitLinear
+    M, N, K = 1500, 8192, 1024
+    g = torch.Generator().manual_seed(8)
+    lin = SplitLinear((torch.randn(N, K, generator=g) * 0.02).to(torch.bfloat16).cuda())
+    y = lin(activations("hot", M, K, 3)).clone()
+    pro = lin._ws[M].pro
+    assert pro.sparse is not None
+    out = torch.empty_like(y)
+    ops.set_gemm_pair_mode(mode)
+    try:
+        ops.split_gemm_mma(pro.a_q8, pro.body_scale, lin.w.b_col, lin.w.w_scale, out, w_rot=lin.w.w_rot, pro=pro, R=lin.R)
+        assert torch.equal(out, y) and torch.equal(lin.compute(lin._ws[M], M), y)
+    finally:
+        ops.set_gemm_pair_mode(-1)
+
+
 def test_swiglu_of_every_gate():
     """The quotient of the epilogue rounds like a division: all 2^16 gates (through the finisher of the split-K path), against
     fp64 rounded once to fp32 and then to bf16."""

@@ -132,9 +132,10 @@ def _held(pro):
     return sum(b for b, ts in bits.items() if ts[0] is not None)
 
 
-def _asked(M, N, K, R, kind, engine, shared):
+def _asked(M, N, K, R, kind, engine, shared, sparse=False):
+    """`sparse`: beside the 2:4-sparse form of the tail."""
     import ctypes
-    call = _lib.LinearCall(M=M, N=N, K=K, R=R, had_kind=kind, engine=engine)
+    call = _lib.LinearCall(M=M, N=N, K=K, R=R, had_kind=kind, engine=engine, sp_val=1 if sparse else None)
     return _lib.load().tq_linear_outputs(ctypes.byref(call), shared)
 
 
@@ -166,7 +167,8 @@ def test_workspaces_hold_what_the_library_asks_for(fake, M, mode):
     try:
         for lin in (layer(), layer(N=24576, K=512, rms_weight=None), layer(ratio=0.0), layer(K=2048), layer(tail_engine="gather")):
             ws = lin.workspace(M)
-            assert _held(ws.pro) == _asked(M, lin.N, lin.K, lin.R, lin.w.had_kind, ws.engine, int(lin.tail_engine == "mma"))
+            assert _held(ws.pro) == _asked(M, lin.N, lin.K, lin.R, lin.w.had_kind, ws.engine, int(lin.tail_engine == "mma"),
+                                           ws.pro.sparse is not None)
     finally:
         ops.set_gemm_pair_mode(-1)
 
@@ -179,10 +181,11 @@ def test_a_forward_allocates_what_it_reads(fake, M):
         x = claimed(M, lin.K, dtype=torch.bfloat16)
         lin(x)
         ws = lin._ws[M]
-        assert _held(ws.pro) == _asked(M, lin.N, lin.K, lin.R, lin.w.had_kind, ws.engine, 0)
+        assert _held(ws.pro) == _asked(M, lin.N, lin.K, lin.R, lin.w.had_kind, ws.engine, 0, ws.pro.sparse is not None)
         before = {f.name: getattr(ws.pro, f.name) for f in dataclasses.fields(ws.pro)}
         assert lin.prologue(x) is ws
-        assert _held(ws.pro) == _asked(M, lin.N, lin.K, lin.R, lin.w.had_kind, ws.engine, int(lin.tail_engine == "mma"))
+        assert _held(ws.pro) == _asked(M, lin.N, lin.K, lin.R, lin.w.had_kind, ws.engine, int(lin.tail_engine == "mma"),
+                                       ws.pro.sparse is not None)
         assert all(v is None or getattr(ws.pro, n) is v for n, v in before.items())
         name, c = fake.calls[-1]
         assert name == PROLOGUE and c["a_q8"] == (ws.pro.a_q8.data_ptr() if ws.pro.a_q8 is not None else None)

@@ -144,3 +144,46 @@ def test_a_sparse_operand_of_another_size_is_refused(fake):  # noqa: F811
         ops.split_prologue(claimed(900, 512, dtype=torch.bfloat16), lin.w.had_kind, lin.R, lin.descending_rank,
                            out=lin.workspace(1500).pro)
     assert not fake.calls
+
+
+def named(c, pro):
+    """The outputs of `pro` that the call `c` names, and those it does not."""
+    fields = dict(a_pack="a_pack", a_q8="a_q8", tail_idx="tail_idx16", tail_val="tail_val", tail_ptr="tail_ptr",
+                  tail_rec="tail_rec", tail_cnt="tail_cnt", tail_dense="tail_dense")
+    pairs = [(getattr(pro, f), c[g]) for f, g in fields.items()] + list(zip(pro.sparse or (), (c[f] for f in ops.SPARSE_FIELDS)))
+    return all((t.data_ptr() if t is not None else None) == at for t, at in pairs) and (pro.sparse or not c["sp_val"])
+
+
+@pytest.mark.parametrize("M", [1, 40, 200, 1000, 1500, 5000])
+@pytest.mark.parametrize("N,K", [(24576, 512), (256, 512), (1024, 4096), (256, 2048)])
+def test_what_a_workspace_shows_is_what_the_last_call_filled(fake, M, N, K):  # noqa: F811
+    """A kernel takes its operand by what it finds: nothing of another call may be among it."""
+    lin = layer(N=N, K=K, rms_weight=None)
+    x = claimed(M, K, dtype=torch.bfloat16)
+    shown = {}
+    for run in ("forward", "prologue", "forward", "prologue", "split_prologue"):
+        if run == "split_prologue":
+            if lin._ws[M].pro.sparse is None:
+                continue   # (its entry point takes the outputs one by one)
+            ops.split_prologue(x, lin.w.had_kind, lin.R, lin.descending_rank, out=lin.workspace(M).pro)
+        else:
+            getattr(lin, run)(x)
+        pro = lin._ws[M].pro
+        assert named(fake.calls[-1][1], pro), run
+        assert shown.setdefault(run, pro) is pro
+    assert lin._ws[M].held.a_q8 is lin._ws[M].pro.a_q8
+
+
+def test_a_forward_on_the_sparse_form_holds_no_other_operand(fake):  # noqa: F811
+    lin = layer(N=24576, K=512, rms_weight=None)
+    lin(claimed(1500, 512, dtype=torch.bfloat16))
+    held = lin._ws[1500].held
+    assert held.sparse is not None and held.tail_rec is None and held.tail_cnt is None and held.tail_dense is None
+
+
+def test_records_are_left_out_where_the_other_forms_are_there(fake):  # noqa: F811
+    """Up to 1024 rows a shared prologue leaves the sparse form and the zero-filled matrix; beyond, records and not the matrix."""
+    lin = layer(N=24576, K=512, rms_weight=None)
+    few, many = lin.workspace(1000).pro, lin.workspace(1500).pro
+    assert few.sparse is not None and few.tail_dense is not None and few.tail_rec is None
+    assert many.sparse is not None and many.tail_dense is None and many.tail_rec is not None
