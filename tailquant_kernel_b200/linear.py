@@ -54,6 +54,7 @@ class _Workspace:
         self.call = None   # (a reference to) the native description of a forward out of these buffers; what it was filled in from
         self.call_pro = None
         self.call_src = ()
+        self.call_t = None
         self.rot_version = None   # of w_rot, where the description rests on its transpose
 
     _FIELDS = {_lib.TQ_OUT_PACK: ("a_pack",), _lib.TQ_OUT_Q8: ("a_q8",), _lib.TQ_OUT_LISTS: ("tail_idx", "tail_val"),
@@ -291,9 +292,14 @@ class SplitLinear:
 
     def prepare_decode(self) -> None:
         """Builds the [K, N] transpose of the rotated weights that the small-M tail reads, ahead of the first small-M
-        forward (which otherwise builds it: an allocation inside that call)."""
-        if self.R and self.w.w_t is None:
+        forward (which otherwise builds it: an allocation inside that call).  Not inside a stream capture: nothing would have
+        written it before the first replay, and every replay would write it again."""
+        if self.R and self.w.w_t is None and not self._capturing():
             self.w.w_t = self._transposed()
+
+    @staticmethod
+    def _capturing() -> bool:
+        return _lib.load().tq_stream_capture_id(ops._stream()) != 0
 
     def _transposed(self, into: Optional[torch.Tensor] = None) -> torch.Tensor:
         r = self.w.w_rot
@@ -305,16 +311,20 @@ class SplitLinear:
         r = self.w.w_rot
         return -1 if r is None or r.is_inference() else r._version
 
-    def _prepare_sparse(self, own: _Workspace) -> None:
+    def _prepare_sparse(self, own: _Workspace) -> bool:
         """The transpose that the left-over entries of the sparse tail are read from.  A layer that had none did not ask for it
         and is not expected to keep it in line: it is made again when `w_rot` was replaced or changed since, in the same memory
-        where `w_rot` is the same tensor (a graph captured before names both)."""
+        where `w_rot` is the same tensor (a graph captured before names both).  False where it would have to be made inside a
+        stream capture: the kernel then reads `w_rot`, and the next call outside makes it."""
         w = self.w
         if w.w_rot is None:
-            return   # (refused with the other parts)
+            return False   # (refused with the other parts)
         version = self._rot_version()
         t, rot, v, place = self._t_of
-        if w.w_t is not None and w.w_t is t and (w.w_rot is not rot or (version, rot.data_ptr()) != (v, place)):
+        changed = w.w_t is not None and w.w_t is t and (w.w_rot is not rot or (version, rot.data_ptr()) != (v, place))
+        if (changed or w.w_t is None) and self._capturing():
+            return False
+        if changed:
             if w.w_rot is rot and tuple(t.shape) == tuple(reversed(rot.shape)) and t.dtype == rot.dtype and t.device == rot.device:
                 self._transposed(t)
             else:
@@ -322,6 +332,7 @@ class SplitLinear:
         self.prepare_decode()
         self._t_of = (w.w_t, w.w_rot, version, w.w_rot.data_ptr())
         own.rot_version = version
+        return True
 
     def _described(self, own: _Workspace) -> bool:
         """Whether `own.call` still names what this layer consists of.  All of it can be replaced between two forwards, and a
@@ -336,8 +347,8 @@ class SplitLinear:
                 and (own.rot_version is None or own.rot_version == self._rot_version())
                 and kind == w.had_kind and rank == self.descending_rank and eps == self.rms_eps and act == self.epilogue)
 
-    def _check_parts(self, engine: int, transposed: bool = False) -> None:
-        """Types, layout and sizes of what a forward reads (`transposed`: w_t beside w_rot): the kernels take it for granted."""
+    def _check_parts(self, engine: int, w_t: Optional[torch.Tensor]) -> None:
+        """Types, layout and sizes of what a forward reads (`w_t`: the transpose it is given): the kernels take it for granted."""
         w, N, K = self.w, self.N, self.K
         ops._check_cuda(w.b_col, "b_col", torch.uint8)
         ops._check(tuple(w.b_col.shape) == (N, K // 2), "b_col must be [N, K/2]")
@@ -346,9 +357,9 @@ class SplitLinear:
         if self.R and engine == _lib.TQ_LINEAR_FUSED:
             ops._check_cuda(w.w_rot, "w_rot", torch.bfloat16)
             ops._check(tuple(w.w_rot.shape) == (N, K), "w_rot must be [N, K]")
-        if self.R and (transposed or engine != _lib.TQ_LINEAR_FUSED):
-            ops._check_cuda(w.w_t, "w_t", torch.bfloat16)
-            ops._check(tuple(w.w_t.shape) == (K, N), "w_t must be [K, N]")
+        if self.R and (w_t is not None or engine != _lib.TQ_LINEAR_FUSED):
+            ops._check_cuda(w_t, "w_t", torch.bfloat16)
+            ops._check(tuple(w_t.shape) == (K, N), "w_t must be [K, N]")
         if w.bias is not None:
             ops._check_cuda(w.bias, "bias", torch.float32)
             ops._check(w.bias.numel() >= N, "bias must have N elements")
@@ -361,16 +372,23 @@ class SplitLinear:
         `own`."""
         if own.call is not None and own.call_pro is pro and self._described(own):
             return own.call
-        own.rot_version = None
+        own.rot_version = own.call = None   # (a part that is refused must not leave the former description in force)
+        w, p = self.w, ops._ptr
+        keep, w_t = True, w.w_t
         if own.engine == _lib.TQ_LINEAR_DECODE:
             self.prepare_decode()
-        elif own.engine == _lib.TQ_LINEAR_FUSED and pro.sparse is not None and \
-                ops.takes_sparse(own.M, self.N, self.K, self.R, self.w.had_kind):
-            self._prepare_sparse(own)
-        own.call = None   # (a part that is refused must not leave the former description in force)
-        self._check_parts(own.engine, own.rot_version is not None)
-        w, p = self.w, ops._ptr
-        own.call_pro = pro
+            w_t = w.w_t
+            if self.R and w_t is None and w.w_rot is not None:   # in a stream capture, for this call of it only
+                keep, w_t = False, self._transposed()
+        elif own.engine == _lib.TQ_LINEAR_FUSED and pro.sparse is not None:
+            if ops.takes_sparse(own.M, self.N, self.K, self.R, w.had_kind):
+                keep = self._prepare_sparse(own)
+                w_t = w.w_t if keep else None
+            elif w_t is self._t_of[0]:
+                w_t = None   # (where the sparse form is all there is, `w_rot` is what is certain to be in line)
+        self._check_parts(own.engine, w_t if own.engine != _lib.TQ_LINEAR_FUSED or own.rot_version is not None else None)
+        own.call_pro = pro if keep else None
+        own.call_t = w_t   # (lives as long as its address is in `call`)
         src = (w.b_col, w.w_scale, w.w_rot, w.w_t, w.bias, self.rms_weight)
         own.call_src = (*src, w.had_kind, self.descending_rank, self.rms_eps, self.epilogue, *map(p, src))
         own.call = ctypes.byref(_lib.LinearCall(
@@ -378,7 +396,7 @@ class SplitLinear:
             engine=own.engine, act=1 if self.epilogue == "swiglu" else 0,
             tail_ld=pro.tail_idx.shape[1] if pro.tail_idx is not None else 0,
             ptr_ld=pro.tail_ptr.shape[1] if pro.tail_ptr is not None else 0, eps=ops.EPS, rms_eps=self.rms_eps,
-            b_col=p(w.b_col), w_scale=p(w.w_scale), w_rot=p(w.w_rot), w_t=p(w.w_t), bias=p(w.bias),
+            b_col=p(w.b_col), w_scale=p(w.w_scale), w_rot=p(w.w_rot), w_t=p(w_t), bias=p(w.bias),
             rms_weight=p(self.rms_weight), a_pack=p(pro.a_pack), a_q8=p(pro.a_q8), body_scale=p(pro.body_scale),
             top_scale=p(pro.top_scale), tail_idx16=p(pro.tail_idx), tail_val=p(pro.tail_val), tail_ptr=p(pro.tail_ptr),
             tail_rec=p(pro.tail_rec), tail_cnt=p(pro.tail_cnt), tail_dense=p(pro.tail_dense), tail=p(own.tail),

@@ -189,6 +189,28 @@ def test_a_prologue_into_a_used_workspace(M):
     assert torch.equal(out, y) and torch.equal(lin.compute(ws, M), y)
 
 
+@pytest.mark.parametrize("M", [1, 1500])
+def test_a_capture_that_is_the_first_call_on_the_transposed_weights(M):
+    """Eager calls between the capture and its first replay read a transpose of their own."""
+    from tailquant_kernel_b200 import SplitLinear
+    N, K = 8192, 1024
+    g = torch.Generator().manual_seed(5)
+    lin = SplitLinear((torch.randn(N, K, generator=g) * 0.02).to(torch.bfloat16).cuda())
+    fresh = SplitLinear.from_prepared(ops.PreparedWeight(**{**vars(lin.w), "w_t": None}))
+    lin(activations("plain", 300, K, 1)), torch.cuda.synchronize()
+    x, out = activations("few_levels", M, K, 2), []
+    lin.w.w_t = None
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        out.append(lin(x))
+    assert lin.w.w_t is None
+    want = fresh(x)
+    assert torch.equal(lin(x), want) and torch.equal(lin.w.w_t, lin.w.w_rot.t())
+    out[0].zero_()
+    graph.replay()
+    assert torch.equal(out[0], want)
+
+
 def outputs(pro):
     return [t for t in (pro.a_pack, pro.a_q8, pro.body_scale, pro.tail_idx, pro.tail_val, pro.tail_ptr, pro.tail_rec, pro.tail_cnt,
                         pro.tail_dense, *(pro.sparse or ())) if t is not None]

@@ -187,3 +187,57 @@ def test_records_are_left_out_where_the_other_forms_are_there(fake):  # noqa: F8
     few, many = lin.workspace(1000).pro, lin.workspace(1500).pro
     assert few.sparse is not None and few.tail_dense is not None and few.tail_rec is None
     assert many.sparse is not None and many.tail_dense is None and many.tail_rec is not None
+
+
+def test_a_capture_makes_no_transpose(fake):  # noqa: F811
+    """It would be written by no kernel before the first replay: the captured call reads `w_rot`, later ones make the transpose."""
+    lin = layer(N=24576, K=512, rms_weight=None)
+    lin.w.w_t = None
+    x = claimed(1500, 512, dtype=torch.bfloat16)
+    fake.capture = 7
+    for _ in range(2):
+        lin(x)
+        assert fake.calls[-1][1]["sp_val"] and not fake.calls[-1][1]["w_t"] and lin.w.w_t is None
+    lin.prepare_decode()
+    assert lin.w.w_t is None
+    fake.capture = 0
+    lin(x)
+    t = lin.w.w_t
+    assert t is not None and fake.calls[-1][1]["w_t"] == t.data_ptr()
+    fake.capture = 8
+    lin(x)
+    assert fake.calls[-1][1]["w_t"] == t.data_ptr()
+    lin.w.w_rot.fill_(2.0)
+    lin(x)
+    assert not fake.calls[-1][1]["w_t"] and float(t[3, 5]) == 0.0
+    fake.capture = 0
+    lin(x)
+    assert fake.calls[-1][1]["w_t"] == t.data_ptr() and lin.w.w_t is t and float(t[3, 5]) == 2.0
+
+
+def test_a_captured_decode_call_keeps_its_transpose_to_itself(fake):  # noqa: F811
+    lin = layer(rms_weight=None)
+    lin.w.w_t = None
+    x = claimed(1, 512, dtype=torch.bfloat16)
+    fake.capture = 7
+    lin(x)
+    assert fake.calls[-1][1]["engine"] == _lib.TQ_LINEAR_DECODE and fake.calls[-1][1]["w_t"] and lin.w.w_t is None
+    fake.capture = 0
+    lin(x)
+    assert lin.w.w_t is not None and fake.calls[-1][1]["w_t"] == lin.w.w_t.data_ptr()
+
+
+@pytest.mark.parametrize("how", ["in_place", "replaced"])
+def test_a_sparse_form_that_is_all_there_is_reads_weights_in_line(fake, how):  # noqa: F811
+    lin = layer(N=24576, K=512, rms_weight=None)
+    lin.w.w_t = None
+    lin(claimed(1500, 512, dtype=torch.bfloat16))
+    lin.w.w_rot.fill_(2.0)
+    if how == "replaced":
+        lin.w.w_rot = torch.full_like(lin.w.w_rot, 2.0)
+    ops.set_gemm_pair_mode(1)
+    try:
+        lin.compute(lin._ws[1500], 1500)
+    finally:
+        ops.set_gemm_pair_mode(-1)
+    assert fake.calls[-1][1]["sp_val"] and not fake.calls[-1][1]["w_t"]
