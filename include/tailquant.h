@@ -331,7 +331,7 @@ typedef struct tq_linear_call {
   int sp_over_ld;         /* at least (R + 1) / 2 */
 } tq_linear_call;
 
-/* Prologue outputs that the workspace of a call should hold, as a sum of these; reads M, N, K, R, had_kind and engine of
+/* Prologue outputs that the workspace of a call should hold, as a sum of these; reads M, N, K, R, had_kind, engine and act of
  * `call`, and whether sp_val is NULL: with sp_val the answer is what is needed beside the sp_* arrays, where tq_linear_sparse
  * says 1.  shared = 0: what tq_linear_forward of this call reads and writes.  shared = 1: what tq_linear_prologue should
  * leave for linears of any width (a wide and a narrow layer can be on different kernels; up to 64 rows also on the decode

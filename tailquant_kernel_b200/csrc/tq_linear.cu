@@ -19,12 +19,15 @@ bool linear_streams(const tq_linear_call& c) {
 // Rows beyond which the zero-filled matrix is not kept whatever it would save (layers whose pair kernel reads it excepted).
 constexpr int DENSE_MAX_ROWS = 4096;
 
+// Whether the kernel is built for the sizes of the call (its stores of SwiGLU outputs are 16 bytes wide).
+bool sparse_fits(const tq_linear_call& c) { return c.K % 512 == 0 && c.N % (c.act ? 16 : 8) == 0 && c.K <= 65536; }
+
 // Whether a linear can take its tail as a 2:4-sparse operand: a full rotation, which spreads the entries over K, and few enough of
 // them that a group of four rarely holds more than two.  (At R = 0.1 K the left-over entries outweigh what the sparse product
 // saves, and rows with a few large channels have twice as many.)
 bool tail_can_be_sparse(const tq_linear_call& c) {
-  return c.engine == TQ_LINEAR_FUSED && (c.had_kind == TQ_HAD_WHT || c.had_kind == TQ_HAD_KRON12) && c.R > 0 && c.K % 512 == 0 &&
-         c.N % 8 == 0 && (long)c.R * 100 <= 7l * c.K;
+  return c.engine == TQ_LINEAR_FUSED && (c.had_kind == TQ_HAD_WHT || c.had_kind == TQ_HAD_KRON12) && c.R > 0 && sparse_fits(c) &&
+         (long)c.R * 100 <= 7l * c.K;
 }
 
 // Whether the sparse form is the fastest for this call.
@@ -145,9 +148,10 @@ int linear_compute(const tq_linear_call& c, void* out, bool early, void* stream)
     if (!c.a_q8 || !c.body_scale || !c.b_col || !c.w_scale || !c.w_rot || !out || !c.sp_meta || !c.sp_over_cnt ||
         !c.sp_over || c.sp_over_ld < (c.R + 1) / 2 || c.N <= 0 || c.K <= 0 || c.R >= c.K)
       return TQ_ERR_BAD_ARG;
-    if (c.K % 512 != 0 || c.N % 8 != 0 || c.K > 65536) return TQ_ERR_UNSUPPORTED;
+    if (!sparse_fits(c)) return TQ_ERR_UNSUPPORTED;
     if (!aligned16(c.a_q8) || !aligned16(c.b_col) || !aligned16(out) || !aligned16(c.w_scale) || !aligned16(c.w_rot) ||
-        !aligned16(c.w_t) || !aligned16(c.sp_over_cnt) || (c.bias && !aligned16(c.bias)))
+        !aligned16(c.w_t) || !aligned16(c.sp_over_cnt) || !aligned16(c.sp_val) || !aligned16(c.sp_meta) ||
+        (c.bias && !aligned16(c.bias)))
       return TQ_ERR_MISALIGNED;
     return run_sparse_gemm(c.a_q8, c.body_scale, c.b_col, c.w_scale, c.w_rot, c.w_t, linear_sparse_tail(c), c.bias, out, nullptr,
                            nullptr, c.M, c.N, c.K, c.act, early, (cudaStream_t)stream);

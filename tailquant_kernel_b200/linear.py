@@ -251,7 +251,8 @@ class SplitLinear:
         layer with the exact-order engine only shares with its like).  Asked when the one follows the other, and again under
         another forced kernel."""
         lib, any_width = _lib.load(), int(shared and self.tail_engine == "mma")
-        c = _lib.LinearCall(M=ws.M, N=self.N, K=self.K, R=self.R, had_kind=self.w.had_kind, engine=ws.engine)
+        c = _lib.LinearCall(M=ws.M, N=self.N, K=self.K, R=self.R, had_kind=self.w.had_kind, engine=ws.engine,
+                            act=int(self.epilogue == "swiglu"))
         sparse = lib.tq_linear_sparse(ctypes.byref(c), any_width) > 0
         c.sp_val = 1 if sparse else None   # (asks for what is needed beside it)
         bits = lib.tq_linear_outputs(ctypes.byref(c), any_width)
@@ -381,7 +382,7 @@ class SplitLinear:
             if self.R and w_t is None and w.w_rot is not None:   # in a stream capture, for this call of it only
                 keep, w_t = False, self._transposed()
         elif own.engine == _lib.TQ_LINEAR_FUSED and pro.sparse is not None:
-            if ops.takes_sparse(own.M, self.N, self.K, self.R, w.had_kind):
+            if ops.takes_sparse(own.M, self.N, self.K, self.R, w.had_kind, int(self.epilogue == "swiglu")):
                 keep = self._prepare_sparse(own)
                 w_t = w.w_t if keep else None
             elif w_t is self._t_of[0]:

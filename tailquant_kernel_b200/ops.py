@@ -331,9 +331,9 @@ def split_gemm_fused(A_pack, body_scale, B_pack, w_scale, out, tail=None, bias=N
     return out
 
 
-def takes_sparse(M: int, N: int, K: int, R: int, had_kind: int = TQ_HAD_WHT) -> bool:
+def takes_sparse(M: int, N: int, K: int, R: int, had_kind: int = TQ_HAD_WHT, act: int = 0) -> bool:
     """Whether a fused linear reads the tail in its 2:4-sparse form where it finds it (the rule of tq_linear_compute)."""
-    c = _lib.LinearCall(M=M, N=N, K=K, R=R, had_kind=had_kind, engine=_lib.TQ_LINEAR_FUSED)
+    c = _lib.LinearCall(M=M, N=N, K=K, R=R, had_kind=had_kind, engine=_lib.TQ_LINEAR_FUSED, act=act)
     return _lib.load().tq_linear_sparse(ctypes.byref(c), 0) > 0
 
 
@@ -361,7 +361,7 @@ def split_gemm_mma(a_q8, body_scale, B_pack, w_scale, out, w_rot=None, pro: Opti
         _check(tuple(w_rot.shape) == (N, K), "w_rot must be [N, K]")
         _check(pro is not None, "the prologue outputs are needed when R > 0")
         # (what the prologue of another kernel left unfilled is not in `pro`: its sparse form serves where nothing else is there)
-        if pro.sparse is not None and (takes_sparse(M, N, K, R) or (pro.tail_rec is None and pro.tail_dense is None)):
+        if pro.sparse is not None and (takes_sparse(M, N, K, R, act=int(act == "swiglu")) or (pro.tail_rec is None and pro.tail_dense is None)):
             _check(tuple(pro.sparse[0].shape) == (M, K // 2), "the sparse tail operand has the wrong shape")
             rc = _lib.load().tq_split_gemm_sparse(
                 _ptr(a_q8), _ptr(body_scale), _ptr(B_pack), _ptr(w_scale), _ptr(w_rot), None, int(R), *map(_ptr, pro.sparse),

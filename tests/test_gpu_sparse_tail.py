@@ -149,6 +149,29 @@ def test_layer_with_swiglu_on_the_sparse_tail(M, N, K):
     assert float((d != 0).float().mean()) < 1e-3 and bool((d <= ref.abs() * 2.0 ** -7 + 1e-4).all())
 
 
+def test_swiglu_of_a_width_that_the_sparse_kernel_does_not_store():
+    """N % 16 == 8: the kernel on records, whatever else the prologue left."""
+    M, N, K = 1500, 8200, 1024
+    x = activations("hot", M, K, 3)
+    g = torch.Generator().manual_seed(9)
+    w = ops.prepare_weight((torch.randn(N, K, generator=g) * 0.02).to(torch.bfloat16).cuda(), t16=False, keep_w_rot=True)
+    from tailquant_kernel_b200 import SplitLinear
+    plain = SplitLinear.from_prepared(w)
+    y, pro = plain(x).clone(), plain.workspace(M).pro
+    assert pro.sparse is not None and ops.takes_sparse(M, N, K, plain.R) and not ops.takes_sparse(M, N, K, plain.R, act=1)
+    ops.split_prologue(x, w.had_kind, plain.R, plain.descending_rank, out=pro)
+    h = torch.empty((M, N // 2), dtype=torch.bfloat16, device="cuda")
+    ops.split_gemm_mma(pro.a_q8, pro.body_scale, w.b_col, w.w_scale, h, w_rot=w.w_rot, pro=pro, R=plain.R, act="swiglu")
+    gate, up = y[:, 0::2].float(), y[:, 1::2].float()
+    silu = torch.nn.functional.silu(gate)
+    want = (silu.to(torch.bfloat16).float() * up).to(torch.bfloat16).float()
+    # other order of the tail sum: a gate or an up value moves by a last place now and then, 2^-7 of it at most (|silu'| <= 1.1),
+    # and silu and the product are rounded again
+    bound = 2.0 ** -7 * (1.1 * (gate * up).abs() + 3 * (silu * up).abs()) + 1e-30
+    diff = (want - h.float()).abs()
+    assert float((diff != 0).float().mean()) < 2e-3 and bool((diff <= bound).all())
+
+
 def test_weights_changed_in_place_reach_the_left_over_entries():
     """The transposed weights are a copy that the layer made: it follows `w_rot`."""
     from tailquant_kernel_b200 import SplitLinear

@@ -241,3 +241,29 @@ def test_a_sparse_form_that_is_all_there_is_reads_weights_in_line(fake, how):  #
     finally:
         ops.set_gemm_pair_mode(-1)
     assert fake.calls[-1][1]["sp_val"] and not fake.calls[-1][1]["w_t"]
+
+
+def described(**fields):
+    """A call on the sparse kernel at 2048 x N x 4096 whose arrays lie at addresses that are never read here."""
+    pointers = ("b_col", "w_scale", "w_rot", "w_t", "a_q8", "body_scale", "top_scale", *ops.SPARSE_FIELDS)
+    return _lib.LinearCall(**{**dict(M=2048, N=4096, K=4096, R=205, had_kind=1, descending_rank=206, sp_over_ld=104,
+                                     engine=_lib.TQ_LINEAR_FUSED), **{f: 0x10000 for f in pointers}, **fields})
+
+
+@pytest.mark.parametrize("field", ["sp_val", "sp_meta", "sp_over_cnt", "a_q8", "w_t", "w_rot"])
+def test_misaligned_operands_are_refused(field):
+    c = described(**{field: 0x10008})
+    assert _lib.load().tq_linear_compute(ctypes.byref(c), 0x10000, 0) == -3
+
+
+@pytest.mark.parametrize("N,act,takes", [(4096, 1, 1), (4104, 0, 1), (4104, 1, 0), (4100, 0, 0)])
+def test_swiglu_needs_whole_stores(N, act, takes):
+    """16 bytes of SwiGLU outputs are 16 channel pairs: other widths stay on the kernels that store them in halves, and where there
+    is nothing but the sparse form they are refused."""
+    lib, c = _lib.load(), described(N=N, act=act)
+    assert lib.tq_linear_sparse(ctypes.byref(c), 0) == takes
+    assert ops.takes_sparse(2048, N, 4096, 205, act=act) == bool(takes)
+    bits = lib.tq_linear_outputs(ctypes.byref(c), 0)
+    assert bool(bits & _lib.TQ_OUT_RECORDS) == (not takes)
+    if not takes:
+        assert lib.tq_linear_compute(ctypes.byref(c), 0x10000, 0) == -2
