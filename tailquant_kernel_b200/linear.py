@@ -298,6 +298,18 @@ class SplitLinear:
         if self.R and self.w.w_t is None and not self._capturing():
             self.w.w_t = self._transposed()
 
+    def refresh(self) -> None:
+        """Makes the [K, N] transpose again, where there is one, after `w_rot` was written by something that its version counter
+        does not see: collectives (`torch.distributed.broadcast`, `all_reduce`), `.data.copy_()`, raw pointers, and every
+        write to tensors made in inference mode.  In the same memory, so that captured graphs follow; not inside a capture.
+        Nothing else of a layer is a copy."""
+        w = self.w
+        if self.R == 0 or w.w_t is None or w.w_rot is None:
+            return
+        if self._capturing():
+            raise RuntimeError("refresh() cannot run inside a stream capture")
+        self._transposed(w.w_t)
+
     @staticmethod
     def _capturing() -> bool:
         return _lib.load().tq_stream_capture_id(ops._stream()) != 0

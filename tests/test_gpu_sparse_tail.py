@@ -212,6 +212,25 @@ def test_a_prologue_into_a_used_workspace(M):
     assert torch.equal(out, y) and torch.equal(lin.compute(ws, M), y)
 
 
+def test_refresh_after_a_write_that_is_not_counted():
+    """As a collective into `w_rot` leaves it; a captured graph follows, since the transpose stays where it is."""
+    from tailquant_kernel_b200 import SplitLinear
+    M, N, K = 1500, 8192, 1024
+    g = torch.Generator().manual_seed(7)
+    a, b = ((torch.randn(N, K, generator=g) * 0.02).to(torch.bfloat16).cuda() for _ in range(2))
+    lin, other = SplitLinear(a), SplitLinear(b)
+    x = activations("few_levels", M, K, 2)
+    lin(x)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        y = lin(x)
+    for f in ("w_rot", "b_col", "w_scale"):
+        getattr(lin.w, f).data.copy_(getattr(other.w, f))
+    lin.refresh()
+    graph.replay()
+    assert torch.equal(y, other(x)) and torch.equal(lin(x), other(x))
+
+
 @pytest.mark.parametrize("M", [1, 1500])
 def test_a_capture_that_is_the_first_call_on_the_transposed_weights(M):
     """Eager calls between the capture and its first replay read a transpose of their own."""

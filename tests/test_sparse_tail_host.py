@@ -267,3 +267,34 @@ def test_swiglu_needs_whole_stores(N, act, takes):
     assert bool(bits & _lib.TQ_OUT_RECORDS) == (not takes)
     if not takes:
         assert lib.tq_linear_compute(ctypes.byref(c), 0x10000, 0) == -2
+
+
+@pytest.mark.parametrize("write", ["data", "inference"])
+def test_refresh_after_a_write_that_is_not_counted(fake, write):  # noqa: F811
+    lin = layer(N=24576, K=512, rms_weight=None)
+    lin.w.w_t = None
+    if write == "inference":
+        with torch.inference_mode():
+            lin.w.w_rot = claimed(24576, 512, dtype=torch.bfloat16)
+    lin.refresh()
+    assert lin.w.w_t is None
+    x = claimed(1500, 512, dtype=torch.bfloat16)
+    lin(x)
+    t = lin.w.w_t
+    with torch.inference_mode():
+        lin.w.w_rot.data.fill_(2.0)
+    lin.refresh()
+    assert lin.w.w_t is t and float(t[3, 5]) == 2.0
+    lin(x)
+    assert fake.calls[-1][1]["w_t"] == t.data_ptr()
+    fake.capture = 7
+    with pytest.raises(RuntimeError, match="capture"):
+        lin.refresh()
+
+
+def test_refresh_of_a_transpose_that_cannot_follow(fake):  # noqa: F811
+    """Another matrix under `w_rot`: an error instead of a half-written transpose."""
+    lin = layer(N=256, K=512, rms_weight=None)
+    lin.w.w_rot = claimed(256, 256, dtype=torch.bfloat16)
+    with pytest.raises(RuntimeError):
+        lin.refresh()
