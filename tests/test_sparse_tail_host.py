@@ -179,6 +179,7 @@ def test_a_forward_on_the_sparse_form_holds_no_other_operand(fake):  # noqa: F81
     lin(claimed(1500, 512, dtype=torch.bfloat16))
     held = lin._ws[1500].held
     assert held.sparse is not None and held.tail_rec is None and held.tail_cnt is None and held.tail_dense is None
+    assert held.tail_idx is None and held.tail_val is None and lin._ws[1500].outputs == _lib.TQ_OUT_Q8
 
 
 def test_records_are_left_out_where_the_other_forms_are_there(fake):  # noqa: F811
