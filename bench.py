@@ -322,7 +322,7 @@ def run_ours(args) -> None:
         torch.cuda.synchronize()
         return e0.elapsed_time(e1) / reps
 
-    wss = [lin.workspace(M_TOKENS) for lin in lins]
+    wss = [lin.workspace(M_TOKENS, shared=False) for lin in lins]   # (the prologue outputs that a forward writes)
     mma = args.tail_engine == "mma"
 
     def pro_call(lin, x, ws):

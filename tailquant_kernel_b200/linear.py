@@ -276,9 +276,10 @@ class SplitLinear:
             self._provide(ws, shared)
         return ws
 
-    def workspace(self, M: int) -> _Workspace:
-        """The buffers for `M` rows, with room for every prologue output that a layer on them may read."""
-        return self._workspace(M, True)
+    def workspace(self, M: int, shared: bool = True) -> _Workspace:
+        """The buffers for `M` rows, with room for every prologue output that a layer on them may read (`shared=False`: with
+        those of this layer's forward)."""
+        return self._workspace(M, shared)
 
     def _own_buffers(self, ws: _Workspace, M: int) -> _Workspace:
         """Output and scratch of THIS layer for a prologue workspace that may belong to another layer."""

@@ -299,3 +299,15 @@ def test_refresh_of_a_transpose_that_cannot_follow(fake):  # noqa: F811
     lin.w.w_rot = claimed(256, 256, dtype=torch.bfloat16)
     with pytest.raises(RuntimeError):
         lin.refresh()
+
+
+def test_the_prologue_outputs_of_a_forward_by_themselves(fake):  # noqa: F811
+    """What the benchmark times as the prologue is what a forward launches."""
+    lin = layer(N=24576, K=512, rms_weight=None)
+    x = claimed(1500, 512, dtype=torch.bfloat16)
+    lin(x)
+    pro = lin._ws[1500].pro
+    assert lin.workspace(1500, shared=False).pro is pro
+    ops.split_prologue(x, lin.w.had_kind, lin.R, lin.descending_rank, out=pro)
+    c = fake.calls[-1][1]
+    assert c["sp_val"] and c["a_q8"] and not c["tail_idx16"] and not c["tail_rec"] and not c["tail_dense"] and not c["a_pack"]
