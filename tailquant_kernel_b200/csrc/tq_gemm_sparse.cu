@@ -410,7 +410,8 @@ sparse_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a8, const __grid_con
     int use = 0, slices = 0;   // uses of the bf16 ring, dense slices so far
     for (int i = 0; ok && i < my_tiles; ++i) {
       const int m0 = 256 * tiles.mt(i), n_tile = tiles.n0(i), n0 = n_tile + rank * (tiles.width(n_tile) >> 1);
-      // entries of rows 8 lane .. 8 lane + 7 of the tile, places of their first ones in its list
+      // entries of rows 8 lane .. 8 lane + 7 of the tile, places of their first ones in its list.  (Counts and indices are held
+      // inside their arrays: outputs that no prologue has filled give wrong sums and no access out of range.)
       int total = 0;
       {
         const int row = m0 + 8 * lane;
@@ -419,10 +420,10 @@ sparse_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a8, const __grid_con
           const uint4 v = *reinterpret_cast<const uint4*>(p.over_cnt + row);
           const uint32_t w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-          for (int j = 0; j < 8; ++j) cnt[j] = (w[j >> 1] >> (16 * (j & 1))) & 0xffffu;
+          for (int j = 0; j < 8; ++j) cnt[j] = min((w[j >> 1] >> (16 * (j & 1))) & 0xffffu, (uint32_t)p.over_ld);
         } else {
 #pragma unroll
-          for (int j = 0; j < 8; ++j) cnt[j] = row + j < p.M ? p.over_cnt[row + j] : 0u;
+          for (int j = 0; j < 8; ++j) cnt[j] = row + j < p.M ? min((uint32_t)p.over_cnt[row + j], (uint32_t)p.over_ld) : 0u;
         }
         uint32_t sum = 0, incl;
 #pragma unroll
@@ -456,6 +457,7 @@ sparse_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a8, const __grid_con
         for (int step = 128; step > 0; step >>= 1)
           if (starts[row + step] <= (uint32_t)at) row += step;
         value = p.over[(size_t)(m0 + (int)row) * p.over_ld + (at - (int)starts[row])];
+        if ((value & 0xffffu) >= (uint32_t)p.K) value = 0u;
       };
       load(lane, v[0], r[0]);
       load(lane + 32, v[1], r[1]);

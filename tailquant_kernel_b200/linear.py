@@ -93,8 +93,8 @@ class _Workspace:
         if outputs & _lib.TQ_OUT_DENSE and p.tail_dense is None:
             p.tail_dense = empty((M, K), torch.bfloat16)
         if sparse and p.sparse is None:
-            p.sparse = (empty((M, K // 2), torch.bfloat16), empty((M, K // 32), torch.int32), empty((M,), torch.int16),
-                        empty((M, (R + 1) // 2), torch.int32))
+            p.sparse = (empty((M, K // 2), torch.bfloat16), empty((M, K // 32), torch.int32),
+                        torch.zeros((M,), dtype=torch.int16, device=device), empty((M, (R + 1) // 2), torch.int32))
 
 
 class SplitLinear:

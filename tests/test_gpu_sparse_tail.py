@@ -149,6 +149,27 @@ def test_layer_with_swiglu_on_the_sparse_tail(M, N, K):
     assert float((d != 0).float().mean()) < 1e-3 and bool((d <= ref.abs() * 2.0 ** -7 + 1e-4).all())
 
 
+@pytest.mark.parametrize("with_t", [True, False])
+def test_outputs_that_no_prologue_filled_are_read_inside_their_arrays(with_t):
+    """Counts beyond the list and indices beyond K, as memory that nothing wrote may hold them: the tail is of no use, the dense
+    part and the status are in order."""
+    M, N, K, R = 300, 264, 512, 26
+    o = prologue(activations("plain", M, K, 5), K, R)
+    o["sp_over_cnt"].fill_(-1)
+    o["sp_over"].copy_(torch.randint(-2 ** 31, 2 ** 31, o["sp_over"].shape, dtype=torch.int64).to(torch.int32).cuda())
+    w = ops.prepare_weight((torch.randn(N, K) * 0.02).to(torch.bfloat16).cuda(), t16=True, keep_w_rot=True)
+    out = torch.empty((M, N), dtype=torch.bfloat16, device="cuda")
+    acc = torch.empty((M, N), dtype=torch.int32, device="cuda")
+    p = lambda t: t.data_ptr()  # noqa: E731
+    _lib.check(_lib.load().tq_split_gemm_sparse(
+        p(o["a_q8"]), p(o["body_scale"]), p(w.b_col), p(w.w_scale), p(w.w_rot), p(w.w_t) if with_t else None, R,
+        *(p(o[f]) for f in ops.SPARSE_FIELDS), o["sp_over"].shape[1], None, p(out), p(acc), None, M, N, K, 0, ops._stream()), "gemm")
+    torch.cuda.synchronize()
+    assert ops.gemm_status() == 0
+    codes = o["a_q8"].cpu().numpy().reshape(M, K // 8, 8)[:, :, [0, 4, 1, 5, 2, 6, 3, 7]].reshape(M, K).astype(np.float64)
+    assert np.array_equal(acc.cpu().numpy(), (codes @ O.unpack_s4(w.b_col.cpu().numpy()).astype(np.float64).T).astype(np.int64))
+
+
 def test_swiglu_of_a_width_that_the_sparse_kernel_does_not_store():
     """N % 16 == 8: the kernel on records, whatever else the prologue left."""
     M, N, K = 1500, 8200, 1024

@@ -311,3 +311,9 @@ def test_the_prologue_outputs_of_a_forward_by_themselves(fake):  # noqa: F811
     ops.split_prologue(x, lin.w.had_kind, lin.R, lin.descending_rank, out=pro)
     c = fake.calls[-1][1]
     assert c["sp_val"] and c["a_q8"] and not c["tail_idx16"] and not c["tail_rec"] and not c["tail_dense"] and not c["a_pack"]
+
+
+def test_counts_that_nothing_wrote_are_zero(fake):  # noqa: F811
+    """`compute` on a workspace that no prologue has filled finds no left-over entries."""
+    lin = layer(N=24576, K=512, rms_weight=None)
+    assert int(lin.workspace(1500).pro.sparse[2].abs().sum()) == 0
