@@ -59,10 +59,10 @@ int linear_outputs(const tq_linear_call& c, bool shared) {
   const bool pair_dense = c.had_kind == TQ_HAD_BLOCK128;   // (the pair kernel loads long runs from it)
   if (few) return o | TQ_OUT_LISTS | TQ_OUT_DENSE;
   if (!fused) return o | TQ_OUT_LISTS;
-  if (c.sp_val && !shared && linear_sparse(c)) return o;
+  if (c.sp_val && !shared && linear_sparse(c)) return o | TQ_OUT_LISTS;
   // (the sparse form and the zero-filled matrix serve every width between them)
   if (c.sp_val && shared && shared_sparse(c) && c.M <= DENSE_ROWS)
-    return o | TQ_OUT_DENSE | linear_outputs(c, false);
+    return o | TQ_OUT_LISTS | TQ_OUT_DENSE | linear_outputs(c, false);
   const bool streams = c.M <= DENSE_MAX_ROWS && stream_is_faster(c.M, c.N, c.K, c.R);
   if (shared || !streams) o |= TQ_OUT_LISTS | TQ_OUT_RECORDS;
   if (streams || pair_dense || (shared && c.M <= DENSE_ROWS)) o |= TQ_OUT_DENSE;
@@ -79,8 +79,6 @@ tq_linear_call linear_own_part(tq_linear_call c) {
   else
     c.a_q8 = nullptr;
   if (fused && takes_sparse(c)) {
-    c.tail_idx16 = nullptr;
-    c.tail_val = nullptr;
     c.tail_dense = nullptr;
     c.tail_ptr = nullptr;
     c.tail_rec = nullptr;

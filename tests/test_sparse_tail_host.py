@@ -179,7 +179,6 @@ def test_a_forward_on_the_sparse_form_holds_no_other_operand(fake):  # noqa: F81
     lin(claimed(1500, 512, dtype=torch.bfloat16))
     held = lin._ws[1500].held
     assert held.sparse is not None and held.tail_rec is None and held.tail_cnt is None and held.tail_dense is None
-    assert held.tail_idx is None and held.tail_val is None and lin._ws[1500].outputs == _lib.TQ_OUT_Q8
 
 
 def test_records_are_left_out_where_the_other_forms_are_there(fake):  # noqa: F811
@@ -310,7 +309,7 @@ def test_the_prologue_outputs_of_a_forward_by_themselves(fake):  # noqa: F811
     assert lin.workspace(1500, shared=False).pro is pro
     ops.split_prologue(x, lin.w.had_kind, lin.R, lin.descending_rank, out=pro)
     c = fake.calls[-1][1]
-    assert c["sp_val"] and c["a_q8"] and not c["tail_idx16"] and not c["tail_rec"] and not c["tail_dense"] and not c["a_pack"]
+    assert c["sp_val"] and c["a_q8"] and not c["tail_rec"] and not c["tail_dense"] and not c["a_pack"]
 
 
 def test_counts_that_nothing_wrote_are_zero(fake):  # noqa: F811
