@@ -15,7 +15,7 @@ from __future__ import annotations
 import ctypes
 import weakref
 from collections import OrderedDict
-from typing import Dict, Optional, Tuple
+from typing import Dict, List, Optional, Tuple
 
 import torch
 
@@ -152,6 +152,7 @@ class SplitLinear:
         self._ws: Dict[int, _Workspace] = {}
         self._ws_shared: Dict[int, _Workspace] = {}
         self._t_of = (None, None, None, None)   # a transpose; the w_rot, its version and place that it belongs to
+        self.split_widths: Optional[List[int]] = None   # of the layers that run on this one's prologues; None: any
 
     @classmethod
     def from_prepared(cls, w: "ops.PreparedWeight", ratio: float = 0.05, activation_percentile: float = 100.0,
@@ -248,19 +249,45 @@ class SplitLinear:
 
     def _provide(self, ws: _Workspace, shared: bool) -> None:
         """Has `ws` show what this layer's forward reads, or with `shared` what any layer on the same prologue may read (a
-        layer with the exact-order engine only shares with its like).  Asked when the one follows the other, and again under
-        another forced kernel."""
-        lib, any_width = _lib.load(), int(shared and self.tail_engine == "mma")
-        c = _lib.LinearCall(M=ws.M, N=self.N, K=self.K, R=self.R, had_kind=self.w.had_kind, engine=ws.engine,
-                            act=int(self.epilogue == "swiglu"))
-        sparse = lib.tq_linear_sparse(ctypes.byref(c), any_width) > 0
-        c.sp_val = 1 if sparse else None   # (asks for what is needed beside it)
-        bits = lib.tq_linear_outputs(ctypes.byref(c), any_width)
-        if bits < 0:
-            _lib.check(bits, self._what(ws.M))
+        layer with the exact-order engine only shares with its like).  The 2:4-sparse form is for layers of any width too, unless
+        `split_widths` says which ones follow: then it is there where one of them takes it.  Asked when a forward follows a
+        prologue or the other way round, and again under another forced kernel."""
+        any_width = shared and self.tail_engine == "mma"
+        if any_width and self.split_widths:
+            asked = [self._ask(ws, n, False) for n in self.split_widths]
+            sparse = any(s for _, s in asked)
+            bits, _ = self._ask(ws, self.N, True, sparse)
+            for b, _ in asked:
+                bits |= b
+        else:
+            bits, sparse = self._ask(ws, self.N, any_width)
         ws.show(bits, sparse)
         now = ops.gemm_pair_mode_changes
         ws.forward_for, ws.shared_for = (-1, now) if shared else (now, -1)
+
+    def _ask(self, ws: _Workspace, N: int, any_width: bool, sparse: Optional[bool] = None) -> Tuple[int, bool]:
+        """Prologue outputs for a layer of N channels (`any_width`: for others too), and whether the 2:4-sparse form is one
+        (`sparse`: as given)."""
+        lib = _lib.load()
+        c = _lib.LinearCall(M=ws.M, N=N, K=self.K, R=self.R, had_kind=self.w.had_kind, engine=ws.engine,
+                            act=int(self.epilogue == "swiglu"))
+        if sparse is None:
+            sparse = lib.tq_linear_sparse(ctypes.byref(c), int(any_width)) > 0
+        c.sp_val = 1 if sparse else None   # (asks for what is needed beside it)
+        bits = lib.tq_linear_outputs(ctypes.byref(c), int(any_width))
+        if bits < 0:
+            _lib.check(bits, self._what(ws.M))
+        return bits, sparse
+
+    def serves(self, ws: _Workspace, N: int) -> bool:
+        """Whether the prologue outputs in `ws` are what a layer of N channels takes.  If not, the next prologue's are."""
+        if self.split_widths is None or N in self.split_widths:
+            return True
+        self.split_widths.append(N)
+        bits, sparse = self._ask(ws, N, False) if ws.M > 64 else (0, False)
+        for w in self._ws.values():
+            w.shared_for = -1
+        return not (bits & ~ws.outputs or (sparse and ws.pro.sparse is None))
 
     def _new_workspace(self, M: int, with_pro: bool) -> _Workspace:
         engine = self._engine(M)
@@ -477,7 +504,7 @@ class _Entry:
 
 _CACHE: "OrderedDict[Tuple, _Entry]" = OrderedDict()
 _CACHE_MAX = 1024        # prepared layers kept (a 36-layer model has 252 target linears)
-_SHARED: Dict[Tuple, Tuple] = {}  # (input, shape of the split, stream, capture) -> (x weakref, workspace)
+_SHARED: Dict[Tuple, Tuple] = {}  # (input, shape of the split, stream, capture) -> (x weakref, workspace, its layer)
 
 
 def _drop(key) -> None:
@@ -501,6 +528,7 @@ def _cached_layer(weight: torch.Tensor, bias: Optional[torch.Tensor], ratio: flo
         return e.lin
     e = _Entry()
     e.lin = SplitLinear(weight, bias, ratio, reuse_output=True)
+    e.lin.split_widths = [e.lin.N]   # (others are added as they come)
     e.wref = weakref.ref(weight, lambda _r, k=key: _drop(k))  # the entry goes when the weight does
     e.bref = None if bias is None else weakref.ref(bias)
     _CACHE[key] = e
@@ -540,13 +568,16 @@ def split_linear_forward(x: torch.Tensor, weight: torch.Tensor, bias: Optional[t
     skey = (x.device.index, x2d.data_ptr(), x._version if known else 0, M, lin.K, lin.R, lin.descending_rank, lin.w.had_kind, stream,
             _lib.load().tq_stream_capture_id(stream))
     hit = _SHARED.get(skey) if known else None
-    if hit is not None and hit[0]() is x:
+    owner = hit[2]() if hit is not None and hit[0]() is x else None
+    if owner is not None:
         ws = hit[1]
+        if not owner.serves(ws, lin.N):   # (the first time that this width follows)
+            ws = owner.prologue(x2d)
     else:
         _SHARED.clear()   # one entry: the prologue outputs live in a workspace that the next prologue of that layer
         ws = lin.prologue(x2d)                    # overwrites, whatever its input
         if known:
-            _SHARED[skey] = (weakref.ref(x), ws)
+            _SHARED[skey] = (weakref.ref(x), ws, weakref.ref(lin))
     y = lin.compute(ws, M, torch.empty((M, lin.N_out), dtype=torch.bfloat16, device=x2d.device))
     y = y.view(*x.shape[:-1], lin.N_out)
     return y if y.dtype == x.dtype else y.to(x.dtype)

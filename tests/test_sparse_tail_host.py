@@ -316,3 +316,57 @@ def test_counts_that_nothing_wrote_are_zero(fake):  # noqa: F811
     """`compute` on a workspace that no prologue has filled finds no left-over entries."""
     lin = layer(N=24576, K=512, rms_weight=None)
     assert int(lin.workspace(1500).pro.sparse[2].abs().sum()) == 0
+
+
+@pytest.fixture
+def patched(fake, monkeypatch):  # noqa: F811
+    """`split_linear_forward` on prepared layers of the given widths, as it would make them; reports the prologues that ran."""
+    from tailquant_kernel_b200 import linear
+    layers = {}
+    monkeypatch.setattr(linear, "_cached_layer", lambda w, b, r: layers[id(w)])
+    monkeypatch.setattr(ops, "_check_cuda", lambda *a, **k: None)
+    linear.clear_cache()
+
+    def make(*widths, K=512):
+        weights = [claimed(n, K, dtype=torch.bfloat16) for n in widths]
+        for w in weights:
+            layers[id(w)] = layer(N=w.shape[0], K=K, rms_weight=None)
+            layers[id(w)].split_widths = [w.shape[0]]
+
+        def call(M):
+            x = claimed(M, K, dtype=torch.bfloat16)
+            fake.calls.clear()
+            for w in weights:
+                linear.split_linear_forward(x, w)
+            return [(name, c["N"], bool(c["sp_val"])) for name, c in fake.calls], [layers[id(w)] for w in weights]
+        return call
+    yield make
+    linear.clear_cache()
+
+
+def test_a_split_that_takes_no_sparse_operand_gets_none(patched):
+    """777 x {4096, 1024, 1024}: none of them does, whatever a wider layer would."""
+    call = patched(4096, 1024, 1024, K=4096)
+    for _ in range(2):
+        calls, lins = call(777)
+        assert [c[0] for c in calls] == ["tq_linear_prologue", *["tq_linear_compute"] * 3] and not any(c[2] for c in calls)
+        assert lins[0]._ws[777].held.sparse is None and lins[0]._ws[777].pro.tail_dense is not None
+    assert lins[0].workspace(300).pro.sparse is None and lins[1].workspace(777).pro.sparse is None
+
+
+@pytest.mark.parametrize("widths", [(24576, 24576), (24576, 1024)])
+def test_a_split_whose_first_linear_takes_it(patched, widths):
+    calls, lins = patched(*widths)(1000)
+    assert [c[0] for c in calls] == ["tq_linear_prologue", "tq_linear_compute", "tq_linear_compute"]
+    assert lins[0]._ws[1000].pro.sparse is not None and calls[0][2]
+
+
+def test_a_split_whose_later_linear_takes_it(patched):
+    """The prologue runs once more when that width follows for the first time: every pass then has the same operands."""
+    call = patched(256, 24576)
+    calls, lins = call(300)
+    assert [c[0].split("_")[-1] for c in calls] == ["prologue", "compute", "prologue", "compute"]
+    assert calls[2][1] == 256 and calls[2][2] and calls[3][2]
+    calls, lins = call(300)
+    assert [c[0].split("_")[-1] for c in calls] == ["prologue", "compute", "compute"] and all(c[2] for c in calls)
+    assert call(300)[1][0].split_widths == [256, 24576]
