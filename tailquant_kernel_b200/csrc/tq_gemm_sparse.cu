@@ -449,7 +449,7 @@ sparse_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a8, const __grid_con
       }
       // This lane's two entries of a dense slice: place `at` of the tile's list, its row by bisection of the first places (so
       // that a row with many entries is loaded by many lanes); beyond the last one zeros of row 0.
-      uint32_t v[2], r[2];
+      uint32_t v[2], r[2], nv[2], nr[2];
       auto load = [&](int at, uint32_t& value, uint32_t& row) {
         value = row = 0u;
         if (at >= total) return;
@@ -457,15 +457,20 @@ sparse_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a8, const __grid_con
         for (int step = 128; step > 0; step >>= 1)
           if (starts[row + step] <= (uint32_t)at) row += step;
         value = p.over[(size_t)(m0 + (int)row) * p.over_ld + (at - (int)starts[row])];
-        if ((value & 0xffffu) >= (uint32_t)p.K) value = 0u;
       };
-      load(lane, v[0], r[0]);
-      load(lane + 32, v[1], r[1]);
+      load(lane, nv[0], nr[0]);
+      load(lane + 32, nv[1], nr[1]);
       ok = __all_sync(0xffffffffu, mbar_wait(b.last_placed(i & 1), (uint32_t)((i >> 1) & 1), abort_flag, 0x1000000u));
       use += kbt;
       // (the slots of the uses from here on are at most one release behind what is waited for)
       for (int q = 0; ok && 64 * q < total; ++q, ++use, ++slices) {
         const int s = use % S::SB, l = slices % S::LISTS;
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          v[j] = (nv[j] & 0xffffu) < (uint32_t)p.K ? nv[j] : 0u;
+          r[j] = nr[j];
+          load(64 * (q + 1) + lane + 32 * j, nv[j], nr[j]);   // (on its way while this slice is built)
+        }
         ok = __all_sync(0xffffffffu, mbar_wait(b.empty_b(s), (uint32_t)((use / S::SB) & 1) ^ 1u, abort_flag, 0x2000000u));
         if (!ok) break;
         tc_fence_after();
@@ -499,8 +504,6 @@ sparse_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a8, const __grid_con
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncwarp();
         if (lane == 0) mbar_arrive(b.built(l));
-        load(64 * (q + 1) + lane, v[0], r[0]);
-        load(64 * (q + 1) + lane + 32, v[1], r[1]);
       }
     }
   } else if (warp == 15) {
