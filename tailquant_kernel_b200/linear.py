@@ -151,7 +151,6 @@ class SplitLinear:
         self.reuse_output = bool(reuse_output)
         self._ws: Dict[int, _Workspace] = {}
         self._ws_shared: Dict[int, _Workspace] = {}
-        self._t_of = (None, None, None, None)   # a transpose; the w_rot, its version and place that it belongs to
         self.split_widths: Optional[List[int]] = None   # of the layers that run on this one's prologues; None: any
 
     @classmethod
@@ -173,6 +172,7 @@ class SplitLinear:
             raise RuntimeError("the tensor-core tail needs the rotated bf16 weights (w_rot)")
         if R > 0 and tail_engine == "gather" and w.w_t is None and w.w_rot is not None:
             w.w_t = w.w_rot.t().contiguous()  # the gather engine reads the [K, N] transpose
+            w.t_of = (w.w_t, w.w_rot, cls._version(w.w_rot), w.w_rot.data_ptr())
         if R > 0 and w.w_t is None and w.w_rot is None:
             raise RuntimeError("a tail needs the rotated bf16 weights (w_rot or w_t)")
         self = cls.__new__(cls)
@@ -323,8 +323,8 @@ class SplitLinear:
         """Builds the [K, N] transpose of the rotated weights that the small-M tail reads, ahead of the first small-M
         forward (which otherwise builds it: an allocation inside that call).  Not inside a stream capture: nothing would have
         written it before the first replay, and every replay would write it again."""
-        if self.R and self.w.w_t is None and not self._capturing():
-            self.w.w_t = self._transposed()
+        if self.R:
+            self._follow_w_rot()
 
     def refresh(self) -> None:
         """Makes the [K, N] transpose again, where there is one, after `w_rot` was written by something that its version counter
@@ -348,31 +348,33 @@ class SplitLinear:
             return ops.transpose_bf16(r, into)
         return r.t().contiguous() if into is None else into.copy_(r.t())
 
-    def _rot_version(self) -> int:
-        r = self.w.w_rot
-        return -1 if r is None or r.is_inference() else r._version
+    @staticmethod
+    def _version(t: Optional[torch.Tensor]) -> int:
+        return -1 if t is None or t.is_inference() else t._version
 
-    def _prepare_sparse(self, own: _Workspace) -> bool:
-        """The transpose that the left-over entries of the sparse tail are read from.  A layer that had none did not ask for it
-        and is not expected to keep it in line: it is made again when `w_rot` was replaced or changed since, in the same memory
-        where `w_rot` is the same tensor (a graph captured before names both).  False where it would have to be made inside a
-        stream capture: the kernel then reads `w_rot`, and the next call outside makes it."""
-        w = self.w
-        if w.w_rot is None:
-            return False   # (refused with the other parts)
-        version = self._rot_version()
-        t, rot, v, place = self._t_of
-        changed = w.w_t is not None and w.w_t is t and (w.w_rot is not rot or (version, rot.data_ptr()) != (v, place))
+    def _rot_version(self) -> int:
+        return self._version(self.w.w_rot)
+
+    def _follow_w_rot(self) -> bool:
+        """Has `w_t` be there and, from the first call that finds it there, in line with `w_rot`: it is made again when `w_rot` was
+        replaced or changed since, in the same memory where `w_rot` is the same tensor (a graph captured before names both).
+        One that was replaced with it counts as its transpose.  False where it would have to be made inside a stream capture:
+        that call does without, and the next one outside makes it."""
+        w, rot = self.w, self.w.w_rot
+        if rot is None:
+            return w.w_t is not None
+        version, (t, of, v, place) = self._rot_version(), w.t_of
+        changed = w.w_t is not None and w.w_t is t and (rot is not of or (version, rot.data_ptr()) != (v, place))
         if (changed or w.w_t is None) and self._capturing():
             return False
         if changed:
-            if w.w_rot is rot and tuple(t.shape) == tuple(reversed(rot.shape)) and t.dtype == rot.dtype and t.device == rot.device:
+            if rot is of and tuple(t.shape) == tuple(reversed(rot.shape)) and t.dtype == rot.dtype and t.device == rot.device:
                 self._transposed(t)
             else:
                 w.w_t = None
-        self.prepare_decode()
-        self._t_of = (w.w_t, w.w_rot, version, w.w_rot.data_ptr())
-        own.rot_version = version
+        if w.w_t is None:
+            w.w_t = self._transposed()
+        w.t_of = (w.w_t, rot, version, rot.data_ptr())
         return True
 
     def _described(self, own: _Workspace) -> bool:
@@ -416,17 +418,15 @@ class SplitLinear:
         own.rot_version = own.call = None   # (a part that is refused must not leave the former description in force)
         w, p = self.w, ops._ptr
         keep, w_t = True, w.w_t
-        if own.engine == _lib.TQ_LINEAR_DECODE:
-            self.prepare_decode()
-            w_t = w.w_t
-            if self.R and w_t is None and w.w_rot is not None:   # in a stream capture, for this call of it only
-                keep, w_t = False, self._transposed()
-        elif own.engine == _lib.TQ_LINEAR_FUSED and pro.sparse is not None:
-            if ops.takes_sparse(own.M, self.N, self.K, self.R, w.had_kind, int(self.epilogue == "swiglu")):
-                keep = self._prepare_sparse(own)
-                w_t = w.w_t if keep else None
-            elif w_t is self._t_of[0]:
-                w_t = None   # (where the sparse form is all there is, `w_rot` is what is certain to be in line)
+        if self.R and (own.engine != _lib.TQ_LINEAR_FUSED or (pro.sparse is not None and ops.takes_sparse(
+                own.M, self.N, self.K, self.R, w.had_kind, int(self.epilogue == "swiglu")))):
+            keep, w_t = self._follow_w_rot(), w.w_t
+            if not keep:   # in a stream capture: the sparse GEMM reads `w_rot`, the others a transpose for this call of it only
+                w_t = self._transposed() if own.engine != _lib.TQ_LINEAR_FUSED and w.w_rot is not None else None
+            elif w.w_rot is not None:
+                own.rot_version = self._rot_version()
+        elif pro.sparse is not None and w_t is w.t_of[0]:
+            w_t = None   # (where the sparse form is all there is, `w_rot` is what is certain to be in line)
         self._check_parts(own.engine, w_t if own.engine != _lib.TQ_LINEAR_FUSED or own.rot_version is not None else None)
         own.call_pro = pro if keep else None
         own.call_t = w_t   # (lives as long as its address is in `call`)

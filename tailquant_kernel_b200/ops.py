@@ -20,7 +20,7 @@ from __future__ import annotations
 
 import ctypes
 import math
-from dataclasses import dataclass
+from dataclasses import dataclass, field
 from typing import Optional, Tuple
 
 import torch
@@ -237,6 +237,8 @@ class PreparedWeight:
     b_row: Optional[torch.Tensor]     # [K, N/2] u8   (T4 tail)
     w_rot: Optional[torch.Tensor]     # [N, K] bf16
     bias: Optional[torch.Tensor] = None  # [N] f32
+    # a w_t, and the w_rot, its version and place that it is the transpose of (kept here: layers on one weight share both)
+    t_of: Tuple = field(default=(None, None, None, None), repr=False, compare=False)
 
 
 def prepare_weight(W: torch.Tensor, had_kind: Optional[int] = None, eps: float = EPS, t16: bool = True,

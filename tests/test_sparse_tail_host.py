@@ -4,8 +4,8 @@ import ctypes
 import pytest
 import torch
 
-from tailquant_kernel_b200 import _lib, ops
-from test_linear_host import claimed, fake, layer  # noqa: F401
+from tailquant_kernel_b200 import SplitLinear, _lib, ops
+from test_linear_host import claimed, fake, layer, weight  # noqa: F401
 
 
 def sparse(M, N, K, R, kind=1, engine=_lib.TQ_LINEAR_FUSED, shared=0):
@@ -370,3 +370,45 @@ def test_a_split_whose_later_linear_takes_it(patched):
     calls, lins = call(300)
     assert [c[0].split("_")[-1] for c in calls] == ["prologue", "compute", "compute"] and all(c[2] for c in calls)
     assert call(300)[1][0].split_widths == [256, 24576]
+
+
+@pytest.mark.parametrize("how", ["in_place", "replaced"])
+@pytest.mark.parametrize("first,later", [(1, 1500), (1500, 1), (1, 1), (0, 1500), (0, 1), (0, 0)])
+def test_the_transpose_follows_whichever_call_made_it(fake, first, later, how):  # noqa: F811
+    """Rows of the call that makes it and of the one after `w_rot` has changed; 0: prepare_decode()."""
+    lin = layer(N=8192, K=1024, rms_weight=None)
+    lin.w.w_t = None
+    call = lambda M: lin(claimed(M, 1024, dtype=torch.bfloat16)) if M else lin.prepare_decode()  # noqa: E731
+    call(first)
+    t = lin.w.w_t
+    assert t is not None
+    if how == "in_place":
+        lin.w.w_rot.fill_(2.0)
+    else:
+        lin.w.w_rot = torch.full_like(lin.w.w_rot, 2.0)
+    call(later)
+    assert float(lin.w.w_t[3, 5]) == 2.0 and (how == "replaced" or lin.w.w_t is t)
+    assert later == 0 or fake.calls[-1][1]["w_t"] == lin.w.w_t.data_ptr()
+
+
+@pytest.mark.parametrize("M", [1, 200])
+def test_the_exact_order_engine_follows_w_rot(fake, M):  # noqa: F811
+    w = weight(256, 512)
+    w.w_t = None
+    lin = SplitLinear.from_prepared(w, tail_engine="gather")
+    lin.w.w_rot.fill_(2.0)
+    lin(claimed(M, 512, dtype=torch.bfloat16))
+    assert float(w.w_t[3, 5]) == 2.0 and fake.calls[-1][1]["w_t"] == w.w_t.data_ptr()
+
+
+def test_layers_on_one_weight_share_its_transpose(fake):  # noqa: F811
+    w = weight(8192, 1024)
+    w.w_t = None
+    a, b = (SplitLinear.from_prepared(w) for _ in range(2))
+    a(claimed(1, 1024, dtype=torch.bfloat16))
+    t = w.w_t
+    w.w_rot.fill_(2.0)
+    b(claimed(1500, 1024, dtype=torch.bfloat16))
+    assert w.w_t is t and float(t[3, 5]) == 2.0
+    a(claimed(1, 1024, dtype=torch.bfloat16))
+    assert fake.calls[-1][1]["w_t"] == t.data_ptr()
