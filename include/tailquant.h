@@ -377,6 +377,8 @@ int tq_int4_linear_splitk_noalloc(const uint8_t* a_pack, const float* body_scale
  * output is not valid).  Synchronises the device, returns TQ_ERR_DEVICE_STATUS when the word is non-zero and
  * clears it, so poll it at a synchronisation point after the launches whose result matters. */
 int tq_gemm_status(unsigned int* status);
+/* For tests: g / (1 + exp(-g)) of all 2^16 bf16 gates, as the SwiGLU epilogues evaluate it and by IEEE division (65536 fp32 each). */
+int tq_swiglu_quotients(float* quotient, float* divided, void* stream);
 
 #ifdef __cplusplus
 }

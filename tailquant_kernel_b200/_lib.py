@@ -68,6 +68,7 @@ SIGNATURES = {
     "tq_linear_prologue": [_P, _P, _P],
     "tq_linear_compute": [_P, _P, _P],
     "tq_stream_capture_id": [_P],
+    "tq_swiglu_quotients": [_P, _P, _P],
     "tq_gemm_status": [_P],
 }
 _CHAR_P_RETURNS = {"tq_error_string", "tq_last_cuda_error"}

@@ -248,6 +248,13 @@ int t4_launch(int mode, const int32_t* C, const float* bs, const int8_t* top_q, 
   return check_launch();
 }
 
+__global__ void swiglu_quotients_kernel(float* __restrict__ quotient, float* __restrict__ divided) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;   // < 2^16
+  const float g = bf16_bits_to_f32(i);
+  quotient[i] = swiglu_quotient(g);
+  divided[i] = __fdiv_rn(g, __fadd_rn(1.0f, expf(-g)));
+}
+
 }  // namespace
 
 int run_transpose_bf16(const void* in, void* out, int N, int K, cudaStream_t st) {
@@ -278,6 +285,12 @@ extern "C" int tq_transpose_bf16(const void* in, void* out, int N, int K, void* 
   if (!in || !out || N < 0 || K < 0) return TQ_ERR_BAD_ARG;
   if (N == 0 || K == 0) return TQ_OK;
   return tq::run_transpose_bf16(in, out, N, K, (cudaStream_t)stream);
+}
+
+extern "C" int tq_swiglu_quotients(float* quotient, float* divided, void* stream) {
+  if (!quotient || !divided) return TQ_ERR_BAD_ARG;
+  tq::swiglu_quotients_kernel<<<256, 256, 0, (cudaStream_t)stream>>>(quotient, divided);
+  return tq::check_launch();
 }
 
 extern "C" int tq_dequant_finish(const int32_t* C, const float* body_scale, const float* w_scale, const float* tail,

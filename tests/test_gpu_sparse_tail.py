@@ -36,8 +36,9 @@ def activations(what, M, K, seed):
     return x.to(torch.bfloat16).cuda()
 
 
-def prologue(x, K, R, wide=False):
-    """All tail forms of one prologue call, through the native description."""
+def prologue(x, K, R, wide=False, gamma=None, sparse=True):
+    """All tail forms of one prologue call, through the native description (`wide`: of the kernel for 16 elements a thread;
+    without `sparse` the others)."""
     M = x.shape[0]
     kind = ops.default_had_kind(K)
     e = lambda *s, t: torch.empty(s, dtype=t, device="cuda")  # noqa: E731
@@ -45,9 +46,12 @@ def prologue(x, K, R, wide=False):
                tail_idx16=e(M, (R + 7) // 8 * 8, t=torch.int16), tail_val=e(M, (R + 7) // 8 * 8, t=torch.bfloat16),
                tail_dense=e(M, K, t=torch.bfloat16), sp_val=e(M, K // 2, t=torch.bfloat16), sp_meta=e(M, K // 32, t=torch.int32),
                sp_over_cnt=e(M, t=torch.int16), sp_over=e(M, (R + 1) // 2, t=torch.int32))
+    if not sparse:
+        out = {k: v for k, v in out.items() if k not in ops.SPARSE_FIELDS}
     c = _lib.LinearCall(M=M, N=8, K=K, R=R, had_kind=kind, descending_rank=ops.split_select_params(K, R)[1],
                         engine=_lib.TQ_LINEAR_FUSED, eps=ops.EPS, tail_ld=out["tail_idx16"].shape[1],
-                        sp_over_ld=out["sp_over"].shape[1], **{k: v.data_ptr() for k, v in out.items()})
+                        sp_over_ld=(R + 1) // 2,
+                        rms_weight=None if gamma is None else gamma.data_ptr(), rms_eps=1e-6, **{k: v.data_ptr() for k, v in out.items()})
     lib = _lib.load()
     lib.tq_set_prologue_mode(0 if wide else -1)
     try:
@@ -58,16 +62,24 @@ def prologue(x, K, R, wide=False):
     return out
 
 
-CASES = [("plain", 3, 512, 26), ("hot", 300, 4096, 205), ("few_levels", 130, 4096, 287), ("one_row", 300, 4096, 205),
-         ("zeros", 20, 1024, 52), ("plain", 9, 2048, 1), ("hot", 140, 12288, 615), ("one_row", 33, 6144, 400),
-         ("few_levels", 40, 8192, 410)]
+# (what, rows, K, R, kernel): the kernel of 16 elements a thread, or that of 64, which K = 4096 takes beyond 256 rows and K = 12288
+# beyond 128 and which can be kept off
+CASES = [("plain", 3, 512, 26, 16), ("one_row", 300, 4096, 205, 16), ("few_levels", 130, 4096, 287, 16), ("zeros", 20, 1024, 52, 16),
+         ("plain", 9, 2048, 1, 16), ("hot", 20, 12288, 615, 16), ("zeros", 140, 12288, 615, 16), ("one_row", 33, 6144, 400, 16),
+         ("few_levels", 40, 8192, 410, 16), ("hot", 300, 4096, 205, 64), ("one_row", 300, 4096, 205, 64),
+         ("few_levels", 300, 4096, 287, 64), ("zeros", 300, 4096, 205, 64), ("hot", 140, 12288, 615, 64), ("few_levels", 140, 12288, 860, 64), ("zeros", 140, 12288, 615, 64)]
 
 
-@pytest.mark.parametrize("what,M,K,R", CASES)
-@pytest.mark.parametrize("wide", [False, True])
-def test_prologue_writes_the_tail_in_sparse_form(what, M, K, R, wide):
-    """The first two entries of each group in order with their places, all others in the row's list; only zeros are left out."""
-    o = prologue(activations(what, M, K, 11), K, R, wide)
+@pytest.mark.parametrize("what,M,K,R,elements", CASES)
+@pytest.mark.parametrize("norm", [False, True])
+def test_prologue_writes_the_tail_in_sparse_form(what, M, K, R, elements, norm):
+    """The first two entries of each group in order with their places, all others in the row's list; only zeros are left out.
+    What else is written has the bits of a prologue without the sparse form (which is compared with the oracle)."""
+    gamma = (1 + 0.1 * torch.randn(K, generator=torch.Generator().manual_seed(1))).to(torch.bfloat16).cuda() if norm else None
+    x = activations(what, M, K, 11)
+    o = prologue(x, K, R, elements == 16, gamma)
+    for name, t in prologue(x, K, R, elements == 16, gamma, sparse=False).items():
+        assert torch.equal(t.view(torch.uint8), o[name].view(torch.uint8)), name
     want = o["tail_dense"].view(torch.int16).cpu().numpy().astype(np.int64) & 0xffff
     member = np.zeros((M, K), bool)
     np.put_along_axis(member, o["tail_idx16"].cpu().numpy()[:, :R].astype(np.int64) & 0xffff, True, 1)
@@ -325,19 +337,17 @@ def test_another_kernel_after_a_forward_on_the_sparse_form(mode):
 
 
 def test_swiglu_of_every_gate():
-    """The quotient of the epilogue rounds like a division: all 2^16 gates (through the finisher of the split-K path), against
-    fp64 rounded once to fp32 and then to bf16."""
-    g = torch.arange(65536, dtype=torch.int32).to(torch.int16).view(torch.bfloat16).float()
-    g = g[torch.isfinite(g) & (g.abs() < 3e38)]
-    n = g.numel() // 8 * 8
-    g = g[:n].cuda()
+    """The epilogues' quotient has the bits of the IEEE division for every bf16 gate, infinities and the largest ones among them
+    (NaN where that is NaN); the finisher of the split-K path rounds it to bf16."""
+    q, d = torch.empty(65536, device="cuda"), torch.empty(65536, device="cuda")
+    _lib.check(_lib.load().tq_swiglu_quotients(q.data_ptr(), d.data_ptr(), ops._stream()), "quotients")
+    nan = torch.isnan(d)
+    assert torch.equal(torch.isnan(q), nan) and torch.equal(q.view(torch.int32)[~nan], d.view(torch.int32)[~nan])
+    g = torch.arange(65536, dtype=torch.int32).to(torch.int16).view(torch.bfloat16).float().cuda()
+    n = g.numel()
     y = torch.stack((g, torch.ones_like(g)), 1).reshape(1, -1).contiguous()
     acc, one = torch.zeros((1, 1, 2 * n), dtype=torch.int32, device="cuda"), torch.ones(2 * n, device="cuda")
     out = torch.empty((1, n), dtype=torch.bfloat16, device="cuda")
     _lib.check(_lib.load().tq_dequant_finish_partials(acc.data_ptr(), 1, one.data_ptr(), one.data_ptr(), y.data_ptr(), None,
                                                       out.data_ptr(), 1, 2 * n, 1, ops._stream()), "finish")
-    e = torch.exp(-g)                                        # (fp32, as the kernel's)
-    want = (g.double() / (1.0 + e).double()).float().to(torch.bfloat16)
-    # torch's exp may differ from the kernel's by an ulp or two, which moves a bf16 result now and then
-    d = (out[0].float() - want.float()).abs()
-    assert float((d > 0).float().mean()) < 2e-3 and bool((d <= want.float().abs() * 2.0 ** -7).all())
+    assert torch.equal(torch.isnan(out[0]), nan) and torch.equal(out[0][~nan], d[~nan].to(torch.bfloat16))
