@@ -79,7 +79,10 @@ def test_prologue_writes_the_tail_in_sparse_form(what, M, K, R, elements, norm):
     x = activations(what, M, K, 11)
     o = prologue(x, K, R, elements == 16, gamma)
     for name, t in prologue(x, K, R, elements == 16, gamma, sparse=False).items():
-        assert torch.equal(t.view(torch.uint8), o[name].view(torch.uint8)), name
+        mine = o[name]
+        if name in ("tail_idx16", "tail_val"):   # (padded to whole stores)
+            t, mine = t[:, :R].contiguous(), mine[:, :R].contiguous()
+        assert torch.equal(t.view(torch.uint8), mine.view(torch.uint8)), name
     want = o["tail_dense"].view(torch.int16).cpu().numpy().astype(np.int64) & 0xffff
     member = np.zeros((M, K), bool)
     np.put_along_axis(member, o["tail_idx16"].cpu().numpy()[:, :R].astype(np.int64) & 0xffff, True, 1)
