@@ -491,14 +491,25 @@ sparse_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a8, const __grid_con
                 (uint16_t)(v[j] >> 16);
         }
         if (!p.w_t) {
-          for (int item = lane; item < 64 * SPG_BH / 8; item += 32) {   // 64 entries x 14 pieces of eight channels
-            const int e = item / (SPG_BH / 8), c = item - e * (SPG_BH / 8), n = n0 + 8 * c;
-            const size_t k = list[l * S::LIST + e] & 0xffffu;
-            uint32_t w[4] = {0u, 0u, 0u, 0u};
-            if (n < p.N)
+          // 64 entries x 14 pieces of eight channels, two bytes at a time: a sector each, so the loads of four pieces are in
+          // flight together: 2048 x 6144 x 4096, 0.7 left-over entries a row, 272 -> 209 us (with w_t 106, the CTA pairs 124)
+          for (int item = lane; item < 64 * SPG_BH / 8; item += 128) {
+            uint32_t w[4][8];
 #pragma unroll
-              for (int j = 0; j < 8; ++j) w[j >> 1] |= (uint32_t)p.w_rot[(size_t)(n + j) * p.K + k] << (16 * (j & 1));
-            st_shared_v4(smem_u32(a) + S::A + (uint32_t)((c >> 3) * 8192 + (e >> 3) * 1024 + (e & 7) * 128 + (((c & 7) ^ (e & 7)) << 4)), w);
+            for (int u = 0; u < 4; ++u) {
+              const int i = item + 32 * u, e = i / (SPG_BH / 8), n = min(n0 + 8 * (i - e * (SPG_BH / 8)), p.N - 8);
+              const uint16_t* const at = p.w_rot + (size_t)n * p.K + (list[l * S::LIST + e] & 0xffffu);
+#pragma unroll
+              for (int j = 0; j < 8; ++j) w[u][j] = at[(size_t)j * p.K];
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+              const int i = item + 32 * u, e = i / (SPG_BH / 8), c = i - e * (SPG_BH / 8);
+              uint32_t v4[4];
+#pragma unroll
+              for (int j = 0; j < 4; ++j) v4[j] = n0 + 8 * c < p.N ? w[u][2 * j] | w[u][2 * j + 1] << 16 : 0u;
+              st_shared_v4(smem_u32(a) + S::A + (uint32_t)((c >> 3) * 8192 + (e >> 3) * 1024 + (e & 7) * 128 + (((c & 7) ^ (e & 7)) << 4)), v4);
+            }
           }
         }
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");

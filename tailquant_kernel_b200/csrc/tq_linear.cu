@@ -42,7 +42,8 @@ bool takes_sparse(const tq_linear_call& c) {
   if (!c.sp_val || c.M == 0 || c.R == 0) return false;
   if (linear_sparse(c)) return true;
   if (has_records(c)) return false;
-  return !c.tail_dense || (shared_sparse(c) && sparse_us(c.M, c.N, c.K, c.R) < plan_stream(c.M, c.N, c.K, ST_TAIL).us);
+  // (without w_t the left-over entries cost more than the zero-filled matrix does)
+  return !c.tail_dense || (c.w_t && shared_sparse(c) && sparse_us(c.M, c.N, c.K, c.R) < plan_stream(c.M, c.N, c.K, ST_TAIL).us);
 }
 
 SparseTail linear_sparse_tail(const tq_linear_call& c) {

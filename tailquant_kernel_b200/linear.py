@@ -261,8 +261,11 @@ class SplitLinear:
                 bits |= b
         else:
             bits, sparse = self._ask(ws, self.N, any_width)
-        ws.show(bits, sparse)
         now = ops.gemm_pair_mode_changes
+        if sparse and not shared and not self._follow_w_rot():   # (a captured call without the transpose: the CTA pairs, for now)
+            bits, sparse = self._ask(ws, self.N, False, False)
+            now = -1
+        ws.show(bits, sparse)
         ws.forward_for, ws.shared_for = (-1, now) if shared else (now, -1)
 
     def _ask(self, ws: _Workspace, N: int, any_width: bool, sparse: Optional[bool] = None) -> Tuple[int, bool]:

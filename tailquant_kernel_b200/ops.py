@@ -340,9 +340,10 @@ def takes_sparse(M: int, N: int, K: int, R: int, had_kind: int = TQ_HAD_WHT, act
 
 
 def split_gemm_mma(a_q8, body_scale, B_pack, w_scale, out, w_rot=None, pro: Optional[PrologueOut] = None,
-                   R: int = 0, bias=None, dbg_acc=None, dbg_tail=None, act: str = "none"):
+                   R: int = 0, bias=None, dbg_acc=None, dbg_tail=None, act: str = "none", w_t=None):
     """One kernel: dense INT4 x INT4 part on tcgen05 kind::i8 plus the tail as a bf16 tensor-core product
-    over the zero-filled tail matrix, fused dequant + bias, bf16 out.  act="swiglu": the weight rows are
+    over the zero-filled tail matrix, fused dequant + bias, bf16 out.  `w_t`: the [K, N] transpose of w_rot, read for
+    the entries that the 2:4-sparse form of the tail leaves over; without it they come from w_rot, several times as slowly.  act="swiglu": the weight rows are
     interleaved (gate_i, up_i) pairs and out is [M, N/2] = bf16(bf16(silu(gate)) * up)."""
     _check(act in ("none", "swiglu"), "act must be 'none' or 'swiglu'")
     _check_cuda(a_q8, "a_q8", torch.int8)
@@ -362,11 +363,14 @@ def split_gemm_mma(a_q8, body_scale, B_pack, w_scale, out, w_rot=None, pro: Opti
         _check_cuda(w_rot, "w_rot", torch.bfloat16)
         _check(tuple(w_rot.shape) == (N, K), "w_rot must be [N, K]")
         _check(pro is not None, "the prologue outputs are needed when R > 0")
+        if w_t is not None:
+            _check_cuda(w_t, "w_t", torch.bfloat16)
+            _check(tuple(w_t.shape) == (K, N), "w_t must be [K, N]")
         # (what the prologue of another kernel left unfilled is not in `pro`: its sparse form serves where nothing else is there)
         if pro.sparse is not None and (takes_sparse(M, N, K, R, act=int(act == "swiglu")) or (pro.tail_rec is None and pro.tail_dense is None)):
             _check(tuple(pro.sparse[0].shape) == (M, K // 2), "the sparse tail operand has the wrong shape")
             rc = _lib.load().tq_split_gemm_sparse(
-                _ptr(a_q8), _ptr(body_scale), _ptr(B_pack), _ptr(w_scale), _ptr(w_rot), None, int(R), *map(_ptr, pro.sparse),
+                _ptr(a_q8), _ptr(body_scale), _ptr(B_pack), _ptr(w_scale), _ptr(w_rot), _ptr(w_t), int(R), *map(_ptr, pro.sparse),
                 pro.sparse[3].shape[1], _ptr(bias), _ptr(out), _ptr(dbg_acc), _ptr(dbg_tail), M, N, K, int(act == "swiglu"), _stream())
             _lib.check(rc, f"split_gemm_mma(M={M}, N={N}, K={K}, R={R})")
             return out

@@ -269,7 +269,8 @@ def test_refresh_after_a_write_that_is_not_counted():
 
 @pytest.mark.parametrize("M", [1, 1500])
 def test_a_capture_that_is_the_first_call_on_the_transposed_weights(M):
-    """Eager calls between the capture and its first replay read a transpose of their own."""
+    """Eager calls between the capture and its first replay read a transpose of their own; the captured one sums the tail on
+    another kernel (a bf16 step apart where a sum lies near the middle)."""
     from tailquant_kernel_b200 import SplitLinear
     N, K = 8192, 1024
     g = torch.Generator().manual_seed(5)
@@ -286,7 +287,9 @@ def test_a_capture_that_is_the_first_call_on_the_transposed_weights(M):
     assert torch.equal(lin(x), want) and torch.equal(lin.w.w_t, lin.w.w_rot.t())
     out[0].zero_()
     graph.replay()
-    assert torch.equal(out[0], want)
+    d, want = (out[0].float() - want.float()).abs(), want.float().abs()
+    sums = 1e-5 * lin.R * (4 * 300 / K ** 0.5 + 6) * float(lin.w.w_rot.abs().max())   # (a few_levels row's largest rotated value)
+    assert float((d != 0).float().mean()) < 1e-3 and bool((d <= want * 2.0 ** -7 + sums).all())
 
 
 def outputs(pro):

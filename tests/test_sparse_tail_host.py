@@ -190,20 +190,23 @@ def test_records_are_left_out_where_the_other_forms_are_there(fake):  # noqa: F8
 
 
 def test_a_capture_makes_no_transpose(fake):  # noqa: F811
-    """It would be written by no kernel before the first replay: the captured call reads `w_rot`, later ones make the transpose."""
+    """It would be written by no kernel before the first replay: the captured forward takes the CTA pairs, later ones make it."""
     lin = layer(N=24576, K=512, rms_weight=None)
     lin.w.w_t = None
     x = claimed(1500, 512, dtype=torch.bfloat16)
     fake.capture = 7
     for _ in range(2):
         lin(x)
-        assert fake.calls[-1][1]["sp_val"] and not fake.calls[-1][1]["w_t"] and lin.w.w_t is None
+        c = fake.calls[-1][1]
+        assert c["tail_rec"] and not c["sp_val"] and not c["w_t"] and lin.w.w_t is None
     lin.prepare_decode()
     assert lin.w.w_t is None
+    lin.compute(lin.prologue(x), 1500)   # (what several linears read: the sparse form too)
+    assert fake.calls[-1][1]["sp_val"] and not fake.calls[-1][1]["w_t"] and lin.w.w_t is None
     fake.capture = 0
     lin(x)
     t = lin.w.w_t
-    assert t is not None and fake.calls[-1][1]["w_t"] == t.data_ptr()
+    assert t is not None and fake.calls[-1][1]["sp_val"] and fake.calls[-1][1]["w_t"] == t.data_ptr()
     fake.capture = 8
     lin(x)
     assert fake.calls[-1][1]["w_t"] == t.data_ptr()
