@@ -173,6 +173,7 @@ class SplitLinear:
         if R > 0 and tail_engine == "gather" and w.w_t is None and w.w_rot is not None:
             w.w_t = w.w_rot.t().contiguous()  # the gather engine reads the [K, N] transpose
             w.t_of = (w.w_t, w.w_rot, cls._version(w.w_rot), w.w_rot.data_ptr())
+            w.t_made = ops.Made() if w.w_t.device.type == "cuda" else None
         if R > 0 and w.w_t is None and w.w_rot is None:
             raise RuntimeError("a tail needs the rotated bf16 weights (w_rot or w_t)")
         self = cls.__new__(cls)
@@ -339,7 +340,7 @@ class SplitLinear:
             return
         if self._capturing():
             raise RuntimeError("refresh() cannot run inside a stream capture")
-        self._transposed(w.w_t)
+        self._make_transpose(w.w_t)
 
     @staticmethod
     def _capturing() -> bool:
@@ -350,6 +351,11 @@ class SplitLinear:
         if r.device.type == "cuda" and r.is_contiguous():
             return ops.transpose_bf16(r, into)
         return r.t().contiguous() if into is None else into.copy_(r.t())
+
+    def _make_transpose(self, into: Optional[torch.Tensor] = None) -> None:
+        w = self.w
+        w.w_t = self._transposed(into)
+        w.t_made = ops.Made() if w.w_t.device.type == "cuda" else None
 
     @staticmethod
     def _version(t: Optional[torch.Tensor]) -> int:
@@ -371,12 +377,10 @@ class SplitLinear:
         if (changed or w.w_t is None) and self._capturing():
             return False
         if changed:
-            if rot is of and tuple(t.shape) == tuple(reversed(rot.shape)) and t.dtype == rot.dtype and t.device == rot.device:
-                self._transposed(t)
-            else:
-                w.w_t = None
-        if w.w_t is None:
-            w.w_t = self._transposed()
+            same = rot is of and tuple(t.shape) == tuple(reversed(rot.shape)) and t.dtype == rot.dtype and t.device == rot.device
+            self._make_transpose(t if same else None)
+        elif w.w_t is None:
+            self._make_transpose()
         w.t_of = (w.w_t, rot, version, rot.data_ptr())
         return True
 
@@ -426,8 +430,11 @@ class SplitLinear:
             keep, w_t = self._follow_w_rot(), w.w_t
             if not keep:   # in a stream capture: the sparse GEMM reads `w_rot`, the others a transpose for this call of it only
                 w_t = self._transposed() if own.engine != _lib.TQ_LINEAR_FUSED and w.w_rot is not None else None
-            elif w.w_rot is not None:
-                own.rot_version = self._rot_version()
+            else:
+                if w.w_rot is not None:
+                    own.rot_version = self._rot_version()
+                if w.t_made is not None and not self._capturing():   # (a capture begins behind what it depends on)
+                    w.t_made.order(w_t)
         elif pro.sparse is not None and w_t is w.t_of[0]:
             w_t = None   # (where the sparse form is all there is, `w_rot` is what is certain to be in line)
         self._check_parts(own.engine, w_t if own.engine != _lib.TQ_LINEAR_FUSED or own.rot_version is not None else None)

@@ -226,6 +226,25 @@ def threshold_topr_pack(A, R, descending_rank, A_pack, body_scale, top_scale, to
 
 
 # --------------------------------------------------------------------------- weights
+class Made:
+    """What the current stream has written so far, for calls on others."""
+    __slots__ = ("event", "stream")
+
+    def __init__(self):
+        self.event, self.stream = torch.cuda.Event(), _stream()
+        self.event.record()
+
+    def order(self, t: torch.Tensor) -> None:
+        """Has the current stream, where it is another, wait for that before it reads `t`."""
+        if self.stream != _stream():
+            here = torch.cuda.current_stream()
+            here.wait_event(self.event)
+            t.record_stream(here)
+
+    def __reduce__(self):
+        return type(None), ()   # (a copy is made by its reader)
+
+
 @dataclass
 class PreparedWeight:
     N: int
@@ -239,6 +258,7 @@ class PreparedWeight:
     bias: Optional[torch.Tensor] = None  # [N] f32
     # a w_t, and the w_rot, its version and place that it is the transpose of (kept here: layers on one weight share both)
     t_of: Tuple = field(default=(None, None, None, None), repr=False, compare=False)
+    t_made: Optional[Made] = field(default=None, repr=False, compare=False)   # where a layer made w_t
 
 
 def prepare_weight(W: torch.Tensor, had_kind: Optional[int] = None, eps: float = EPS, t16: bool = True,

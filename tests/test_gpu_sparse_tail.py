@@ -267,6 +267,26 @@ def test_refresh_after_a_write_that_is_not_counted():
     assert torch.equal(y, other(x)) and torch.equal(lin(x), other(x))
 
 
+@pytest.mark.parametrize("M", [1, 700, 1500])
+def test_a_transpose_made_on_another_stream_is_waited_for(M):
+    """The call that makes it is held up on its stream; the next one, of another row count, comes on a stream of its own."""
+    from tailquant_kernel_b200 import SplitLinear
+    N, K = 8192, 1024
+    g = torch.Generator().manual_seed(5)
+    lin = SplitLinear((torch.randn(N, K, generator=g) * 0.02).to(torch.bfloat16).cuda())
+    fresh = SplitLinear.from_prepared(ops.PreparedWeight(**{**vars(lin.w), "w_t": None}))
+    x, first = activations("few_levels", M, K, 2), activations("plain", 1000, K, 1)
+    want = fresh(x).clone()
+    torch.empty((K, N), dtype=torch.bfloat16, device="cuda").fill_(7.0)   # (what the transpose's memory may have held)
+    side = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(side):
+        torch.cuda._sleep(20_000_000)   # (some 10 ms)
+        lin(first)
+    assert lin.w.w_t is not None
+    assert torch.equal(lin(x), want)
+
+
 @pytest.mark.parametrize("M", [1, 1500])
 def test_a_capture_that_is_the_first_call_on_the_transposed_weights(M):
     """Eager calls between the capture and its first replay read a transpose of their own; the captured one sums the tail on

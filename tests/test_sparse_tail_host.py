@@ -1,5 +1,7 @@
 """When a layer takes its tail as a 2:4-sparse operand, and what it holds for it (no GPU; see test_linear_host.py)."""
+import copy
 import ctypes
+import pickle
 
 import pytest
 import torch
@@ -415,3 +417,12 @@ def test_layers_on_one_weight_share_its_transpose(fake):  # noqa: F811
     assert w.w_t is t and float(t[3, 5]) == 2.0
     a(claimed(1, 1024, dtype=torch.bfloat16))
     assert fake.calls[-1][1]["w_t"] == t.data_ptr()
+
+
+def test_a_prepared_weight_can_be_copied():
+    """What orders streams is not part of a copy."""
+    made = object.__new__(ops.Made)
+    rot, t = torch.zeros(8, 64), torch.zeros(64, 8)
+    w = ops.PreparedWeight(8, 64, 1, torch.zeros(8, 32), torch.zeros(8), t, None, rot, t_of=(t, rot, 0, rot.data_ptr()), t_made=made)
+    for twin in (copy.deepcopy(w), pickle.loads(pickle.dumps(w))):
+        assert twin.t_made is None and twin.w_t is not t and twin.t_of[0] is twin.w_t and twin.t_of[1] is twin.w_rot
