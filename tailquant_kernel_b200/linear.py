@@ -276,7 +276,7 @@ class SplitLinear:
         c = _lib.LinearCall(M=ws.M, N=N, K=self.K, R=self.R, had_kind=self.w.had_kind, engine=ws.engine,
                             act=int(self.epilogue == "swiglu"))
         if sparse is None:
-            sparse = lib.tq_linear_sparse(ctypes.byref(c), int(any_width)) > 0
+            sparse = ws.engine == _lib.TQ_LINEAR_FUSED and lib.tq_linear_sparse(ctypes.byref(c), int(any_width)) > 0
         c.sp_val = 1 if sparse else None   # (asks for what is needed beside it)
         bits = lib.tq_linear_outputs(ctypes.byref(c), int(any_width))
         if bits < 0:
@@ -372,8 +372,10 @@ class SplitLinear:
         w, rot = self.w, self.w.w_rot
         if rot is None:
             return w.w_t is not None
-        version, (t, of, v, place) = self._rot_version(), w.t_of
-        changed = w.w_t is not None and w.w_t is t and (rot is not of or (version, rot.data_ptr()) != (v, place))
+        version, address, (t, of, v, place) = self._rot_version(), rot.data_ptr(), w.t_of
+        if w.w_t is t and rot is of and version == v and address == place:
+            return True
+        changed = w.w_t is not None and w.w_t is t
         if (changed or w.w_t is None) and self._capturing():
             return False
         if changed:
@@ -381,7 +383,7 @@ class SplitLinear:
             self._make_transpose(t if same else None)
         elif w.w_t is None:
             self._make_transpose()
-        w.t_of = (w.w_t, rot, version, rot.data_ptr())
+        w.t_of = (w.w_t, rot, version, address)
         return True
 
     def _described(self, own: _Workspace) -> bool:
@@ -432,9 +434,9 @@ class SplitLinear:
                 w_t = self._transposed() if own.engine != _lib.TQ_LINEAR_FUSED and w.w_rot is not None else None
             else:
                 if w.w_rot is not None:
-                    own.rot_version = self._rot_version()
-                if w.t_made is not None and not self._capturing():   # (a capture begins behind what it depends on)
-                    w.t_made.order(w_t)
+                    own.rot_version = w.t_of[2]
+                if w.t_made is not None:
+                    w.t_made.order()
         elif pro.sparse is not None and w_t is w.t_of[0]:
             w_t = None   # (where the sparse form is all there is, `w_rot` is what is certain to be in line)
         self._check_parts(own.engine, w_t if own.engine != _lib.TQ_LINEAR_FUSED or own.rot_version is not None else None)

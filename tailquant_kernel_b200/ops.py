@@ -234,12 +234,12 @@ class Made:
         self.event, self.stream = torch.cuda.Event(), _stream()
         self.event.record()
 
-    def order(self, t: torch.Tensor) -> None:
-        """Has the current stream, where it is another, wait for that before it reads `t`."""
-        if self.stream != _stream():
-            here = torch.cuda.current_stream()
-            here.wait_event(self.event)
-            t.record_stream(here)
+    def order(self) -> None:
+        """Has the current stream, where it is another, wait for that; not inside a capture, which begins behind what it depends
+        on.  (Memory is given back on the stream it came from, as that of every other part of a layer.)"""
+        stream = _stream()
+        if self.stream != stream and not _lib.load().tq_stream_capture_id(stream):
+            torch.cuda.current_stream().wait_event(self.event)
 
     def __reduce__(self):
         return type(None), ()   # (a copy is made by its reader)
