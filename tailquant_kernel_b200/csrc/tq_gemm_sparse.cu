@@ -9,8 +9,9 @@
 // The entries left over (one row in two has one at R = 0.05 K, K = 4096) follow behind the K slices of a tile, 64 of them at a
 // time, as one more dense slice: warp 0 collects them from the lists of the tile's 256 rows while the K slices run and builds A,
 // one value per column; B are rows of w_t, gathered by TMA.  A dense slice takes about 0.8 us.  (Added in the epilogue instead,
-// where nothing hides the loads, the left-over entries cost 30 % of the GEMM.)  Rows that consist of a few equal values have
-// many: with 26 in every row of 2048 x 6144 x 4096 this kernel takes 454 us where the dense product takes 121.
+// where nothing hides the loads, the left-over entries cost 30 % of the GEMM.)  Their number is without bound, and rows that
+// consist of a few equal values have many: 2048 x 6144 x 4096 with three equal large channels, whose indices agree in the last two
+// bits, (7.3 left over in every row) 197 us, with four (26) 457, where the dense product takes 125 and 130.
 //
 // Tile: 256 rows x up to 224 channels per pair.  The two accumulators (int32, fp32) of 224 columns leave 64 columns of tensor
 // memory for the places (16 per K slice); 256 channels would leave none.  The last tile of a row of tiles is as narrow as its
@@ -790,8 +791,10 @@ int run_sparse_gemm(const int8_t* a_q8, const float* body_scale, const uint8_t* 
 }  // namespace tq
 
 extern "C" int tq_split_gemm_sparse(const int8_t* a_q8, const float* body_scale, const uint8_t* b_col, const float* w_scale,
-                                    const void* w_rot, const void* w_t, int R, void* sp_val, uint32_t* sp_meta, uint16_t* sp_over_cnt, uint32_t* sp_over, int sp_over_ld, const float* bias, void* out_bf16,
-                                    int32_t* dbg_acc, float* dbg_tail, int M, int N, int K, int act, void* stream) {
+                                    const void* w_rot, const void* w_t, int R, void* sp_val, uint32_t* sp_meta,
+                                    uint16_t* sp_over_cnt, uint32_t* sp_over, int sp_over_ld, const float* bias,
+                                    void* out_bf16, int32_t* dbg_acc, float* dbg_tail, int M, int N, int K, int act,
+                                    void* stream) {
   using namespace tq;
   if (!a_q8 || !body_scale || !b_col || !w_scale || !w_rot || R <= 0 || R >= K || sp_over_ld < (R + 1) / 2 ||
       !sp_val || !sp_meta || !sp_over_cnt || !sp_over || !out_bf16 || M < 0 || N <= 0 || K <= 0 || (act & ~1))

@@ -131,7 +131,11 @@ static bool stream_is_faster(int M, int N, int K, int R) {
 // tiles take as long as full ones), a share of the weight stream, and 0.08 us for each left-over entry among four rows of a
 // tile; 5.5 us around it, 1.5 of them in the prologue.  `e`: left-over entries of a row whose R entries lie independently.  Fit
 // to 200 shapes (80..2048 rows, N = 1024..28672, K = 1024, 4096, 12288, R = 0.05 K): 5 % off on average, 0.4 % lost by the
-// choice.  300 x 24576 x 4096: 88 us, 118 and 122 on the other two; 2048 x 4096 x 4096: 68 against 81 on pairs.
+// choice.  300 x 24576 x 4096: 88 us, 118 and 122 on the other two; 2048 x 4096 x 4096: 68 against 81 on pairs.  At the ends, whole
+// linears on 13 shapes (128..4096 rows, K = 512..12288) each at R = 0.001, 0.01, 0.05, 0.069 K: 0.9 % lost on average, nearly all
+// of it by staying with the pairs where many entries make few rounds look long (1500 x 28672 x 512, 0.069 K: 124 us, 101
+// here; 4096 x 2048 x 1024 62 and 54); where the rule takes this kernel the best of the others is at most 2.4 % ahead (520 x 4096 x
+// 8192, 0.05 K: 85 against 83), and without left-over entries (0.001 K) 2048 x 6144 x 4096 takes 120 against 144.
 static float sparse_us(int M, int N, int K, int R) {
   const int rounds = (((M + 255) / 256) * ((N + 223) / 224) + 73) / 74;
   const float q = (float)R / (float)K, e = (float)K * q * q * q * (1.0f - 0.5f * q);
