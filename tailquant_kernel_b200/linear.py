@@ -13,6 +13,7 @@ a forward is capturable in a CUDA graph after its first call, as the reference's
 from __future__ import annotations
 
 import ctypes
+import threading
 import weakref
 from collections import OrderedDict
 from typing import Dict, List, Optional, Tuple
@@ -20,6 +21,9 @@ from typing import Dict, List, Optional, Tuple
 import torch
 
 from . import _lib, ops
+
+
+_MAKING = threading.Lock()   # held while a transpose of rotated weights is made
 
 
 def interleave_gate_up(w_gate: torch.Tensor, w_up: torch.Tensor) -> torch.Tensor:
@@ -353,9 +357,9 @@ class SplitLinear:
         return r.t().contiguous() if into is None else into.copy_(r.t())
 
     def _make_transpose(self, into: Optional[torch.Tensor] = None) -> None:
-        w = self.w
-        w.w_t = self._transposed(into)
-        w.t_made = ops.Made() if w.w_t.device.type == "cuda" else None
+        t = self._transposed(into)
+        self.w.t_made = ops.Made() if t.device.type == "cuda" else None
+        self.w.w_t = t
 
     @staticmethod
     def _version(t: Optional[torch.Tensor]) -> int:
@@ -375,15 +379,17 @@ class SplitLinear:
         version, address, (t, of, v, place) = self._rot_version(), rot.data_ptr(), w.t_of
         if w.w_t is t and rot is of and version == v and address == place:
             return True
-        changed = w.w_t is not None and w.w_t is t
-        if (changed or w.w_t is None) and self._capturing():
-            return False
-        if changed:
-            same = rot is of and tuple(t.shape) == tuple(reversed(rot.shape)) and t.dtype == rot.dtype and t.device == rot.device
-            self._make_transpose(t if same else None)
-        elif w.w_t is None:
-            self._make_transpose()
-        w.t_of = (w.w_t, rot, version, address)
+        with _MAKING:   # (threads on streams of their own: one of them makes it, and says so last)
+            t, of, v, place = w.t_of
+            changed = w.w_t is not None and w.w_t is t and (rot is not of or (version, address) != (v, place))
+            if (changed or w.w_t is None) and self._capturing():
+                return False
+            if changed:
+                same = rot is of and tuple(t.shape) == tuple(reversed(rot.shape)) and t.dtype == rot.dtype and t.device == rot.device
+                self._make_transpose(t if same else None)
+            elif w.w_t is None:
+                self._make_transpose()
+            w.t_of = (w.w_t, rot, version, address)
         return True
 
     def _described(self, own: _Workspace) -> bool:

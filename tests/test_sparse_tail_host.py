@@ -2,6 +2,8 @@
 import copy
 import ctypes
 import pickle
+import threading
+import time
 
 import pytest
 import torch
@@ -426,3 +428,22 @@ def test_a_prepared_weight_can_be_copied():
     w = ops.PreparedWeight(8, 64, 1, torch.zeros(8, 32), torch.zeros(8), t, None, rot, t_of=(t, rot, 0, rot.data_ptr()), t_made=made)
     for twin in (copy.deepcopy(w), pickle.loads(pickle.dumps(w))):
         assert twin.t_made is None and twin.w_t is not t and twin.t_of[0] is twin.w_t and twin.t_of[1] is twin.w_rot
+
+
+def test_threads_make_one_transpose(fake, monkeypatch):  # noqa: F811
+    """Each would read the other's, made on a stream that it does not wait for."""
+    lin = layer(N=8192, K=1024, rms_weight=None)
+    lin.w.w_t = None
+    made, transposed = [], SplitLinear._transposed
+
+    def slow(self, into=None):
+        time.sleep(0.05)
+        made.append(transposed(self, into))
+        return made[-1]
+    monkeypatch.setattr(SplitLinear, "_transposed", slow)
+    threads = [threading.Thread(target=lin, args=(claimed(M, 1024, dtype=torch.bfloat16),)) for M in (1, 1500, 700)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert len(made) == 1 and {c["w_t"] for _, c in fake.calls} == {made[0].data_ptr()} and len(fake.calls) == 3
