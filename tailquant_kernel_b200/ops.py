@@ -122,6 +122,14 @@ class PrologueOut:
     sparse: Optional[Tuple[torch.Tensor, ...]] = None
 
 
+def _check_sparse(sparse, M: int, K: int, R: int) -> None:
+    val, meta, over_cnt, over = sparse
+    _check([t.dtype for t in sparse] == [torch.bfloat16, torch.int32, torch.int16, torch.int32] and
+           all(t.is_contiguous() for t in sparse), "the sparse tail operand has the wrong types or strides")
+    _check(R > 0 and tuple(val.shape) == (M, K // 2) and tuple(meta.shape) == (M, K // 32) and over_cnt.numel() == M and
+           over.dim() == 2 and over.shape[0] == M and over.shape[1] >= (R + 1) // 2, "the sparse tail operand has the wrong shape")
+
+
 def split_prologue(x: torch.Tensor, had_kind: int, R: int, descending_rank: Optional[int] = None,
                    eps: float = EPS, t16: bool = True, t4: bool = False, want_x_rot: bool = False,
                    want_q8: bool = False, want_pack: bool = True, out: Optional[PrologueOut] = None,
@@ -164,15 +172,13 @@ def split_prologue(x: torch.Tensor, had_kind: int, R: int, descending_rank: Opti
     if out.sparse is not None:   # (a linear prefers it to the other forms of the tail, so it must not keep an earlier input's)
         _check(out.idx32 is None and out.top_q is None and out.x_rot is None,
                "the sparse tail operand comes without T4 outputs and without x_rot")
-        val, meta, over_cnt, over = out.sparse
-        _check(R > 0 and tuple(val.shape) == (M, K // 2) and tuple(meta.shape) == (M, K // 32) and over_cnt.numel() == M and
-               over.shape[0] == M, "the sparse tail operand has the wrong shape")
+        _check_sparse(out.sparse, M, K, R)
         c = _lib.LinearCall(
             M=M, N=8, K=K, R=R, had_kind=had_kind, descending_rank=descending_rank, engine=_lib.TQ_LINEAR_FUSED, tail_ld=ld,
             ptr_ld=pld, eps=eps, rms_eps=float(rms_eps), rms_weight=_ptr(rms_weight), a_pack=_ptr(out.a_pack), a_q8=_ptr(out.a_q8),
             body_scale=_ptr(out.body_scale), top_scale=_ptr(out.top_scale), tail_idx16=_ptr(out.tail_idx),
             tail_val=_ptr(out.tail_val), tail_ptr=_ptr(out.tail_ptr), tail_rec=_ptr(out.tail_rec), tail_cnt=_ptr(out.tail_cnt),
-            tail_dense=_ptr(out.tail_dense), sp_over_ld=over.shape[1], **dict(zip(SPARSE_FIELDS, map(_ptr, out.sparse))))
+            tail_dense=_ptr(out.tail_dense), sp_over_ld=out.sparse[3].shape[1], **dict(zip(SPARSE_FIELDS, map(_ptr, out.sparse))))
         _lib.check(_lib.load().tq_linear_prologue(ctypes.byref(c), _ptr(x), _stream()),
                    f"split_prologue(M={M}, K={K}, had_kind={had_kind}, R={R})")
         return out
@@ -362,9 +368,10 @@ def takes_sparse(M: int, N: int, K: int, R: int, had_kind: int = TQ_HAD_WHT, act
 def split_gemm_mma(a_q8, body_scale, B_pack, w_scale, out, w_rot=None, pro: Optional[PrologueOut] = None,
                    R: int = 0, bias=None, dbg_acc=None, dbg_tail=None, act: str = "none", w_t=None):
     """One kernel: dense INT4 x INT4 part on tcgen05 kind::i8 plus the tail as a bf16 tensor-core product
-    over the zero-filled tail matrix, fused dequant + bias, bf16 out.  `w_t`: the [K, N] transpose of w_rot, read for
-    the entries that the 2:4-sparse form of the tail leaves over; without it they come from w_rot, several times as slowly.  act="swiglu": the weight rows are
-    interleaved (gate_i, up_i) pairs and out is [M, N/2] = bf16(bf16(silu(gate)) * up)."""
+    over the zero-filled tail matrix, fused dequant + bias, bf16 out.  act="swiglu": the weight rows are
+    interleaved (gate_i, up_i) pairs and out is [M, N/2] = bf16(bf16(silu(gate)) * up).  `w_t`: the [K, N] transpose of
+    w_rot, read for the entries that the 2:4-sparse form of the tail leaves over; without it they come from w_rot, several
+    times as slowly."""
     _check(act in ("none", "swiglu"), "act must be 'none' or 'swiglu'")
     _check_cuda(a_q8, "a_q8", torch.int8)
     _check_cuda(B_pack, "B_pack", torch.uint8)
@@ -388,7 +395,7 @@ def split_gemm_mma(a_q8, body_scale, B_pack, w_scale, out, w_rot=None, pro: Opti
             _check(tuple(w_t.shape) == (K, N), "w_t must be [K, N]")
         # (what the prologue of another kernel left unfilled is not in `pro`: its sparse form serves where nothing else is there)
         if pro.sparse is not None and (takes_sparse(M, N, K, R, act=int(act == "swiglu")) or (pro.tail_rec is None and pro.tail_dense is None)):
-            _check(tuple(pro.sparse[0].shape) == (M, K // 2), "the sparse tail operand has the wrong shape")
+            _check_sparse(pro.sparse, M, K, R)
             rc = _lib.load().tq_split_gemm_sparse(
                 _ptr(a_q8), _ptr(body_scale), _ptr(B_pack), _ptr(w_scale), _ptr(w_rot), _ptr(w_t), int(R), *map(_ptr, pro.sparse),
                 pro.sparse[3].shape[1], _ptr(bias), _ptr(out), _ptr(dbg_acc), _ptr(dbg_tail), M, N, K, int(act == "swiglu"), _stream())

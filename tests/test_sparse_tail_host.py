@@ -1,6 +1,7 @@
 """When a layer takes its tail as a 2:4-sparse operand, and what it holds for it (no GPU; see test_linear_host.py)."""
 import copy
 import ctypes
+import dataclasses
 import pickle
 import threading
 import time
@@ -447,3 +448,16 @@ def test_threads_make_one_transpose(fake, monkeypatch):  # noqa: F811
     for t in threads:
         t.join()
     assert len(made) == 1 and {c["w_t"] for _, c in fake.calls} == {made[0].data_ptr()} and len(fake.calls) == 3
+
+
+@pytest.mark.parametrize("which", range(4))
+def test_a_gemm_refuses_a_sparse_operand_of_another_size(fake, which):  # noqa: F811
+    lin = layer(N=24576, K=512, rms_weight=None)
+    lin(claimed(1500, 512, dtype=torch.bfloat16))
+    pro, w = lin._ws[1500].pro, lin.w
+    sparse = list(pro.sparse)
+    sparse[which] = sparse[which][:-1].clone()
+    with pytest.raises(RuntimeError, match="sparse"):
+        ops.split_gemm_mma(*(t.as_subclass(type(w.b_col)) for t in (pro.a_q8, pro.body_scale)), w.b_col, w.w_scale,
+                           claimed(1500, 24576, dtype=torch.bfloat16), w_rot=w.w_rot, pro=dataclasses.replace(pro, sparse=tuple(sparse)),
+                           R=lin.R)
