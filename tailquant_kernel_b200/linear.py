@@ -288,9 +288,8 @@ class SplitLinear:
         return bits, sparse
 
     def serves(self, ws: _Workspace, N: int) -> bool:
-        """Whether the prologue outputs in `ws` are what a layer of N channels takes.  If not, the next prologue's are."""
-        if self.split_widths is None or N in self.split_widths:
-            return True
+        """Whether the prologue outputs in `ws` are what a layer of N channels takes, a width not in `split_widths` so far.  If
+        not, the next prologue's are."""
         self.split_widths.append(N)
         bits, sparse = self._ask(ws, N, False) if ws.M > 64 else (0, False)
         for w in self._ws.values():
@@ -402,10 +401,10 @@ class SplitLinear:
                 and r is w.w_rot and (r is None or r.data_ptr() == pr) and t is w.w_t and (t is None or t.data_ptr() == pt)
                 and i is w.bias and (i is None or i.data_ptr() == pi)
                 and g is self.rms_weight and (g is None or g.data_ptr() == pg)
-                and (own.rot_version is None or own.rot_version == self._rot_version())
+                and (own.rot_version is None or own.rot_version == r._version)
                 and kind == w.had_kind and rank == self.descending_rank and eps == self.rms_eps and act == self.epilogue)
 
-    def _check_parts(self, engine: int, w_t: Optional[torch.Tensor]) -> None:
+    def _check_parts(self, engine: int, w_t: Optional[torch.Tensor], reads_t: bool) -> None:
         """Types, layout and sizes of what a forward reads (`w_t`: the transpose it is given): the kernels take it for granted."""
         w, N, K = self.w, self.N, self.K
         ops._check_cuda(w.b_col, "b_col", torch.uint8)
@@ -415,7 +414,7 @@ class SplitLinear:
         if self.R and engine == _lib.TQ_LINEAR_FUSED:
             ops._check_cuda(w.w_rot, "w_rot", torch.bfloat16)
             ops._check(tuple(w.w_rot.shape) == (N, K), "w_rot must be [N, K]")
-        if self.R and (w_t is not None or engine != _lib.TQ_LINEAR_FUSED):
+        if reads_t:
             ops._check_cuda(w_t, "w_t", torch.bfloat16)
             ops._check(tuple(w_t.shape) == (K, N), "w_t must be [K, N]")
         if w.bias is not None:
@@ -433,19 +432,20 @@ class SplitLinear:
         own.rot_version = own.call = None   # (a part that is refused must not leave the former description in force)
         w, p = self.w, ops._ptr
         keep, w_t = True, w.w_t
-        if self.R and (own.engine != _lib.TQ_LINEAR_FUSED or (pro.sparse is not None and ops.takes_sparse(
-                own.M, self.N, self.K, self.R, w.had_kind, int(self.epilogue == "swiglu")))):
+        reads_t = self.R > 0 and (own.engine != _lib.TQ_LINEAR_FUSED or (pro.sparse is not None and ops.takes_sparse(
+            own.M, self.N, self.K, self.R, w.had_kind, int(self.epilogue == "swiglu"))))
+        if reads_t:
             keep, w_t = self._follow_w_rot(), w.w_t
             if not keep:   # in a stream capture: the sparse GEMM reads `w_rot`, the others a transpose for this call of it only
                 w_t = self._transposed() if own.engine != _lib.TQ_LINEAR_FUSED and w.w_rot is not None else None
             else:
-                if w.w_rot is not None:
+                if w.w_rot is not None and not w.w_rot.is_inference():
                     own.rot_version = w.t_of[2]
                 if w.t_made is not None:
                     w.t_made.order()
         elif pro.sparse is not None and w_t is w.t_of[0]:
             w_t = None   # (where the sparse form is all there is, `w_rot` is what is certain to be in line)
-        self._check_parts(own.engine, w_t if own.engine != _lib.TQ_LINEAR_FUSED or own.rot_version is not None else None)
+        self._check_parts(own.engine, w_t, reads_t and (keep or own.engine != _lib.TQ_LINEAR_FUSED))
         own.call_pro = pro if keep else None
         own.call_t = w_t   # (lives as long as its address is in `call`)
         src = (w.b_col, w.w_scale, w.w_rot, w.w_t, w.bias, self.rms_weight)
@@ -589,7 +589,8 @@ def split_linear_forward(x: torch.Tensor, weight: torch.Tensor, bias: Optional[t
     owner = hit[2]() if hit is not None and hit[0]() is x else None
     if owner is not None:
         ws = hit[1]
-        if not owner.serves(ws, lin.N):   # (the first time that this width follows)
+        known_widths = owner.split_widths
+        if known_widths is not None and lin.N not in known_widths and not owner.serves(ws, lin.N):   # (a width's first time)
             ws = owner.prologue(x2d)
     else:
         _SHARED.clear()   # one entry: the prologue outputs live in a workspace that the next prologue of that layer

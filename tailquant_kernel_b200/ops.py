@@ -233,18 +233,21 @@ def threshold_topr_pack(A, R, descending_rank, A_pack, body_scale, top_scale, to
 
 # --------------------------------------------------------------------------- weights
 class Made:
-    """What the current stream has written so far, for calls on others."""
+    """What the current stream has written so far, for calls on others.  The event costs 13 us, so that of the default stream, which
+    always lives, is recorded when another asks (and stands for a little more)."""
     __slots__ = ("event", "stream")
 
     def __init__(self):
-        self.event, self.stream = torch.cuda.Event(), _stream()
-        self.event.record()
+        self.stream = _stream()
+        self.event = torch.cuda.current_stream().record_event() if self.stream else None
 
     def order(self) -> None:
         """Has the current stream, where it is another, wait for that; not inside a capture, which begins behind what it depends
         on.  (Memory is given back on the stream it came from, as that of every other part of a layer.)"""
         stream = _stream()
         if self.stream != stream and not _lib.load().tq_stream_capture_id(stream):
+            if self.event is None:
+                self.event = torch.cuda.default_stream().record_event()
             torch.cuda.current_stream().wait_event(self.event)
 
     def __reduce__(self):

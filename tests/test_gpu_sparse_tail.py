@@ -268,7 +268,8 @@ def test_refresh_after_a_write_that_is_not_counted():
 
 
 @pytest.mark.parametrize("M", [1, 700, 1500])
-def test_a_transpose_made_on_another_stream_is_waited_for(M):
+@pytest.mark.parametrize("maker", ["default", "side"])
+def test_a_transpose_made_on_another_stream_is_waited_for(M, maker):
     """The call that makes it is held up on its stream; the next one, of another row count, comes on a stream of its own."""
     from tailquant_kernel_b200 import SplitLinear
     N, K = 8192, 1024
@@ -278,13 +279,15 @@ def test_a_transpose_made_on_another_stream_is_waited_for(M):
     x, first = activations("few_levels", M, K, 2), activations("plain", 1000, K, 1)
     want = fresh(x).clone()
     torch.empty((K, N), dtype=torch.bfloat16, device="cuda").fill_(7.0)   # (what the transpose's memory may have held)
-    side = torch.cuda.Stream()
+    side, default = torch.cuda.Stream(), torch.cuda.current_stream()
     torch.cuda.synchronize()
-    with torch.cuda.stream(side):
+    with torch.cuda.stream(side if maker == "side" else default):
         torch.cuda._sleep(20_000_000)   # (some 10 ms)
         lin(first)
     assert lin.w.w_t is not None
-    assert torch.equal(lin(x), want)
+    with torch.cuda.stream(default if maker == "side" else side):
+        y = lin(x)
+        assert torch.equal(y, want)
 
 
 @pytest.mark.parametrize("M", [1, 1500])
