@@ -198,7 +198,7 @@ int tq_split_gemm_mma_swiglu(const int8_t* a_q8, const float* body_scale, const 
  * tq_linear_call: sp_val has the first two entries of each group of four (zeros where there are fewer), sp_meta their places,
  * four bits per group (the lower place, the higher one << 2); sp_over the entries beyond two of a group (index | bf16 << 16,
  * ascending), sp_over_cnt how many there are.
- * w_t may be NULL: the left-over entries are then read from w_rot two bytes at a time (2048 x 6144 x 4096 at R = 0.05 K 209 us
+ * w_t may be NULL: the left-over entries are then read from w_rot two bytes at a time (2048 x 6144 x 4096 at R = 0.05 K 272 us
  * instead of 106).  act = 1: SwiGLU, out [M, N/2]. */
 int tq_split_gemm_sparse(const int8_t* a_q8, const float* body_scale, const uint8_t* b_col, const float* w_scale,
                          const void* w_rot, const void* w_t, int R, void* sp_val, uint32_t* sp_meta,

@@ -11,7 +11,7 @@
 // one value per column; B are rows of w_t, gathered by TMA.  A dense slice takes about 0.8 us.  (Added in the epilogue instead,
 // where nothing hides the loads, the left-over entries cost 30 % of the GEMM.)  Their number is without bound, and rows that
 // consist of a few equal values have many: 2048 x 6144 x 4096 with three equal large channels, whose indices agree in the last two
-// bits, (7.3 left over in every row) 197 us, with four (26) 457, where the dense product takes 125 and 130.
+// bits, (7.4 left over in every row) 203 us, with four (26) 471, where the dense product takes 125 and 130.
 //
 // Tile: 256 rows x up to 224 channels per pair.  The two accumulators (int32, fp32) of 224 columns leave 64 columns of tensor
 // memory for the places (16 per K slice); 256 channels would leave none.  The last tile of a row of tiles is as narrow as its
@@ -470,7 +470,6 @@ sparse_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a8, const __grid_con
         for (int j = 0; j < 2; ++j) {
           v[j] = (nv[j] & 0xffffu) < (uint32_t)p.K ? nv[j] : 0u;
           r[j] = nr[j];
-          load(64 * (q + 1) + lane + 32 * j, nv[j], nr[j]);   // (on its way while this slice is built)
         }
         ok = __all_sync(0xffffffffu, mbar_wait(b.empty_b(s), (uint32_t)((use / S::SB) & 1) ^ 1u, abort_flag, 0x2000000u));
         if (!ok) break;
@@ -481,6 +480,10 @@ sparse_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a8, const __grid_con
         list[l * S::LIST + lane + 32] = v[1];
         __syncwarp();
         if (lane == 0) mbar_arrive(b.listed(l));   // warps 14 and 15 load the rows of w_t
+        // (the next slice's entries, on their way while this one is built: 26 a row 538 -> 471 us; asked for in front of the wait
+        // for the slot they cost the kernel 1.2 % with plain rows)
+#pragma unroll
+        for (int j = 0; j < 2; ++j) load(64 * (q + 1) + lane + 32 * j, nv[j], nr[j]);
 #pragma unroll 8
         for (int c = 0; c < S::A / 512; ++c) *reinterpret_cast<uint4*>(a + c * 512 + lane * 16) = make_uint4(0u, 0u, 0u, 0u);
         __syncwarp();
@@ -492,25 +495,14 @@ sparse_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a8, const __grid_con
                 (uint16_t)(v[j] >> 16);
         }
         if (!p.w_t) {
-          // 64 entries x 14 pieces of eight channels, two bytes at a time: a sector each, so the loads of four pieces are in
-          // flight together: 2048 x 6144 x 4096, 0.7 left-over entries a row, 272 -> 209 us (with w_t 106, the CTA pairs 124)
-          for (int item = lane; item < 64 * SPG_BH / 8; item += 128) {
-            uint32_t w[4][8];
+          for (int item = lane; item < 64 * SPG_BH / 8; item += 32) {   // 64 entries x 14 pieces of eight channels
+            const int e = item / (SPG_BH / 8), c = item - e * (SPG_BH / 8), n = n0 + 8 * c;
+            const size_t k = list[l * S::LIST + e] & 0xffffu;
+            uint32_t w[4] = {0u, 0u, 0u, 0u};
+            if (n < p.N)
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
-              const int i = item + 32 * u, e = i / (SPG_BH / 8), n = min(n0 + 8 * (i - e * (SPG_BH / 8)), p.N - 8);
-              const uint16_t* const at = p.w_rot + (size_t)n * p.K + (list[l * S::LIST + e] & 0xffffu);
-#pragma unroll
-              for (int j = 0; j < 8; ++j) w[u][j] = at[(size_t)j * p.K];
-            }
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-              const int i = item + 32 * u, e = i / (SPG_BH / 8), c = i - e * (SPG_BH / 8);
-              uint32_t v4[4];
-#pragma unroll
-              for (int j = 0; j < 4; ++j) v4[j] = n0 + 8 * c < p.N ? w[u][2 * j] | w[u][2 * j + 1] << 16 : 0u;
-              st_shared_v4(smem_u32(a) + S::A + (uint32_t)((c >> 3) * 8192 + (e >> 3) * 1024 + (e & 7) * 128 + (((c & 7) ^ (e & 7)) << 4)), v4);
-            }
+              for (int j = 0; j < 8; ++j) w[j >> 1] |= (uint32_t)p.w_rot[(size_t)(n + j) * p.K + k] << (16 * (j & 1));
+            st_shared_v4(smem_u32(a) + S::A + (uint32_t)((c >> 3) * 8192 + (e >> 3) * 1024 + (e & 7) * 128 + (((c & 7) ^ (e & 7)) << 4)), w);
           }
         }
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
