@@ -128,7 +128,7 @@ def run_reference(args) -> None:
         "scaling": "weak", "vs_baseline": None, "dtype": "int4 x int4 -> int32, fp32 dequant, bf16 out",
         "data": "synthetic",
         "config": {"workload": "Qwen3-8B decoder layer linears: qkv 4096->6144, o 4096->4096, gate_up 4096->24576, "
-                               "down 12288->4096 (BASELINE configs[1])",
+                               "down 12288->4096",
                    "rows_per_step": CPU_SAMPLE_ROWS, "rows_of_the_gpu_arm": M_TOKENS, "tail_ratio": RATIO,
                    "same_config": CPU_SAMPLE_ROWS == M_TOKENS,
                    "note": "a bounded sample of the rows; throughput (TOPS) is per row and comparable, ms_per_step is not"},
@@ -526,7 +526,7 @@ def run_ours(args) -> None:
         "dtype": "int4 x int4 -> int32 (tcgen05 kind::i8), bf16 tail, fp32 dequant, bf16 out",
         "data": "synthetic",
         "config": {"workload": "Qwen3-8B decoder layer linears: qkv 4096->6144, o 4096->4096, gate_up 4096->24576, "
-                               "down 12288->4096 (BASELINE configs[1])",
+                               "down 12288->4096",
                    "rows_per_gpu": M_TOKENS, "global_rows": M_TOKENS * world, "tail_ratio": RATIO,
                    "tail_engine": args.tail_engine,
                    "parallelism": f"token-row shard x{world}, replicated weights, no collective",
@@ -962,7 +962,7 @@ def main() -> None:
                     help="mma: tail on the tensor cores inside the GEMM kernel; gather: exact-order CUDA-core kernel")
     ap.add_argument("--workload", default="layer",
                     choices=["layer", "decode", "llama_sweep", "single", "latency_table", "prefill36", "probe"],
-                    help="layer = the benchmark proper (baseline configs[1]); the others print secondary figures")
+                    help="layer = the benchmark proper at 2048 rows; the others print secondary figures")
     ap.add_argument("--reference-rows", type=int, default=CPU_SAMPLE_ROWS,
                     help="token rows of the 2048 that the CPU arm (and the cpu_baseline leg) works through per step")
     ap.add_argument("--only", default="", help="decode / probe: restrict to one linear (qkv_proj, o_proj, gate_up_proj, down_proj)")
